@@ -219,7 +219,8 @@ class Engine {
   std::vector<int> clusterOf_, clusterBoxes_, renderBoxes_;
   void buildClusters();
   std::vector<int> sourceBoxes_;  // lo xyz, hi xyz per source
-  DeviceBuffer renderField_, renderSmoke_, sceneDepth_, slices_, lighting_, occupancy_, lut_, renderParams_, image_, anchors_, lightSums_, renderBoxesD_;
+  DeviceBuffer renderField_, renderSmoke_, sceneDepth_, slices_, lighting_, occupancy_, lut_, renderParams_, image_, anchors_, lightSums_, renderBoxesD_,
+      renderPages_;
   SimParams* renderParamsH_ = nullptr;
   // The blackbody table and the render parameters of the latest state (device).
   int renderInputs();

@@ -20,65 +20,76 @@ namespace {
 
 constexpr int RTHREADS = 128;
 
-// A thread's current box (the pages its samples read) and its last two brick lookups (samples
-// near a brick's face alternate between two bricks).
-struct SlotCache {
-  int bx, by, bz, slot;
-  int bx2, by2, bz2, slot2;
-  int lo[3], hi[3];  // the current box in bricks, inclusive
+// A thread's current box: the bricks its samples read.
+struct BoxCursor {
+  int lo[3], hi[3];  // in bricks, inclusive
+  int first;         // its first entry in FpRender::pages
 };
-FP_DEV SlotCache noBox() {
-  SlotCache c;
-  c.bx = c.bx2 = 1 << 30;
-  c.by = c.bz = c.by2 = c.bz2 = 0;
-  c.slot = c.slot2 = -1;
+FP_DEV BoxCursor noBox() {
+  BoxCursor c;
   for (int a = 0; a < 3; a++) {
     c.lo[a] = 0;
     c.hi[a] = -1;
   }
+  c.first = 0;
   return c;
 }
-// Box k becomes the current one; the lookup cache starts over (pages are per box).
-FP_DEV void useBox(const FpRender& R, SlotCache& c, int k) {
+// Box k becomes the current one.
+FP_DEV void useBox(const FpRender& R, BoxCursor& c, int k) {
   for (int a = 0; a < 3; a++) {
-    c.lo[a] = R.boxes[6 * k + a];
-    c.hi[a] = R.boxes[6 * k + 3 + a];
+    c.lo[a] = R.boxes[FP_BOX_INTS * k + a];
+    c.hi[a] = R.boxes[FP_BOX_INTS * k + 3 + a];
   }
-  c.bx = c.bx2 = 1 << 30;
+  c.first = R.boxes[FP_BOX_INTS * k + 6];
 }
-FP_DEV bool inBox(const SlotCache& c, int bx, int by, int bz) {
+FP_DEV bool inBox(const BoxCursor& c, int bx, int by, int bz) {
   return bx >= c.lo[0] && bx <= c.hi[0] && by >= c.lo[1] && by <= c.hi[1] && bz >= c.lo[2] && bz <= c.hi[2];
 }
+// The slot of world brick b, or -1, through the tile hash.
+FP_DEV int hashedSlot(const SimParams& P, int bx, int by, int bz) {
+  int t = hashFind(P, bx >> 2, by >> 2, bz >> 2);
+  if (t < 0) return -1;
+  return checkSlot(P, FP_SITE_ENTRY, entryPage(P.entries[t * 64 + (((bz & 3) * 4 + (by & 3)) * 4 + (bx & 3))]));
+}
+// The entry of brick b of the current box in its table.
+FP_DEV int pageIndex(const BoxCursor& c, int bx, int by, int bz) {
+  return c.first + ((bz - c.lo[2]) * (c.hi[1] - c.lo[1] + 1) + (by - c.lo[1])) * (c.hi[0] - c.lo[0] + 1) + (bx - c.lo[0]);
+}
 // fireProPage: the slot of world brick b inside the current box, or -1.
-FP_DEV int slotAt(const SimParams& P, const FpRender& R, SlotCache& c, int bx, int by, int bz) {
-  if (bx == c.bx && by == c.by && bz == c.bz) return c.slot;
-  if (bx == c.bx2 && by == c.by2 && bz == c.bz2) return c.slot2;
-  c.bx2 = c.bx;
-  c.by2 = c.by;
-  c.bz2 = c.bz;
-  c.slot2 = c.slot;
-  int s = -1;
-  if (inBox(c, bx, by, bz)) {
-    int t = hashFind(P, bx >> 2, by >> 2, bz >> 2);
-    if (t >= 0) s = checkSlot(P, FP_SITE_ENTRY, entryPage(P.entries[t * 64 + (((bz & 3) * 4 + (by & 3)) * 4 + (bx & 3))]));
+FP_DEV int slotAt(const SimParams& P, const FpRender& R, BoxCursor& c, int bx, int by, int bz) {
+  if (!inBox(c, bx, by, bz)) return -1;
+  return R.pages ? __ldg(&R.pages[pageIndex(c, bx, by, bz)]) : hashedSlot(P, bx, by, bz);
+}
+// The slots of the bricks that the cells from (x,y,z) to n further on each axis lie in: s[k] for
+// the low (bit clear) or high (bit set) brick on x, y, z (bits 0, 1, 2). n is less than a brick,
+// `sh` the log2 of a brick's cells on the lattice asked about. False unless every one lies in the
+// current box and has a slot. The common case of a sample: its taps then need no lookup each.
+FP_DEV bool slots8(const FpRender& R, const BoxCursor& c, int sh, int x, int y, int z, int n, int* s) {
+  const int bx = x >> sh, by = y >> sh, bz = z >> sh, ex = (x + n) >> sh, ey = (y + n) >> sh, ez = (z + n) >> sh;
+  if (!R.pages || bx < c.lo[0] || by < c.lo[1] || bz < c.lo[2] || ex > c.hi[0] || ey > c.hi[1] || ez > c.hi[2])
+    return false;
+  const int nx = c.hi[0] - c.lo[0] + 1, nxy = nx * (c.hi[1] - c.lo[1] + 1);
+  const int* p = R.pages + pageIndex(c, bx, by, bz);
+  const int dx = ex - bx, dy = ey != by ? nx : 0, dz = ez != bz ? nxy : 0;
+  int all = 0;
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    s[k] = __ldg(p + ((k & 1) ? dx : 0) + ((k & 2) ? dy : 0) + ((k & 4) ? dz : 0));
+    all |= s[k];
   }
-  c.bx = bx;
-  c.by = by;
-  c.bz = bz;
-  c.slot = s;
-  return s;
+  return all >= 0;
 }
 
 FP_DEV float glowOf(float life) { return fminf(fmaxf(life * 5.f, 0.f), 1.f); }  // fireProGlow
 
 // The simulation's smoke at a world cell: zero outside the box or without a slot.
-FP_DEV float rawSmoke(const SimParams& P, const FpRender& R, SlotCache& c, int x, int y, int z) {
+FP_DEV float rawSmoke(const SimParams& P, const FpRender& R, BoxCursor& c, int x, int y, int z) {
   int s = slotAt(P, R, c, x >> P.shift, y >> P.shift, z >> P.shift);
   if (s < 0) return 0.f;
   return ldHalf(P.fld, (size_t)s * 4 * P.N + localCell(P, x, y, z), P.scalarHalf != 0);
 }
 // fireProField of the smoke at `q` in cells: clamped to the box, trilinear.
-FP_DEV float smokeSample(const SimParams& P, const FpRender& R, SlotCache& c, float qx, float qy, float qz) {
+FP_DEV float smokeSample(const SimParams& P, const FpRender& R, BoxCursor& c, float qx, float qy, float qz) {
   float B = (float)P.B;
   qx = fminf(fmaxf(qx, (float)c.lo[0] * B + .5f), (float)(c.hi[0] + 1) * B - .5f);
   qy = fminf(fmaxf(qy, (float)c.lo[1] * B + .5f), (float)(c.hi[1] + 1) * B - .5f);
@@ -95,7 +106,7 @@ FP_DEV float smokeSample(const SimParams& P, const FpRender& R, SlotCache& c, fl
   return v;
 }
 // smoothSmoke's [1,2,1]/4 density at a world cell: eight half-offset samples.
-FP_DEV float smoothedSmoke(const SimParams& P, const FpRender& R, SlotCache& c, int x, int y, int z) {
+FP_DEV float smoothedSmoke(const SimParams& P, const FpRender& R, BoxCursor& c, int x, int y, int z) {
   float d = 0.f;
   for (int k = 0; k < 8; k++)
     d += smokeSample(P, R, c, (float)(x + (k & 1)), (float)(y + ((k >> 1) & 1)), (float)(z + (k >> 2)));
@@ -104,14 +115,14 @@ FP_DEV float smoothedSmoke(const SimParams& P, const FpRender& R, SlotCache& c, 
 
 // The coarse smoke grid (smoke_divisor d > 1): 2^P.smokeShift cells a brick side.
 // The simulation's coarse density at a coarse cell: zero outside the box or without a slot.
-FP_DEV float rawCoarse(const SimParams& P, const FpRender& R, SlotCache& c, int x, int y, int z) {
+FP_DEV float rawCoarse(const SimParams& P, const FpRender& R, BoxCursor& c, int x, int y, int z) {
   const int sh = P.smokeShift, m = (1 << sh) - 1;
   int s = slotAt(P, R, c, x >> sh, y >> sh, z >> sh);
   if (s < 0) return 0.f;
   return ldHalf(P.smk, (size_t)s * P.smokeCells + (((z & m) << sh | (y & m)) << sh | (x & m)), P.scalarHalf != 0);
 }
 // fireProField of the coarse density at `q` in coarse cells: clamped to the box, trilinear.
-FP_DEV float coarseSample(const SimParams& P, const FpRender& R, SlotCache& c, float qx, float qy, float qz) {
+FP_DEV float coarseSample(const SimParams& P, const FpRender& R, BoxCursor& c, float qx, float qy, float qz) {
   float S = (float)(1 << P.smokeShift);
   qx = fminf(fmaxf(qx, (float)c.lo[0] * S + .5f), (float)(c.hi[0] + 1) * S - .5f);
   qy = fminf(fmaxf(qy, (float)c.lo[1] * S + .5f), (float)(c.hi[1] + 1) * S - .5f);
@@ -128,7 +139,7 @@ FP_DEV float coarseSample(const SimParams& P, const FpRender& R, SlotCache& c, f
   return v;
 }
 // smoothCoarseSmoke (lighting.wgsl:104-129): the [1,2,1]/4 density at a coarse cell.
-FP_DEV float smoothedCoarse(const SimParams& P, const FpRender& R, SlotCache& c, int x, int y, int z) {
+FP_DEV float smoothedCoarse(const SimParams& P, const FpRender& R, BoxCursor& c, int x, int y, int z) {
   float d = 0.f;
   for (int k = 0; k < 8; k++)
     d += coarseSample(P, R, c, (float)(x + (k & 1)), (float)(y + ((k >> 1) & 1)), (float)(z + (k >> 2)));
@@ -136,7 +147,7 @@ FP_DEV float smoothedCoarse(const SimParams& P, const FpRender& R, SlotCache& c,
 }
 // The smoothed coarse density at a coarse cell: the pool in a brick with a slot, else what a
 // sample based in a slotted brick reads from its apron (`apron`), else zero.
-FP_DEV float renderSmokeCell(const SimParams& P, const FpRender& R, SlotCache& c, int x, int y, int z, bool apron) {
+FP_DEV float renderSmokeCell(const SimParams& P, const FpRender& R, BoxCursor& c, int x, int y, int z, bool apron) {
   const int sh = P.smokeShift, m = (1 << sh) - 1;
   int s = slotAt(P, R, c, x >> sh, y >> sh, z >> sh);
   if (s >= 0) return R.renderSmoke[(size_t)s * P.smokeCells + (((z & m) << sh | (y & m)) << sh | (x & m))];
@@ -144,7 +155,7 @@ FP_DEV float renderSmokeCell(const SimParams& P, const FpRender& R, SlotCache& c
 }
 // renderSmokeAt (volume-common.wgsl:74-78): fireProField of the smoothed coarse density at `q`
 // in coarse cells.
-FP_DEV float renderSmokeAt(const SimParams& P, const FpRender& R, SlotCache& c, float qx, float qy, float qz) {
+FP_DEV float renderSmokeAt(const SimParams& P, const FpRender& R, BoxCursor& c, float qx, float qy, float qz) {
   const int sh = P.smokeShift;
   float S = (float)(1 << sh);
   qx = fminf(fmaxf(qx, (float)c.lo[0] * S + .5f), (float)(c.hi[0] + 1) * S - .5f);
@@ -153,8 +164,20 @@ FP_DEV float renderSmokeAt(const SimParams& P, const FpRender& R, SlotCache& c, 
   float gx = qx - .5f, gy = qy - .5f, gz = qz - .5f;
   int x0 = (int)floorf(gx), y0 = (int)floorf(gy), z0 = (int)floorf(gz);
   float fx = gx - (float)x0, fy = gy - (float)y0, fz = gz - (float)z0;
-  bool based = slotAt(P, R, c, x0 >> sh, y0 >> sh, z0 >> sh) >= 0;
   float v = 0.f;
+  int slots[8];
+  if (slots8(R, c, sh, x0, y0, z0, 1, slots)) {
+    const int m = (1 << sh) - 1;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      int dx = k & 1, dy = (k >> 1) & 1, dz = k >> 2;
+      float w = (dx ? fx : 1.f - fx) * (dy ? fy : 1.f - fy) * (dz ? fz : 1.f - fz);
+      v += __ldg(&R.renderSmoke[(size_t)slots[k] * P.smokeCells +
+                                ((((z0 + dz) & m) << sh | ((y0 + dy) & m)) << sh | ((x0 + dx) & m))]) * w;
+    }
+    return v;
+  }
+  bool based = slotAt(P, R, c, x0 >> sh, y0 >> sh, z0 >> sh) >= 0;
   for (int k = 0; k < 8; k++) {
     int dx = k & 1, dy = (k >> 1) & 1, dz = k >> 2;
     float w = (dx ? fx : 1.f - fx) * (dy ? fy : 1.f - fy) * (dz ? fz : 1.f - fz);
@@ -164,7 +187,7 @@ FP_DEV float renderSmokeAt(const SimParams& P, const FpRender& R, SlotCache& c, 
 }
 // cachedSmokeCell (lighting.wgsl:133-156): the smoothed coarse density a conservative bound
 // reads at coarse cell (x,y,z): the pool, else the apron a previous neighbour holds.
-FP_DEV float cachedSmokeCell(const SimParams& P, const FpRender& R, SlotCache& c, int x, int y, int z) {
+FP_DEV float cachedSmokeCell(const SimParams& P, const FpRender& R, BoxCursor& c, int x, int y, int z) {
   const int sh = P.smokeShift, m = (1 << sh) - 1;
   int bx = x >> sh, by = y >> sh, bz = z >> sh;
   int s = slotAt(P, R, c, bx, by, bz);
@@ -182,12 +205,9 @@ FP_DEV float cachedSmokeCell(const SimParams& P, const FpRender& R, SlotCache& c
 // brick without one reads as the apron of a sample based in a slotted brick would hold it
 // (`apron`: the smoothed density, no heat, flame or fuel; all zero with coarse smoke, whose
 // field apron holds no neighbour), else zero.
-FP_DEV float4 renderCell(const SimParams& P, const FpRender& R, SlotCache& c, int x, int y, int z, bool apron) {
+FP_DEV float4 renderCell(const SimParams& P, const FpRender& R, BoxCursor& c, int x, int y, int z, bool apron) {
   int s = slotAt(P, R, c, x >> P.shift, y >> P.shift, z >> P.shift);
-  if (s >= 0) {
-    size_t i = (size_t)s * 4 * P.N + localCell(P, x, y, z);
-    return make_float4(R.renderField[i], R.renderField[i + P.N], R.renderField[i + 2 * P.N], R.renderField[i + 3 * P.N]);
-  }
+  if (s >= 0) return __ldg(&R.renderField[(size_t)s * P.N + localCell(P, x, y, z)]);
   if (!apron || P.smokeDiv > 1) return make_float4(0.f, 0.f, 0.f, 0.f);
   return make_float4(smoothedSmoke(P, R, c, x, y, z), 0.f, 0.f, 0.f);
 }
@@ -197,15 +217,11 @@ FP_DEV void add4(float4& a, const float4& b, float w) {
   a.z += b.z * w;
   a.w += b.w * w;
 }
-// fireProField of the render field at `q` in cells (fireProSample, volume-bricks.wgsl).
-FP_DEV float4 renderSample(const SimParams& P, const FpRender& R, SlotCache& c, float qx, float qy, float qz) {
-  float B = (float)P.B;
-  qx = fminf(fmaxf(qx, (float)c.lo[0] * B + .5f), (float)(c.hi[0] + 1) * B - .5f);
-  qy = fminf(fmaxf(qy, (float)c.lo[1] * B + .5f), (float)(c.hi[1] + 1) * B - .5f);
-  qz = fminf(fmaxf(qz, (float)c.lo[2] * B + .5f), (float)(c.hi[2] + 1) * B - .5f);
-  float gx = qx - .5f, gy = qy - .5f, gz = qz - .5f;
-  int x0 = (int)floorf(gx), y0 = (int)floorf(gy), z0 = (int)floorf(gz);
-  float fx = gx - (float)x0, fy = gy - (float)y0, fz = gz - (float)z0;
+// The trilinear sample of the 2x2x2 block from cell (x0,y0,z0) when a cell of it has no slot or
+// lies past the box: a lookup a cell. Out of line, so that the rare path costs the march and the
+// lighting neither registers nor instruction-cache space.
+static __device__ __noinline__ float4 renderSampleFar(const SimParams& P, const FpRender& R, BoxCursor c, int x0, int y0,
+                                                      int z0, float fx, float fy, float fz) {
   bool based = slotAt(P, R, c, x0 >> P.shift, y0 >> P.shift, z0 >> P.shift) >= 0;
   float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
   for (int k = 0; k < 8; k++) {
@@ -215,11 +231,93 @@ FP_DEV float4 renderSample(const SimParams& P, const FpRender& R, SlotCache& c, 
   }
   return v;
 }
+// fireProField of the render field at `q` in cells (fireProSample, volume-bricks.wgsl).
+FP_DEV float4 renderSample(const SimParams& P, const FpRender& R, BoxCursor& c, float qx, float qy, float qz) {
+  float B = (float)P.B;
+  qx = fminf(fmaxf(qx, (float)c.lo[0] * B + .5f), (float)(c.hi[0] + 1) * B - .5f);
+  qy = fminf(fmaxf(qy, (float)c.lo[1] * B + .5f), (float)(c.hi[1] + 1) * B - .5f);
+  qz = fminf(fmaxf(qz, (float)c.lo[2] * B + .5f), (float)(c.hi[2] + 1) * B - .5f);
+  float gx = qx - .5f, gy = qy - .5f, gz = qz - .5f;
+  int x0 = (int)floorf(gx), y0 = (int)floorf(gy), z0 = (int)floorf(gz);
+  float fx = gx - (float)x0, fy = gy - (float)y0, fz = gz - (float)z0;
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  int slots[8];
+  if (slots8(R, c, P.shift, x0, y0, z0, 1, slots)) {
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      int dx = k & 1, dy = (k >> 1) & 1, dz = k >> 2;
+      float w = (dx ? fx : 1.f - fx) * (dy ? fy : 1.f - fy) * (dz ? fz : 1.f - fz);
+      add4(v, __ldg(&R.renderField[(size_t)slots[k] * P.N + localCell(P, x0 + dx, y0 + dy, z0 + dz)]), w);
+    }
+    return v;
+  }
+  return renderSampleFar(P, R, c, x0, y0, z0, fx, fy, fz);
+}
 
-// fireProReconstruct (volume-reconstruction.wgsl:5-95): 0 trilinear; 1 quadratic and 2 cubic
-// B-splines from eight trilinear samples.
-FP_DEV float4 reconstruct(const SimParams& P, const FpRender& R, SlotCache& c, float px, float py, float pz, int mode) {
-  if (mode == 0) return renderSample(P, R, c, px, py, pz);
+// Two FP32 multiply-adds an instruction (fma.rn.f32x2): a render-field cell is two pairs.
+struct Pair4 {
+  unsigned long long a, b;
+};
+FP_DEV unsigned long long both(float w) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(w));
+  return r;
+}
+FP_DEV void fma4(Pair4& v, const Pair4& t, unsigned long long w) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(v.a) : "l"(t.a), "l"(w));
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(v.b) : "l"(t.b), "l"(w));
+}
+// The tensor-product sum of the NT^3 cells from (x0,y0,z0) with weights w[axis][tap], all in
+// slotted bricks of the box (slots8's answer). x innermost, then y, then z.
+template <int NT>
+FP_DEV float4 tensorSample(const SimParams& P, const FpRender& R, const int* slots, int x0, int y0, int z0,
+                           const float (*w)[4]) {
+  const int sh = P.shift, m = P.B - 1, bx = x0 >> sh, by = y0 >> sh, bz = z0 >> sh;
+  unsigned base[8];
+#pragma unroll
+  for (int k = 0; k < 8; k++) base[k] = (unsigned)slots[k] * (unsigned)P.N;
+  const ulonglong2* F = reinterpret_cast<const ulonglong2*>(R.renderField);
+  unsigned long long wx[NT];
+  unsigned ox[NT];
+  bool hx[NT];
+#pragma unroll
+  for (int i = 0; i < NT; i++) {
+    wx[i] = both(w[0][i]);
+    ox[i] = (unsigned)((x0 + i) & m);
+    hx[i] = ((x0 + i) >> sh) != bx;
+  }
+  Pair4 v{0ull, 0ull};
+#pragma unroll
+  for (int k = 0; k < NT; k++) {
+    const bool hz = ((z0 + k) >> sh) != bz;
+    const unsigned lz = (unsigned)((z0 + k) & m) << (2 * sh);
+    const unsigned b00 = hz ? base[4] : base[0], b10 = hz ? base[5] : base[1], b01 = hz ? base[6] : base[2],
+                   b11 = hz ? base[7] : base[3];
+    Pair4 plane{0ull, 0ull};
+#pragma unroll
+    for (int j = 0; j < NT; j++) {
+      const bool hy = ((y0 + j) >> sh) != by;
+      const unsigned l = lz + ((unsigned)((y0 + j) & m) << sh), r0 = (hy ? b01 : b00) + l, r1 = (hy ? b11 : b10) + l;
+      Pair4 row{0ull, 0ull};
+#pragma unroll
+      for (int i = 0; i < NT; i++) {
+        const ulonglong2 q = __ldg(F + ((hx[i] ? r1 : r0) + ox[i]));
+        fma4(row, Pair4{q.x, q.y}, wx[i]);
+      }
+      fma4(plane, row, both(w[1][j]));
+    }
+    fma4(v, plane, both(w[2][k]));
+  }
+  float4 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v.a));
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.z), "=f"(r.w) : "l"(v.b));
+  return r;
+}
+
+// The B-spline as eight trilinear samples, when a cell of its block has no slot or lies past the
+// box (each sample then decides by itself what the missing cells hold and where it clamps).
+static __device__ __noinline__ float4 reconstructFar(const SimParams& P, const FpRender& R, BoxCursor c, float px,
+                                                     float py, float pz, int mode) {
   float pos[2][3], wt[2][3];
   float p[3] = {px, py, pz};
   for (int a = 0; a < 3; a++) {
@@ -247,6 +345,45 @@ FP_DEV float4 reconstruct(const SimParams& P, const FpRender& R, SlotCache& c, f
     int ix = (i >> 2) & 1, iy = (i >> 1) & 1, iz = i & 1;
     add4(v, renderSample(P, R, c, pos[ix][0], pos[iy][1], pos[iz][2]), wt[ix][0] * wt[iy][1] * wt[iz][2]);
   }
+  return make_float4(fmaxf(v.x, 0.f), fmaxf(v.y, 0.f), fmaxf(v.z, 0.f), fmaxf(v.w, 0.f));
+}
+
+// fireProReconstruct (volume-reconstruction.wgsl:5-95): 0 trilinear; 1 quadratic and 2 cubic
+// B-splines. The reference takes eight trilinear samples, a sampler's filtering being free there.
+// Here a sample is eight loads and as many lookups, and the eight touch just the 3^3 or 4^3 cells
+// under the spline once each: with every one of them in a slotted brick of the box (the window then
+// clamps nowhere) the same sum is taken over the cells directly, one vector load and two packed
+// multiply-adds a cell.
+FP_DEV float4 reconstruct(const SimParams& P, const FpRender& R, BoxCursor& c, float px, float py, float pz, int mode) {
+  if (mode == 0) return renderSample(P, R, c, px, py, pz);
+  float w[3][4];
+  int first[3];
+  const float p[3] = {px, py, pz};
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+    const float g = p[a] - .5f;
+    if (mode == 1) {
+      const float center = floorf(g + .5f), delta = g - center;
+      first[a] = (int)center - 1;
+      w[a][0] = .5f * (.5f - delta) * (.5f - delta);
+      w[a][1] = .75f - delta * delta;
+      w[a][2] = .5f * (.5f + delta) * (.5f + delta);
+      w[a][3] = 0.f;
+    } else {
+      const float base = floorf(g), q = g - base, inv = 1.f - q;
+      first[a] = (int)base - 1;
+      w[a][0] = inv * inv * inv / 6.f;
+      w[a][1] = (3.f * q * q * q - 6.f * q * q + 4.f) / 6.f;
+      w[a][2] = (-3.f * q * q * q + 3.f * q * q + 3.f * q + 1.f) / 6.f;
+      w[a][3] = q * q * q / 6.f;
+    }
+  }
+  int slots[8];
+  // The quadratic's eight samples look at a fourth cell too, with weight zero: what it holds does
+  // not matter, where the box clamps them does.
+  if (!slots8(R, c, P.shift, first[0], first[1], first[2], 3, slots)) return reconstructFar(P, R, c, px, py, pz, mode);
+  const float4 v = mode == 1 ? tensorSample<3>(P, R, slots, first[0], first[1], first[2], w)
+                             : tensorSample<4>(P, R, slots, first[0], first[1], first[2], w);
   return make_float4(fmaxf(v.x, 0.f), fmaxf(v.y, 0.f), fmaxf(v.z, 0.f), fmaxf(v.w, 0.f));
 }
 
@@ -281,7 +418,7 @@ FP_DEV float3 emissionOf(const FpRender& R, const float4& f) {
 
 // sampleWorld (volume-common.wgsl:33-43): the render field at world point p, zero outside
 // the box.
-FP_DEV float4 sampleWorld(const SimParams& P, const FpRender& R, SlotCache& c, float px, float py, float pz) {
+FP_DEV float4 sampleWorld(const SimParams& P, const FpRender& R, BoxCursor& c, float px, float py, float pz) {
   float size = (float)P.B * P.h;
   if (px < (float)c.lo[0] * size || py < (float)c.lo[1] * size || pz < (float)c.lo[2] * size ||
       px > (float)(c.hi[0] + 1) * size || py > (float)(c.hi[1] + 1) * size || pz > (float)(c.hi[2] + 1) * size)
@@ -295,7 +432,7 @@ FP_DEV float4 sampleWorld(const SimParams& P, const FpRender& R, SlotCache& c, f
 }
 
 // exitDistance (lighting.wgsl:248-255).
-FP_DEV float exitDistance(const SimParams& P, const SlotCache& c, float px, float py, float pz, float dx, float dy,
+FP_DEV float exitDistance(const SimParams& P, const BoxCursor& c, float px, float py, float pz, float dx, float dy,
                           float dz) {
   float size = (float)P.B * P.h;
   float p[3] = {px, py, pz}, d[3] = {dx, dy, dz}, m = 1e30f;
@@ -315,7 +452,7 @@ FP_DEV float integratedTransmission(float extinction, float distance, float atte
 }
 
 // incidentLight (lighting.wgsl:257-310): glow RGB and the sun's transmittance at p.
-FP_DEV float4 incidentLight(const SimParams& P, const FpRender& R, SlotCache& c, float px, float py, float pz) {
+FP_DEV float4 incidentLight(const SimParams& P, const FpRender& R, BoxCursor& c, float px, float py, float pz) {
   float4 local = sampleWorld(P, R, c, px, py, pz);
   if (local.x + glowOf(local.z) < 1e-5f) return make_float4(0.f, 0.f, 0.f, 1.f);
   float ln = sqrtf(R.light[0] * R.light[0] + R.light[1] * R.light[1] + R.light[2] * R.light[2]);
@@ -360,7 +497,7 @@ FP_DEV float4 incidentLight(const SimParams& P, const FpRender& R, SlotCache& c,
 // the same cursor): the lanes take the shadow samples (32 at a time) and the six glow
 // directions, and every lane then adds their terms in the order of the serial loops, with the
 // serial early stop of the shadow sum, so all lanes return the serial result's value.
-FP_DEV float4 incidentLightWarp(const SimParams& P, const FpRender& R, SlotCache& c, float px, float py, float pz) {
+FP_DEV float4 incidentLightWarp(const SimParams& P, const FpRender& R, BoxCursor& c, float px, float py, float pz) {
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   float4 local = sampleWorld(P, R, c, px, py, pz);
@@ -430,7 +567,7 @@ FP_DEV float4 incidentLightWarp(const SimParams& P, const FpRender& R, SlotCache
 
 // The brick of computing brick `i` inside a box, that box made the current one, with its
 // slot; false when no box holds it.
-FP_DEV bool boxBrick(const SimParams& P, const FpRender& R, SlotCache& c, uint32_t i, int& bx, int& by, int& bz,
+FP_DEV bool boxBrick(const SimParams& P, const FpRender& R, BoxCursor& c, uint32_t i, int& bx, int& by, int& bz,
                      int& slot) {
   uint32_t id = P.active[i];
   if (!homeOk(P, id)) return false;  // the bounds-checked build only
@@ -441,7 +578,7 @@ FP_DEV bool boxBrick(const SimParams& P, const FpRender& R, SlotCache& c, uint32
   bz = t.z * 4 + (l >> 4);
   int k = 0;
   for (; k < R.boxCount; k++) {
-    const int* b = R.boxes + 6 * k;
+    const int* b = R.boxes + FP_BOX_INTS * k;
     if (bx >= b[0] && bx <= b[3] && by >= b[1] && by <= b[4] && bz >= b[2] && bz <= b[5]) break;
   }
   if (k == R.boxCount) return false;
@@ -450,23 +587,34 @@ FP_DEV bool boxBrick(const SimParams& P, const FpRender& R, SlotCache& c, uint32
   return slot >= 0;
 }
 
+// The boxes' brick tables: a hash lookup a brick of a box, once a render, in place of one at every
+// brick a ray or a light sample enters.
+__global__ void __launch_bounds__(256) k_render_pages(const SimParams* __restrict__ Pp, const __grid_constant__ FpRender R) {
+  const SimParams& P = *Pp;
+  for (int k = blockIdx.y; k < R.boxCount; k += gridDim.y) {
+    const int* b = R.boxes + FP_BOX_INTS * k;
+    const int nx = b[3] - b[0] + 1, ny = b[4] - b[1] + 1, nz = b[5] - b[2] + 1, total = nx * ny * nz;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x)
+      R.pages[b[6] + i] = hashedSlot(P, b[0] + i % nx, b[1] + i / nx % ny, b[2] + i / (nx * ny));
+  }
+}
+
 // smoothSmoke: each boxed brick's render field, the smoothed density with heat, lifetime and
 // fuel as they are.
-__global__ void __launch_bounds__(RTHREADS) k_render_field(const SimParams* __restrict__ Pp, FpRender R) {
+__global__ void __launch_bounds__(RTHREADS) k_render_field(const SimParams* __restrict__ Pp, const __grid_constant__ FpRender R) {
   const SimParams& P = *Pp;
   uint32_t total = P.counters->active;
   const bool half = P.scalarHalf != 0;
   for (uint32_t i = blockIdx.x; i < total; i += gridDim.x) {
-    SlotCache c = noBox();
+    BoxCursor c = noBox();
     int bx, by, bz, slot;
     if (!boxBrick(P, R, c, i, bx, by, bz, slot)) continue;
     for (int k = threadIdx.x; k < P.N; k += blockDim.x) {
       int x = bx * P.B + (k & (P.B - 1)), y = by * P.B + ((k >> P.shift) & (P.B - 1)), z = bz * P.B + (k >> (2 * P.shift));
       size_t o = (size_t)slot * 4 * P.N + k;
-      R.renderField[o] = P.smokeDiv > 1 ? ldHalf(P.fld, o, half) : smoothedSmoke(P, R, c, x, y, z);
-      R.renderField[o + P.N] = ldHalf(P.fld, o + P.N, half);
-      R.renderField[o + 2 * P.N] = ldHalf(P.fld, o + 2 * P.N, half);
-      R.renderField[o + 3 * P.N] = ldHalf(P.fld, o + 3 * P.N, half);
+      R.renderField[(size_t)slot * P.N + k] =
+          make_float4(P.smokeDiv > 1 ? ldHalf(P.fld, o, half) : smoothedSmoke(P, R, c, x, y, z),
+                      ldHalf(P.fld, o + P.N, half), ldHalf(P.fld, o + 2 * P.N, half), ldHalf(P.fld, o + 3 * P.N, half));
     }
     if (P.smokeDiv > 1) {  // smoothCoarseSmoke on the brick's coarse cells
       const int sh = P.smokeShift, S = 1 << sh;
@@ -479,7 +627,7 @@ __global__ void __launch_bounds__(RTHREADS) k_render_field(const SimParams* __re
 }
 
 // buildOccupancy and buildLighting of each boxed brick, from the render field.
-__global__ void __launch_bounds__(RTHREADS) k_render_light(const SimParams* __restrict__ Pp, FpRender R) {
+__global__ void __launch_bounds__(RTHREADS) k_render_light(const SimParams* __restrict__ Pp, const __grid_constant__ FpRender R) {
   const SimParams& P = *Pp;
   __shared__ int flags;
   __shared__ int glowBits, smokeBits;  // the coarse bound's maxima (nonnegative floats' bits)
@@ -489,7 +637,7 @@ __global__ void __launch_bounds__(RTHREADS) k_render_light(const SimParams* __re
   const float texel = P.h * (float)(P.B >> R.lightShift);
   const int per = P.B / 8, blocks = per * per * per;
   for (uint32_t i = blockIdx.x; i < total; i += gridDim.x) {
-    SlotCache c = noBox();
+    BoxCursor c = noBox();
     int bx, by, bz, slot;
     if (!boxBrick(P, R, c, i, bx, by, bz, slot)) continue;  // the same for the whole CTA
     // Each 8-cell block with a halo of two cells, in units of 2x2x2 cells: a unit in a
@@ -553,28 +701,19 @@ __global__ void __launch_bounds__(RTHREADS) k_render_light(const SimParams* __re
       float4 light = incidentLightWarp(P, R, c, ((float)(bx * L + lx) + .5f) * texel,
                                        ((float)(by * L + ly) + .5f) * texel, ((float)(bz * L + lz) + .5f) * texel);
       if ((threadIdx.x & 31) == 0) {
-        size_t o = (size_t)slot * 4 * L3 + k;
-        R.lighting[o] = light.x;
-        R.lighting[o + L3] = light.y;
-        R.lighting[o + 2 * L3] = light.z;
-        R.lighting[o + 3 * L3] = light.w;
+        R.lighting[(size_t)slot * L3 + k] = light;
       }
     }
   }
 }
 
-// fireProLight (volume-bricks.wgsl:158-178) at `q` in lighting texels.
-FP_DEV float4 lightSample(const SimParams& P, const FpRender& R, SlotCache& c, float qx, float qy, float qz) {
+// The lighting sample whose texels' bricks are not all slotted: out of line, rare.
+static __device__ __noinline__ float4 lightSampleFar(const SimParams& P, const FpRender& R, BoxCursor c, int x0, int y0,
+                                                     int z0, float fx, float fy, float fz) {
   const int L = 1 << R.lightShift, L3 = L * L * L;
   const float texel = P.h * (float)(P.B >> R.lightShift);
-  qx = fminf(fmaxf(qx, (float)c.lo[0] * L + .5f), (float)(c.hi[0] + 1) * L - .5f);
-  qy = fminf(fmaxf(qy, (float)c.lo[1] * L + .5f), (float)(c.hi[1] + 1) * L - .5f);
-  qz = fminf(fmaxf(qz, (float)c.lo[2] * L + .5f), (float)(c.hi[2] + 1) * L - .5f);
-  float gx = qx - .5f, gy = qy - .5f, gz = qz - .5f;
-  int x0 = (int)floorf(gx), y0 = (int)floorf(gy), z0 = (int)floorf(gz);
   if (slotAt(P, R, c, x0 >> R.lightShift, y0 >> R.lightShift, z0 >> R.lightShift) < 0)
     return make_float4(0.f, 0.f, 0.f, 1.f);
-  float fx = gx - (float)x0, fy = gy - (float)y0, fz = gz - (float)z0;
   float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
   for (int k = 0; k < 8; k++) {
     int dx = k & 1, dy = (k >> 1) & 1, dz = k >> 2;
@@ -583,15 +722,37 @@ FP_DEV float4 lightSample(const SimParams& P, const FpRender& R, SlotCache& c, f
     int s = slotAt(P, R, c, x >> R.lightShift, y >> R.lightShift, z >> R.lightShift);
     float4 t;
     if (s >= 0) {
-      int m = L - 1;
-      size_t o = (size_t)s * 4 * L3 + (((z & m) * L + (y & m)) * L + (x & m));
-      t = make_float4(R.lighting[o], R.lighting[o + L3], R.lighting[o + 2 * L3], R.lighting[o + 3 * L3]);
+      const int m = L - 1;
+      t = __ldg(&R.lighting[(size_t)s * L3 + (((z & m) * L + (y & m)) * L + (x & m))]);
     } else {  // the apron of a neighbour without a slot: lit where it stands
       t = incidentLight(P, R, c, ((float)x + .5f) * texel, ((float)y + .5f) * texel, ((float)z + .5f) * texel);
     }
     add4(v, t, w);
   }
   return v;
+}
+// fireProLight (volume-bricks.wgsl:158-178) at `q` in lighting texels.
+FP_DEV float4 lightSample(const SimParams& P, const FpRender& R, BoxCursor& c, float qx, float qy, float qz) {
+  const int L = 1 << R.lightShift, L3 = L * L * L;
+  qx = fminf(fmaxf(qx, (float)c.lo[0] * L + .5f), (float)(c.hi[0] + 1) * L - .5f);
+  qy = fminf(fmaxf(qy, (float)c.lo[1] * L + .5f), (float)(c.hi[1] + 1) * L - .5f);
+  qz = fminf(fmaxf(qz, (float)c.lo[2] * L + .5f), (float)(c.hi[2] + 1) * L - .5f);
+  float gx = qx - .5f, gy = qy - .5f, gz = qz - .5f;
+  int x0 = (int)floorf(gx), y0 = (int)floorf(gy), z0 = (int)floorf(gz);
+  float fx = gx - (float)x0, fy = gy - (float)y0, fz = gz - (float)z0;
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  int slots[8];
+  if (slots8(R, c, R.lightShift, x0, y0, z0, 1, slots)) {
+    const int m = L - 1;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      int dx = k & 1, dy = (k >> 1) & 1, dz = k >> 2;
+      float w = (dx ? fx : 1.f - fx) * (dy ? fy : 1.f - fy) * (dz ? fz : 1.f - fz);
+      add4(v, __ldg(&R.lighting[(size_t)slots[k] * L3 + ((((z0 + dz) & m) * L + ((y0 + dy) & m)) * L + ((x0 + dx) & m))]), w);
+    }
+    return v;
+  }
+  return lightSampleFar(P, R, c, x0, y0, z0, fx, fy, fz);
 }
 
 // fireProJitter (volume-march.wgsl:94-102).
@@ -617,7 +778,7 @@ struct Ray {
 };
 // fireProHit: where the ray enters and leaves box k (entry after exit when it misses).
 FP_DEV float2 boxHit(const FpRender& R, const Ray& r, int k, float brickSize) {
-  const int* b = R.boxes + 6 * k;
+  const int* b = R.boxes + FP_BOX_INTS * k;
   float lo = 0.f, hi = 1e30f;
   for (int a = 0; a < 3; a++) {
     float ta = ((float)b[a] * brickSize - r.ro[a]) / r.safe[a];
@@ -675,7 +836,7 @@ FP_DEV bool rayOf(const SimParams& P, const FpRender& R, float ux, float uy, Ray
 // fireProEnter (fireProNext): the box the ray is in at t, or the next one it enters, becomes the
 // current one with its exit, and t moves to its entry; false past the last box. Boxes never
 // overlap, so of the boxes the ray has not left, the one it enters first is the one.
-FP_DEV bool enterBox(const SimParams& P, const FpRender& R, const Ray& r, float& t, float& exit, SlotCache& c) {
+FP_DEV bool enterBox(const SimParams& P, const FpRender& R, const Ray& r, float& t, float& exit, BoxCursor& c) {
   const float brickSize = P.h * (float)P.B;
   float entry = 1e30f, out = 0.f;
   int best = -1;
@@ -694,16 +855,25 @@ FP_DEV bool enterBox(const SimParams& P, const FpRender& R, const Ray& r, float&
   return true;
 }
 
-// One step of fireProMarch (volume-march.wgsl:178-268) at t, ds long, in the current box (which
-// the ray leaves at `exit`): past an empty block a skip of whole steps up to the exit, else the
-// shaded sample. Returns the next t.
-FP_DEV float marchStep(const SimParams& P, const FpRender& R, SlotCache& c, const Ray& r, float t, float ds, float exit,
-                       float& trans, float* rad) {
-  const float brickSize = P.h * (float)P.B, lightRatio = (float)(P.B >> R.lightShift);
+// One sample of fireProMarch (volume-march.wgsl:178-268) at t, ds long, in the current box (which
+// the ray leaves at `exit`).
+struct Sample {
+  bool lit;        // its block may hold something visible; else the ray goes on at `next`
+  float next;      // past an empty block: whole steps beyond it, up to the exit
+  float cell[3];   // the sample point in field cells
+  int filter;      // the reconstruction filter of its block
+};
+FP_DEV Sample sampleAt(const SimParams& P, const FpRender& R, BoxCursor& c, const Ray& r, float t, float ds, float exit) {
+  const float brickSize = P.h * (float)P.B;
+  Sample s;
   float tt = t + r.jitter * ds;
   float p[3] = {r.ro[0] + r.rd[0] * tt, r.ro[1] + r.rd[1] * tt, r.ro[2] + r.rd[2] * tt};
-  float cell[3] = {p[0] / P.h, p[1] / P.h, p[2] / P.h};
-  int ci[3] = {(int)floorf(cell[0]), (int)floorf(cell[1]), (int)floorf(cell[2])};
+  int ci[3];
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+    s.cell[a] = p[a] / P.h;
+    ci[a] = (int)floorf(s.cell[a]);
+  }
   int slot = slotAt(P, R, c, ci[0] >> P.shift, ci[1] >> P.shift, ci[2] >> P.shift);
   float size = brickSize;
   int flags = 0;
@@ -713,92 +883,208 @@ FP_DEV float marchStep(const SimParams& P, const FpRender& R, SlotCache& c, cons
     flags = R.occupancy[(size_t)slot * per * per * per + block];
     size = P.h * 8.f;
   }
-  if (!(flags & 2)) {
+  s.lit = (flags & 2) != 0;
+  s.filter = (flags & 1) ? R.filter : 0;
+  s.next = t;
+  if (!s.lit) {
     // Skip whole steps past the empty block, keeping the lattice.
     float dist = 1e30f;
+#pragma unroll
     for (int a = 0; a < 3; a++) dist = fminf(dist, ((floorf(p[a] / size) + r.exitSide[a]) * size - p[a]) / r.safe[a]);
-    return fminf(t + fmaxf(1.f, floorf(dist / r.stepSize) + 1.f) * r.stepSize, exit);
+    s.next = fminf(t + fmaxf(1.f, floorf(dist / r.stepSize) + 1.f) * r.stepSize, exit);
   }
-  float4 f = reconstruct(P, R, c, cell[0], cell[1], cell[2], (flags & 1) ? R.filter : 0);
+  return s;
+}
+// The radiance a sample ds long adds per unit of the transmittance before it, and the factor it
+// leaves of that transmittance.
+FP_DEV float4 shade(const SimParams& P, const FpRender& R, BoxCursor& c, const Ray& r, const Sample& s, float ds) {
+  const float lightRatio = (float)(P.B >> R.lightShift);
+  float4 f = reconstruct(P, R, c, s.cell[0], s.cell[1], s.cell[2], s.filter);
   if (P.smokeDiv > 1) {  // fireProRenderField: the smoothed coarse density, trilinear
     const float q = 1.f / (float)P.smokeDiv;
-    f.x = renderSmokeAt(P, R, c, cell[0] * q, cell[1] * q, cell[2] * q);
+    f.x = renderSmokeAt(P, R, c, s.cell[0] * q, s.cell[1] * q, s.cell[2] * q);
   }
-  if (f.x + glowOf(f.z) > .002f) {
-    // fireProShade
-    float3 glow = emissionOf(R, f);
-    float density = fmaxf(0.f, f.x) * R.optical[0];
-    float sc[3] = {0.f, 0.f, 0.f};
-    if (density > 0.f) {
-      float4 inc = lightSample(P, R, c, cell[0] / lightRatio, cell[1] / lightRatio, cell[2] / lightRatio);
-      sc[0] = R.smoke[0] * (R.ambient[0] + r.direct[0] * inc.w + inc.x * .65f) * density;
-      sc[1] = R.smoke[1] * (R.ambient[1] + r.direct[1] * inc.w + inc.y * .65f) * density;
-      sc[2] = R.smoke[2] * (R.ambient[2] + r.direct[2] * inc.w + inc.z * .65f) * density;
+  if (!(f.x + glowOf(f.z) > .002f)) return make_float4(0.f, 0.f, 0.f, 1.f);
+  // fireProShade
+  float3 glow = emissionOf(R, f);
+  float density = fmaxf(0.f, f.x) * R.optical[0];
+  float sc[3] = {0.f, 0.f, 0.f};
+  if (density > 0.f) {
+    float4 inc = lightSample(P, R, c, s.cell[0] / lightRatio, s.cell[1] / lightRatio, s.cell[2] / lightRatio);
+    sc[0] = R.smoke[0] * (R.ambient[0] + r.direct[0] * inc.w + inc.x * .65f) * density;
+    sc[1] = R.smoke[1] * (R.ambient[1] + r.direct[1] * inc.w + inc.y * .65f) * density;
+    sc[2] = R.smoke[2] * (R.ambient[2] + r.direct[2] * inc.w + inc.z * .65f) * density;
+  }
+  float ext = extinctionOf(R, f);
+  float tau = ext * ds;
+  float integral = ds * (1.f - .5f * tau + tau * tau / 6.f);
+  if (tau >= .001f) integral = (1.f - expf(-tau)) / ext;
+  return make_float4((sc[0] + glow.x) * integral, (sc[1] + glow.y) * integral, (sc[2] + glow.z) * integral,
+                     1.f - fminf(1.f, ext * integral));
+}
+
+// A ray is marched by a group of G lanes of a warp, a lane a step: the next G steps of the ray's
+// lattice are looked up together, those before the first empty block (or the end) are shaded
+// together, and their colours and transmittances are composed over the lanes. A serial march is a
+// chain of dependent lookups and loads a few hundred instructions long a step, and an image of a
+// few tens of thousands of rays leaves the chip idle waiting for it; along the ray the lanes also
+// read neighbouring cells and mostly agree on the filter. All lanes of a group hold the same ray
+// state. Steps past the first empty one, and those past the point where the ray turns opaque, are
+// dropped, so the samples that count are the serial march's, at the same positions.
+// Every lane of the warp calls this together, those without work with `alive` false.
+constexpr float OPAQUE = .008f;
+struct March {
+  float t, exit, trans, rad[3];
+};
+template <int G>
+FP_DEV void marchGroup(const SimParams& P, const FpRender& R, BoxCursor& c, const Ray& r, float limit, bool alive, March& m) {
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & (G - 1);
+  float t = m.t;
+#pragma unroll
+  for (int j = 0; j < G - 1; j++)  // the serial march's own sums
+    if (j < lane) t += r.stepSize;
+  const float ds = fminf(r.stepSize, limit - t);
+  const bool live = alive && t < limit;
+  Sample s;
+  s.lit = false;
+  s.next = t;
+  if (live) s = sampleAt(P, R, c, r, t, ds, m.exit);
+  int n = G;  // the lanes before the first empty or absent step
+  float next;
+  if constexpr (G > 1) {
+    const unsigned group = (__ballot_sync(full, !(live && s.lit)) >> ((threadIdx.x & 31) & ~(G - 1))) & ((1u << G) - 1u);
+    n = group ? __ffs(group) - 1 : G;
+  } else {
+    n = s.lit ? 1 : 0;
+  }
+  float4 q = make_float4(0.f, 0.f, 0.f, 1.f);
+  if (live && lane < n) q = shade(P, R, c, r, s, ds);
+  // Where the ray goes on: past the last shaded step, or past the empty block after it.
+  next = (live && s.lit) ? t + ds : s.next;
+  if constexpr (G > 1) {
+    const bool absent = !__shfl_sync(full, live ? 1 : 0, n < G ? n : G - 1, G);  // the step after the last is past the limit
+    const float empty = __shfl_sync(full, next, n < G ? n : G - 1, G);
+    const float lastEnd = __shfl_sync(full, next, n > 0 ? n - 1 : 0, G);
+    next = (n < G && !absent) ? empty : lastEnd;
+    // The transmittance before each lane's step: an exclusive product over the group.
+    float incl = q.w;
+#pragma unroll
+    for (int o = 1; o < G; o <<= 1) {
+      const float v = __shfl_up_sync(full, incl, o, G);
+      if (lane >= o) incl *= v;
     }
-    float ext = extinctionOf(R, f);
-    float tau = ext * ds;
-    float integral = ds * (1.f - .5f * tau + tau * tau / 6.f);
-    if (tau >= .001f) integral = (1.f - expf(-tau)) / ext;
-    rad[0] += trans * (sc[0] + glow.x) * integral;
-    rad[1] += trans * (sc[1] + glow.y) * integral;
-    rad[2] += trans * (sc[2] + glow.z) * integral;
-    trans *= 1.f - fminf(1.f, ext * integral);
+    const float before = __shfl_up_sync(full, incl, 1, G);
+    const float tb = lane == 0 ? m.trans : m.trans * before;
+    const bool counts = tb >= OPAQUE;  // falls along the group: a prefix of it
+    float x = counts ? tb * q.x : 0.f, y = counts ? tb * q.y : 0.f, z = counts ? tb * q.z : 0.f;
+    float left = counts ? tb * q.w : m.trans;
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) {
+      x += __shfl_xor_sync(full, x, o, G);
+      y += __shfl_xor_sync(full, y, o, G);
+      z += __shfl_xor_sync(full, z, o, G);
+      left = fminf(left, __shfl_xor_sync(full, left, o, G));
+    }
+    if (alive) {
+      m.rad[0] += x;
+      m.rad[1] += y;
+      m.rad[2] += z;
+      m.trans = left;
+      m.t = next;
+    }
+  } else if (alive) {
+    m.rad[0] += m.trans * q.x;
+    m.rad[1] += m.trans * q.y;
+    m.rad[2] += m.trans * q.z;
+    m.trans *= q.w;
+    m.t = next;
   }
-  return t + ds;
+}
+
+// The pixel of a thread's group: a CTA covers a tile of pixels, so that the rays of a warp and of
+// a CTA read neighbouring bricks.
+template <int G>
+FP_DEV void groupPixel(int& px, int& py) {
+  constexpr int RAYS = RTHREADS / G, TX = RAYS >= 64 ? 16 : (RAYS >= 16 ? 4 : 2), WX = 32 / G >= 8 ? 8 : (32 / G >= 2 ? 2 : 1);
+  constexpr int WY = (32 / G) / WX;  // a warp's rays: WX x WY
+  const int warp = threadIdx.x >> 5, g = (threadIdx.x & 31) / G;
+  constexpr int PER = TX / WX;  // warps a row of the CTA's tile
+  px = blockIdx.x * TX + (warp % PER) * WX + g % WX;
+  py = blockIdx.y * (RAYS / TX) + (warp / PER) * WY + g / WX;
+}
+template <int G>
+static dim3 groupGrid(int w, int h) {
+  constexpr int RAYS = RTHREADS / G, TX = RAYS >= 64 ? 16 : (RAYS >= 16 ? 4 : 2), TY = RAYS / TX;
+  return dim3((unsigned)((w + TX - 1) / TX), (unsigned)((h + TY - 1) / TY));
 }
 
 // buildSlices (volume-slices.wgsl:28-122): a ray per half-resolution pixel marches from the
 // first box entry to the last exit, box by box, recording radiance and opacity at FP_SLICES
 // evenly spaced depths; depths passed by a skip or a jump between boxes keep the values of the
-// moment, those past the exit or an opaque ray the final ones.
-__global__ void __launch_bounds__(RTHREADS) k_slices(const SimParams* __restrict__ Pp, FpRender R) {
+// moment, those past the exit or an opaque ray the final ones. Without a scene depth every pixel
+// resumes from the last slice, so only that one is stored.
+template <int G>
+__global__ void __launch_bounds__(RTHREADS) k_slices(const SimParams* __restrict__ Pp, const __grid_constant__ FpRender R) {
   const SimParams& P = *Pp;
-  int pix = blockIdx.x * blockDim.x + threadIdx.x;
-  if (pix >= R.sliceW * R.sliceH) return;
-  int px = pix % R.sliceW, py = pix / R.sliceW;
-  float4* out = reinterpret_cast<float4*>(R.slices) + (size_t)pix * FP_SLICES;
-  float trans = 1.f, rad[3] = {0.f, 0.f, 0.f};
+  int px, py;
+  groupPixel<G>(px, py);
+  const bool inside = px < R.sliceW && py < R.sliceH;
+  const size_t plane = (size_t)R.sliceW * R.sliceH;
+  float4* out = R.slices + (size_t)py * R.sliceW + px;
+  const bool writes = inside && (threadIdx.x & (G - 1)) == 0;
+  March m{0.f, 0.f, 1.f, {0.f, 0.f, 0.f}};
   int recorded = 0;
+  auto record = [&]() {
+    if (writes && (R.depth || recorded == FP_SLICES - 1))
+      out[(size_t)recorded * plane] = make_float4(m.rad[0], m.rad[1], m.rad[2], 1.f - m.trans);
+    recorded++;
+  };
   Ray r;
-  if (R.boxCount > 0 && rayOf(P, R, ((float)px + .5f) / (float)R.sliceW, ((float)py + .5f) / (float)R.sliceH, r)) {
+  bool alive = inside && R.boxCount > 0 &&
+               rayOf(P, R, ((float)px + .5f) / (float)R.sliceW, ((float)py + .5f) / (float)R.sliceH, r);
+  float spacing = 0.f, depth = 0.f;
+  if (alive) {
     r.jitter = jitterOf((uint32_t)px, (uint32_t)py, R.time);
-    const float spacing = fmaxf(r.hi - r.lo, 0.f) / (float)FP_SLICES;
-    SlotCache c = noBox();
-    float t = r.lo, depth = r.lo + spacing, exit = t;
-    while (recorded < FP_SLICES && t < r.hi && trans >= .008f) {
-      if (t >= exit) {
-        if (!enterBox(P, R, r, t, exit, c)) break;
-      } else {
-        float ds = fminf(r.stepSize, fminf(depth, exit) - t);
-        t = marchStep(P, R, c, r, t, ds, exit, trans, rad);
-      }
-      while (recorded < FP_SLICES && t >= depth) {
-        out[recorded] = make_float4(rad[0], rad[1], rad[2], 1.f - trans);
-        recorded++;
-        depth = r.lo + spacing * (float)(recorded + 1);
-      }
+    spacing = fmaxf(r.hi - r.lo, 0.f) / (float)FP_SLICES;
+    m.t = m.exit = r.lo;
+    depth = r.lo + spacing;
+  }
+  BoxCursor c = noBox();
+  while (true) {
+    alive = alive && recorded < FP_SLICES && m.t < r.hi && m.trans >= OPAQUE;
+    bool steps = alive;
+    if (alive && m.t >= m.exit) {
+      steps = false;
+      alive = enterBox(P, R, r, m.t, m.exit, c);
+    }
+    if (!__any_sync(0xffffffffu, alive)) break;
+    if (__any_sync(0xffffffffu, steps)) marchGroup<G>(P, R, c, r, fminf(depth, m.exit), steps, m);
+    while (alive && recorded < FP_SLICES && m.t >= depth) {
+      record();
+      depth = r.lo + spacing * (float)(recorded + 1);
     }
   }
-  for (; recorded < FP_SLICES; recorded++) out[recorded] = make_float4(rad[0], rad[1], rad[2], 1.f - trans);
+  while (recorded < FP_SLICES) record();
 }
 
 // fireProSceneVolume (scene-volume.wgsl:39-44, 146-167): the march of each pixel's ray up to
 // the scene's depth through the boxes, from the last half-resolution slice in front of it when
 // slices exist.
-__global__ void __launch_bounds__(RTHREADS) k_march(const SimParams* __restrict__ Pp, FpRender R) {
+template <int G>
+__global__ void __launch_bounds__(RTHREADS) k_march(const SimParams* __restrict__ Pp, const __grid_constant__ FpRender R) {
   const SimParams& P = *Pp;
-  int pix = blockIdx.x * blockDim.x + threadIdx.x;
-  if (pix >= R.width * R.height) return;
-  int px = pix % R.width, py = pix / R.width;
-  float4* out = reinterpret_cast<float4*>(R.image) + pix;
-  *out = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (R.boxCount == 0) return;
+  int px, py;
+  groupPixel<G>(px, py);
+  const bool inside = px < R.width && py < R.height;
+  const size_t pix = (size_t)py * R.width + px;
   const float ux = ((float)px + .5f) / (float)R.width, uy = ((float)py + .5f) / (float)R.height;
+  March m{0.f, 0.f, 1.f, {0.f, 0.f, 0.f}};
   Ray r;
-  if (!rayOf(P, R, ux, uy, r)) return;
+  bool alive = inside && R.boxCount > 0 && rayOf(P, R, ux, uy, r);
   // fireProSceneDistance (volume-march.wgsl:76-89): the scene's depth ends the ray.
-  float end = r.hi;
-  if (R.depth) {
+  float end = alive ? r.hi : 0.f;
+  if (alive && R.depth) {
     const float d = R.depth[pix];
     if (d < .999999f) {
       const float cx = ux * 2.f - 1.f, cy = 1.f - uy * 2.f;
@@ -810,48 +1096,54 @@ __global__ void __launch_bounds__(RTHREADS) k_march(const SimParams* __restrict_
       end = fminf(end, dist);
     }
   }
-  if (end <= r.lo) return;
-  r.jitter = jitterOf((uint32_t)px, (uint32_t)py, R.time);
-  float t = r.lo, trans = 1.f;
-  float rad[3] = {0.f, 0.f, 0.f};
-  if (R.slices) {
-    // Resume from the last slice in front of the scene: the half-resolution texels
-    // interpolated bilinearly (clamped at the edges) on that slice.
-    const float count = (float)FP_SLICES;
-    const float slice = floorf((end - r.lo) / (r.hi - r.lo) * count);
-    if (slice >= 1.f) {
-      const int layer = (int)fminf(slice, count) - 1;
-      float gx = ux * (float)R.sliceW - .5f, gy = uy * (float)R.sliceH - .5f;
-      float fx0 = floorf(gx), fy0 = floorf(gy);
-      float wx = gx - fx0, wy = gy - fy0;
-      int x0 = (int)fx0, y0 = (int)fy0;
-      int xs[2] = {min(max(x0, 0), R.sliceW - 1), min(max(x0 + 1, 0), R.sliceW - 1)};
-      int ys[2] = {min(max(y0, 0), R.sliceH - 1), min(max(y0 + 1, 0), R.sliceH - 1)};
-      const float4* S = reinterpret_cast<const float4*>(R.slices);
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      for (int k = 0; k < 4; k++) {
-        int ix = k & 1, iy = k >> 1;
-        add4(v, S[((size_t)ys[iy] * R.sliceW + xs[ix]) * FP_SLICES + layer], (ix ? wx : 1.f - wx) * (iy ? wy : 1.f - wy));
+  alive = alive && end > r.lo;
+  if (alive) {
+    r.jitter = jitterOf((uint32_t)px, (uint32_t)py, R.time);
+    m.t = r.lo;
+    if (R.slices) {
+      // Resume from the last slice in front of the scene: the half-resolution texels
+      // interpolated bilinearly (clamped at the edges) on that slice.
+      const float count = (float)FP_SLICES;
+      const float slice = R.depth ? floorf((end - r.lo) / (r.hi - r.lo) * count) : count;
+      if (slice >= 1.f) {
+        const int layer = (int)fminf(slice, count) - 1;
+        float gx = ux * (float)R.sliceW - .5f, gy = uy * (float)R.sliceH - .5f;
+        float fx0 = floorf(gx), fy0 = floorf(gy);
+        float wx = gx - fx0, wy = gy - fy0;
+        int x0 = (int)fx0, y0 = (int)fy0;
+        int xs[2] = {min(max(x0, 0), R.sliceW - 1), min(max(x0 + 1, 0), R.sliceW - 1)};
+        int ys[2] = {min(max(y0, 0), R.sliceH - 1), min(max(y0 + 1, 0), R.sliceH - 1)};
+        const float4* S = R.slices + (size_t)layer * R.sliceW * R.sliceH;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int k = 0; k < 4; k++) {
+          int ix = k & 1, iy = k >> 1;
+          add4(v, S[(size_t)ys[iy] * R.sliceW + xs[ix]], (ix ? wx : 1.f - wx) * (iy ? wy : 1.f - wy));
+        }
+        m.t = slice >= count ? r.hi : r.lo + (r.hi - r.lo) * slice / count;  // the last slice ends the ray
+        m.trans = 1.f - v.w;
+        m.rad[0] = v.x;
+        m.rad[1] = v.y;
+        m.rad[2] = v.z;
       }
-      t = r.lo + (r.hi - r.lo) * fminf(slice, count) / count;
-      trans = 1.f - v.w;
-      rad[0] = v.x;
-      rad[1] = v.y;
-      rad[2] = v.z;
     }
   }
   // fireProMarch: the cursor starts exited, so the first pass enters the box at t.
-  SlotCache c = noBox();
-  float exit = t;
-  while (t < end && trans >= .008f) {
-    if (t >= exit) {
-      if (!enterBox(P, R, r, t, exit, c)) break;
-      continue;
+  const bool drawn = alive;
+  BoxCursor c = noBox();
+  m.exit = m.t;
+  while (true) {
+    alive = alive && m.t < end && m.trans >= OPAQUE;
+    bool steps = alive;
+    if (alive && m.t >= m.exit) {
+      steps = false;
+      alive = enterBox(P, R, r, m.t, m.exit, c);
     }
-    float ds = fminf(r.stepSize, fminf(end, exit) - t);
-    t = marchStep(P, R, c, r, t, ds, exit, trans, rad);
+    if (!__any_sync(0xffffffffu, alive)) break;
+    if (__any_sync(0xffffffffu, steps)) marchGroup<G>(P, R, c, r, fminf(end, m.exit), steps, m);
   }
-  *out = make_float4(rad[0], rad[1], rad[2], 1.f - trans);
+  if (inside && (threadIdx.x & (G - 1)) == 0)
+    reinterpret_cast<float4*>(R.image)[pix] =
+        drawn ? make_float4(m.rad[0], m.rad[1], m.rad[2], 1.f - m.trans) : make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
 // collectLights (scene-lights.wgsl:37-106): a CTA of 64 lanes per computing brick, a lane per
@@ -859,7 +1151,7 @@ __global__ void __launch_bounds__(RTHREADS) k_march(const SimParams* __restrict_
 // anchor is the nearest to its centre (height above an anchor counting a quarter; ties to the
 // lower index); the lanes' luminance, luminance-weighted offsets and RGB are summed in shared
 // memory and seven lanes add the totals to the anchor's floats.
-__global__ void __launch_bounds__(64) k_collect_lights(const SimParams* __restrict__ Pp, FpRender R,
+__global__ void __launch_bounds__(64) k_collect_lights(const SimParams* __restrict__ Pp, const __grid_constant__ FpRender R,
                                                        const float* __restrict__ anchors, int count, float* sums) {
   const SimParams& P = *Pp;
   __shared__ float2 nearest[64];
@@ -962,12 +1254,18 @@ void fp_launch_collect_lights(const SimParams* dP, const FpRender& R, const floa
 }
 
 void fp_launch_render(const SimParams* dP, const FpRender& R, int sms, cudaStream_t st) {
+  if (R.pages) {
+    const int rows = R.boxCount < 64 ? R.boxCount : 64;
+    const long long blocks = (R.pageCount / rows + 255) / 256;
+    k_render_pages<<<dim3((unsigned)(blocks < 1 ? 1 : (blocks < sms * 8 ? blocks : sms * 8)), rows), 256, 0, st>>>(dP, R);
+  }
   k_render_field<<<sms * 8, RTHREADS, 0, st>>>(dP, R);
   k_render_light<<<sms * 8, RTHREADS, 0, st>>>(dP, R);
   if (R.slices) {
-    int half = R.sliceW * R.sliceH;
-    k_slices<<<(half + RTHREADS - 1) / RTHREADS, RTHREADS, 0, st>>>(dP, R);
+    k_slices<8><<<groupGrid<8>(R.sliceW, R.sliceH), RTHREADS, 0, st>>>(dP, R);
+    // Every pixel resumes at its last slice: at most an eighth of its ray is left to march.
+    k_march<1><<<groupGrid<1>(R.width, R.height), RTHREADS, 0, st>>>(dP, R);
+  } else {
+    k_march<8><<<groupGrid<8>(R.width, R.height), RTHREADS, 0, st>>>(dP, R);
   }
-  int pixels = R.width * R.height;
-  k_march<<<(pixels + RTHREADS - 1) / RTHREADS, RTHREADS, 0, st>>>(dP, R);
 }

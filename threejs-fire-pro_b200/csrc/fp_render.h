@@ -12,6 +12,12 @@
 // Depths a half-resolution pass records (VolumeSlices.ts DEPTH_SLICES).
 #define FP_SLICES 8
 
+// The render boxes' brick tables (FpRender::pages): rows of the box list, and the most bricks the
+// boxes may hold together for the tables to be built (64 MB; a box is the span of a cluster's
+// content, so thinly spread content can span far more bricks than it holds).
+#define FP_BOX_INTS 8
+#define FP_MAX_PAGES (1ll << 24)
+
 struct FpRender {
   float ivp[16];  // clip to world, column-major
   int width, height;
@@ -21,18 +27,23 @@ struct FpRender {
   float flameOpacity;
   int shadowSamples, raySteps, filter;
   int lightShift;       // lighting texels per brick side = 1 << lightShift
-  const int* boxes;     // the render boxes: lo xyz, hi xyz in bricks (inclusive), six ints each;
-                        // boxes never overlap, each lies in one cluster of tiles
+  const int* boxes;     // the render boxes, FP_BOX_INTS ints each: lo xyz, hi xyz in bricks
+                        // (inclusive), the box's first entry in `pages`; boxes never overlap, each
+                        // lies in one cluster of tiles
   int boxCount;
-  float* renderField;   // [slot][4][cells]: smoothed smoke, heat, lifetime, fuel (coarse smoke:
-                        // the simulation's fields as they are)
+  int* pages;           // per box, x fastest, each brick's slot or -1; null when the boxes hold more
+                        // than FP_MAX_PAGES bricks (lookups then go through the tile hash)
+  long long pageCount;
+  float4* renderField;  // [slot][cell]: smoothed smoke, heat, lifetime, fuel (coarse smoke: the
+                        // simulation's fields as they are)
   float* renderSmoke;   // coarse smoke (smokeDiv > 1): [slot][smoke cells], the smoothed density
-  float* lighting;      // [slot][4][texels]: glow RGB, sun transmittance
+  float4* lighting;     // [slot][texel]: glow RGB, sun transmittance
   uint8_t* occupancy;   // [slot]: bit 0 flame glow, bit 1 anything visible, in the block and halo
   const float4* lut;    // blackbody: peak-normalised linear RGB, log2 radiance
   float* image;         // width x height x 4
   const float* depth;   // the scene's depth buffer (width x height, clip z 0..1), or null
-  float* slices;        // half resolution: sliceW x sliceH x FP_SLICES x 4, or null (full resolution)
+  float4* slices;       // half resolution: FP_SLICES x sliceH x sliceW, or null (full resolution);
+                        // without a scene depth only the last of them is read, and written
   int sliceW, sliceH;
 };
 

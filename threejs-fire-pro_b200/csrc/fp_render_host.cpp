@@ -296,23 +296,40 @@ int Engine::render(const fp_camera& cam, const fp_render_settings& rs, float* im
   R.raySteps = (int)rs.ray_steps;
   R.filter = rs.filter;
   R.lightShift = lightShift;
-  // The boxes of the latest step (none before the first).
+  // The boxes of the latest step (none before the first) and their brick tables.
   R.boxCount = steps_ > 0 ? (int)(renderBoxes_.size() / 6) : 0;
   if (R.boxCount > 0) {
-    const size_t bytes = renderBoxes_.size() * 4;
-    if (renderBoxesD_.bytes < bytes && !alloc(renderBoxesD_, std::max<size_t>(bytes, 64 * 24), false)) return FP_ENOMEM;
-    if ((rc = check(cudaMemcpyAsync(renderBoxesD_.ptr, renderBoxes_.data(), bytes, cudaMemcpyHostToDevice, stream()),
-                    "render")))
+    std::vector<int> rows((size_t)R.boxCount * FP_BOX_INTS, 0);
+    long long pages = 0;
+    for (int k = 0; k < R.boxCount; k++) {
+      const int* box = &renderBoxes_[(size_t)k * 6];
+      int* row = &rows[(size_t)k * FP_BOX_INTS];
+      std::memcpy(row, box, 24);
+      row[6] = (int)std::min(pages, FP_MAX_PAGES);
+      long long bricks = 1;
+      for (int a = 0; a < 3; a++) bricks = std::min(bricks * std::max(0, box[3 + a] - box[a] + 1), FP_MAX_PAGES + 1);
+      pages = std::min(pages + bricks, FP_MAX_PAGES + 1);
+    }
+    const size_t bytes = rows.size() * 4;
+    if (renderBoxesD_.bytes < bytes && !alloc(renderBoxesD_, std::max<size_t>(bytes, 64 * FP_BOX_INTS * 4), false))
+      return FP_ENOMEM;
+    if ((rc = check(cudaMemcpyAsync(renderBoxesD_.ptr, rows.data(), bytes, cudaMemcpyHostToDevice, stream()), "render")))
       return rc;
+    // Grown by half again, so that boxes that widen from frame to frame seldom allocate.
+    if (pages <= FP_MAX_PAGES) {
+      if (renderPages_.bytes < (size_t)pages * 4 && !alloc(renderPages_, (size_t)pages * 6, false)) return FP_ENOMEM;
+      R.pages = (int*)renderPages_.ptr;
+      R.pageCount = pages;
+    }
   }
   R.boxes = (const int*)renderBoxesD_.ptr;
   R.depth = depth;
-  R.slices = cam.half_resolution ? (float*)slices_.ptr : nullptr;
+  R.slices = cam.half_resolution ? (float4*)slices_.ptr : nullptr;
   R.sliceW = sliceW;
   R.sliceH = sliceH;
-  R.renderField = (float*)renderField_.ptr;
+  R.renderField = (float4*)renderField_.ptr;
   R.renderSmoke = (float*)renderSmoke_.ptr;
-  R.lighting = (float*)lighting_.ptr;
+  R.lighting = (float4*)lighting_.ptr;
   R.occupancy = (uint8_t*)occupancy_.ptr;
   R.lut = (const float4*)lut_.ptr;
   R.image = out;
