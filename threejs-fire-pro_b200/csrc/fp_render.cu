@@ -19,6 +19,7 @@
 namespace {
 
 constexpr int RTHREADS = 128;
+constexpr int MARCH_CTAS = 3;
 
 // A thread's current box: the bricks its samples read.
 struct BoxCursor {
@@ -55,10 +56,37 @@ FP_DEV int hashedSlot(const SimParams& P, int bx, int by, int bz) {
 FP_DEV int pageIndex(const BoxCursor& c, int bx, int by, int bz) {
   return c.first + ((bz - c.lo[2]) * (c.hi[1] - c.lo[1] + 1) + (by - c.lo[1])) * (c.hi[0] - c.lo[0] + 1) + (bx - c.lo[0]);
 }
-// fireProPage: the slot of world brick b inside the current box, or -1.
+// fireProPage: the slot of world brick b inside the current box, or less than 0 (FpRender::pages).
 FP_DEV int slotAt(const SimParams& P, const FpRender& R, BoxCursor& c, int bx, int by, int bz) {
   if (!inBox(c, bx, by, bz)) return -1;
   return R.pages ? __ldg(&R.pages[pageIndex(c, bx, by, bz)]) : hashedSlot(P, bx, by, bz);
+}
+// Of a low-face cell (lx,ly,lz) of a brick of `side` cells a side, its place in the brick's three
+// apron planes.
+FP_DEV int apronIndex(int side, int lx, int ly, int lz) {
+  if (lx == 0) return lz * side + ly;
+  if (ly == 0) return (side + lz) * side + lx;
+  return (2 * side + ly) * side + lx;
+}
+// The cell at place i of a brick's apron planes; false for a place that stands for none (a cell on
+// two faces has one place) and for cells that no sample based in a slotted brick reads: `before`
+// has bit k set when the brick k's set bits (x, y, z) before this one on those axes has a slot.
+FP_DEV bool apronCell(int side, int i, unsigned before, int& lx, int& ly, int& lz) {
+  const int face = i / (side * side), a = i % side, b = (i / side) % side;
+  lx = face == 0 ? 0 : a;
+  ly = face == 1 ? 0 : (face == 0 ? a : b);
+  lz = face == 2 ? 0 : b;
+  if ((face >= 1 && lx == 0) || (face == 2 && ly == 0)) return false;
+  const unsigned on = (lx == 0 ? 1u : 0u) | (ly == 0 ? 2u : 0u) | (lz == 0 ? 4u : 0u);
+  for (unsigned k = 1; k < 8; k++)
+    if ((k & ~on) == 0u && ((before >> k) & 1u)) return true;
+  return false;
+}
+FP_DEV unsigned slottedBefore(const SimParams& P, const FpRender& R, BoxCursor& c, int bx, int by, int bz) {
+  unsigned before = 0;
+  for (int k = 1; k < 8; k++)
+    if (slotAt(P, R, c, bx - (k & 1), by - ((k >> 1) & 1), bz - (k >> 2)) >= 0) before |= 1u << k;
+  return before;
 }
 // The slots of the bricks that the cells from (x,y,z) to n further on each axis lie in: s[k] for
 // the low (bit clear) or high (bit set) brick on x, y, z (bits 0, 1, 2). n is less than a brick,
@@ -151,7 +179,9 @@ FP_DEV float renderSmokeCell(const SimParams& P, const FpRender& R, BoxCursor& c
   const int sh = P.smokeShift, m = (1 << sh) - 1;
   int s = slotAt(P, R, c, x >> sh, y >> sh, z >> sh);
   if (s >= 0) return R.renderSmoke[(size_t)s * P.smokeCells + (((z & m) << sh | (y & m)) << sh | (x & m))];
-  return apron ? smoothedCoarse(P, R, c, x, y, z) : 0.f;
+  if (!apron) return 0.f;
+  if (s <= -2) return R.apronSmoke[(size_t)(-2 - s) * 3 * (m + 1) * (m + 1) + apronIndex(m + 1, x & m, y & m, z & m)];
+  return smoothedCoarse(P, R, c, x, y, z);
 }
 // renderSmokeAt (volume-common.wgsl:74-78): fireProField of the smoothed coarse density at `q`
 // in coarse cells.
@@ -196,7 +226,7 @@ FP_DEV float cachedSmokeCell(const SimParams& P, const FpRender& R, BoxCursor& c
   for (int k = 1; k < 8; k++) {
     if (((k & 1) && l[0] != 0) || ((k & 2) && l[1] != 0) || ((k & 4) && l[2] != 0)) continue;
     if (slotAt(P, R, c, bx - (k & 1), by - ((k >> 1) & 1), bz - ((k >> 2) & 1)) >= 0)
-      return smoothedCoarse(P, R, c, x, y, z);
+      return renderSmokeCell(P, R, c, x, y, z, true);
   }
   return 0.f;
 }
@@ -209,6 +239,10 @@ FP_DEV float4 renderCell(const SimParams& P, const FpRender& R, BoxCursor& c, in
   int s = slotAt(P, R, c, x >> P.shift, y >> P.shift, z >> P.shift);
   if (s >= 0) return __ldg(&R.renderField[(size_t)s * P.N + localCell(P, x, y, z)]);
   if (!apron || P.smokeDiv > 1) return make_float4(0.f, 0.f, 0.f, 0.f);
+  if (s <= -2) {
+    const int m = P.B - 1;
+    return make_float4(R.apronField[(size_t)(-2 - s) * 3 * P.B * P.B + apronIndex(P.B, x & m, y & m, z & m)], 0.f, 0.f, 0.f);
+  }
   return make_float4(smoothedSmoke(P, R, c, x, y, z), 0.f, 0.f, 0.f);
 }
 FP_DEV void add4(float4& a, const float4& b, float w) {
@@ -243,11 +277,15 @@ FP_DEV float4 renderSample(const SimParams& P, const FpRender& R, BoxCursor& c, 
   float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
   int slots[8];
   if (slots8(R, c, P.shift, x0, y0, z0, 1, slots)) {
+    const unsigned sh = P.shift, m = P.B - 1;
+    const unsigned lx[2] = {x0 & m, (x0 + 1) & m}, ly[2] = {(y0 & m) << sh, ((y0 + 1) & m) << sh},
+                   lz[2] = {(z0 & m) << (2 * sh), ((z0 + 1) & m) << (2 * sh)};
+    const unsigned N = P.N;
 #pragma unroll
     for (int k = 0; k < 8; k++) {
       int dx = k & 1, dy = (k >> 1) & 1, dz = k >> 2;
       float w = (dx ? fx : 1.f - fx) * (dy ? fy : 1.f - fy) * (dz ? fz : 1.f - fz);
-      add4(v, __ldg(&R.renderField[(size_t)slots[k] * P.N + localCell(P, x0 + dx, y0 + dy, z0 + dz)]), w);
+      add4(v, __ldg(&R.renderField[(unsigned)slots[k] * N + (lx[dx] + ly[dy] + lz[dz])]), w);
     }
     return v;
   }
@@ -287,7 +325,9 @@ FP_DEV float4 tensorSample(const SimParams& P, const FpRender& R, const int* slo
     hx[i] = ((x0 + i) >> sh) != bx;
   }
   Pair4 v{0ull, 0ull};
-#pragma unroll
+  // A plane of the block at a time: its loads in flight together, and the code of one plane only
+  // (the whole block unrolled cost the march a fifth of its issue slots in instruction misses).
+#pragma unroll 1
   for (int k = 0; k < NT; k++) {
     const bool hz = ((z0 + k) >> sh) != bz;
     const unsigned lz = (unsigned)((z0 + k) & m) << (2 * sh);
@@ -306,7 +346,7 @@ FP_DEV float4 tensorSample(const SimParams& P, const FpRender& R, const int* slo
       }
       fma4(plane, row, both(w[1][j]));
     }
-    fma4(v, plane, both(w[2][k]));
+    fma4(v, plane, both(k == 0 ? w[2][0] : (k == 1 ? w[2][1] : (k == 2 ? w[2][2] : w[2][3]))));
   }
   float4 r;
   asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v.a));
@@ -391,7 +431,17 @@ FP_DEV float4 reconstruct(const SimParams& P, const FpRender& R, BoxCursor& c, f
 FP_DEV float extinctionOf(const FpRender& R, const float4& f) {
   return fmaxf(0.f, f.x) * R.optical[0] + glowOf(f.z) * R.flameOpacity;
 }
-FP_DEV float3 emissionOf(const FpRender& R, const float4& f) {
+// What the fire's tint makes of the blackbody colour, the same for every sample.
+struct Tint {
+  float peak, saturation;
+};
+FP_DEV Tint tintOf(const FpRender& R) {
+  Tint t;
+  t.peak = fmaxf(R.fire[0], fmaxf(R.fire[1], R.fire[2]));
+  t.saturation = 1.f - fminf(R.fire[0], fminf(R.fire[1], R.fire[2])) / fmaxf(t.peak, 1e-6f);
+  return t;
+}
+FP_DEV float3 emissionOf(const FpRender& R, const Tint& tint, const float4& f) {
   if (R.optical[1] <= 0.f) return make_float3(0.f, 0.f, 0.f);
   float s = fmaxf(0.f, f.x) * R.optical[0], flame = glowOf(f.z) * R.flameOpacity;
   float3 source = make_float3((1.f - R.smoke[0]) * s * R.smoke[3] + flame, (1.f - R.smoke[1]) * s * R.smoke[3] + flame,
@@ -407,8 +457,7 @@ FP_DEV float3 emissionOf(const FpRender& R, const float4& f) {
   float4 spec = make_float4(mixf(a.x, b.x, fr), mixf(a.y, b.y, fr), mixf(a.z, b.z, fr), mixf(a.w, b.w, fr));
   float scale = exp2f(fminf(fmaxf(spec.w, -24.f), 10.f));
   float3 thermal = make_float3(spec.x * scale, spec.y * scale, spec.z * scale);
-  float tintPeak = fmaxf(R.fire[0], fmaxf(R.fire[1], R.fire[2]));
-  float saturation = 1.f - fminf(R.fire[0], fminf(R.fire[1], R.fire[2])) / fmaxf(tintPeak, 1e-6f);
+  const float tintPeak = tint.peak, saturation = tint.saturation;
   float peak = fmaxf(thermal.x, fmaxf(thermal.y, thermal.z));
   float k = R.optical[1];
   return make_float3(mixf(thermal.x * tintPeak, R.fire[0] * peak, saturation) * source.x * k,
@@ -453,6 +502,7 @@ FP_DEV float integratedTransmission(float extinction, float distance, float atte
 
 // incidentLight (lighting.wgsl:257-310): glow RGB and the sun's transmittance at p.
 FP_DEV float4 incidentLight(const SimParams& P, const FpRender& R, BoxCursor& c, float px, float py, float pz) {
+  const Tint tint = tintOf(R);
   float4 local = sampleWorld(P, R, c, px, py, pz);
   if (local.x + glowOf(local.z) < 1e-5f) return make_float4(0.f, 0.f, 0.f, 1.f);
   float ln = sqrtf(R.light[0] * R.light[0] + R.light[1] * R.light[1] + R.light[2] * R.light[2]);
@@ -479,7 +529,7 @@ FP_DEV float4 incidentLight(const SimParams& P, const FpRender& R, BoxCursor& c,
         float4 f = sampleWorld(P, R, c, px + dirs[d][0] * q, py + dirs[d][1] * q, pz + dirs[d][2] * q);
         float ext = extinctionOf(R, f);
         float att = expf(-ext * interval);
-        float3 e = emissionOf(R, f);
+        float3 e = emissionOf(R, tint, f);
         float w = transmission * integratedTransmission(ext, interval, att) / 6.f;
         glow.x += e.x * w;
         glow.y += e.y * w;
@@ -500,6 +550,7 @@ FP_DEV float4 incidentLight(const SimParams& P, const FpRender& R, BoxCursor& c,
 FP_DEV float4 incidentLightWarp(const SimParams& P, const FpRender& R, BoxCursor& c, float px, float py, float pz) {
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
+  const Tint tint = tintOf(R);
   float4 local = sampleWorld(P, R, c, px, py, pz);
   if (local.x + glowOf(local.z) < 1e-5f) return make_float4(0.f, 0.f, 0.f, 1.f);
   float ln = sqrtf(R.light[0] * R.light[0] + R.light[1] * R.light[1] + R.light[2] * R.light[2]);
@@ -542,7 +593,7 @@ FP_DEV float4 incidentLightWarp(const SimParams& P, const FpRender& R, BoxCursor
         float4 f = sampleWorld(P, R, c, px + dirs[lane][0] * q, py + dirs[lane][1] * q, pz + dirs[lane][2] * q);
         float ext = extinctionOf(R, f);
         float att = expf(-ext * interval);
-        float3 e = emissionOf(R, f);
+        float3 e = emissionOf(R, tint, f);
         ew[k] = transmission * integratedTransmission(ext, interval, att) / 6.f;
         ex[k] = e.x;
         ey[k] = e.y;
@@ -591,6 +642,7 @@ FP_DEV bool boxBrick(const SimParams& P, const FpRender& R, BoxCursor& c, uint32
 // brick a ray or a light sample enters.
 __global__ void __launch_bounds__(256) k_render_pages(const SimParams* __restrict__ Pp, const __grid_constant__ FpRender R) {
   const SimParams& P = *Pp;
+  if (R.apronCap && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *R.apronCount = 0;
   for (int k = blockIdx.y; k < R.boxCount; k += gridDim.y) {
     const int* b = R.boxes + FP_BOX_INTS * k;
     const int nx = b[3] - b[0] + 1, ny = b[4] - b[1] + 1, nz = b[5] - b[2] + 1, total = nx * ny * nz;
@@ -598,16 +650,59 @@ __global__ void __launch_bounds__(256) k_render_pages(const SimParams* __restric
       R.pages[b[6] + i] = hashedSlot(P, b[0] + i % nx, b[1] + i / nx % ny, b[2] + i / (nx * ny));
   }
 }
+// The apron bricks of the boxes, numbered in the order they are met (what one holds depends on its
+// place alone, not on its number). The tables are written while they are read: only from -1 to
+// less, and a neighbour's sign is all that is read.
+__global__ void __launch_bounds__(256) k_render_aprons(const __grid_constant__ FpRender R) {
+  const volatile int* pages = R.pages;
+  for (int k = blockIdx.y; k < R.boxCount; k += gridDim.y) {
+    const int* b = R.boxes + FP_BOX_INTS * k;
+    const int nx = b[3] - b[0] + 1, ny = b[4] - b[1] + 1, nz = b[5] - b[2] + 1, total = nx * ny * nz;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+      if (pages[b[6] + i] != -1) continue;
+      const int x = i % nx, y = i / nx % ny, z = i / (nx * ny);
+      bool after = false;
+#pragma unroll
+      for (int q = 1; q < 8; q++) {
+        const int dx = q & 1, dy = (q >> 1) & 1, dz = q >> 2;
+        if (x >= dx && y >= dy && z >= dz && pages[b[6] + i - dx - dy * nx - dz * nx * ny] >= 0) after = true;
+      }
+      if (!after) continue;
+      const int g = atomicAdd(R.apronCount, 1);
+      if (g >= R.apronCap) continue;
+      R.apronBricks[g] = make_int4(b[0] + x, b[1] + y, b[2] + z, k);
+      R.pages[b[6] + i] = -2 - g;
+    }
+  }
+}
+FP_DEV uint32_t apronTotal(const FpRender& R) { return R.apronCap ? (uint32_t)min(*R.apronCount, R.apronCap) : 0u; }
 
 // smoothSmoke: each boxed brick's render field, the smoothed density with heat, lifetime and
 // fuel as they are.
 __global__ void __launch_bounds__(RTHREADS) k_render_field(const SimParams* __restrict__ Pp, const __grid_constant__ FpRender R) {
   const SimParams& P = *Pp;
-  uint32_t total = P.counters->active;
+  const uint32_t total = P.counters->active, aprons = apronTotal(R);
   const bool half = P.scalarHalf != 0;
-  for (uint32_t i = blockIdx.x; i < total; i += gridDim.x) {
+  for (uint32_t i = blockIdx.x; i < total + aprons; i += gridDim.x) {
     BoxCursor c = noBox();
     int bx, by, bz, slot;
+    if (i >= total) {
+      const uint32_t g = i - total;
+      const int4 q = R.apronBricks[g];
+      useBox(R, c, q.w);
+      const unsigned before = slottedBefore(P, R, c, q.x, q.y, q.z);
+      const int side = P.smokeDiv > 1 ? 1 << P.smokeShift : P.B, planes = 3 * side * side;
+      for (int k = threadIdx.x; k < planes; k += blockDim.x) {
+        int lx, ly, lz;
+        if (!apronCell(side, k, before, lx, ly, lz)) continue;
+        const int x = q.x * side + lx, y = q.y * side + ly, z = q.z * side + lz;
+        if (P.smokeDiv > 1)
+          R.apronSmoke[(size_t)g * planes + k] = smoothedCoarse(P, R, c, x, y, z);
+        else
+          R.apronField[(size_t)g * planes + k] = smoothedSmoke(P, R, c, x, y, z);
+      }
+      continue;
+    }
     if (!boxBrick(P, R, c, i, bx, by, bz, slot)) continue;
     for (int k = threadIdx.x; k < P.N; k += blockDim.x) {
       int x = bx * P.B + (k & (P.B - 1)), y = by * P.B + ((k >> P.shift) & (P.B - 1)), z = bz * P.B + (k >> (2 * P.shift));
@@ -632,13 +727,27 @@ __global__ void __launch_bounds__(RTHREADS) k_render_light(const SimParams* __re
   __shared__ int flags;
   __shared__ int glowBits, smokeBits;  // the coarse bound's maxima (nonnegative floats' bits)
   if (threadIdx.x == 0) glowBits = smokeBits = 0;
-  uint32_t total = P.counters->active;
+  const uint32_t total = P.counters->active, aprons = apronTotal(R);
   const int L = 1 << R.lightShift, L3 = L * L * L;
   const float texel = P.h * (float)(P.B >> R.lightShift);
   const int per = P.B / 8, blocks = per * per * per;
-  for (uint32_t i = blockIdx.x; i < total; i += gridDim.x) {
+  for (uint32_t i = blockIdx.x; i < total + aprons; i += gridDim.x) {
     BoxCursor c = noBox();
     int bx, by, bz, slot;
+    if (i >= total) {
+      const int4 q = R.apronBricks[i - total];
+      useBox(R, c, q.w);
+      const unsigned before = slottedBefore(P, R, c, q.x, q.y, q.z);
+      const int planes = 3 * L * L;
+      for (int k = threadIdx.x >> 5; k < planes; k += blockDim.x >> 5) {
+        int lx, ly, lz;
+        if (!apronCell(L, k, before, lx, ly, lz)) continue;
+        float4 light = incidentLightWarp(P, R, c, ((float)(q.x * L + lx) + .5f) * texel,
+                                         ((float)(q.y * L + ly) + .5f) * texel, ((float)(q.z * L + lz) + .5f) * texel);
+        if ((threadIdx.x & 31) == 0) R.apronLight[(size_t)(i - total) * planes + k] = light;
+      }
+      continue;
+    }
     if (!boxBrick(P, R, c, i, bx, by, bz, slot)) continue;  // the same for the whole CTA
     // Each 8-cell block with a halo of two cells, in units of 2x2x2 cells: a unit in a
     // slotted brick looks at its corner cells of the render field.
@@ -724,6 +833,9 @@ static __device__ __noinline__ float4 lightSampleFar(const SimParams& P, const F
     if (s >= 0) {
       const int m = L - 1;
       t = __ldg(&R.lighting[(size_t)s * L3 + (((z & m) * L + (y & m)) * L + (x & m))]);
+    } else if (s <= -2) {
+      const int m = L - 1;
+      t = __ldg(&R.apronLight[(size_t)(-2 - s) * 3 * L * L + apronIndex(L, x & m, y & m, z & m)]);
     } else {  // the apron of a neighbour without a slot: lit where it stands
       t = incidentLight(P, R, c, ((float)x + .5f) * texel, ((float)y + .5f) * texel, ((float)z + .5f) * texel);
     }
@@ -733,7 +845,7 @@ static __device__ __noinline__ float4 lightSampleFar(const SimParams& P, const F
 }
 // fireProLight (volume-bricks.wgsl:158-178) at `q` in lighting texels.
 FP_DEV float4 lightSample(const SimParams& P, const FpRender& R, BoxCursor& c, float qx, float qy, float qz) {
-  const int L = 1 << R.lightShift, L3 = L * L * L;
+  const int L = 1 << R.lightShift;
   qx = fminf(fmaxf(qx, (float)c.lo[0] * L + .5f), (float)(c.hi[0] + 1) * L - .5f);
   qy = fminf(fmaxf(qy, (float)c.lo[1] * L + .5f), (float)(c.hi[1] + 1) * L - .5f);
   qz = fminf(fmaxf(qz, (float)c.lo[2] * L + .5f), (float)(c.hi[2] + 1) * L - .5f);
@@ -743,12 +855,14 @@ FP_DEV float4 lightSample(const SimParams& P, const FpRender& R, BoxCursor& c, f
   float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
   int slots[8];
   if (slots8(R, c, R.lightShift, x0, y0, z0, 1, slots)) {
-    const int m = L - 1;
+    const unsigned sh = R.lightShift, m = (1u << sh) - 1u;
+    const unsigned lx[2] = {x0 & m, (x0 + 1) & m}, ly[2] = {(y0 & m) << sh, ((y0 + 1) & m) << sh},
+                   lz[2] = {(z0 & m) << (2 * sh), ((z0 + 1) & m) << (2 * sh)};
 #pragma unroll
     for (int k = 0; k < 8; k++) {
       int dx = k & 1, dy = (k >> 1) & 1, dz = k >> 2;
       float w = (dx ? fx : 1.f - fx) * (dy ? fy : 1.f - fy) * (dz ? fz : 1.f - fz);
-      add4(v, __ldg(&R.lighting[(size_t)slots[k] * L3 + ((((z0 + dz) & m) * L + ((y0 + dy) & m)) * L + ((x0 + dx) & m))]), w);
+      add4(v, __ldg(&R.lighting[((unsigned)slots[k] << (3 * sh)) + (lx[dx] + ly[dy] + lz[dz])]), w);
     }
     return v;
   }
@@ -772,17 +886,19 @@ FP_DEV float jitterOf(uint32_t px, uint32_t py, float time) {
 // A pixel's march (fireProSceneVolume with fireProMarch), a thread a pixel.
 // A camera ray through the boxes (fireProRay, fireProSpan) and what its march keeps fixed.
 struct Ray {
-  float ro[3], rd[3], safe[3], exitSide[3];
+  float ro[3], rd[3];
   float lo, hi;  // the first box entry and the last exit
-  float stepSize, jitter, direct[3];
+  float stepSize, jitter, direct;  // direct: the sun's factor (fireProDirect over sceneLight)
+  float perSafe[3], perStep;       // 1 / safeAxis(rd), 1 / stepSize
 };
+FP_DEV float safeAxis(float d) { return fabsf(d) > 1e-6f ? d : 1e-6f; }
 // fireProHit: where the ray enters and leaves box k (entry after exit when it misses).
 FP_DEV float2 boxHit(const FpRender& R, const Ray& r, int k, float brickSize) {
   const int* b = R.boxes + FP_BOX_INTS * k;
   float lo = 0.f, hi = 1e30f;
   for (int a = 0; a < 3; a++) {
-    float ta = ((float)b[a] * brickSize - r.ro[a]) / r.safe[a];
-    float tb = ((float)(b[3 + a] + 1) * brickSize - r.ro[a]) / r.safe[a];
+    float ta = ((float)b[a] * brickSize - r.ro[a]) / safeAxis(r.rd[a]);
+    float tb = ((float)(b[3 + a] + 1) * brickSize - r.ro[a]) / safeAxis(r.rd[a]);
     lo = fmaxf(lo, fminf(ta, tb));
     hi = fminf(hi, fmaxf(ta, tb));
   }
@@ -805,10 +921,7 @@ FP_DEV bool rayOf(const SimParams& P, const FpRender& R, float ux, float uy, Ray
   float rl = sqrtf(r.rd[0] * r.rd[0] + r.rd[1] * r.rd[1] + r.rd[2] * r.rd[2]);
   for (int a = 0; a < 3; a++) r.rd[a] /= rl;
   const float brickSize = P.h * (float)P.B;
-  for (int a = 0; a < 3; a++) {
-    r.safe[a] = fabsf(r.rd[a]) > 1e-6f ? r.rd[a] : 1e-6f;
-    r.exitSide[a] = r.rd[a] > 0.f ? 1.f : 0.f;
-  }
+  for (int a = 0; a < 3; a++) r.perSafe[a] = 1.f / safeAxis(r.rd[a]);
   // fireProSpan: the first entry, the last exit and the length inside every box.
   r.lo = 1e30f;
   r.hi = 0.f;
@@ -823,13 +936,13 @@ FP_DEV bool rayOf(const SimParams& P, const FpRender& R, float ux, float uy, Ray
   }
   if (!(r.hi > r.lo)) return false;
   r.stepSize = fmaxf(P.h * .5f, length / (float)R.raySteps);
+  r.perStep = 1.f / r.stepSize;
   // fireProDirect
   float ln = sqrtf(R.light[0] * R.light[0] + R.light[1] * R.light[1] + R.light[2] * R.light[2]);
   float g = R.optical[3];
   float mu = (r.rd[0] * R.light[0] + r.rd[1] * R.light[1] + r.rd[2] * R.light[2]) / ln;
   float phase = (1.f - g * g) / powf(fmaxf(.05f, 1.f + g * g - 2.f * g * mu), 1.5f);
-  float dk = R.light[3] * (.35f + phase * .3f);
-  for (int a = 0; a < 3; a++) r.direct[a] = R.sceneLight[a] * dk;
+  r.direct = R.light[3] * (.35f + phase * .3f);
   return true;
 }
 
@@ -864,41 +977,53 @@ struct Sample {
   int filter;      // the reconstruction filter of its block
 };
 FP_DEV Sample sampleAt(const SimParams& P, const FpRender& R, BoxCursor& c, const Ray& r, float t, float ds, float exit) {
-  const float brickSize = P.h * (float)P.B;
   Sample s;
   float tt = t + r.jitter * ds;
   float p[3] = {r.ro[0] + r.rd[0] * tt, r.ro[1] + r.rd[1] * tt, r.ro[2] + r.rd[2] * tt};
   int ci[3];
 #pragma unroll
   for (int a = 0; a < 3; a++) {
-    s.cell[a] = p[a] / P.h;
+    s.cell[a] = p[a] / P.h;  // divided: which block a sample on its face falls in is a decision
     ci[a] = (int)floorf(s.cell[a]);
   }
   int slot = slotAt(P, R, c, ci[0] >> P.shift, ci[1] >> P.shift, ci[2] >> P.shift);
-  float size = brickSize;
+  int shift = P.shift;  // log2 cells of what is empty together: the brick, or the 8-cell block
   int flags = 0;
   if (slot >= 0) {  // fireProOccupancy: the sample's 8-cell block of the brick
-    const int per = P.B / 8, m = P.B - 1;
-    int block = ((((ci[2] & m) >> 3) * per) + ((ci[1] & m) >> 3)) * per + ((ci[0] & m) >> 3);
-    flags = R.occupancy[(size_t)slot * per * per * per + block];
-    size = P.h * 8.f;
+    const int per = P.shift - 3, m = (1 << per) - 1;
+    const int block = (((((ci[2] >> 3) & m) << per) | ((ci[1] >> 3) & m)) << per) | ((ci[0] >> 3) & m);
+    flags = __ldg(&R.occupancy[((size_t)slot << (3 * per)) + block]);
+    shift = 3;
   }
   s.lit = (flags & 2) != 0;
   s.filter = (flags & 1) ? R.filter : 0;
   s.next = t;
   if (!s.lit) {
-    // Skip whole steps past the empty block, keeping the lattice.
-    float dist = 1e30f;
+    // Skip whole steps past the empty block, keeping the lattice. The count of steps is a decision
+    // too: from reciprocals, unless it is near a whole number.
+    float away[3], dist = 1e30f;
 #pragma unroll
-    for (int a = 0; a < 3; a++) dist = fminf(dist, ((floorf(p[a] / size) + r.exitSide[a]) * size - p[a]) / r.safe[a]);
-    s.next = fminf(t + fmaxf(1.f, floorf(dist / r.stepSize) + 1.f) * r.stepSize, exit);
+    for (int a = 0; a < 3; a++) {
+      const int edge = ((ci[a] >> shift) + (r.rd[a] > 0.f ? 1 : 0)) << shift;
+      away[a] = (float)edge * P.h - p[a];
+      dist = fminf(dist, away[a] * r.perSafe[a]);
+    }
+    float steps = dist * r.perStep;
+    if (!(fabsf(steps - rintf(steps)) > 1e-3f)) {
+      dist = 1e30f;
+#pragma unroll
+      for (int a = 0; a < 3; a++) dist = fminf(dist, away[a] / safeAxis(r.rd[a]));
+      steps = dist / r.stepSize;
+    }
+    s.next = fminf(t + fmaxf(1.f, floorf(steps) + 1.f) * r.stepSize, exit);
   }
   return s;
 }
 // The radiance a sample ds long adds per unit of the transmittance before it, and the factor it
 // leaves of that transmittance.
-FP_DEV float4 shade(const SimParams& P, const FpRender& R, BoxCursor& c, const Ray& r, const Sample& s, float ds) {
-  const float lightRatio = (float)(P.B >> R.lightShift);
+FP_DEV float4 shade(const SimParams& P, const FpRender& R, BoxCursor& c, const Ray& r, const Tint& tint, const Sample& s,
+                    float ds) {
+  const float texels = 1.f / (float)(P.B >> R.lightShift);  // lighting texels a cell: a power of two, exact
   float4 f = reconstruct(P, R, c, s.cell[0], s.cell[1], s.cell[2], s.filter);
   if (P.smokeDiv > 1) {  // fireProRenderField: the smoothed coarse density, trilinear
     const float q = 1.f / (float)P.smokeDiv;
@@ -906,14 +1031,14 @@ FP_DEV float4 shade(const SimParams& P, const FpRender& R, BoxCursor& c, const R
   }
   if (!(f.x + glowOf(f.z) > .002f)) return make_float4(0.f, 0.f, 0.f, 1.f);
   // fireProShade
-  float3 glow = emissionOf(R, f);
+  float3 glow = emissionOf(R, tint, f);
   float density = fmaxf(0.f, f.x) * R.optical[0];
   float sc[3] = {0.f, 0.f, 0.f};
   if (density > 0.f) {
-    float4 inc = lightSample(P, R, c, s.cell[0] / lightRatio, s.cell[1] / lightRatio, s.cell[2] / lightRatio);
-    sc[0] = R.smoke[0] * (R.ambient[0] + r.direct[0] * inc.w + inc.x * .65f) * density;
-    sc[1] = R.smoke[1] * (R.ambient[1] + r.direct[1] * inc.w + inc.y * .65f) * density;
-    sc[2] = R.smoke[2] * (R.ambient[2] + r.direct[2] * inc.w + inc.z * .65f) * density;
+    float4 inc = lightSample(P, R, c, s.cell[0] * texels, s.cell[1] * texels, s.cell[2] * texels);
+    sc[0] = R.smoke[0] * (R.ambient[0] + R.sceneLight[0] * r.direct * inc.w + inc.x * .65f) * density;
+    sc[1] = R.smoke[1] * (R.ambient[1] + R.sceneLight[1] * r.direct * inc.w + inc.y * .65f) * density;
+    sc[2] = R.smoke[2] * (R.ambient[2] + R.sceneLight[2] * r.direct * inc.w + inc.z * .65f) * density;
   }
   float ext = extinctionOf(R, f);
   float tau = ext * ds;
@@ -924,49 +1049,65 @@ FP_DEV float4 shade(const SimParams& P, const FpRender& R, BoxCursor& c, const R
 }
 
 // A ray is marched by a group of G lanes of a warp, a lane a step: the next G steps of the ray's
-// lattice are looked up together, those before the first empty block (or the end) are shaded
+// lattice are looked up together, those before the first empty block (or the limit) are shaded
 // together, and their colours and transmittances are composed over the lanes. A serial march is a
 // chain of dependent lookups and loads a few hundred instructions long a step, and an image of a
 // few tens of thousands of rays leaves the chip idle waiting for it; along the ray the lanes also
 // read neighbouring cells and mostly agree on the filter. All lanes of a group hold the same ray
-// state. Steps past the first empty one, and those past the point where the ray turns opaque, are
-// dropped, so the samples that count are the serial march's, at the same positions.
-// Every lane of the warp calls this together, those without work with `alive` false.
+// state. The samples that count are the serial march's, at the very same positions; those past the
+// point where the ray turns opaque are dropped.
+// Every lane of the warp calls the two halves together, those without work with `on` false.
 constexpr float OPAQUE = .008f;
 struct March {
   float t, exit, trans, rad[3];
 };
 template <int G>
-FP_DEV void marchGroup(const SimParams& P, const FpRender& R, BoxCursor& c, const Ray& r, float limit, bool alive, March& m) {
+struct Steps {
+  float t, ds;   // this lane's step
+  float next;    // where the ray goes on after the group's steps
+  bool lit, any; // this lane's block may hold something; some lane's of the group
+  Sample s;
+};
+// The group's next steps before `limit`, looked up.
+template <int G>
+FP_DEV Steps<G> lookAhead(const SimParams& P, const FpRender& R, BoxCursor& c, const Ray& r, float limit, bool on,
+                          const March& m) {
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & (G - 1);
-  float t = m.t;
+  Steps<G> a;
+  a.t = m.t;
 #pragma unroll
   for (int j = 0; j < G - 1; j++)  // the serial march's own sums
-    if (j < lane) t += r.stepSize;
-  const float ds = fminf(r.stepSize, limit - t);
-  const bool live = alive && t < limit;
-  Sample s;
-  s.lit = false;
-  s.next = t;
-  if (live) s = sampleAt(P, R, c, r, t, ds, m.exit);
-  int n = G;  // the lanes before the first empty or absent step
-  float next;
+    if (j < lane) a.t += r.stepSize;
+  a.ds = fminf(r.stepSize, limit - a.t);
+  const bool live = on && a.t < limit;
+  a.s.lit = false;
+  a.s.next = a.t;
+  if (live) a.s = sampleAt(P, R, c, r, a.t, a.ds, m.exit);
+  a.lit = live && a.s.lit;
+  // Where the ray goes on: past the last step to shade, or past the empty block of the step after it.
+  a.next = a.lit ? a.t + a.ds : a.s.next;
+  a.any = a.lit;
   if constexpr (G > 1) {
-    const unsigned group = (__ballot_sync(full, !(live && s.lit)) >> ((threadIdx.x & 31) & ~(G - 1))) & ((1u << G) - 1u);
-    n = group ? __ffs(group) - 1 : G;
-  } else {
-    n = s.lit ? 1 : 0;
+    const int shift = (threadIdx.x & 31) & ~(G - 1);
+    const unsigned lanes = (__ballot_sync(full, live) >> shift) & ((1u << G) - 1u);
+    const unsigned dark = (~__ballot_sync(full, a.lit) >> shift) & ((1u << G) - 1u);
+    const int n = dark ? __ffs((int)dark) - 1 : G;  // the steps to shade
+    a.lit = a.lit && lane < n;
+    a.any = n > 0;
+    a.next = __shfl_sync(full, a.next, (n < G && ((lanes >> n) & 1u)) ? n : max(0, n - 1), G);
   }
+  return a;
+}
+// The group's lit steps shaded and composed into the ray.
+template <int G>
+FP_DEV void shadeSteps(const SimParams& P, const FpRender& R, BoxCursor& c, const Ray& r, const Tint& tint, bool on,
+                       const Steps<G>& a, March& m) {
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & (G - 1);
   float4 q = make_float4(0.f, 0.f, 0.f, 1.f);
-  if (live && lane < n) q = shade(P, R, c, r, s, ds);
-  // Where the ray goes on: past the last shaded step, or past the empty block after it.
-  next = (live && s.lit) ? t + ds : s.next;
+  if (on && a.lit) q = shade(P, R, c, r, tint, a.s, a.ds);
   if constexpr (G > 1) {
-    const bool absent = !__shfl_sync(full, live ? 1 : 0, n < G ? n : G - 1, G);  // the step after the last is past the limit
-    const float empty = __shfl_sync(full, next, n < G ? n : G - 1, G);
-    const float lastEnd = __shfl_sync(full, next, n > 0 ? n - 1 : 0, G);
-    next = (n < G && !absent) ? empty : lastEnd;
     // The transmittance before each lane's step: an exclusive product over the group.
     float incl = q.w;
 #pragma unroll
@@ -986,37 +1127,87 @@ FP_DEV void marchGroup(const SimParams& P, const FpRender& R, BoxCursor& c, cons
       z += __shfl_xor_sync(full, z, o, G);
       left = fminf(left, __shfl_xor_sync(full, left, o, G));
     }
-    if (alive) {
+    if (on) {
       m.rad[0] += x;
       m.rad[1] += y;
       m.rad[2] += z;
       m.trans = left;
-      m.t = next;
     }
-  } else if (alive) {
+  } else if (on) {
     m.rad[0] += m.trans * q.x;
     m.rad[1] += m.trans * q.y;
     m.rad[2] += m.trans * q.z;
     m.trans *= q.w;
-    m.t = next;
+  }
+}
+// The march of the warp's rays, each from m.t to `end`: `limitOf()` gives the depth at which a
+// ray's lattice starts over before the exit, `arrived()` is called whenever a ray has moved on.
+// The rays of a warp cross their empty stretches together, by lookups alone, before any shades: a
+// ray in empty space then does not wait, step by step, for the others' shading.
+// What bounds it is instruction issue (cells come from L1): about 98 % L1 hits, DRAM idle. Slice
+// pass, us: 14,400 rays of a small plume 2103 -> 85; 129,600 rays of a 1.8k-brick jet 8954 -> 845;
+// 518,400 rays of 3.7k bricks 20,889 -> 3025; full resolution, 231,401 rays, quadratic 12,807 -> 800.
+template <int G, class Limit, class Arrived>
+FP_DEV void marchRays(const SimParams& P, const FpRender& R, const Ray& r, bool alive, float end, March& m, Limit limitOf,
+                      Arrived arrived) {
+  const unsigned full = 0xffffffffu;
+  const Tint tint = tintOf(R);
+  BoxCursor c = noBox();
+  while (true) {
+    Steps<G> a;
+    bool ready = false;  // this group's steps hold a lit one
+    a.next = 0.f;
+    while (true) {
+      alive = alive && m.t < end && m.trans >= OPAQUE;
+      bool on = alive && !ready;
+      if (on && m.t >= m.exit) {
+        alive = enterBox(P, R, r, m.t, m.exit, c);
+        on = alive && m.t < m.exit;
+        if (alive) arrived();
+      }
+      if (!__any_sync(full, on)) {
+        if (!__any_sync(full, alive && !ready)) break;
+        continue;
+      }
+      Steps<G> b = lookAhead<G>(P, R, c, r, fminf(limitOf(), m.exit), on, m);
+      if (on) {
+        a = b;
+        ready = b.any;
+        if (!ready) {
+          m.t = b.next;
+          arrived();
+        }
+      }
+    }
+    if (!__any_sync(full, ready)) break;
+    shadeSteps<G>(P, R, c, r, tint, ready, a, m);
+    if (ready) {
+      m.t = a.next;
+      arrived();
+    }
   }
 }
 
-// The pixel of a thread's group: a CTA covers a tile of pixels, so that the rays of a warp and of
-// a CTA read neighbouring bricks.
+// The pixel of a thread's group. A warp's rays and a CTA's four warps cover square tiles of the
+// image, so that they read neighbouring bricks.
+template <int G>
+struct RayTile {
+  static constexpr int RAYS = 32 / G;  // a warp's
+  static constexpr int WX = RAYS >= 32 ? 8 : (RAYS >= 8 ? 4 : (RAYS >= 2 ? 2 : 1)), WY = RAYS / WX;
+  static constexpr int TX = 2 * WX, TY = 2 * WY;
+  static_assert(RTHREADS == 128, "four warps a CTA");
+};
 template <int G>
 FP_DEV void groupPixel(int& px, int& py) {
-  constexpr int RAYS = RTHREADS / G, TX = RAYS >= 64 ? 16 : (RAYS >= 16 ? 4 : 2), WX = 32 / G >= 8 ? 8 : (32 / G >= 2 ? 2 : 1);
-  constexpr int WY = (32 / G) / WX;  // a warp's rays: WX x WY
+  using T = RayTile<G>;
   const int warp = threadIdx.x >> 5, g = (threadIdx.x & 31) / G;
-  constexpr int PER = TX / WX;  // warps a row of the CTA's tile
-  px = blockIdx.x * TX + (warp % PER) * WX + g % WX;
-  py = blockIdx.y * (RAYS / TX) + (warp / PER) * WY + g / WX;
+  px = blockIdx.x * T::TX + (warp & 1) * T::WX + g % T::WX;
+  py = blockIdx.y * T::TY + (warp >> 1) * T::WY + g / T::WX;
 }
 template <int G>
 static dim3 groupGrid(int w, int h) {
-  constexpr int RAYS = RTHREADS / G, TX = RAYS >= 64 ? 16 : (RAYS >= 16 ? 4 : 2), TY = RAYS / TX;
-  return dim3((unsigned)((w + TX - 1) / TX), (unsigned)((h + TY - 1) / TY));
+  using T = RayTile<G>;
+  return dim3((unsigned)((w + T::TX - 1) / T::TX), (unsigned)((h + T::TY - 1) / T::TY));
 }
 
 // buildSlices (volume-slices.wgsl:28-122): a ray per half-resolution pixel marches from the
@@ -1025,7 +1216,7 @@ static dim3 groupGrid(int w, int h) {
 // moment, those past the exit or an opaque ray the final ones. Without a scene depth every pixel
 // resumes from the last slice, so only that one is stored.
 template <int G>
-__global__ void __launch_bounds__(RTHREADS) k_slices(const SimParams* __restrict__ Pp, const __grid_constant__ FpRender R) {
+__global__ void __launch_bounds__(RTHREADS, MARCH_CTAS) k_slices(const SimParams* __restrict__ Pp, const __grid_constant__ FpRender R) {
   const SimParams& P = *Pp;
   int px, py;
   groupPixel<G>(px, py);
@@ -1050,21 +1241,13 @@ __global__ void __launch_bounds__(RTHREADS) k_slices(const SimParams* __restrict
     m.t = m.exit = r.lo;
     depth = r.lo + spacing;
   }
-  BoxCursor c = noBox();
-  while (true) {
-    alive = alive && recorded < FP_SLICES && m.t < r.hi && m.trans >= OPAQUE;
-    bool steps = alive;
-    if (alive && m.t >= m.exit) {
-      steps = false;
-      alive = enterBox(P, R, r, m.t, m.exit, c);
-    }
-    if (!__any_sync(0xffffffffu, alive)) break;
-    if (__any_sync(0xffffffffu, steps)) marchGroup<G>(P, R, c, r, fminf(depth, m.exit), steps, m);
-    while (alive && recorded < FP_SLICES && m.t >= depth) {
-      record();
-      depth = r.lo + spacing * (float)(recorded + 1);
-    }
-  }
+  marchRays<G>(P, R, r, alive, r.hi, m, [&]() { return depth; },
+               [&]() {
+                 while (recorded < FP_SLICES && m.t >= depth) {
+                   record();
+                   depth = r.lo + spacing * (float)(recorded + 1);
+                 }
+               });
   while (recorded < FP_SLICES) record();
 }
 
@@ -1072,7 +1255,7 @@ __global__ void __launch_bounds__(RTHREADS) k_slices(const SimParams* __restrict
 // the scene's depth through the boxes, from the last half-resolution slice in front of it when
 // slices exist.
 template <int G>
-__global__ void __launch_bounds__(RTHREADS) k_march(const SimParams* __restrict__ Pp, const __grid_constant__ FpRender R) {
+__global__ void __launch_bounds__(RTHREADS, MARCH_CTAS) k_march(const SimParams* __restrict__ Pp, const __grid_constant__ FpRender R) {
   const SimParams& P = *Pp;
   int px, py;
   groupPixel<G>(px, py);
@@ -1129,18 +1312,8 @@ __global__ void __launch_bounds__(RTHREADS) k_march(const SimParams* __restrict_
   }
   // fireProMarch: the cursor starts exited, so the first pass enters the box at t.
   const bool drawn = alive;
-  BoxCursor c = noBox();
   m.exit = m.t;
-  while (true) {
-    alive = alive && m.t < end && m.trans >= OPAQUE;
-    bool steps = alive;
-    if (alive && m.t >= m.exit) {
-      steps = false;
-      alive = enterBox(P, R, r, m.t, m.exit, c);
-    }
-    if (!__any_sync(0xffffffffu, alive)) break;
-    if (__any_sync(0xffffffffu, steps)) marchGroup<G>(P, R, c, r, fminf(end, m.exit), steps, m);
-  }
+  marchRays<G>(P, R, r, alive, end, m, [&]() { return end; }, []() {});
   if (inside && (threadIdx.x & (G - 1)) == 0)
     reinterpret_cast<float4*>(R.image)[pix] =
         drawn ? make_float4(m.rad[0], m.rad[1], m.rad[2], 1.f - m.trans) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1161,6 +1334,7 @@ __global__ void __launch_bounds__(64) k_collect_lights(const SimParams* __restri
   const int lane = threadIdx.x, stride = P.B >> 2;
   const bool half = P.scalarHalf != 0;
   const float side = (float)P.B * P.h;
+  const Tint tint = tintOf(R);
   for (uint32_t i = blockIdx.x; i < total; i += gridDim.x) {
     const uint32_t id = P.active[i];
     if (!homeOk(P, id)) continue;  // the bounds-checked build only
@@ -1203,7 +1377,7 @@ __global__ void __launch_bounds__(64) k_collect_lights(const SimParams* __restri
       }
       f.x = v;
     }
-    const float3 rgb = emissionOf(R, f);
+    const float3 rgb = emissionOf(R, tint, f);
     const float luminance = rgb.x * .2126f + rgb.y * .7152f + rgb.z * .0722f;
     const float cx = ((float)b[0] + .5f) * side, cy = ((float)b[1] + .5f) * side, cz = ((float)b[2] + .5f) * side;
     float2 best = make_float2(1e38f, 0.f);
@@ -1253,19 +1427,38 @@ void fp_launch_collect_lights(const SimParams* dP, const FpRender& R, const floa
   k_collect_lights<<<sms * 16, 64, 0, st>>>(dP, R, anchors, count, sums);
 }
 
+// Lanes a ray (marchRays): enough that the rays' lanes fill the chip several times over (148 SMs x
+// 12 warps), no more, since a group's lanes share the ray's own work and its last steps leave lanes
+// idle. Slice pass, us by lanes 1 / 2 / 4 / 8 / 16: 14,400 rays 308 / 198 / 138 / 112 / 82; 129,600
+// rays 925 / 818 / 940 / 1159 / 1429; 518,400 rays 2913 / 2958 / 3501 / 4363 / 5844; full
+// resolution with 231,401 rays 1046 / 773 / 714 / 798 / 1141.
+template <int G>
+static void marchLaunch(const SimParams* dP, const FpRender& R, cudaStream_t st) {
+  if (R.slices) {
+    k_slices<G><<<groupGrid<G>(R.sliceW, R.sliceH), RTHREADS, 0, st>>>(dP, R);
+    // Every pixel resumes at its last slice: at most an eighth of its ray is left to march.
+    k_march<1><<<groupGrid<1>(R.width, R.height), RTHREADS, 0, st>>>(dP, R);
+  } else {
+    k_march<G><<<groupGrid<G>(R.width, R.height), RTHREADS, 0, st>>>(dP, R);
+  }
+}
 void fp_launch_render(const SimParams* dP, const FpRender& R, int sms, cudaStream_t st) {
   if (R.pages) {
     const int rows = R.boxCount < 64 ? R.boxCount : 64;
     const long long blocks = (R.pageCount / rows + 255) / 256;
     k_render_pages<<<dim3((unsigned)(blocks < 1 ? 1 : (blocks < sms * 8 ? blocks : sms * 8)), rows), 256, 0, st>>>(dP, R);
+    if (R.apronCap)
+      k_render_aprons<<<dim3((unsigned)(blocks < 1 ? 1 : (blocks < sms * 8 ? blocks : sms * 8)), rows), 256, 0, st>>>(R);
   }
   k_render_field<<<sms * 8, RTHREADS, 0, st>>>(dP, R);
   k_render_light<<<sms * 8, RTHREADS, 0, st>>>(dP, R);
-  if (R.slices) {
-    k_slices<8><<<groupGrid<8>(R.sliceW, R.sliceH), RTHREADS, 0, st>>>(dP, R);
-    // Every pixel resumes at its last slice: at most an eighth of its ray is left to march.
-    k_march<1><<<groupGrid<1>(R.width, R.height), RTHREADS, 0, st>>>(dP, R);
-  } else {
-    k_march<8><<<groupGrid<8>(R.width, R.height), RTHREADS, 0, st>>>(dP, R);
-  }
+  const long long rays = R.slices ? (long long)R.sliceW * R.sliceH : (long long)R.width * R.height;
+  if (rays >= 125000)
+    marchLaunch<2>(dP, R, st);
+  else if (rays >= 62500)
+    marchLaunch<4>(dP, R, st);
+  else if (rays >= 31250)
+    marchLaunch<8>(dP, R, st);
+  else
+    marchLaunch<16>(dP, R, st);
 }

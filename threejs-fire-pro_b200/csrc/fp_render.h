@@ -31,9 +31,21 @@ struct FpRender {
                         // (inclusive), the box's first entry in `pages`; boxes never overlap, each
                         // lies in one cluster of tiles
   int boxCount;
-  int* pages;           // per box, x fastest, each brick's slot or -1; null when the boxes hold more
-                        // than FP_MAX_PAGES bricks (lookups then go through the tile hash)
+  int* pages;           // per box, x fastest, each brick's slot, -1 without one, or -2 - g for
+                        // apron brick g; null when the boxes hold more than FP_MAX_PAGES bricks
+                        // (lookups then go through the tile hash)
   long long pageCount;
+  // Apron bricks: those without a slot that a brick with one precedes on some axes, so that a
+  // sample based in that one reads them. The cells and texels such a sample can reach (those on
+  // the brick's low faces) are computed once a render, per apron brick three planes (x = 0, then
+  // y = 0, then z = 0, the axes left in x, y, z order). Past apronCap they are computed where a
+  // sample needs them.
+  int apronCap;
+  int* apronCount;      // how many there are (it may exceed apronCap)
+  int4* apronBricks;    // x, y, z, box
+  float* apronField;    // the smoothed smoke of the field cells (no coarse smoke)
+  float* apronSmoke;    // coarse smoke: the smoothed density of the coarse cells
+  float4* apronLight;   // the incident light of the lighting texels
   float4* renderField;  // [slot][cell]: smoothed smoke, heat, lifetime, fuel (coarse smoke: the
                         // simulation's fields as they are)
   float* renderSmoke;   // coarse smoke (smokeDiv > 1): [slot][smoke cells], the smoothed density

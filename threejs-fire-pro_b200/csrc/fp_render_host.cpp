@@ -233,6 +233,15 @@ int Engine::renderInputs() {
   return FP_OK;
 }
 
+// Room of at least `need` bytes in a buffer that a render can do without: `want` bytes when it has
+// to be allocated. False without it, the device's error state cleared.
+bool Engine::spare(DeviceBuffer& b, size_t need, size_t want) {
+  if (b.ptr && b.bytes >= need) return true;
+  if (alloc(b, want, false)) return true;
+  cudaGetLastError();
+  return false;
+}
+
 // The optical model's settings (fire-emission.wgsl's uniforms).
 static void optics(FpRender& R, const fp_render_settings& rs) {
   std::memcpy(R.optical, rs.optical, sizeof(R.optical));
@@ -316,10 +325,21 @@ int Engine::render(const fp_camera& cam, const fp_render_settings& rs, float* im
     if ((rc = check(cudaMemcpyAsync(renderBoxesD_.ptr, rows.data(), bytes, cudaMemcpyHostToDevice, stream()), "render")))
       return rc;
     // Grown by half again, so that boxes that widen from frame to frame seldom allocate.
-    if (pages <= FP_MAX_PAGES) {
-      if (renderPages_.bytes < (size_t)pages * 4 && !alloc(renderPages_, (size_t)pages * 6, false)) return FP_ENOMEM;
+    if (pages <= FP_MAX_PAGES && spare(renderPages_, (size_t)pages * 4, (size_t)pages * 6)) {
       R.pages = (int*)renderPages_.ptr;
       R.pageCount = pages;
+      // Apron bricks: twice the slots is more than a connected volume's surface takes.
+      const int SB = smokeDiv_ > 1 ? 1 << sshift_ : 0;
+      const size_t plane = smokeDiv_ > 1 ? (size_t)SB * SB : (size_t)B_ * B_, perBrick = 3 * (plane * 4 + (size_t)L * L * 16);
+      const size_t room = 2 * (size_t)slots_, cap = std::min<size_t>(room, (size_t)pages);
+      if (spare(apronList_, 16 + cap * 16, 16 + room * 16) && spare(apronPools_, cap * perBrick, room * perBrick)) {
+        R.apronCap = (int)cap;
+        R.apronCount = (int*)apronList_.ptr;
+        R.apronBricks = (int4*)apronList_.ptr + 1;
+        R.apronLight = (float4*)apronPools_.ptr;
+        float* cells = (float*)apronPools_.ptr + cap * 3 * L * L * 4;
+        (smokeDiv_ > 1 ? R.apronSmoke : R.apronField) = cells;
+      }
     }
   }
   R.boxes = (const int*)renderBoxesD_.ptr;
