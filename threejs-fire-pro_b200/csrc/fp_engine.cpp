@@ -184,7 +184,7 @@ Engine::~Engine() {
   cudaStreamSynchronize(stream());
   freeAll();
   DeviceBuffer* render[] = {&renderField_, &renderSmoke_, &sceneDepth_, &slices_, &lighting_, &occupancy_, &lut_, &renderParams_, &image_, &anchors_, &lightSums_, &renderBoxesD_,
-                            &renderPages_, &apronList_, &apronPools_};
+                            &renderPages_, &apronList_, &apronPools_, &renderUnits_};
   for (DeviceBuffer* b : render)
     if (b->ptr) cudaFree(b->ptr);
   if (renderParamsH_) cudaFreeHost(renderParamsH_);

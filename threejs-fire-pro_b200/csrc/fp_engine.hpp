@@ -220,7 +220,7 @@ class Engine {
   void buildClusters();
   std::vector<int> sourceBoxes_;  // lo xyz, hi xyz per source
   DeviceBuffer renderField_, renderSmoke_, sceneDepth_, slices_, lighting_, occupancy_, lut_, renderParams_, image_, anchors_, lightSums_, renderBoxesD_,
-      renderPages_, apronList_, apronPools_;
+      renderPages_, apronList_, apronPools_, renderUnits_;
   SimParams* renderParamsH_ = nullptr;
   // The blackbody table and the render parameters of the latest state (device).
   bool spare(DeviceBuffer& b, size_t need, size_t want);

@@ -19,6 +19,8 @@
 namespace {
 
 constexpr int RTHREADS = 128;
+// Resident CTAs an SM the march is compiled for (168 registers): four (128, spills) and five lost
+// 7 % and 20 % on the slice pass, two 15 %.
 constexpr int MARCH_CTAS = 3;
 
 // A thread's current box: the bricks its samples read.
@@ -500,6 +502,13 @@ FP_DEV float integratedTransmission(float extinction, float distance, float atte
   return (1.f - attenuation) / extinction;
 }
 
+// The glow's six rays.
+FP_DEV float glowRay(int d, int axis) {
+  const float sign = (d & 1) ? -1.f : 1.f;
+  if (d < 2) return sign * (axis == 0 ? .36f : (axis == 1 ? .48f : -.8f));
+  if (d < 4) return sign * (axis == 0 ? -.8f : (axis == 1 ? .6f : 0.f));
+  return sign * (axis == 0 ? .48f : (axis == 1 ? .64f : .6f));
+}
 // incidentLight (lighting.wgsl:257-310): glow RGB and the sun's transmittance at p.
 FP_DEV float4 incidentLight(const SimParams& P, const FpRender& R, BoxCursor& c, float px, float py, float pz) {
   const Tint tint = tintOf(R);
@@ -518,15 +527,13 @@ FP_DEV float4 incidentLight(const SimParams& P, const FpRender& R, BoxCursor& c,
       if (depth > 9.f) break;
     }
   }
-  const float dirs[6][3] = {{.36f, .48f, -.8f}, {-.36f, -.48f, .8f}, {-.8f, .6f, 0.f},
-                            {.8f, -.6f, 0.f},   {.48f, .64f, .6f},   {-.48f, -.64f, -.6f}};
   float3 glow = make_float3(0.f, 0.f, 0.f);
   if (R.optical[1] > 0.f && local.x > 1e-5f) {
     for (int d = 0; d < 6; d++) {
       float t = 0.f, interval = .075f, transmission = 1.f;
       for (int s = 0; s < 6; s++) {
         float q = t + interval * .5f;
-        float4 f = sampleWorld(P, R, c, px + dirs[d][0] * q, py + dirs[d][1] * q, pz + dirs[d][2] * q);
+        float4 f = sampleWorld(P, R, c, px + glowRay(d, 0) * q, py + glowRay(d, 1) * q, pz + glowRay(d, 2) * q);
         float ext = extinctionOf(R, f);
         float att = expf(-ext * interval);
         float3 e = emissionOf(R, tint, f);
@@ -537,79 +544,6 @@ FP_DEV float4 incidentLight(const SimParams& P, const FpRender& R, BoxCursor& c,
         transmission *= att;
         t += interval;
         interval *= 1.65f;
-      }
-    }
-  }
-  return make_float4(glow.x, glow.y, glow.z, expf(-depth));
-}
-
-// incidentLight with a whole warp, every lane passing the same position (and its own copy of
-// the same cursor): the lanes take the shadow samples (32 at a time) and the six glow
-// directions, and every lane then adds their terms in the order of the serial loops, with the
-// serial early stop of the shadow sum, so all lanes return the serial result's value.
-FP_DEV float4 incidentLightWarp(const SimParams& P, const FpRender& R, BoxCursor& c, float px, float py, float pz) {
-  const unsigned full = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
-  const Tint tint = tintOf(R);
-  float4 local = sampleWorld(P, R, c, px, py, pz);
-  if (local.x + glowOf(local.z) < 1e-5f) return make_float4(0.f, 0.f, 0.f, 1.f);
-  float ln = sqrtf(R.light[0] * R.light[0] + R.light[1] * R.light[1] + R.light[2] * R.light[2]);
-  float sx = R.light[0] / ln, sy = R.light[1] / ln, sz = R.light[2] / ln;
-  int count = R.shadowSamples;
-  float ds = exitDistance(P, c, px, py, pz, sx, sy, sz) / (float)count;
-  float depth = 0.f;
-  if (R.light[3] > 0.f) {
-    bool stop = false;
-    for (int base = 0; base < count && !stop; base += 32) {
-      const int i = base + lane;
-      float v = 0.f;
-      if (i < count) {
-        float t = ((float)i + .5f) * ds;
-        float4 f = sampleWorld(P, R, c, px + sx * t, py + sy * t, pz + sz * t);
-        v = (fmaxf(0.f, f.x) * R.optical[2] + glowOf(f.z) * R.flameOpacity) * ds;
-      }
-      const int n = min(32, count - base);
-      for (int j = 0; j < n; j++) {
-        const float vj = __shfl_sync(full, v, j);
-        if (!stop) {
-          depth += vj;
-          stop = depth > 9.f;
-        }
-      }
-    }
-  }
-  float3 glow = make_float3(0.f, 0.f, 0.f);
-  if (R.optical[1] > 0.f && local.x > 1e-5f) {
-    const float dirs[6][3] = {{.36f, .48f, -.8f}, {-.36f, -.48f, .8f}, {-.8f, .6f, 0.f},
-                              {.8f, -.6f, 0.f},   {.48f, .64f, .6f},   {-.48f, -.64f, -.6f}};
-    float ex[6], ey[6], ez[6], ew[6];  // lane d < 6: direction d's six steps
-#pragma unroll
-    for (int k = 0; k < 6; k++) ex[k] = ey[k] = ez[k] = ew[k] = 0.f;
-    if (lane < 6) {
-      float t = 0.f, interval = .075f, transmission = 1.f;
-#pragma unroll
-      for (int k = 0; k < 6; k++) {
-        float q = t + interval * .5f;
-        float4 f = sampleWorld(P, R, c, px + dirs[lane][0] * q, py + dirs[lane][1] * q, pz + dirs[lane][2] * q);
-        float ext = extinctionOf(R, f);
-        float att = expf(-ext * interval);
-        float3 e = emissionOf(R, tint, f);
-        ew[k] = transmission * integratedTransmission(ext, interval, att) / 6.f;
-        ex[k] = e.x;
-        ey[k] = e.y;
-        ez[k] = e.z;
-        transmission *= att;
-        t += interval;
-        interval *= 1.65f;
-      }
-    }
-    for (int d = 0; d < 6; d++) {
-#pragma unroll
-      for (int k = 0; k < 6; k++) {
-        const float w = __shfl_sync(full, ew[k], d);
-        glow.x += __shfl_sync(full, ex[k], d) * w;
-        glow.y += __shfl_sync(full, ey[k], d) * w;
-        glow.z += __shfl_sync(full, ez[k], d) * w;
       }
     }
   }
@@ -677,142 +611,316 @@ __global__ void __launch_bounds__(256) k_render_aprons(const __grid_constant__ F
 }
 FP_DEV uint32_t apronTotal(const FpRender& R) { return R.apronCap ? (uint32_t)min(*R.apronCount, R.apronCap) : 0u; }
 
-// smoothSmoke: each boxed brick's render field, the smoothed density with heat, lifetime and
-// fuel as they are.
+// The [1,2,1]/4 density of a block of side `bs` cells (8, or a coarse brick's 2 or 4) whose first
+// cell is (ox,oy,oz), on a lattice of 2^sh cells a brick: smoothSmoke's and smoothCoarseSmoke's
+// eight half-offset samples a cell share their corners, so the block's (bs + 2)^3 cells are staged
+// once, the (bs + 1)^3 corner samples taken from the stage, and each cell's eight of them summed.
+// The sums and their order are smoothedSmoke's; `raw` reads a cell (zero outside the box or
+// without a slot) and `put` takes cell k of the block and its density. Every thread of the CTA
+// calls it.
+// What bounds it: reading a cell through the brick tables cost 64 lookups and loads a cell when
+// every cell took its own eight samples (427 us on 3.7k bricks of 8^3, 216 us on 1.8k).
+struct SmoothStage {
+  float cells[1000], corners[729];
+};
+template <class Raw, class Put>
+FP_DEV void smoothBlock(const BoxCursor& c, SmoothStage& st, int sh, int ox, int oy, int oz, int bs, Raw raw, Put put) {
+  const int S = bs + 2, C = bs + 1;
+  for (int i = threadIdx.x; i < S * S * S; i += RTHREADS)
+    st.cells[i] = raw(ox - 1 + i % S, oy - 1 + i / S % S, oz - 1 + i / (S * S));
+  __syncthreads();
+  // Corner i of an axis lies between cells i - 1 and i of the block; at the box's own faces the
+  // sample clamps to the centre of the cell inside it.
+  const int o[3] = {ox, oy, oz};
+  for (int i = threadIdx.x; i < C * C * C; i += RTHREADS) {
+    const int q[3] = {i % C, i / C % C, i / (C * C)};
+    int f0[3];
+    float fr[3];
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      const bool low = o[a] + q[a] == (c.lo[a] << sh), high = o[a] + q[a] == ((c.hi[a] + 1) << sh);
+      f0[a] = low ? q[a] + 1 : q[a];  // the staged place of the sample's first cell
+      fr[a] = low || high ? 0.f : .5f;
+    }
+    float v = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      const int dx = k & 1, dy = (k >> 1) & 1, dz = k >> 2;
+      const float w = (dx ? fr[0] : 1.f - fr[0]) * (dy ? fr[1] : 1.f - fr[1]) * (dz ? fr[2] : 1.f - fr[2]);
+      if (w != 0.f) v += st.cells[((f0[2] + dz) * S + f0[1] + dy) * S + f0[0] + dx] * w;
+    }
+    st.corners[i] = v;
+  }
+  __syncthreads();
+  for (int k = threadIdx.x; k < bs * bs * bs; k += RTHREADS) {
+    const int x = k % bs, y = k / bs % bs, z = k / (bs * bs);
+    float d = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; j++) d += st.corners[((z + (j >> 2)) * C + y + ((j >> 1) & 1)) * C + x + (j & 1)];
+    put(k, fmaxf(0.f, d * .125f));
+  }
+}
+
+// smoothSmoke: the render field of each boxed brick, the smoothed density with heat, lifetime and
+// fuel as they are; the coarse density smoothed on its own lattice; the aprons of both; and each
+// 2x2x2 cells' maxima for the occupancy. A CTA an 8^3 block, so that bricks of 16^3 and 32^3 spread
+// over the chip too.
 __global__ void __launch_bounds__(RTHREADS) k_render_field(const SimParams* __restrict__ Pp, const __grid_constant__ FpRender R) {
   const SimParams& P = *Pp;
+  __shared__ SmoothStage st;
+  __shared__ float2 cellMax[512];
   const uint32_t total = P.counters->active, aprons = apronTotal(R);
-  const bool half = P.scalarHalf != 0;
-  for (uint32_t i = blockIdx.x; i < total + aprons; i += gridDim.x) {
+  const bool half = P.scalarHalf != 0, coarse = P.smokeDiv > 1;
+  const int per = P.B / 8, blocks = per * per * per;
+  const int ssh = P.smokeShift, SB = 1 << ssh, sbs = SB < 8 ? SB : 8, sper = coarse ? SB / sbs : 0, sblocks = sper * sper * sper;
+  for (uint32_t item = blockIdx.x; item < (total + aprons) * (uint32_t)blocks; item += gridDim.x) {
+    const uint32_t i = item / blocks;
+    const int b = item % blocks, ox = b % per * 8, oy = b / per % per * 8, oz = b / (per * per) * 8;
+    const int sx = coarse ? b % sper * sbs : 0, sy = coarse ? b / sper % sper * sbs : 0,
+              sz = coarse ? b / (sper * sper) * sbs : 0;  // the coarse block b, when there are that many
     BoxCursor c = noBox();
-    int bx, by, bz, slot;
+    auto fine = [&](int x, int y, int z) { return rawSmoke(P, R, c, x, y, z); };
+    auto thin = [&](int x, int y, int z) { return rawCoarse(P, R, c, x, y, z); };
+    __syncthreads();  // the previous block's stage has been read
     if (i >= total) {
+      // An apron brick: its cells on the low faces.
       const uint32_t g = i - total;
       const int4 q = R.apronBricks[g];
       useBox(R, c, q.w);
-      const unsigned before = slottedBefore(P, R, c, q.x, q.y, q.z);
-      const int side = P.smokeDiv > 1 ? 1 << P.smokeShift : P.B, planes = 3 * side * side;
-      for (int k = threadIdx.x; k < planes; k += blockDim.x) {
-        int lx, ly, lz;
-        if (!apronCell(side, k, before, lx, ly, lz)) continue;
-        const int x = q.x * side + lx, y = q.y * side + ly, z = q.z * side + lz;
-        if (P.smokeDiv > 1)
-          R.apronSmoke[(size_t)g * planes + k] = smoothedCoarse(P, R, c, x, y, z);
-        else
-          R.apronField[(size_t)g * planes + k] = smoothedSmoke(P, R, c, x, y, z);
-      }
+      const int side = coarse ? SB : P.B, bs = coarse ? sbs : 8, cx = coarse ? sx : ox, cy = coarse ? sy : oy,
+                cz = coarse ? sz : oz;
+      if ((coarse && b >= sblocks) || (cx > 0 && cy > 0 && cz > 0)) continue;  // the same for the whole CTA
+      float* out = (coarse ? R.apronSmoke : R.apronField) + (size_t)g * 3 * side * side;
+      auto put = [&](int k, float d) {
+        const int lx = cx + k % bs, ly = cy + k / bs % bs, lz = cz + k / (bs * bs);
+        if (lx == 0 || ly == 0 || lz == 0) out[apronIndex(side, lx, ly, lz)] = d;
+      };
+      if (coarse)
+        smoothBlock(c, st, ssh, q.x * side + cx, q.y * side + cy, q.z * side + cz, bs, thin, put);
+      else
+        smoothBlock(c, st, P.shift, q.x * side + cx, q.y * side + cy, q.z * side + cz, bs, fine, put);
       continue;
     }
-    if (!boxBrick(P, R, c, i, bx, by, bz, slot)) continue;
-    for (int k = threadIdx.x; k < P.N; k += blockDim.x) {
-      int x = bx * P.B + (k & (P.B - 1)), y = by * P.B + ((k >> P.shift) & (P.B - 1)), z = bz * P.B + (k >> (2 * P.shift));
-      size_t o = (size_t)slot * 4 * P.N + k;
-      R.renderField[(size_t)slot * P.N + k] =
-          make_float4(P.smokeDiv > 1 ? ldHalf(P.fld, o, half) : smoothedSmoke(P, R, c, x, y, z),
-                      ldHalf(P.fld, o + P.N, half), ldHalf(P.fld, o + 2 * P.N, half), ldHalf(P.fld, o + 3 * P.N, half));
-    }
-    if (P.smokeDiv > 1) {  // smoothCoarseSmoke on the brick's coarse cells
-      const int sh = P.smokeShift, S = 1 << sh;
-      for (int k = threadIdx.x; k < P.smokeCells; k += blockDim.x) {
-        int x = bx * S + (k & (S - 1)), y = by * S + ((k >> sh) & (S - 1)), z = bz * S + (k >> (2 * sh));
-        R.renderSmoke[(size_t)slot * P.smokeCells + k] = smoothedCoarse(P, R, c, x, y, z);
+    int bx, by, bz, slot;
+    if (!boxBrick(P, R, c, i, bx, by, bz, slot)) continue;  // the same for the whole CTA
+    auto put = [&](int k, float d) {
+      const int cell = (((oz + (k >> 6)) << P.shift) + oy + ((k >> 3) & 7)) * P.B + ox + (k & 7);
+      const size_t o = (size_t)slot * 4 * P.N + cell;
+      const float4 f = make_float4(d, ldHalf(P.fld, o + P.N, half), ldHalf(P.fld, o + 2 * P.N, half),
+                                   ldHalf(P.fld, o + 3 * P.N, half));
+      R.renderField[(size_t)slot * P.N + cell] = f;
+      const float glow = glowOf(f.z);
+      cellMax[k] = make_float2(glow, (coarse ? 0.f : f.x) + glow);
+    };
+    if (coarse) {
+      for (int k = threadIdx.x; k < 512; k += RTHREADS) {
+        const int cell = (((oz + (k >> 6)) << P.shift) + oy + ((k >> 3) & 7)) * P.B + ox + (k & 7);
+        put(k, ldHalf(P.fld, (size_t)slot * 4 * P.N + cell, half));
       }
+      if (b < sblocks)
+        smoothBlock(c, st, ssh, bx * SB + sx, by * SB + sy, bz * SB + sz, sbs, thin, [&](int k, float d) {
+          const int x = sx + k % sbs, y = sy + k / sbs % sbs, z = sz + k / (sbs * sbs);
+          R.renderSmoke[(size_t)slot * P.smokeCells + ((((z << ssh) | y) << ssh) | x)] = d;
+        });
+    } else {
+      smoothBlock(c, st, P.shift, bx * P.B + ox, by * P.B + oy, bz * P.B + oz, 8, fine, put);
+    }
+    __syncthreads();
+    if (threadIdx.x < 64) {
+      const int u = threadIdx.x, first = ((u >> 4) * 2 * 8 + ((u >> 2) & 3) * 2) * 8 + (u & 3) * 2;
+      float2 m = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int k = 0; k < 8; k++) {
+        const float2 v = cellMax[first + ((k >> 2) * 8 + ((k >> 1) & 1)) * 8 + (k & 1)];
+        m.x = fmaxf(m.x, v.x);
+        m.y = fmaxf(m.y, v.y);
+      }
+      R.units[((size_t)slot * blocks + b) * 64 + u] = m;
     }
   }
 }
 
-// buildOccupancy and buildLighting of each boxed brick, from the render field.
-__global__ void __launch_bounds__(RTHREADS) k_render_light(const SimParams* __restrict__ Pp, const __grid_constant__ FpRender R) {
+// buildOccupancy (lighting.wgsl:149-244), a warp an 8^3 block: what is visible in the block and two
+// cells around it, from the maxima of 2x2x2 cells (216 of them; each lies in one brick).
+__global__ void __launch_bounds__(RTHREADS) k_render_occupancy(const SimParams* __restrict__ Pp,
+                                                               const __grid_constant__ FpRender R) {
   const SimParams& P = *Pp;
-  __shared__ int flags;
-  __shared__ int glowBits, smokeBits;  // the coarse bound's maxima (nonnegative floats' bits)
-  if (threadIdx.x == 0) glowBits = smokeBits = 0;
-  const uint32_t total = P.counters->active, aprons = apronTotal(R);
-  const int L = 1 << R.lightShift, L3 = L * L * L;
-  const float texel = P.h * (float)(P.B >> R.lightShift);
-  const int per = P.B / 8, blocks = per * per * per;
-  for (uint32_t i = blockIdx.x; i < total + aprons; i += gridDim.x) {
+  const uint32_t total = P.counters->active;
+  const int per = P.B / 8, blocks = per * per * per, lane = threadIdx.x & 31;
+  const bool coarse = P.smokeDiv > 1;
+  for (uint32_t item = blockIdx.x * (RTHREADS / 32) + (threadIdx.x >> 5); item < total * (uint32_t)blocks;
+       item += gridDim.x * (RTHREADS / 32)) {
     BoxCursor c = noBox();
     int bx, by, bz, slot;
-    if (i >= total) {
-      const int4 q = R.apronBricks[i - total];
+    if (!boxBrick(P, R, c, item / blocks, bx, by, bz, slot)) continue;  // the same for the whole warp
+    const int b = item % blocks;
+    const int ox = bx * P.B + b % per * 8 - 2, oy = by * P.B + b / per % per * 8 - 2, oz = bz * P.B + b / (per * per) * 8 - 2;
+    float glow = 0.f, seen = 0.f;
+#pragma unroll
+    for (int u = lane; u < 216; u += 32) {
+      const int ux = ox + (u % 6) * 2, uy = oy + ((u / 6) % 6) * 2, uz = oz + (u / 36) * 2, m = P.B - 1;
+      const int s = slotAt(P, R, c, ux >> P.shift, uy >> P.shift, uz >> P.shift);
+      if (s < 0) continue;
+      const int block = (((uz & m) >> 3) * per + ((uy & m) >> 3)) * per + ((ux & m) >> 3);
+      const int unit = (((uz & 7) >> 1) * 4 + ((uy & 7) >> 1)) * 4 + ((ux & 7) >> 1);
+      const float2 v = __ldg(&R.units[((size_t)s * blocks + block) * 64 + unit]);
+      glow = fmaxf(glow, v.x);
+      seen = fmaxf(seen, v.y);
+    }
+    float smoke = 0.f;
+    if (coarse) {
+      // Every trilinear donor of coarse density in the block and halo (lighting.wgsl:222-238).
+      const int d = P.smokeDiv, S = 1 << P.smokeShift;
+      const float ratio = (float)d;
+      int lo[3], size[3], boxLo[3], boxHi[3];
+      const int o[3] = {ox, oy, oz};
+#pragma unroll
+      for (int a = 0; a < 3; a++) {
+        lo[a] = (int)floorf((float)o[a] / ratio - .5f);
+        size[a] = (int)floorf((float)(o[a] + 12) / ratio - .5f) + 2 - lo[a];
+        boxLo[a] = c.lo[a] * S;
+        boxHi[a] = (c.hi[a] + 1) * S - 1;
+      }
+      for (int q = lane; q < size[0] * size[1] * size[2]; q += 32) {
+        int cq[3] = {lo[0] + q % size[0], lo[1] + (q / size[0]) % size[1], lo[2] + q / (size[0] * size[1])};
+#pragma unroll
+        for (int a = 0; a < 3; a++) cq[a] = min(max(cq[a], boxLo[a]), boxHi[a]);
+        smoke = fmaxf(smoke, cachedSmokeCell(P, R, c, cq[0], cq[1], cq[2]));
+      }
+    }
+    // Nonnegative floats order as their bits.
+    glow = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(glow)));
+    seen = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(seen)));
+    if (coarse) smoke = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(smoke)));
+    if (lane == 0)
+      R.occupancy[(size_t)slot * blocks + b] =
+          (uint8_t)((glow > .002f ? 1 : 0) | (seen > .002f || (coarse && smoke + glow > .002f) ? 2 : 0));
+  }
+}
+
+// buildLighting of each boxed brick and of the aprons, LIGHT_TEXELS texels of a brick a CTA. An
+// incident light (incidentLight) is a sample where it stands, up to 256 samples towards the sun and
+// six rays of six samples, each at a place known beforehand: the CTA takes the texels' samples as
+// one flat list, a thread each, into shared memory; then four lanes a texel add them up in the
+// serial order, one the sun's depth (with its early stop) and one each colour of the glow.
+// A warp a texel left 26 lanes idle while six walked the rays: 1.9 -> 0.46 ms on the default
+// grid's 640 bricks of 64 texels, 0.66 -> 0.21 ms on 3.7k bricks of 8.
+constexpr int LIGHT_TEXELS = 16, GLOW_SAMPLES = 36, SUN_SAMPLES = 256;
+struct LightStage {
+  float sun[LIGHT_TEXELS][SUN_SAMPLES];
+  float glow[LIGHT_TEXELS][5][GLOW_SAMPLES];  // emission RGB, the integrated transmission, the attenuation
+  float4 at[LIGHT_TEXELS];                    // the lit texels: position, the sun samples' spacing
+  float4* out[LIGHT_TEXELS];
+  int glows[LIGHT_TEXELS];
+  int count;
+};
+__global__ void __launch_bounds__(RTHREADS) k_render_light(const SimParams* __restrict__ Pp, const __grid_constant__ FpRender R) {
+  const SimParams& P = *Pp;
+  __shared__ LightStage st;
+  const uint32_t total = P.counters->active, aprons = apronTotal(R);
+  const int L = 1 << R.lightShift, L3 = L * L * L, planes = 3 * L * L;
+  const uint32_t chunks = (L3 + LIGHT_TEXELS - 1) / LIGHT_TEXELS, apronChunks = (planes + LIGHT_TEXELS - 1) / LIGHT_TEXELS;
+  const float texel = P.h * (float)(P.B >> R.lightShift);
+  const Tint tint = tintOf(R);
+  const float ln = sqrtf(R.light[0] * R.light[0] + R.light[1] * R.light[1] + R.light[2] * R.light[2]);
+  const float sx = R.light[0] / ln, sy = R.light[1] / ln, sz = R.light[2] / ln;
+  const int count = R.light[3] > 0.f ? R.shadowSamples : 0, perTexel = count + (R.optical[1] > 0.f ? GLOW_SAMPLES : 0);
+  for (uint32_t item = blockIdx.x; item < total * chunks + aprons * apronChunks; item += gridDim.x) {
+    BoxCursor c = noBox();
+    int bx, by, bz, slot = 0;
+    unsigned before = 0;
+    const bool apron = item >= total * chunks;
+    const uint32_t brick = apron ? (item - total * chunks) / apronChunks : item / chunks;
+    const int first = (int)(apron ? (item - total * chunks) % apronChunks : item % chunks) * LIGHT_TEXELS;
+    if (apron) {
+      const int4 q = R.apronBricks[brick];
       useBox(R, c, q.w);
-      const unsigned before = slottedBefore(P, R, c, q.x, q.y, q.z);
-      const int planes = 3 * L * L;
-      for (int k = threadIdx.x >> 5; k < planes; k += blockDim.x >> 5) {
-        int lx, ly, lz;
-        if (!apronCell(L, k, before, lx, ly, lz)) continue;
-        float4 light = incidentLightWarp(P, R, c, ((float)(q.x * L + lx) + .5f) * texel,
-                                         ((float)(q.y * L + ly) + .5f) * texel, ((float)(q.z * L + lz) + .5f) * texel);
-        if ((threadIdx.x & 31) == 0) R.apronLight[(size_t)(i - total) * planes + k] = light;
-      }
-      continue;
+      bx = q.x;
+      by = q.y;
+      bz = q.z;
+      before = slottedBefore(P, R, c, bx, by, bz);
+    } else if (!boxBrick(P, R, c, brick, bx, by, bz, slot)) {
+      continue;  // the same for the whole CTA
     }
-    if (!boxBrick(P, R, c, i, bx, by, bz, slot)) continue;  // the same for the whole CTA
-    // Each 8-cell block with a halo of two cells, in units of 2x2x2 cells: a unit in a
-    // slotted brick looks at its corner cells of the render field.
-    for (int b = 0; b < blocks; b++) {
-      if (threadIdx.x == 0) flags = 0;
-      __syncthreads();
-      int ox = bx * P.B + (b % per) * 8 - 2, oy = by * P.B + ((b / per) % per) * 8 - 2, oz = bz * P.B + (b / (per * per)) * 8 - 2;
-      int mine = 0;
-      const bool coarse = P.smokeDiv > 1;
-      float glowMax = 0.f, smokeMax = 0.f;
-      for (int u = threadIdx.x; u < 216; u += blockDim.x) {
-        int ux = ox + (u % 6) * 2, uy = oy + ((u / 6) % 6) * 2, uz = oz + (u / 36) * 2;
-        if (slotAt(P, R, c, ux >> P.shift, uy >> P.shift, uz >> P.shift) < 0) continue;
-        for (int k = 0; k < 8; k++) {
-          float4 f = renderCell(P, R, c, ux + (k & 1), uy + ((k >> 1) & 1), uz + (k >> 2), true);
-          float g = glowOf(f.z);
-          mine |= (g > .002f ? 1 : 0) | ((coarse ? 0.f : f.x) + g > .002f ? 2 : 0);
-          glowMax = fmaxf(glowMax, g);
+    // The texels that anything is at: the others see the open sun and no glow.
+    if (threadIdx.x < 32) {
+      const int k = first + (int)threadIdx.x;
+      bool lit = false;
+      float4 at = make_float4(0.f, 0.f, 0.f, 0.f), local = at;
+      float4* out = nullptr;
+      if (threadIdx.x < LIGHT_TEXELS && k < (apron ? planes : L3)) {
+        int lx = k % L, ly = (k / L) % L, lz = k / (L * L);
+        if (!apron || apronCell(L, k, before, lx, ly, lz)) {
+          out = apron ? R.apronLight + (size_t)brick * planes + k : R.lighting + (size_t)slot * L3 + k;
+          at = make_float4(((float)(bx * L + lx) + .5f) * texel, ((float)(by * L + ly) + .5f) * texel,
+                           ((float)(bz * L + lz) + .5f) * texel, 0.f);
+          local = sampleWorld(P, R, c, at.x, at.y, at.z);
+          lit = !(local.x + glowOf(local.z) < 1e-5f);
+          if (!lit) *out = make_float4(0.f, 0.f, 0.f, 1.f);
         }
       }
-      if (coarse) {
-        // Every trilinear donor of coarse density in the block and halo (lighting.wgsl:222-238).
-        const int d = P.smokeDiv, S = 1 << P.smokeShift;
-        const float ratio = (float)d;
-        int lo[3], hi[3], size[3], boxLo[3], boxHi[3];
-        const int o[3] = {ox, oy, oz};
-        for (int a = 0; a < 3; a++) {
-          lo[a] = (int)floorf((float)o[a] / ratio - .5f);
-          hi[a] = (int)floorf((float)(o[a] + 12) / ratio - .5f) + 1;
-          size[a] = hi[a] - lo[a] + 1;
-          boxLo[a] = c.lo[a] * S;
-          boxHi[a] = (c.hi[a] + 1) * S - 1;
-        }
-        for (int q = threadIdx.x; q < size[0] * size[1] * size[2]; q += blockDim.x) {
-          int cq[3] = {lo[0] + q % size[0], lo[1] + (q / size[0]) % size[1], lo[2] + q / (size[0] * size[1])};
-          for (int a = 0; a < 3; a++) cq[a] = min(max(cq[a], boxLo[a]), boxHi[a]);
-          smokeMax = fmaxf(smokeMax, cachedSmokeCell(P, R, c, cq[0], cq[1], cq[2]));
-        }
-        glowMax = fmaxf(glowMax, __shfl_xor_sync(0xffffffffu, glowMax, 16));
-        for (int w = 8; w > 0; w >>= 1) glowMax = fmaxf(glowMax, __shfl_xor_sync(0xffffffffu, glowMax, w));
-        for (int w = 16; w > 0; w >>= 1) smokeMax = fmaxf(smokeMax, __shfl_xor_sync(0xffffffffu, smokeMax, w));
-        if ((threadIdx.x & 31) == 0) {
-          atomicMax(&glowBits, __float_as_int(glowMax));
-          atomicMax(&smokeBits, __float_as_int(smokeMax));
-        }
+      const unsigned mask = __ballot_sync(0xffffffffu, lit);
+      if (lit) {
+        const int j = __popc(mask & ((1u << threadIdx.x) - 1u));
+        at.w = exitDistance(P, c, at.x, at.y, at.z, sx, sy, sz) / (float)R.shadowSamples;
+        st.at[j] = at;
+        st.out[j] = out;
+        st.glows[j] = R.optical[1] > 0.f && local.x > 1e-5f;
       }
-      if (mine) atomicOr(&flags, mine);
-      __syncthreads();
-      if (coarse && threadIdx.x == 0 && __int_as_float(smokeBits) + __int_as_float(glowBits) > .002f) flags |= 2;
-      if (threadIdx.x == 0) {
-        R.occupancy[(size_t)slot * blocks + b] = (uint8_t)flags;
-        glowBits = 0;
-        smokeBits = 0;
-      }
-      __syncthreads();
+      if (threadIdx.x == 0) st.count = __popc(mask);
     }
-    // The brick's texels of the lighting lattice, a warp a texel.
-    for (int k = threadIdx.x >> 5; k < L3; k += blockDim.x >> 5) {
-      int lx = k % L, ly = (k / L) % L, lz = k / (L * L);
-      float4 light = incidentLightWarp(P, R, c, ((float)(bx * L + lx) + .5f) * texel,
-                                       ((float)(by * L + ly) + .5f) * texel, ((float)(bz * L + lz) + .5f) * texel);
-      if ((threadIdx.x & 31) == 0) {
-        R.lighting[(size_t)slot * L3 + k] = light;
+    __syncthreads();
+    const int n = st.count;
+    for (int q = threadIdx.x; q < n * perTexel; q += RTHREADS) {
+      const int j = q / perTexel, i = q - j * perTexel;
+      const float4 at = st.at[j];
+      if (i < count) {
+        const float t = ((float)i + .5f) * at.w;
+        const float4 f = sampleWorld(P, R, c, at.x + sx * t, at.y + sy * t, at.z + sz * t);
+        st.sun[j][i] = (fmaxf(0.f, f.x) * R.optical[2] + glowOf(f.z) * R.flameOpacity) * at.w;
+      } else if (st.glows[j]) {
+        const int s = i - count, d = s / 6, k = s - d * 6;
+        float t = 0.f, interval = .075f;
+        for (int e = 0; e < k; e++) {
+          t += interval;
+          interval *= 1.65f;
+        }
+        const float p = t + interval * .5f;
+        const float4 f = sampleWorld(P, R, c, at.x + glowRay(d, 0) * p, at.y + glowRay(d, 1) * p, at.z + glowRay(d, 2) * p);
+        const float ext = extinctionOf(R, f), att = expf(-ext * interval);
+        const float3 e = emissionOf(R, tint, f);
+        st.glow[j][0][s] = e.x;
+        st.glow[j][1][s] = e.y;
+        st.glow[j][2][s] = e.z;
+        st.glow[j][3][s] = integratedTransmission(ext, interval, att);
+        st.glow[j][4][s] = att;
       }
     }
+    __syncthreads();
+    for (int q = threadIdx.x; q < n * 4; q += RTHREADS) {
+      const int j = q >> 2, role = q & 3;
+      float v = 0.f;
+      if (role == 3) {
+        float depth = 0.f;
+        for (int i = 0; i < count; i++) {
+          depth += st.sun[j][i];
+          if (depth > 9.f) break;
+        }
+        v = expf(-depth);
+      } else if (st.glows[j]) {
+        for (int d = 0; d < 6; d++) {
+          float transmission = 1.f;
+#pragma unroll
+          for (int k = 0; k < 6; k++) {
+            const int s = d * 6 + k;
+            v += st.glow[j][role][s] * (transmission * st.glow[j][3][s] / 6.f);
+            transmission *= st.glow[j][4][s];
+          }
+        }
+      }
+      reinterpret_cast<float*>(st.out[j])[role] = v;
+    }
+    __syncthreads();  // the stage is read before the next texels' samples
   }
 }
 
@@ -1450,8 +1558,11 @@ void fp_launch_render(const SimParams* dP, const FpRender& R, int sms, cudaStrea
     if (R.apronCap)
       k_render_aprons<<<dim3((unsigned)(blocks < 1 ? 1 : (blocks < sms * 8 ? blocks : sms * 8)), rows), 256, 0, st>>>(R);
   }
-  k_render_field<<<sms * 8, RTHREADS, 0, st>>>(dP, R);
-  k_render_light<<<sms * 8, RTHREADS, 0, st>>>(dP, R);
+  k_render_field<<<sms * 24, RTHREADS, 0, st>>>(dP, R);
+  // More CTAs than reside: texels that nothing is at cost little, so equal shares of them are not
+  // equal work (5 CTAs an SM 536 us, 20 474, 40 464 on the default grid).
+  k_render_light<<<sms * 40, RTHREADS, 0, st>>>(dP, R);
+  k_render_occupancy<<<sms * 8, RTHREADS, 0, st>>>(dP, R);
   const long long rays = R.slices ? (long long)R.sliceW * R.sliceH : (long long)R.width * R.height;
   if (rays >= 125000)
     marchLaunch<2>(dP, R, st);

@@ -272,6 +272,7 @@ int Engine::render(const fp_camera& cam, const fp_render_settings& rs, float* im
             (lighting_.bytes >= (size_t)slots_ * 4 * L * L * L * 4 ||
              grow(lighting_, (size_t)slots_ * 4 * L * L * L * 4, 0)) &&
             (occupancy_.bytes >= (size_t)slots_ * blocks || grow(occupancy_, (size_t)slots_ * blocks, 0)) &&
+            (renderUnits_.bytes >= (size_t)slots_ * N_ || grow(renderUnits_, (size_t)slots_ * N_, 0)) &&
             (smokeDiv_ == 1 || renderSmoke_.bytes >= (size_t)slots_ * SN_ * 4 ||
              grow(renderSmoke_, (size_t)slots_ * SN_ * 4, 0)) &&
             (renderParams_.ptr || alloc(renderParams_, sizeof(SimParams), false));
@@ -348,6 +349,7 @@ int Engine::render(const fp_camera& cam, const fp_render_settings& rs, float* im
   R.sliceW = sliceW;
   R.sliceH = sliceH;
   R.renderField = (float4*)renderField_.ptr;
+  R.units = (float2*)renderUnits_.ptr;
   R.renderSmoke = (float*)renderSmoke_.ptr;
   R.lighting = (float4*)lighting_.ptr;
   R.occupancy = (uint8_t*)occupancy_.ptr;
