@@ -53,6 +53,16 @@ struct Field {
 template <int SS>
 FP_DEV int stagedAt(const Stage<SS>& G, int x, int y, int z) { return ((z - G.oz) * G.S + (y - G.oy)) * G.S + (x - G.ox); }
 
+// The world position of a cell's centre, rounded: not to be folded into the sums it is used in, which
+// would make a position differ with the expression it stands in.
+FP_DEV float centreOf(int cell, float h) { return __fmul_rn((float)cell + 0.5f, h); }
+// The numbers of a lattice a cell's arithmetic uses again and again, in registers: read through
+// SimParams they are loaded anew after every store.
+struct Lat {
+  float h, invH, dt;
+};
+FP_DEV Lat latOf(const SimParams& P) { return Lat{P.h, P.invH, P.dt}; }
+
 // A cell within HALO cells of the home brick: the staged box always holds it, so no check.
 template <int SS>
 FP_DEV float nearCell(const SimParams& P, const Home& H, const Stage<SS>& G, const Field& f, int c, int x, int y, int z) {
@@ -129,35 +139,70 @@ FP_DEV float fieldSample(const SimParams& P, const Home& H, const Stage<SS>& G, 
   }
 }
 
-// Copy channels [0, nch) of a pool of `ch` channels over the staged box into shared memory,
-// zero where no slot, with asynchronous 4-byte copies (cp.async): every thread keeps all its
-// copies in flight and the caller waits once. A brick without a slot reads nothing (source
-// size 0 zero-fills). A half pool is widened to FP32 on the way (plain loads: cp.async moves
-// at least 4 bytes).
-template <int SS>
-FP_DEV void stageField(const SimParams& P, const Home& H, const Stage<SS>& G, float* sm, const float* pool, int ch,
-                       bool half = false, int nch = 0) {
-  constexpr int S = SS > 0 ? SS : 1, S3 = SS * SS * SS;
-  if constexpr (SS == 0) return;
-  if (nch <= 0) nch = ch;
-  for (int i = threadIdx.x; i < S3; i += blockDim.x) {
-    int lx = i % S, ly = (i / S) % S, lz = i / (S * S);
-    int x = G.ox + lx, y = G.oy + ly, z = G.oz + lz;
-    int s = brickSlot(P, H, x >> P.shift, y >> P.shift, z >> P.shift);
+// Copy channels [0, NCH) of a pool of `ch` channels of N cells a slot into shared memory, zero where
+// no slot, with asynchronous copies: every thread keeps all its copies in flight and the caller
+// waits once. A staged box is rows of PITCH floats, and the rows' 8 inner cells start where a brick
+// or a cube of a brick starts: an inner row is two 16-byte copies and a rim two cells or 8 bytes of
+// the neighbour's row, so an address serves 2 to 4 cells of every channel. (A copy a cell, each
+// with its own address, was a quarter of the predictor's instructions.) A brick without a slot
+// reads nothing (source size 0 zero-fills). A half pool is widened on the way by plain loads.
+//   rows  RY0 .. RY0 + NR - 1 of the box on y and z
+//   X0    where the 8 inner cells start in a row: 2 (a rim before them too; `sm` 8 bytes past a
+//         16-byte boundary) or 0 (no rim before them; `sm` on one); two cells after them either way
+//   (ox,oy,oz)  the lattice cell of the box's first place; `sh` the log2 of a brick's cells on it
+constexpr int PITCH = 8 + 2 * HALO;
+FP_DEV void copy8(unsigned dst, const float* g, int bytes) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(dst), "l"(g), "r"(bytes) : "memory");
+}
+FP_DEV void copy16(unsigned dst, const float* g, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(g), "r"(bytes) : "memory");
+}
+template <int NCH, int NR, int RY0, int X0>
+FP_DEV void stageRows(const Home& H, int sh, int N, float* sm, int plane, const float* pool, int ch, bool half, int ox,
+                      int oy, int oz) {
+  constexpr int ROWS = NR * NR, WIDE = 2 * ROWS, ALL = WIDE + (X0 ? 2 : 1) * ROWS;
+  const int m = (1 << sh) - 1;
+  for (int i = threadIdx.x; i < ALL; i += THREADS) {
+    const bool wide = i < WIDE;
+    const int j = wide ? i : i - WIDE, row = (wide || X0) ? j >> 1 : j, e = (wide || X0) ? j & 1 : 1;
+    const int lx = wide ? X0 + 4 * e : (X0 + 8) * e, ly = RY0 + row % NR, lz = RY0 + row / NR;
+    const int x = ox + lx, y = oy + ly, z = oz + lz;
+    const int s = H.nslot[nbrIndex((x >> sh) - H.bx, (y >> sh) - H.by, (z >> sh) - H.bz)];
+    const size_t at = (size_t)(s < 0 ? 0 : s) * (unsigned)(ch * N) + ((((z & m) << sh | (y & m)) << sh) | (x & m));
+    float* to = sm + (lz * PITCH + ly) * PITCH + lx;
     if (half) {
-      size_t base = s < 0 ? 0 : (size_t)s * ch * P.N + localCell(P, x, y, z);
-      for (int c = 0; c < nch; c++) sm[c * S3 + i] = s < 0 ? 0.f : ldHalf(pool, base + (size_t)c * P.N, true);
+      const __half2* g = reinterpret_cast<const __half2*>(reinterpret_cast<const __half*>(pool) + at);
+#pragma unroll
+      for (int c = 0; c < NCH; c++) {
+        float2 v[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+        if (s >= 0) {
+          v[0] = __half22float2(g[(size_t)c * (N / 2)]);
+          if (wide) v[1] = __half22float2(g[(size_t)c * (N / 2) + 1]);
+        }
+        *reinterpret_cast<float2*>(to + c * plane) = v[0];
+        if (wide) *reinterpret_cast<float2*>(to + c * plane + 2) = v[1];
+      }
       continue;
     }
-    const float* src = s < 0 ? pool : pool + (size_t)s * ch * P.N + localCell(P, x, y, z);
-    int bytes = s < 0 ? 0 : 4;
-    for (int c = 0; c < nch; c++) {
-      unsigned dst = (unsigned)__cvta_generic_to_shared(sm + c * S3 + i);
-      const float* g = s < 0 ? pool : src + (size_t)c * P.N;
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(dst), "l"(g), "r"(bytes) : "memory");
+    const float* g = s < 0 ? pool : pool + at;
+    const unsigned dst = (unsigned)__cvta_generic_to_shared(to);
+#pragma unroll
+    for (int c = 0; c < NCH; c++) {
+      if (wide)
+        copy16(dst + 4 * c * plane, g + (size_t)c * N, s < 0 ? 0 : 16);
+      else
+        copy8(dst + 4 * c * plane, g + (size_t)c * N, s < 0 ? 0 : 8);
     }
   }
 }
+// The whole box of the transport kernels: a brick (or cube of a brick) of 8^3 cells and its HALO rim.
+template <int NCH>
+FP_DEV void stageField(const Home& H, int sh, int N, const Stage<PITCH>& G, float* sm, const float* pool, int ch,
+                       bool half = false) {
+  stageRows<NCH, PITCH, 0, HALO>(H, sh, N, sm, Stage<PITCH>::S3, pool, ch, half, G.ox, G.oy, G.oz);
+}
+// The first staged float: 8 bytes past a 16-byte boundary (stageRows).
+constexpr int STAGE_PAD = 2;
 // Wait for this thread's staged copies, then for every thread's.
 FP_DEV void stageWait() {
   asm volatile("cp.async.wait_all;\n" ::: "memory");
@@ -175,9 +220,9 @@ FP_DEV TransportStage<STAGED> stageOf(const SimParams& P, const Home& H) {
 
 // Component c of the staggered velocity at world position p: stored half a cell back along c.
 template <int SS>
-FP_DEV float velComp(const SimParams& P, const Home& H, const Stage<SS>& G, const Field& v, float px, float py, float pz,
-                     int c) {
-  float qx = px * P.invH, qy = py * P.invH, qz = pz * P.invH;
+FP_DEV float velComp(const SimParams& P, const Home& H, const Lat& L, const Stage<SS>& G, const Field& v, float px, float py,
+                     float pz, int c) {
+  float qx = px * L.invH, qy = py * L.invH, qz = pz * L.invH;
   return fieldSample(P, H, G, v, c, c == 0 ? qx - 0.5f : qx, c == 1 ? qy - 0.5f : qy, c == 2 ? qz - 0.5f : qz);
 }
 // velocityAt through the directory, q in cell units.
@@ -195,10 +240,11 @@ static __device__ __noinline__ float3 velocityFar(const SimParams& P, const Home
 // (per axis: unshifted, and shifted half a cell for the component stored along it) and one
 // check that all three blocks are staged.
 template <int SS>
-FP_DEV float3 velocityAt(const SimParams& P, const Home& H, const Stage<SS>& G, const Field& v, float px, float py,
-                         float pz) {
-  const float q[3] = {px * P.invH, py * P.invH, pz * P.invH};
+FP_DEV float3 velocityAt(const SimParams& P, const Home& H, const Lat& L, const Stage<SS>& G, const Field& v, float px,
+                         float py, float pz) {
   if constexpr (SS > 0) {
+    // Rounded products: the three samples and the far path share them.
+    const float q[3] = {__fmul_rn(px, L.invH), __fmul_rn(py, L.invH), __fmul_rn(pz, L.invH)};
     const int o[3] = {G.ox, G.oy, G.oz};
     int i0[3], i1[3];
     float f0[3], f1[3];
@@ -206,9 +252,12 @@ FP_DEV float3 velocityAt(const SimParams& P, const Home& H, const Stage<SS>& G, 
 #pragma unroll
     for (int a = 0; a < 3; a++) {
       float u0 = q[a] - 0.5f, u1 = q[a] - 1.f;
-      float g0 = floorf(u0), g1 = floorf(u1);
+      // u1 is half a cell below u0: its floor is u0's or one less.
+      const float g0 = floorf(u0);
+      const bool same = u1 >= g0;
+      const float g1 = same ? g0 : g0 - 1.f;
       i0[a] = (int)g0 - o[a];
-      i1[a] = (int)g1 - o[a];
+      i1[a] = same ? i0[a] : i0[a] - 1;
       f0[a] = u0 - g0;
       f1[a] = u1 - g1;
       in = in && i1[a] >= 0 && i0[a] < G.S - 1;  // i1 <= i0 <= i1 + 1
@@ -227,6 +276,7 @@ FP_DEV float3 velocityAt(const SimParams& P, const Home& H, const Stage<SS>& G, 
     }
     return velocityFar(P, H, v, q[0], q[1], q[2]);
   } else {
+    const float q[3] = {px * L.invH, py * L.invH, pz * L.invH};
     return velocityCells(P, H, v, q);
   }
 }
@@ -281,53 +331,76 @@ FP_DEV void cellOf(const SimParams& P, const Home& H, int c, int& x, int& y, int
 // the scalars at the start of the step.
 // advectVelocityWithBounds (fluid-velocity-transport.wgsl:28-100) at velocity cell (x,y,z),
 // offset c of its brick's slot, on the velocity lattice P.
-template <int SS>
-FP_DEV void predictVelocity(const SimParams& P, const Home& H, const Stage<SS>& G, const Field& V, size_t slot, int c, int x,
-                            int y, int z) {
-  const size_t N = P.N;
+// CN: the lattice's cells a slot when known at compile time (the staged forms: 8^3), else 0.
+template <int CN, int SS>
+FP_DEV void predictVelocity(const SimParams& P, const Home& H, const Lat& L, const Stage<SS>& G, const Field& V,
+                            float* __restrict__ out, uint16_t* __restrict__ donors, int c, int x, int y, int z) {
+  const int N = CN ? CN : P.N;
   // The limiter's bounds (the forward 2x2x2 block of each donor cell) are taken where the
   // correction needs them, at the donor, from the same start-of-step velocity.
-  const float px = ((float)x + 0.5f) * P.h, py = ((float)y + 0.5f) * P.h, pz = ((float)z + 0.5f) * P.h;
+  const float px = centreOf(x, L.h), py = centreOf(y, L.h), pz = centreOf(z, L.h);
   // solidAt at a cell centre is solidCell of that cell: centre / h + 0.25 floors to it.
   if (solidCell(P, H, x, y, z)) {
-    for (int k = 0; k < 3; k++) P.velP[(slot * 3 + k) * N + c] = 0.f;
+    for (int k = 0; k < 3; k++) out[k * N + c] = 0.f;
   } else {
     float3 orig = make_float3(nearCell(P, H, G, V, 0, x, y, z), nearCell(P, H, G, V, 1, x, y, z),
                               nearCell(P, H, G, V, 2, x, y, z));
 #pragma unroll
     for (int comp = 0; comp < 3; comp++) {
       float face[3] = {px, py, pz};
-      face[comp] += 0.5f * P.h;
+      face[comp] += 0.5f * L.h;
       float3 fv = velocityOnFace(P, H, G, V, x, y, z, comp, orig);
-      float3 vm = velocityAt(P, H, G, V, face[0] - 0.5f * P.dt * fv.x, face[1] - 0.5f * P.dt * fv.y,
-                             face[2] - 0.5f * P.dt * fv.z);
-      float dep[3] = {face[0] - P.dt * vm.x, face[1] - P.dt * vm.y, face[2] - P.dt * vm.z};
+      float3 vm = velocityAt(P, H, L, G, V, face[0] - 0.5f * L.dt * fv.x, face[1] - 0.5f * L.dt * fv.y,
+                             face[2] - 0.5f * L.dt * fv.z);
+      float dep[3] = {face[0] - L.dt * vm.x, face[1] - L.dt * vm.y, face[2] - L.dt * vm.z};
       float sh[3] = {dep[0], dep[1], dep[2]};
-      sh[comp] -= 0.5f * P.h;
+      sh[comp] -= 0.5f * L.h;
       // Divided, not multiplied by 1/h: still air lands exactly on a cell boundary here and
       // the donor cell is an integer decision the oracle repeats.
-      int bx = (int)floorf(sh[0] / P.h - 0.5f), by = (int)floorf(sh[1] / P.h - 0.5f),
-          bz = (int)floorf(sh[2] / P.h - 0.5f);
-      P.donors[(slot * 3 + comp) * N + c] = (uint16_t)packDonor(bx - x, by - y, bz - z);
-      P.velP[(slot * 3 + comp) * N + c] = velComp(P, H, G, V, dep[0], dep[1], dep[2], comp);
+      int bx = (int)floorf(sh[0] / L.h - 0.5f), by = (int)floorf(sh[1] / L.h - 0.5f),
+          bz = (int)floorf(sh[2] / L.h - 0.5f);
+      donors[comp * N + c] = (uint16_t)packDonor(bx - x, by - y, bz - z);
+      out[comp * N + c] = velComp(P, H, L, G, V, dep[0], dep[1], dep[2], comp);
     }
   }
 }
+// Least and greatest of three (one instruction each on sm_100).
+FP_DEV float min3(float a, float b, float c) {
+  float r;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+FP_DEV float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+// What the scalars' predictor writes: the brick's predictor and donor ranges.
+struct ScalarOut {
+  float *pred, *range;
+};
 // advectScalars (fluid-scalar-transport.wgsl:38-142) at field cell (x,y,z), offset c of its
-// brick's slot: P the field lattice, VP the velocity lattice the trace samples.
+// brick's slot: P the field lattice, VP the velocity lattice the trace samples (ONE: the same one).
 // GV: the stage of the velocity (on VP's lattice), GF: the stage of the scalars (on P's).
-template <int SV, int SF>
-FP_DEV void predictScalars(const SimParams& P, const SimParams& VP, const Home& H, const Stage<SV>& GV, const Field& V,
-                           const Stage<SF>& GF, const Field& F, size_t slot, int c, int x, int y, int z) {
-  const size_t N = P.N;
+template <int CN, bool ONE, int SV, int SF>
+FP_DEV void predictScalars(const SimParams& P, const SimParams& VP, const Home& H, const Lat& L, const Lat& VL,
+                           const Stage<SV>& GV, const Field& V, const Stage<SF>& GF, const Field& F, const ScalarOut& O,
+                           bool maccormack, bool noLife, bool noSmoke, int c, int x, int y, int z) {
+  const int N = CN ? CN : P.N;
   // Scalars: a cell-centred RK2 back trace, the predictor and its donors' range.
-  const float px = ((float)x + 0.5f) * P.h, py = ((float)y + 0.5f) * P.h, pz = ((float)z + 0.5f) * P.h;
-  float3 cv = VP.velDiv == 1 ? centreVelocity(VP, H, GV, V, x, y, z) : velocityAt(VP, H, GV, V, px, py, pz);
-  float3 vm = velocityAt(VP, H, GV, V, px - 0.5f * P.dt * cv.x, py - 0.5f * P.dt * cv.y, pz - 0.5f * P.dt * cv.z);
-  float dx_ = px - P.dt * vm.x, dy_ = py - P.dt * vm.y, dz_ = pz - P.dt * vm.z;
+  const float px = centreOf(x, L.h), py = centreOf(y, L.h), pz = centreOf(z, L.h);
+  float3 cv = ONE ? centreVelocity(VP, H, GV, V, x, y, z) : velocityAt(VP, H, VL, GV, V, px, py, pz);
+  // The midpoint: half a step back from the rounded centre, but from the centre itself in the
+  // directory form of a divided lattice.
+  constexpr bool EXACT = !ONE && SF == 0;
+  const float half = 0.5f * L.dt;
+  const float mid[3] = {EXACT ? fmaf((float)x + 0.5f, L.h, -__fmul_rn(half, cv.x)) : fmaf(-half, cv.x, px),
+                        EXACT ? fmaf((float)y + 0.5f, L.h, -__fmul_rn(half, cv.y)) : fmaf(-half, cv.y, py),
+                        EXACT ? fmaf((float)z + 0.5f, L.h, -__fmul_rn(half, cv.z)) : fmaf(-half, cv.z, pz)};
+  float3 vm = velocityAt(VP, H, VL, GV, V, mid[0], mid[1], mid[2]);
+  float dx_ = fmaf(-L.dt, vm.x, px), dy_ = fmaf(-L.dt, vm.y, py), dz_ = fmaf(-L.dt, vm.z, pz);
   // The departure's trilinear block in cell units: corner `base`, fractions `fr`.
-  const float dc[3] = {(float)x + (dx_ - px) * P.invH, (float)y + (dy_ - py) * P.invH,
-                       (float)z + (dz_ - pz) * P.invH};
+  const float dc[3] = {(float)x + (dx_ - px) * L.invH, (float)y + (dy_ - py) * L.invH, (float)z + (dz_ - pz) * L.invH};
   int base[3];
   float fr[3];
 #pragma unroll
@@ -338,33 +411,33 @@ FP_DEV void predictScalars(const SimParams& P, const SimParams& VP, const Home& 
   }
   const float* blk = stagedBlock(GF, F, base[0], base[1], base[2]);
   float out[4];
-  float* sb = P.sb + slot * 8 * N;
 #pragma unroll
   for (int k = 0; k < 4; k++) {
     float t[8];
     blockCells(P, H, GF, F, k, blk, base[0], base[1], base[2], t);
     out[k] = blend8(t, fr[0], fr[1], fr[2]);
-    if (P.maccormack) {
+    if (maccormack) {
       // The donors' range; FP16-finite for smoke, heat and fuel, [0,1]-anchored for lifetime.
       float lo = k == 2 ? 1.f : 65504.f, hi = k == 2 ? 0.f : -65504.f;
 #pragma unroll
-      for (int j = 0; j < 8; j++) {
-        lo = fminf(lo, t[j]);
-        hi = fmaxf(hi, t[j]);
+      for (int j = 0; j < 8; j += 2) {
+        lo = min3(lo, t[j], t[j + 1]);
+        hi = max3(hi, t[j], t[j + 1]);
       }
       const int row = k < 2 ? k : 5 - k;  // rows: smoke, heat, fuel, lifetime
-      sb[row * N + c] = lo;
-      sb[(4 + row) * N + c] = hi;
+      O.range[row * N + c] = lo;
+      O.range[(4 + row) * N + c] = hi;
     }
   }
-  if (!P.maccormack) out[2] = clamp01(out[2]);
-  else if (P.lifetimeZero) out[2] = 0.f;
+  if (!maccormack) out[2] = clamp01(out[2]);
+  else if (noLife) out[2] = 0.f;
   // With coarse smoke the fine smoke channel carries no density
   // (fluid-scalar-transport.wgsl:127, :137).
-  if (P.smokeDiv > 1) out[0] = 0.f;
+  if (noSmoke) out[0] = 0.f;
   // The predictor lives within the step: FP32 in every precision, so the limiter compares
   // the corrected value with unrounded predictions.
-  for (int k = 0; k < 4; k++) P.fldP[(slot * 4 + k) * N + c] = out[k];
+#pragma unroll
+  for (int k = 0; k < 4; k++) O.pred[k * N + c] = out[k];
 }
 
 // Transport kernels' forms. 0: unstaged (any grid). 1: staged, 8^3 bricks on one lattice.
@@ -372,6 +445,7 @@ FP_DEV void predictScalars(const SimParams& P, const SimParams& VP, const Home& 
 // divisor d > 1 with 8 d field cells a brick side): the velocity is staged once over the brick
 // and a HALO-cell rim on its own lattice, the scalars per cube of 8^3 field cells and a HALO rim.
 constexpr int CUBE = 8;
+constexpr int CELLS = CUBE * CUBE * CUBE;  // of a brick (or a cube) of the staged forms
 template <int SS>
 FP_DEV Stage<SS> stageAt(int ox, int oy, int oz) {
   Stage<SS> G;
@@ -407,18 +481,23 @@ FP_DEV void brick_predict(const SimParams* __restrict__ Pp, uint32_t i) {
   if (!homeOk(P, id)) return;  // the bounds-checked build only
   Home H = enterBrick(P, id, nslot);
   size_t slot = (size_t)nslot[13];
+  const Lat L = latOf(P);
+  const ScalarOut O{P.fldP + slot * 4 * P.N, P.sb + slot * 8 * P.N};
+  const bool maccormack = P.maccormack != 0, noLife = P.lifetimeZero != 0, noSmoke = P.smokeDiv > 1;
   if constexpr (MODE == 2) {
     const SimParams& VP = *P.vview;
+    const Lat VL = latOf(VP);
     const TransportStage<true> GV = velocityStage(VP, H);
-    Field V{P.vel, 3, smem};
-    Field F{P.fld, 4, smem + 3 * GV.S3, P.scalarHalf != 0};
-    stageField(VP, H, GV, smem, P.vel, 3);
+    float* st = smem + STAGE_PAD;
+    Field V{P.vel, 3, st};
+    Field F{P.fld, 4, st + 3 * GV.S3, P.scalarHalf != 0};
+    float* out = P.velP + slot * 3 * CELLS;
+    uint16_t* donors = P.donors + slot * 3 * CELLS;
+    stageField<3>(H, 3, CELLS, GV, st, P.vel, 3);
     stageWait();
-    for (int c = threadIdx.x; c < VP.N; c += blockDim.x) {
-      int x, y, z;
-      cellOf(VP, H, c, x, y, z);
-      predictVelocity(VP, H, GV, V, slot, c, x, y, z);
-    }
+    for (int c = threadIdx.x; c < CELLS; c += THREADS)
+      predictVelocity<CELLS>(VP, H, VL, GV, V, out, donors, c, H.bx * 8 + (c & 7), H.by * 8 + ((c >> 3) & 7),
+                             H.bz * 8 + (c >> 6));
     const int cubes = (P.B / CUBE) * (P.B / CUBE) * (P.B / CUBE);
     for (int k = 0; k < cubes; k++) {
       int ox, oy, oz;
@@ -426,44 +505,51 @@ FP_DEV void brick_predict(const SimParams* __restrict__ Pp, uint32_t i) {
       const TransportStage<true> GF =
           stageAt<8 + 2 * HALO>(H.bx * P.B + ox - HALO, H.by * P.B + oy - HALO, H.bz * P.B + oz - HALO);
       __syncthreads();  // the previous cube's stage has been read
-      stageField(P, H, GF, smem + 3 * GV.S3, P.fld, 4, F.half);
+      stageField<4>(H, P.shift, P.N, GF, st + 3 * GV.S3, P.fld, 4, F.half);
       stageWait();
-      for (int q = threadIdx.x; q < CUBE * CUBE * CUBE; q += blockDim.x) {
+      for (int q = threadIdx.x; q < CUBE * CUBE * CUBE; q += THREADS) {
         const int lx = ox + (q & 7), ly = oy + ((q >> 3) & 7), lz = oz + (q >> 6);
-        predictScalars(P, VP, H, GV, V, GF, F, slot, (lz * P.B + ly) * P.B + lx, H.bx * P.B + lx, H.by * P.B + ly,
-                       H.bz * P.B + lz);
+        predictScalars<0, false>(P, VP, H, L, VL, GV, V, GF, F, O, maccormack, noLife, noSmoke,
+                          (lz * P.B + ly) * P.B + lx, H.bx * P.B + lx, H.by * P.B + ly, H.bz * P.B + lz);
       }
+    }
+  } else if constexpr (MODE == 1) {
+    const TransportStage<true> G = stageOf<true>(P, H);
+    float* st = smem + STAGE_PAD;
+    Field V{P.vel, 3, st};
+    Field F{P.fld, 4, st + 3 * G.S3, P.scalarHalf != 0};
+    float* out = P.velP + slot * 3 * CELLS;
+    uint16_t* donors = P.donors + slot * 3 * CELLS;
+    stageField<3>(H, 3, CELLS, G, st, P.vel, 3);
+    stageField<4>(H, 3, CELLS, G, st + 3 * G.S3, P.fld, 4, F.half);
+    stageWait();
+    for (int c = threadIdx.x; c < CELLS; c += THREADS) {
+      const int x = H.bx * 8 + (c & 7), y = H.by * 8 + ((c >> 3) & 7), z = H.bz * 8 + (c >> 6);
+      predictVelocity<CELLS>(P, H, L, G, V, out, donors, c, x, y, z);
+      predictScalars<CELLS, true>(P, P, H, L, L, G, V, G, F, O, maccormack, noLife, noSmoke, c, x, y, z);
     }
   } else {
-    constexpr bool STAGED = MODE == 1;
-    TransportStage<STAGED> G = stageOf<STAGED>(P, H);
-    Field V{P.vel, 3, STAGED ? smem : nullptr};
-    Field F{P.fld, 4, STAGED ? smem + 3 * G.S3 : nullptr, P.scalarHalf != 0};
-    if (STAGED) {
-      stageField(P, H, G, smem, P.vel, 3);
-      stageField(P, H, G, smem + 3 * G.S3, P.fld, 4, F.half);
-      stageWait();
+    const TransportStage<false> G = stageOf<false>(P, H);
+    Field V{P.vel, 3, nullptr};
+    Field F{P.fld, 4, nullptr, P.scalarHalf != 0};
+    // The velocity lattice's cells, then the field lattice's.
+    const SimParams& VP = *P.vview;
+    const Lat VL = latOf(VP);
+    float* out = P.velP + slot * 3 * VP.N;
+    uint16_t* donors = P.donors + slot * 3 * VP.N;
+    const bool one = P.velDiv == 1;
+    for (int c = threadIdx.x; c < VP.N; c += blockDim.x) {
+      int x, y, z;
+      cellOf(VP, H, c, x, y, z);
+      predictVelocity<0>(VP, H, VL, G, V, out, donors, c, x, y, z);
     }
-    if (STAGED || P.velDiv == 1) {
-      for (int c = threadIdx.x; c < P.N; c += blockDim.x) {
-        int x, y, z;
-        cellOf(P, H, c, x, y, z);
-        predictVelocity(P, H, G, V, slot, c, x, y, z);
-        predictScalars(P, P, H, G, V, G, F, slot, c, x, y, z);
-      }
-    } else {
-      // The velocity lattice's cells, then the field lattice's.
-      const SimParams& VP = *P.vview;
-      for (int c = threadIdx.x; c < VP.N; c += blockDim.x) {
-        int x, y, z;
-        cellOf(VP, H, c, x, y, z);
-        predictVelocity(VP, H, G, V, slot, c, x, y, z);
-      }
-      for (int c = threadIdx.x; c < P.N; c += blockDim.x) {
-        int x, y, z;
-        cellOf(P, H, c, x, y, z);
-        predictScalars(P, VP, H, G, V, G, F, slot, c, x, y, z);
-      }
+    for (int c = threadIdx.x; c < P.N; c += blockDim.x) {
+      int x, y, z;
+      cellOf(P, H, c, x, y, z);
+      if (one)
+        predictScalars<0, true>(P, P, H, L, L, G, V, G, F, O, maccormack, noLife, noSmoke, c, x, y, z);
+      else
+        predictScalars<0, false>(P, VP, H, L, VL, G, V, G, F, O, maccormack, noLife, noSmoke, c, x, y, z);
     }
   }
   __syncthreads();
@@ -490,19 +576,29 @@ FP_DEV void brick_correct(const SimParams* __restrict__ Pp, uint32_t i) {
   if (!homeOk(P, id)) return;  // the bounds-checked build only
   Home H = enterBrick(P, id, nslot);
   TransportStage<STAGED> G = stageOf<STAGED>(P, H);
-  Field V{P.vel, 3, STAGED ? smem : nullptr};
-  Field Vp{P.velP, 3, STAGED ? smem + 3 * G.S3 : nullptr};
-  if (STAGED) {
-    stageField(P, H, G, smem, P.vel, 3);
-    stageField(P, H, G, smem + 3 * G.S3, P.velP, 3);
+  float* st = smem + STAGE_PAD;
+  Field V{P.vel, 3, STAGED ? st : nullptr};
+  Field Vp{P.velP, 3, STAGED ? st + 3 * G.S3 : nullptr};
+  if constexpr (STAGED) {
+    stageField<3>(H, 3, CELLS, G, st, P.vel, 3);
+    stageField<3>(H, 3, CELLS, G, st + 3 * G.S3, P.velP, 3);
     stageWait();
   }
   size_t slot = (size_t)nslot[13];
-  const size_t N = P.N;
-  for (int c = threadIdx.x; c < P.N; c += blockDim.x) {
+  const Lat L = latOf(P);
+  const int N = STAGED ? CELLS : P.N, shift = STAGED ? 3 : P.shift;
+  const uint16_t* __restrict__ donors = P.donors + slot * 3 * N;
+  float* __restrict__ out = P.velC + slot * 3 * N;
+  for (int c = threadIdx.x; c < N; c += THREADS) {
     int x, y, z;
-    cellOf(P, H, c, x, y, z);
-    float px = ((float)x + 0.5f) * P.h, py = ((float)y + 0.5f) * P.h, pz = ((float)z + 0.5f) * P.h;
+    if constexpr (STAGED) {
+      x = H.bx * 8 + (c & 7);
+      y = H.by * 8 + ((c >> 3) & 7);
+      z = H.bz * 8 + (c >> 6);
+    } else {
+      cellOf(P, H, c, x, y, z);
+    }
+    float px = centreOf(x, L.h), py = centreOf(y, L.h), pz = centreOf(z, L.h);
     bool solid = solidCell<ONE>(P, H, x, y, z);  // solidAt at the cell centre
     float3 orig = make_float3(nearCell(P, H, G, V, 0, x, y, z), nearCell(P, H, G, V, 1, x, y, z),
                               nearCell(P, H, G, V, 2, x, y, z));
@@ -512,50 +608,50 @@ FP_DEV void brick_correct(const SimParams* __restrict__ Pp, uint32_t i) {
       if (!solid) {
         float predicted = nearCell(P, H, G, Vp, comp, x, y, z);
         float face[3] = {px, py, pz};
-        face[comp] += 0.5f * P.h;
-        uint32_t donor = P.donors[(slot * 3 + comp) * N + c];
+        face[comp] += 0.5f * L.h;
+        uint32_t donor = donors[comp * N + c];
         bool retrace = donor == (1u << 15);
         int base[3] = {x + (int)(donor & 31u) - 16, y + (int)((donor >> 5) & 31u) - 16,
                        z + (int)((donor >> 10) & 31u) - 16};
         float3 fv = make_float3(0.f, 0.f, 0.f);
         if (retrace) {
           fv = velocityOnFace(P, H, G, V, x, y, z, comp, orig);
-          float3 vm = velocityAt(P, H, G, V, face[0] - 0.5f * P.dt * fv.x, face[1] - 0.5f * P.dt * fv.y,
-                                 face[2] - 0.5f * P.dt * fv.z);
-          float dep[3] = {face[0] - P.dt * vm.x, face[1] - P.dt * vm.y, face[2] - P.dt * vm.z};
-          dep[comp] -= 0.5f * P.h;
-          for (int a = 0; a < 3; a++) base[a] = (int)floorf(dep[a] / P.h - 0.5f);  // as in the predictor
+          float3 vm = velocityAt(P, H, L, G, V, face[0] - 0.5f * L.dt * fv.x, face[1] - 0.5f * L.dt * fv.y,
+                                 face[2] - 0.5f * L.dt * fv.z);
+          float dep[3] = {face[0] - L.dt * vm.x, face[1] - L.dt * vm.y, face[2] - L.dt * vm.z};
+          dep[comp] -= 0.5f * L.h;
+          for (int a = 0; a < 3; a++) base[a] = (int)floorf(dep[a] / L.h - 0.5f);  // as in the predictor
         }
         // The bounds of the donor: the start-of-step component over the 2x2x2 block forward of
         // the donor cell (advectVelocityWithBounds' shared-tile min/max,
         // fluid-velocity-transport.wgsl:66-100), zero for a donor brick without a slot.
         float lo = 0.f, hi = 0.f;
-        int bs = brickSlot(P, H, base[0] >> P.shift, base[1] >> P.shift, base[2] >> P.shift);
+        int bs = brickSlot(P, H, base[0] >> shift, base[1] >> shift, base[2] >> shift);
         if (bs >= 0) {
           float t[8];
           blockCells(P, H, G, V, comp, stagedBlock(G, V, base[0], base[1], base[2]), base[0], base[1], base[2], t);
           lo = 1e5f;
           hi = -1e5f;
 #pragma unroll
-          for (int j = 0; j < 8; j++) {
-            lo = fminf(lo, t[j]);
-            hi = fmaxf(hi, t[j]);
+          for (int j = 0; j < 8; j += 2) {
+            lo = min3(lo, t[j], t[j + 1]);
+            hi = max3(hi, t[j], t[j + 1]);
           }
         }
         if (lo == hi && predicted == lo) {
           result = predicted;
         } else {
           if (!retrace) fv = velocityOnFace(P, H, G, V, x, y, z, comp, orig);
-          float3 vm = velocityAt(P, H, G, V, face[0] + 0.5f * P.dt * fv.x, face[1] + 0.5f * P.dt * fv.y,
-                                 face[2] + 0.5f * P.dt * fv.z);
-          float fw[3] = {face[0] + P.dt * vm.x, face[1] + P.dt * vm.y, face[2] + P.dt * vm.z};
-          fw[comp] -= 0.5f * P.h;
-          float reversed = fieldSample(P, H, G, Vp, comp, fw[0] * P.invH, fw[1] * P.invH, fw[2] * P.invH);
+          float3 vm = velocityAt(P, H, L, G, V, face[0] + 0.5f * L.dt * fv.x, face[1] + 0.5f * L.dt * fv.y,
+                                 face[2] + 0.5f * L.dt * fv.z);
+          float fw[3] = {face[0] + L.dt * vm.x, face[1] + L.dt * vm.y, face[2] + L.dt * vm.z};
+          fw[comp] -= 0.5f * L.h;
+          float reversed = fieldSample(P, H, G, Vp, comp, fw[0] * L.invH, fw[1] * L.invH, fw[2] * L.invH);
           float corrected = predicted + 0.5f * (get(orig, comp) - reversed);
           result = (corrected < lo || corrected > hi) ? predicted : corrected;
         }
       }
-      P.velC[(slot * 3 + comp) * N + c] = result;
+      out[comp * N + c] = result;
     }
   }
   __syncthreads();
@@ -589,17 +685,30 @@ FP_DEV void brick_evolve(const SimParams* __restrict__ Pp, uint32_t i) {
   Home H = enterBrick(P, id, nslot);
   constexpr bool STAGED = MODE != 0;
   const SimParams& VP = MODE == 1 ? P : *P.vview;  // the velocity lattice the traces sample
-  Field V{P.vel, 3, STAGED ? smem : nullptr};
-  Field Fp{P.fldP, 4, STAGED ? smem + 3 * TransportStage<true>::S3 : nullptr, false};  // the predictor: FP32
+  float* st = smem + STAGE_PAD;
+  Field V{P.vel, 3, STAGED ? st : nullptr};
+  Field Fp{P.fldP, 4, STAGED ? st + 3 * TransportStage<true>::S3 : nullptr, false};  // the predictor: FP32
   const bool half = P.scalarHalf != 0;  // the state pools
   size_t slot = (size_t)nslot[13];
-  const size_t N = P.N;
+  const int N = MODE == 1 ? CELLS : P.N;
+  // What is the same for every cell, once a brick.
+  const Lat L = latOf(P), VL = latOf(VP);
+  const bool maccormack = P.maccormack != 0, coarse = P.smokeDiv > 1, fuelOn = P.fuelEnabled != 0;
+  const bool oneLattice = MODE == 1 || VP.velDiv == 1;
+  const float ignition = P.ignition, cutoff = P.cutoff, flameStep = P.flame.dt / P.flame.lifespan;
+  const float burnLeft = expf(-P.burnRate * L.dt);
+  const float smokeKept = expf(-P.dissipation * L.dt), smokeHalf = expf(-P.dissipation * L.dt * 0.5f);
+  const float heatKept = expf(-P.cooling * L.dt), heatHalf = expf(-P.cooling * L.dt * 0.5f);
+  const float padMin = fmaxf(2.f, 2.f * (float)P.velDiv);
+  const float* __restrict__ range = P.sb + slot * 8 * N;
+  float* __restrict__ fldN = P.fldN;
+  float* __restrict__ expn = P.expn + slot * N;
   int tile = (int)(id >> 6);
   uint32_t busy = 0;
   bool expands = false;
   // One field cell (x,y,z), offset c of the brick's slot; GV stages the velocity, GF the predictor.
   auto cell = [&](const auto& GV, const auto& GF, int c, int x, int y, int z) {
-      float px = ((float)x + 0.5f) * P.h, py = ((float)y + 0.5f) * P.h, pz = ((float)z + 0.5f) * P.h;
+      float px = centreOf(x, L.h), py = centreOf(y, L.h), pz = centreOf(z, L.h);
       bool solid = solidCell<MODE == 1>(P, H, x, y, z);  // solidAt at the cell centre
       float value[4] = {0.f, 0.f, 0.f, 0.f};
       float expansion = 0.f;
@@ -608,10 +717,10 @@ FP_DEV void brick_evolve(const SimParams* __restrict__ Pp, uint32_t i) {
       float3 cv = make_float3(0.f, 0.f, 0.f);
       if (!solid) {
         float tr[4];
-        if (!P.maccormack) {
+        if (!maccormack) {
           for (int k = 0; k < 4; k++) tr[k] = nearCell(P, H, GF, Fp, k, x, y, z);
         } else {
-          const float* b = P.sb + slot * 8 * N;
+          const float* b = range;
           float mn0 = b[0 * N + c], mn1 = b[1 * N + c], mn3 = b[2 * N + c], lmin = b[3 * N + c];
           float mx0 = b[4 * N + c], mx1 = b[5 * N + c], mx3 = b[6 * N + c], lmax = b[7 * N + c];
           if (mn0 == mx0 && mn1 == mx1 && mn3 == mx3 && lmin == lmax) {
@@ -622,16 +731,16 @@ FP_DEV void brick_evolve(const SimParams* __restrict__ Pp, uint32_t i) {
           } else {
             float a0 = nearCell(P, H, GF, Fp, 0, x, y, z), a1 = nearCell(P, H, GF, Fp, 1, x, y, z),
                   a2 = nearCell(P, H, GF, Fp, 2, x, y, z), a3 = nearCell(P, H, GF, Fp, 3, x, y, z);
-            cv = VP.velDiv == 1 ? centreVelocity(VP, H, GV, V, x, y, z) : velocityAt(VP, H, GV, V, px, py, pz);
+            cv = oneLattice ? centreVelocity(VP, H, GV, V, x, y, z) : velocityAt(VP, H, VL, GV, V, px, py, pz);
             cvSampled = true;
-            float3 vm = velocityAt(VP, H, GV, V, px + 0.5f * P.dt * cv.x, py + 0.5f * P.dt * cv.y, pz + 0.5f * P.dt * cv.z);
-            float fx = px + P.dt * vm.x, fy = py + P.dt * vm.y, fz = pz + P.dt * vm.z;
+            float3 vm = velocityAt(VP, H, VL, GV, V, px + 0.5f * L.dt * cv.x, py + 0.5f * L.dt * cv.y, pz + 0.5f * L.dt * cv.z);
+            float fx = px + L.dt * vm.x, fy = py + L.dt * vm.y, fz = pz + L.dt * vm.z;
             const size_t o = slot * 4 * N + c;
             float o0 = ldHalf(P.fld, o, half), o1 = ldHalf(P.fld, o + N, half), o2 = ldHalf(P.fld, o + 2 * N, half),
                   o3 = ldHalf(P.fld, o + 3 * N, half);
             // The forward trace's trilinear block of the predictor, in cell units.
-            const float fc[3] = {(float)x + (fx - px) * P.invH, (float)y + (fy - py) * P.invH,
-                                 (float)z + (fz - pz) * P.invH};
+            const float fc[3] = {(float)x + (fx - px) * L.invH, (float)y + (fy - py) * L.invH,
+                                 (float)z + (fz - pz) * L.invH};
             int base[3];
             float fr[3];
   #pragma unroll
@@ -663,7 +772,7 @@ FP_DEV void brick_evolve(const SimParams* __restrict__ Pp, uint32_t i) {
         }
         // With coarse smoke the fine smoke channel stages only this step's source production
         // (fluid-scalar-transport.wgsl:190-199).
-        if (P.smokeDiv > 1) tr[0] = 0.f;
+        if (coarse) tr[0] = 0.f;
         float lifetime = tr[2];
         float prodS = 0.f, prodH = 0.f, injectedFuel = 0.f;
         uint2 list = tileList(P, tile, 0);
@@ -673,23 +782,23 @@ FP_DEV void brick_evolve(const SimParams* __restrict__ Pp, uint32_t i) {
           if (w == 0.f) continue;
           float2 var = burstVariation(e, px, py, pz, P.seedBits);
           lifetime = fmaxf(lifetime, e.flame * w * var.y);
-          prodS += e.smoke * w * P.dt;
-          prodH += e.heat * var.x * w * P.dt;
-          injectedFuel += e.fuel * w * P.dt;
+          prodS += e.smoke * w * L.dt;
+          prodH += e.heat * var.x * w * L.dt;
+          injectedFuel += e.fuel * w * L.dt;
         }
         // Mesh emission at this cell (fluid-field-evolution.wgsl:33-36).
         if (const FpMeshSource* ms = meshSourceAt(P, H, x, y, z)) {
           lifetime = fmaxf(lifetime, ms->scalar[0]);
-          prodS += ms->scalar[2] * P.dt;
-          prodH += ms->scalar[1] * P.dt;
-          injectedFuel += ms->scalar[3] * P.dt;
+          prodS += ms->scalar[2] * L.dt;
+          prodH += ms->scalar[1] * L.dt;
+          injectedFuel += ms->scalar[3] * L.dt;
         }
         float remaining = 0.f, burned = 0.f;
-        if (P.fuelEnabled) {
+        if (fuelOn) {
           remaining = tr[3] + injectedFuel;
-          if (tr[1] + prodH >= P.ignition) {
+          if (tr[1] + prodH >= ignition) {
             lifetime = fmaxf(lifetime, fminf(remaining, 1.f));
-            float unburned = remaining * expf(-P.burnRate * P.dt);
+            float unburned = remaining * burnLeft;
             burned = remaining - unburned;
             remaining = unburned;
           }
@@ -699,14 +808,14 @@ FP_DEV void brick_evolve(const SimParams* __restrict__ Pp, uint32_t i) {
         float after = 0.f, f0 = 0.f, f1 = 0.f, f2 = 0.f;
         if (before > 0.f) {
           const FpFlame& F = P.flame;
-          after = fmaxf(0.f, before - F.dt / F.lifespan);
+          after = fmaxf(0.f, before - flameStep);
           f0 = F.smoke * F.lifespan * rampIntegral(F, 0, after, before);
           f1 = F.heat * F.lifespan * rampIntegral(F, 1, after, before);
           f2 = F.expansion * (F.lifespan * rampIntegral(F, 2, after, before) / F.dt);
         }
-        expansion = f2 + P.flame.expansion * burned / P.dt;
-        float dS = tr[0] * expf(-P.dissipation * P.dt) + (prodS + f0) * expf(-P.dissipation * P.dt * 0.5f);
-        float dH = tr[1] * expf(-P.cooling * P.dt) + (prodH + f1) * expf(-P.cooling * P.dt * 0.5f);
+        expansion = f2 + P.flame.expansion * burned / L.dt;
+        float dS = __fmaf_rn(tr[0], smokeKept, __fmul_rn(prodS + f0, smokeHalf));
+        float dH = __fmaf_rn(tr[1], heatKept, __fmul_rn(prodH + f1, heatHalf));
         value[0] = fmaxf(dS, 0.f);
         value[1] = fmaxf(dH, 0.f);
         value[2] = after;
@@ -716,12 +825,12 @@ FP_DEV void brick_evolve(const SimParams* __restrict__ Pp, uint32_t i) {
       // clearDormant (fluid-common.wgsl:8-13)
       if (!injected && value[2] == 0.f && value[0] < 0.001f && value[1] < 0.001f && value[3] < 0.001f)
         value[0] = value[1] = value[2] = value[3] = 0.f;
-      for (int k = 0; k < 4; k++) stHalf(P.fldN, (slot * 4 + k) * N + c, value[k], half);
-      P.expn[slot * N + c] = expansion;
+      for (int k = 0; k < 4; k++) stHalf(fldN, (slot * 4 + k) * N + c, value[k], half);
+      expn[c] = expansion;
       if (expansion != 0.f) expands = true;
       // holdsContent and contentSupport (fluid-content.wgsl:22-39).
-      if (fmaxf(fmaxf(P.smokeDiv > 1 ? 0.f : value[0], value[2]), value[3]) > P.cutoff) {
-        if (!cvSampled) cv = VP.velDiv == 1 ? centreVelocity(VP, H, GV, V, x, y, z) : velocityAt(VP, H, GV, V, px, py, pz);
+      if (fmaxf(fmaxf(coarse ? 0.f : value[0], value[2]), value[3]) > cutoff) {
+        if (!cvSampled) cv = oneLattice ? centreVelocity(VP, H, GV, V, x, y, z) : velocityAt(VP, H, VL, GV, V, px, py, pz);
         int idc[3] = {x, y, z};
         float vv[3] = {cv.x, cv.y, cv.z};
         bool low[3], high[3];
@@ -729,7 +838,7 @@ FP_DEV void brick_evolve(const SimParams* __restrict__ Pp, uint32_t i) {
           float side = (float)P.B;
           float loc = (float)(idc[a] & (P.B - 1)) + 0.5f;
           // two velocity cells of stencil (2 d field cells), and a step of motion
-          float pad = fminf(side, fmaxf(2.f, 2.f * (float)P.velDiv) + fabsf(vv[a]) * P.dt / P.h);
+          float pad = fminf(side, padMin + fabsf(vv[a]) * L.dt / L.h);
           low[a] = loc < pad;
           high[a] = loc + pad >= side;
         }
@@ -740,7 +849,7 @@ FP_DEV void brick_evolve(const SimParams* __restrict__ Pp, uint32_t i) {
   };
   if constexpr (MODE == 2) {
     const TransportStage<true> GV = velocityStage(VP, H);
-    stageField(VP, H, GV, smem, P.vel, 3);
+    stageField<3>(H, 3, CELLS, GV, st, P.vel, 3);
     const int cubes = (P.B / CUBE) * (P.B / CUBE) * (P.B / CUBE);
     for (int k = 0; k < cubes; k++) {
       int ox, oy, oz;
@@ -748,20 +857,21 @@ FP_DEV void brick_evolve(const SimParams* __restrict__ Pp, uint32_t i) {
       const TransportStage<true> GF =
           stageAt<8 + 2 * HALO>(H.bx * P.B + ox - HALO, H.by * P.B + oy - HALO, H.bz * P.B + oz - HALO);
       if (k > 0) __syncthreads();  // the previous cube's stage has been read
-      stageField(P, H, GF, smem + 3 * GV.S3, P.fldP, 4);
+      stageField<4>(H, P.shift, P.N, GF, st + 3 * GV.S3, P.fldP, 4);
       stageWait();
       for (int q = threadIdx.x; q < CUBE * CUBE * CUBE; q += blockDim.x) {
         const int lx = ox + (q & 7), ly = oy + ((q >> 3) & 7), lz = oz + (q >> 6);
         cell(GV, GF, (lz * P.B + ly) * P.B + lx, H.bx * P.B + lx, H.by * P.B + ly, H.bz * P.B + lz);
       }
     }
+  } else if constexpr (MODE == 1) {
+    const TransportStage<true> G = stageOf<true>(P, H);
+    stageField<3>(H, 3, CELLS, G, st, P.vel, 3);
+    stageField<4>(H, 3, CELLS, G, st + 3 * G.S3, P.fldP, 4);
+    stageWait();
+    for (int c = threadIdx.x; c < CELLS; c += THREADS) cell(G, G, c, H.bx * 8 + (c & 7), H.by * 8 + ((c >> 3) & 7), H.bz * 8 + (c >> 6));
   } else {
-    TransportStage<STAGED> G = stageOf<STAGED>(P, H);
-    if (STAGED) {
-      stageField(P, H, G, smem, P.vel, 3);
-      stageField(P, H, G, smem + 3 * G.S3, P.fldP, 4);
-      stageWait();
-    }
+    const TransportStage<false> G = stageOf<false>(P, H);
     for (int c = threadIdx.x; c < P.N; c += blockDim.x) {
       int x, y, z;
       cellOf(P, H, c, x, y, z);
@@ -810,18 +920,18 @@ FP_DEV void brick_curl(const SimParams* __restrict__ Pp, uint32_t i) {
   if (!P.curlOn) return;  // the same for the whole CTA
   if (!homeOk(P, P.active[i])) return;  // the bounds-checked build only
   Home H = enterBrick(P, P.active[i], nslot);
-  Stage<STAGED ? 8 + 2 : 0> G;  // staged: 8^3 bricks and a one-cell rim
-  G.ox = H.bx * P.B - 1;
-  G.oy = H.by * P.B - 1;
-  G.oz = H.bz * P.B - 1;
-  Field V{P.velC, 3, STAGED ? smem : nullptr};
-  if (STAGED) {
-    stageField(P, H, G, smem, P.velC, 3);
+  // Staged: 8^3 bricks; of the transport box's rows those of a one-cell rim.
+  const TransportStage<STAGED> G = stageOf<STAGED>(P, H);
+  Field V{P.velC, 3, STAGED ? smem + STAGE_PAD : nullptr};
+  if constexpr (STAGED) {
+    stageRows<3, 10, 1, HALO>(H, 3, CELLS, smem + STAGE_PAD, G.S3, P.velC, 3, false, G.ox, G.oy, G.oz);
     stageWait();
   }
   size_t slot = (size_t)nslot[13];
-  const size_t N = P.N;
-  for (int c = threadIdx.x; c < P.N; c += blockDim.x) {
+  const int N = STAGED ? CELLS : P.N;
+  const float h = P.h;
+  float* __restrict__ out = P.curl + slot * 4 * N;
+  for (int c = threadIdx.x; c < N; c += THREADS) {
     int x, y, z;
     cellOf(P, H, c, x, y, z);
     auto cc = [&](int qx, int qy, int qz, int comp) {
@@ -829,15 +939,15 @@ FP_DEV void brick_curl(const SimParams* __restrict__ Pp, uint32_t i) {
       r[comp] -= 1;
       return 0.5f * (nearCell(P, H, G, V, comp, qx, qy, qz) + nearCell(P, H, G, V, comp, r[0], r[1], r[2]));
     };
-    float hh = 0.5f / P.h;
+    float hh = 0.5f / h;
     float dx0 = (cc(x + 1, y, z, 1) - cc(x - 1, y, z, 1)) * hh, dx1 = (cc(x + 1, y, z, 2) - cc(x - 1, y, z, 2)) * hh;
     float dy0 = (cc(x, y + 1, z, 0) - cc(x, y - 1, z, 0)) * hh, dy1 = (cc(x, y + 1, z, 2) - cc(x, y - 1, z, 2)) * hh;
     float dz0 = (cc(x, y, z + 1, 0) - cc(x, y, z - 1, 0)) * hh, dz1 = (cc(x, y, z + 1, 1) - cc(x, y, z - 1, 1)) * hh;
     float c0 = dy1 - dz1, c1 = dz0 - dx1, c2 = dx0 - dy0;
-    P.curl[(slot * 4 + 0) * N + c] = c0;
-    P.curl[(slot * 4 + 1) * N + c] = c1;
-    P.curl[(slot * 4 + 2) * N + c] = c2;
-    P.curl[(slot * 4 + 3) * N + c] = sqrtf(c0 * c0 + c1 * c1 + c2 * c2);
+    out[0 * N + c] = c0;
+    out[1 * N + c] = c1;
+    out[2 * N + c] = c2;
+    out[3 * N + c] = sqrtf(c0 * c0 + c1 * c1 + c2 * c2);
   }
   __syncthreads();
 }
@@ -936,7 +1046,7 @@ template <bool ONE, int SC, int SS>
 FP_DEV float3 cellForce(const SimParams& P, const Home& H, const Stage<SC>& Gc, const Field& Fc, const Stage<SS>& Gs,
                         const Field& Fs, int tile, int x, int y, int z) {
   if (brickSlot(P, H, x >> P.shift, y >> P.shift, z >> P.shift) < 0) return make_float3(0.f, 0.f, 0.f);
-  float wx = ((float)x + 0.5f) * P.h, wy = ((float)y + 0.5f) * P.h, wz = ((float)z + 0.5f) * P.h;
+  float wx = centreOf(x, P.h), wy = centreOf(y, P.h), wz = centreOf(z, P.h);
   if (solidCell<ONE>(P, H, x, y, z)) return make_float3(0.f, 0.f, 0.f);  // solidAt at the centre
   // The evolved scalars of this step (the reference swaps field and corrected first); with a
   // velocity divisor d > 1 their mean over the velocity cell (velocityCellAverage).
@@ -1017,6 +1127,7 @@ FP_DEV float sourceVelocity(const SimParams& P, const Home& H, int tile, float v
 // copied to shared memory first.
 // The side of the cubes the force kernel walks a brick in: their force tiles fit shared memory.
 constexpr int FORCE_SUB = 16;
+constexpr int FORCE_TILE = 732;  // float3s of the staged forms' force tile: 9^3, to a 16-byte boundary
 
 // MODE 1: 8^3 bricks on one lattice, curl and scalars staged. MODE 2: a velocity lattice of 8^3
 // cells a brick under a finer field lattice: the curl staged, the scalars' means (fieldAverage)
@@ -1036,22 +1147,24 @@ FP_DEV void brick_forces(const SimParams* __restrict__ Pp, uint32_t i) {
   // brick), each with its centre forces on the cube and one cell beyond its upper faces.
   constexpr bool ONE = MODE == 1, CSTAGED = MODE != 0;
   const int SUB = CSTAGED ? 8 : min(P.B, FORCE_SUB), E = SUB + 1, E3 = E * E * E, per = CSTAGED ? 1 : P.B / SUB;
-  float* stage = reinterpret_cast<float*>(forceTile + E3);
-  // Staged (8^3 bricks: E = 9): the curl over E + 2 cells a side, two scalars over E.
-  Stage<CSTAGED ? 11 : 0> Gc;
-  Stage<ONE ? 9 : 0> Gs;
-  Gc.ox = H.bx * P.B - 1;
-  Gc.oy = H.by * P.B - 1;
-  Gc.oz = H.bz * P.B - 1;
+  float* stage = reinterpret_cast<float*>(forceTile + FORCE_TILE);
+  // Staged: the curl over the cells before the brick to two past it (the transport box), the
+  // evolved smoke and heat from the brick's first cells to one past it.
+  Stage<CSTAGED ? PITCH : 0> Gc;
+  Stage<ONE ? PITCH : 0> Gs;
+  Gc.ox = H.bx * P.B - HALO;
+  Gc.oy = H.by * P.B - HALO;
+  Gc.oz = H.bz * P.B - HALO;
   Gs.ox = H.bx * P.B;
   Gs.oy = H.by * P.B;
   Gs.oz = H.bz * P.B;
   const bool half = P.scalarHalf != 0;
-  Field Fc{P.curl, 4, CSTAGED ? stage : nullptr};
-  Field Fs{P.fldN, 4, ONE ? stage + 4 * Gc.S3 : nullptr, half};
-  if (CSTAGED) {
-    if (P.vorticity != 0.f) stageField(P, H, Gc, stage, P.curl, 4);
-    if (ONE) stageField(P, H, Gs, stage + 4 * Gc.S3, P.fldN, 4, half, 2);  // smoke, heat
+  Field Fc{P.curl, 4, CSTAGED ? stage + STAGE_PAD : nullptr};
+  // Gs's two planes lie S3 apart as every stage's do; of the second only nine layers are held.
+  Field Fs{P.fldN, 4, ONE ? stage + 4 + 4 * Gc.S3 : nullptr, half};
+  if constexpr (CSTAGED) {
+    if (P.vorticity != 0.f) stageRows<4, 11, 1, HALO>(H, 3, CELLS, stage + STAGE_PAD, Gc.S3, P.curl, 4, false, Gc.ox, Gc.oy, Gc.oz);
+    if constexpr (ONE) stageRows<2, 9, 0, 0>(H, 3, CELLS, stage + 4 + 4 * Gc.S3, Gs.S3, P.fldN, 4, half, Gs.ox, Gs.oy, Gs.oz);
     stageWait();
   }
   const float decay = expf(-P.damping * P.dt);
@@ -1072,7 +1185,7 @@ FP_DEV void brick_forces(const SimParams* __restrict__ Pp, uint32_t i) {
       float3 F0 = forceTile[t];
       float f[3] = {0.5f * (F0.x + forceTile[t + 1].x), 0.5f * (F0.y + forceTile[t + E].y),
                     0.5f * (F0.z + forceTile[t + E * E].z)};
-      float px = ((float)x + 0.5f) * P.h, py = ((float)y + 0.5f) * P.h, pz = ((float)z + 0.5f) * P.h;
+      float px = centreOf(x, P.h), py = centreOf(y, P.h), pz = centreOf(z, P.h);
       float out[3];
       for (int a = 0; a < 3; a++) {
         float v = P.velC[(slot * 3 + a) * N + c] * decay + P.dt * f[a];
@@ -1106,10 +1219,10 @@ __global__ void __launch_bounds__(THREADS, FP_TRANSPORT_CTAS) k_forces(FpBatch b
     brick_forces<MODE>(MODE == 1 ? &P : P.vview, i);  // the velocity lattice
   }
 }
-// Shared memory of the staged force kernel: the (B+1)^3 force tile, the curl over (B+3)^3,
-// two scalar channels over (B+1)^3.
-constexpr size_t FORCE_STAGED_BYTES = 729 * sizeof(float3) + (4 * 1331 + 2 * 729) * sizeof(float);
-constexpr size_t FORCE_CURL_STAGED_BYTES = 729 * sizeof(float3) + 4 * 1331 * sizeof(float);  // MODE 2
+// Shared memory of the staged force kernel: the force tile, the curl's box, and of the scalars' box
+// a plane and nine layers.
+constexpr size_t FORCE_CURL_STAGED_BYTES = FORCE_TILE * sizeof(float3) + (4 + 4 * PITCH * PITCH * PITCH) * sizeof(float);  // MODE 2
+constexpr size_t FORCE_STAGED_BYTES = FORCE_CURL_STAGED_BYTES + (PITCH * PITCH * PITCH + 9 * PITCH * PITCH) * sizeof(float);
 
 // pressureUnknown (fluid-forces.wgsl:210-226): the cell's brick and those of its negative
 // neighbours compute.
@@ -1410,9 +1523,9 @@ FP_DEV float smokeSampleS(const SimParams& P, const Home& H, const SmokeStage& G
 // traceBack / traceForward (fluid-advection.wgsl:67-75) from `p` with centre velocity `cv`.
 // G and V: the velocity and its stage (on the velocity lattice), or no stage.
 template <int SS>
-FP_DEV float3 smokeTrace(const SimParams& P, const Home& H, const Stage<SS>& G, const Field& V, const float* p, float3 cv,
-                         float sign) {
-  float3 vm = velocityAt(*P.vview, H, G, V, p[0] + sign * 0.5f * P.dt * cv.x, p[1] + sign * 0.5f * P.dt * cv.y,
+FP_DEV float3 smokeTrace(const SimParams& P, const Home& H, const Lat& VL, const Stage<SS>& G, const Field& V,
+                         const float* p, float3 cv, float sign) {
+  float3 vm = velocityAt(*P.vview, H, VL, G, V, p[0] + sign * 0.5f * P.dt * cv.x, p[1] + sign * 0.5f * P.dt * cv.y,
                          p[2] + sign * 0.5f * P.dt * cv.z);
   return make_float3(p[0] + sign * P.dt * vm.x, p[1] + sign * P.dt * vm.y, p[2] + sign * P.dt * vm.z);
 }
@@ -1437,18 +1550,20 @@ __global__ void __launch_bounds__(VSTAGED ? 256 : SMOKE_THREADS, VSTAGED ? 3 : 8
     const float sp = P.h * (float)P.smokeDiv, invSp = 1.f / sp;
     const bool half = P.scalarHalf != 0;
     const TransportStage<VSTAGED> G = velocityStageIf<VSTAGED>(*P.vview, H);
-    Field V{P.vel, 3, VSTAGED ? smem : nullptr};
-    SmokeStage GS = stageSmoke(P, H, VSTAGED && P.smokeShift == 3, smem + 3 * G.S3, P.smk, half);
-    if (VSTAGED) {
-      stageField(*P.vview, H, G, smem, P.vel, 3);
+    float* st = smem + STAGE_PAD;
+    Field V{P.vel, 3, VSTAGED ? st : nullptr};
+    const Lat VL = latOf(*P.vview);
+    SmokeStage GS = stageSmoke(P, H, VSTAGED && P.smokeShift == 3, st + 3 * G.S3, P.smk, half);
+    if constexpr (VSTAGED) {
+      stageField<3>(H, 3, CELLS, G, st, P.vel, 3);
       stageWait();
     }
     for (int c = threadIdx.x; c < P.smokeCells; c += blockDim.x) {
       SmokeCell s = smokeCellOf(P, H, c);
       float density = 0.f;
       if (!solidAt(P, H, s.p[0], s.p[1], s.p[2])) {
-        float3 cv = velocityAt(*P.vview, H, G, V, s.p[0], s.p[1], s.p[2]);
-        float3 dep = smokeTrace(P, H, G, V, s.p, cv, -1.f);
+        float3 cv = velocityAt(*P.vview, H, VL, G, V, s.p[0], s.p[1], s.p[2]);
+        float3 dep = smokeTrace(P, H, VL, G, V, s.p, cv, -1.f);
         density = smokeSampleS(P, H, GS, P.smk, dep.x * invSp, dep.y * invSp, dep.z * invSp, half);
         if (P.maccormack) {
           // The donor block is an integer decision: divided, as the oracle does.
@@ -1510,10 +1625,12 @@ __global__ void __launch_bounds__(VSTAGED ? 256 : SMOKE_THREADS, VSTAGED ? 3 : 8
     const float sp = P.h * (float)d, invSp = 1.f / sp, volume = (float)(d * d * d / 8);
     const bool half = P.scalarHalf != 0;
     const TransportStage<VSTAGED> G = velocityStageIf<VSTAGED>(*P.vview, H);
-    Field V{P.vel, 3, VSTAGED ? smem : nullptr};
-    SmokeStage GS = stageSmoke(P, H, VSTAGED && P.smokeShift == 3, smem + 3 * G.S3, P.smkP, false);
-    if (VSTAGED) {
-      stageField(*P.vview, H, G, smem, P.vel, 3);
+    float* st = smem + STAGE_PAD;
+    Field V{P.vel, 3, VSTAGED ? st : nullptr};
+    const Lat VL = latOf(*P.vview);
+    SmokeStage GS = stageSmoke(P, H, VSTAGED && P.smokeShift == 3, st + 3 * G.S3, P.smkP, false);
+    if constexpr (VSTAGED) {
+      stageField<3>(H, 3, CELLS, G, st, P.vel, 3);
       stageWait();
     }
     uint32_t busy = 0;
@@ -1521,14 +1638,14 @@ __global__ void __launch_bounds__(VSTAGED ? 256 : SMOKE_THREADS, VSTAGED ? 3 : 8
       SmokeCell s = smokeCellOf(P, H, c);
       float density = 0.f;
       if (!solidAt(P, H, s.p[0], s.p[1], s.p[2])) {
-        float3 cv = velocityAt(*P.vview, H, G, V, s.p[0], s.p[1], s.p[2]);
+        float3 cv = velocityAt(*P.vview, H, VL, G, V, s.p[0], s.p[1], s.p[2]);
         const float predictor = P.smkP[slot * SN + c];
         float bounded = predictor;
         if (P.maccormack) {
           const float lo = P.smkB[(slot * 2 + 0) * SN + c], hi = P.smkB[(slot * 2 + 1) * SN + c];
           if (lo != hi || predictor != lo) {
             const float original = ldHalf(P.smk, slot * SN + c, half);
-            float3 fwd = smokeTrace(P, H, G, V, s.p, cv, 1.f);
+            float3 fwd = smokeTrace(P, H, VL, G, V, s.p, cv, 1.f);
             float reversed = smokeSampleS(P, H, GS, P.smkP, fwd.x * invSp, fwd.y * invSp, fwd.z * invSp, false);
             float corrected = predictor + 0.5f * (original - reversed);
             bounded = (corrected < lo || corrected > hi) ? predictor : corrected;
@@ -1581,7 +1698,7 @@ __global__ void __launch_bounds__(VSTAGED ? 256 : SMOKE_THREADS, VSTAGED ? 3 : 8
 // Staged kernels for 8^3 bricks: `channels` staged fields over (8 + 2 HALO)^3 cells.
 static size_t stagedBytes(int channels) {
   const int S = 8 + 2 * HALO;
-  return (size_t)channels * S * S * S * sizeof(float);
+  return ((size_t)channels * S * S * S + 4) * sizeof(float);  // and STAGE_PAD, to 16 bytes
 }
 // The velocity lattice 8^3 a brick and the smoke grid 8^3 or finer: the staged forms.
 static bool smokeStaged(int B, int vd, int sd) { return B == CUBE * vd && B / sd >= CUBE; }
@@ -1643,7 +1760,7 @@ void fp_launch_evolve(const FpBatch& bt, int B, int vd, int sms, cudaStream_t st
 }
 void fp_launch_curl(const FpBatch& bt, int B, int vd, int sms, cudaStream_t st) {
   if (B == 8 && vd == 1)  // staged: 8^3 bricks, one lattice
-    k_curl<true><<<sms * 6, THREADS, 3 * 10 * 10 * 10 * sizeof(float), st>>>(bt);
+    k_curl<true><<<sms * 6, THREADS, stagedBytes(3), st>>>(bt);
   else
     k_curl<false><<<sms * 6, THREADS, 0, st>>>(bt);
 }
