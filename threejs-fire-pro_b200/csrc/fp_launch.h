@@ -44,6 +44,12 @@ void fp_launch_topology(const FpBatch& bt, bool anyAll, int sms, cudaStream_t st
 void fp_launch_relax(const FpBatch& bt, const MgSel& S, bool tiles, int B, int sms, cudaStream_t st);
 void fp_launch_restrict(const FpBatch& bt, const MgSel& S, bool tiles, int B, int sms, cudaStream_t st);
 void fp_launch_prolong(const FpBatch& bt, const MgSel& S, bool tiles, int B, int sms, cudaStream_t st);
+// Jacobi sweeps several a launch, on the levels fp_sweeps_fused names (B velocity cells a brick):
+// S.pin -> S.pout, the level's other buffer. Down: two sweeps, and the restriction of the result into
+// S.coarse (the level below's right-hand side) and S.cfirst (its first iterate); up: three sweeps.
+bool fp_sweeps_fused(int level, int B);
+void fp_launch_sweeps_down(const FpBatch& bt, const MgSel& S, int B, int sms, cudaStream_t st);
+void fp_launch_sweeps_up(const FpBatch& bt, const MgSel& S, int B, int sms, cudaStream_t st);
 // The bottom level's iterations, a CTA per simulation.
 void fp_launch_bottom(const FpBatch& bt, const MgSel& S, int iterations, int sms, cudaStream_t st);
 // The V-cycle from the second tile level down in one CTA per simulation (k_coarse): S.level is

@@ -485,6 +485,283 @@ FP_DEV Home enterTile(const SimParams& P, int t, int4 rec) {
   return H;
 }
 
+// Several Jacobi sweeps of a level in one launch: a CTA stages a box of values three cells beyond what
+// it owns, and sweeps it there, each sweep a cell less far out, until the last covers its own cells.
+// The cells of the rim are swept by their own CTA too, with the same arithmetic from the same values
+// (each sweep's result rounded as the level stores it), so all agree. The result goes to the level's
+// other buffer, since the neighbours read this one.
+//   DOWN   two sweeps (written: prolongation adds to them) and the restriction of the result
+//   UP     three sweeps
+// A sweep alone is a launch that waits for its work list, its brick's neighbours and one stage: 4 to
+// 5 us however small the level, 24 us at the finest level of 3.1k bricks, most of it latency.
+enum Sweeps { DOWN = 0, UP = 1 };
+// A staged cell's flags: 0 for no unknown (its value becomes zero), else one of
+constexpr uint8_t RIM_OPEN = 0x80;   // an unknown, not solid: the sweeps update it (bits 0-5: its open sides)
+constexpr uint8_t RIM_KEEP = 0x40;   // no part of the solve this step: its value stays
+constexpr uint8_t RIM_SOLID = 0x01;  // an unknown that is solid: zero too
+
+// The shapes: OWN cells a side, pieces of 4 values (16 bytes, or 8 in BF16) a row: one before, one
+// after, so that every piece lies in one owner's row.
+template <int OWN>
+struct Rim {
+  static constexpr int R = 3, S = OWN + 2 * R;       // the box of values
+  static constexpr int PIECES = OWN / 4 + 2, P = OWN == 8 ? 20 : 12;  // a row's pieces; its pitch (bank spread)
+  static constexpr int X0 = 4 - R;                   // the box's first cell in a row
+  static constexpr int C = OWN + 4;                  // the box the first sweep covers
+  static constexpr int THREADS = OWN == 8 ? 256 : 128;
+  static constexpr int VALUES = S * S * P, SWEPT = C * C * P, FLAGS = C * C * P;
+  static constexpr size_t SMEM = (VALUES + 2 * SWEPT) * sizeof(float) + FLAGS;
+};
+
+// Four values of a level from index a.
+FP_DEV float4 ld4(const float* p, long a, bool narrow) {
+  if (!narrow) return *reinterpret_cast<const float4*>(p + a);
+  const __nv_bfloat162* q = reinterpret_cast<const __nv_bfloat162*>(reinterpret_cast<const __nv_bfloat16*>(p) + a);
+  const float2 u = __bfloat1622float2(q[0]), v = __bfloat1622float2(q[1]);
+  return make_float4(u.x, u.y, v.x, v.y);
+}
+
+// Fill the stage of the box of an owner of OWN^3 cells whose 27 neighbours' storage is nbr[] (their
+// slots, -1 none): values from `src`, right-hand sides, and flags from `topo`, `open(n, low, cell)`
+// (whether cell `cell` of neighbour n, on its low faces on the axes of bits `low`, is an unknown) and
+// `keep(n)` (whether n is no part of the solve this step).
+template <int OWN, class Open, class Keep>
+FP_DEV void stageRim(const int* nbr, const float* src, bool srcN, const float* rhs, bool rhsN, const uint8_t* topo,
+                     float* val, float* rh, uint8_t* fl, Open open, Keep keep) {
+  using K = Rim<OWN>;
+  constexpr int M = OWN - 1, CELLS = OWN * OWN * OWN;
+  for (int i = threadIdx.x; i < K::S * K::S * K::PIECES; i += K::THREADS) {
+    const int piece = i % K::PIECES, row = i / K::PIECES, ry = row % K::S, rz = row / K::S;
+    const int y = ry - K::R, z = rz - K::R;
+    const int dx = piece == 0 ? -1 : (piece == K::PIECES - 1 ? 1 : 0), dy = y < 0 ? -1 : (y >= OWN ? 1 : 0),
+              dz = z < 0 ? -1 : (z >= OWN ? 1 : 0);
+    const int n = nbrIndex(dx, dy, dz), s = nbr[n];
+    const int cx = piece == 0 ? OWN - 4 : (dx > 0 ? 0 : (piece - 1) * 4);
+    const long at = (long)s * CELLS + ((z & M) * OWN + (y & M)) * OWN + cx;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (s >= 0) v = ld4(src, at, srcN);
+    *reinterpret_cast<float4*>(val + (rz * K::S + ry) * K::P + piece * 4) = v;
+    if (ry < 1 || ry > K::C || rz < 1 || rz > K::C) continue;
+    // The box of the first sweep: a cell less on every side.
+    const int o = ((rz - 1) * K::C + (ry - 1)) * K::P + piece * 4;
+    float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+    uchar4 f = make_uchar4(0, 0, 0, 0);
+    if (s >= 0) {
+      r = ld4(rhs, at, rhsN);
+      const uchar4 t = *reinterpret_cast<const uchar4*>(topo + at);
+      const unsigned low = ((y & M) == 0 ? 2u : 0u) | ((z & M) == 0 ? 4u : 0u);
+      if (keep(n)) {
+        f = make_uchar4(RIM_KEEP, RIM_KEEP, RIM_KEEP, RIM_KEEP);
+      } else {
+        const int cell = ((z & M) * OWN + (y & M)) * OWN + cx;
+        // The piece before the row starts on no low face that a sweep reaches (OWN > R).
+        const unsigned edge = (cx == 0 && dx >= 0) ? low | 1u : low;
+        auto flag = [](uint8_t t, bool on) {
+          return (uint8_t)(!on ? 0u : ((t & FP_STORED_SOLID) ? RIM_SOLID : (RIM_OPEN | (t & 63u))));
+        };
+        f = make_uchar4(flag(t.x, open(n, edge, cell)), flag(t.y, open(n, low, cell + 1)),
+                        flag(t.z, open(n, low, cell + 2)), flag(t.w, open(n, low, cell + 3)));
+      }
+    }
+    *reinterpret_cast<float4*>(rh + o) = r;
+    *reinterpret_cast<uchar4*>(fl + o) = f;
+  }
+  __syncthreads();
+}
+
+// One sweep over the box `E` cells a side around the owner's (E = OWN + 2 rim): `get` and `put` are
+// given a cell's place from the box's first cell on each axis.
+template <int OWN, int E, class Put>
+FP_DEV void sweepBox(const float* in, int inS, int inOff, const float* rh, const uint8_t* fl, bool narrow, Put put) {
+  using K = Rim<OWN>;
+  constexpr int W = (K::C - E) / 2;  // the sweep's box starts this far into the first sweep's
+  for (int i = threadIdx.x; i < E * E * E; i += K::THREADS) {
+    const int x = i % E, y = i / E % E, z = i / (E * E);
+    const int o = ((z + W) * K::C + y + W) * K::P + x + W + K::X0 + 1;  // in the first sweep's box
+    const int c = ((z + W + inOff) * inS + y + W + inOff) * K::P + x + W + K::X0 + 1;  // in the values read
+    const uint32_t f = fl[o];
+    float v = 0.f;
+    if (f & RIM_OPEN) {
+      const int sy = K::P, sz = inS * K::P;
+      const float v0 = (f & 1u) ? in[c + 1] : 0.f, v1 = (f & 2u) ? in[c - 1] : 0.f;
+      const float v2 = (f & 4u) ? in[c + sy] : 0.f, v3 = (f & 8u) ? in[c - sy] : 0.f;
+      const float v4 = (f & 16u) ? in[c + sz] : 0.f, v5 = (f & 32u) ? in[c - sz] : 0.f;
+      const float sum = (v0 + v1) + (v2 + v3) + (v4 + v5);
+      const float cand = (sum - rh[o]) / fmaxf(diagOf(f & 63u), 1e-12f);
+      v = mixf(in[c], cand, 0.8f);
+      if (narrow) v = __bfloat162float(__float2bfloat16_rn(v));
+    } else if (f & RIM_KEEP) {
+      v = in[c];
+    }
+    put(x, y, z, o, v);
+  }
+}
+
+// The sweeps of a staged box. `own(index in the owner's cells, value)` takes the last sweep's values;
+// DOWN's restriction takes them from shared memory (the box of the second sweep) through `coarse`.
+template <int OWN, int KIND, class Own>
+FP_DEV void sweepAll(float* val, float* rh, const uint8_t* fl, float* other, bool narrow, Own own) {
+  using K = Rim<OWN>;
+  // The first sweep: from the staged values to `other`.
+  sweepBox<OWN, K::C>(val, K::S, 1, rh, fl, narrow, [&](int, int, int, int o, float v) { other[o] = v; });
+  __syncthreads();
+  // The second: back into the staged values' memory, laid out as the first sweep's box.
+  sweepBox<OWN, OWN + 2>(other, K::C, 0, rh, fl, narrow, [&](int x, int y, int z, int o, float v) {
+    val[o] = v;
+    if (KIND == DOWN && x >= 1 && x <= OWN && y >= 1 && y <= OWN && z >= 1 && z <= OWN)
+      own(((z - 1) * OWN + y - 1) * OWN + x - 1, v);
+  });
+  __syncthreads();
+  if (KIND == UP)
+    sweepBox<OWN, OWN>(val, K::C, 0, rh, fl, narrow,
+                       [&](int x, int y, int z, int, float v) { own((z * OWN + y) * OWN + x, v); });
+}
+// The restriction of coarse cell q (of the owner's (OWN / 2)^3) after DOWN's sweeps.
+template <int OWN>
+FP_DEV float restrictRim(const float* val, const float* rh, const uint8_t* fl, int q, bool& every) {
+  using K = Rim<OWN>;
+  constexpr int H = OWN / 2;
+  const int cx = q % H, cy = q / H % H, cz = q / (H * H);
+  float residual = 0.f;
+  every = true;
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    const int x = cx * 2 + (k & 1), y = cy * 2 + ((k >> 1) & 1), z = cz * 2 + (k >> 2);
+    const int o = ((z + 2) * K::C + y + 2) * K::P + x + 2 + K::X0 + 1;
+    const uint32_t f = fl[o];
+    every = every && f != 0u;
+    if (f & RIM_OPEN) {
+      const float v0 = (f & 1u) ? val[o + 1] : 0.f, v1 = (f & 2u) ? val[o - 1] : 0.f;
+      const float v2 = (f & 4u) ? val[o + K::P] : 0.f, v3 = (f & 8u) ? val[o - K::P] : 0.f;
+      const float v4 = (f & 16u) ? val[o + K::C * K::P] : 0.f, v5 = (f & 32u) ? val[o - K::C * K::P] : 0.f;
+      const float sum = (v0 + v1) + (v2 + v3) + (v4 + v5);
+      residual += rh[o] - (sum - diagOf(f & 63u) * val[o]);
+    }
+  }
+  return residual * 0.5f;
+}
+
+// The shared memory of a box, carved.
+template <int OWN>
+struct RimStage {
+  float *val, *rh, *other;
+  uint8_t* fl;
+  FP_DEV explicit RimStage(float* smem) {
+    using K = Rim<OWN>;
+    val = smem;
+    rh = val + K::VALUES;
+    other = rh + K::SWEPT;
+    fl = reinterpret_cast<uint8_t*>(other + K::SWEPT);
+  }
+};
+// What DOWN writes of coarse cell `out` of the level below from restriction r.
+FP_DEV void storeCoarse(const SimParams& P, const Args& A, long out, float r, bool every) {
+  stBf(const_cast<float*>(A.coarse), out, r, A.coarseN);  // the coarse right-hand side
+  float first = 0.f;
+  if (every) {
+    const uint32_t f = expandFlags(P.topo[A.level + 1][out]);
+    if (!(f & SOLIDF)) first = mixf(0.f, (0.f - r) / fmaxf(diagOf(f), 1e-12f), 0.8f);
+  }
+  stBf(A.cfirst, out, first, A.cfirstN);
+}
+
+// Brick levels of OWN^3 cells a brick (8 or 4), a CTA a brick. A.pin: the level's values; A.pout: the
+// result, the other buffer; DOWN: A.coarse the coarse right-hand side, A.cfirst its first iterate.
+template <int OWN, int KIND>
+__global__ void __launch_bounds__(Rim<OWN>::THREADS) k_sweep_bricks(FpBatch bt, MgSel Sl) {
+  __shared__ int nslot[27];
+  __shared__ uint32_t okBits;
+  extern __shared__ __align__(16) float rimSmem[];
+  const RimStage<OWN> st(rimSmem);
+  const int t = threadIdx.x;
+  const uint32_t total = workTotal(bt, FP_WORK_ACTIVE);
+  for (uint32_t item = blockIdx.x; item < total; item += gridDim.x) {
+    uint32_t i;
+    const SimParams& P = *workSim(bt, FP_WORK_ACTIVE, item, i).vview;
+    const Args A = resolve(P, Sl);
+    if (A.skip) continue;  // the same for the whole CTA
+    const uint32_t id = P.active[i];
+    if (!homeOk(P, id)) continue;  // the bounds-checked build only
+    const Home H = homeOf(P, id, nslot);
+    __syncthreads();  // the previous brick's stage has been read
+    if (t < 32) {
+      bool ok = false;
+      if (t < 27) {
+        const int s = checkSlot(P, FP_SITE_RECORD, entryPage(P.records[(size_t)id * FP_RECORD_WORDS + t]));
+        nslot[t] = s;
+        ok = s >= 0 || (P.ground && H.by + (t / 3) % 3 - 1 < 0);
+      }
+      const uint32_t b = __ballot_sync(0xffffffffu, ok);
+      if (t == 0) okBits = b;
+    }
+    __syncthreads();
+    // activeCell: a cell is an unknown when its brick and those before it on the axes of its low
+    // faces compute (below the ground none are asked).
+    const uint32_t ok = okBits;
+    auto open = [&](int n, unsigned low, int) {
+      uint32_t need = 1u << n;
+      if (low & 1u) need |= need >> 1;
+      if (low & 2u) need |= need >> 3;
+      if (low & 4u) need |= need >> 9;
+      return (ok & need) == need;
+    };
+    stageRim<OWN>(nslot, A.pin, A.pinN, A.rhs, A.rhsN, P.topo[A.level], st.val, st.rh, st.fl, open, [](int) { return false; });
+    const long slot = nslot[13];
+    constexpr int CELLS = OWN * OWN * OWN;
+    sweepAll<OWN, KIND>(st.val, st.rh, st.fl, st.other, A.poutN, [&](int c, float v) { stBf(A.pout, slot * CELLS + c, v, A.poutN); });
+    if (KIND == DOWN)
+      for (int q = t; q < CELLS / 8; q += Rim<OWN>::THREADS) {
+        bool every;
+        const float r = restrictRim<OWN>(st.val, st.rh, st.fl, q, every);
+        storeCoarse(P, A, slot * (CELLS / 8) + q, r, every);
+      }
+  }
+}
+
+// The first tile level (4^3 cells a tile, a cell a brick), a CTA a live tile. The cells of neighbour
+// tiles that are not live are no part of the solve.
+template <int KIND>
+__global__ void __launch_bounds__(Rim<4>::THREADS) k_sweep_tiles(FpBatch bt, MgSel Sl) {
+  __shared__ int nbr[27];
+  __shared__ uint64_t masks[27];
+  __shared__ uint32_t liveBits;
+  extern __shared__ __align__(16) float rimSmem[];
+  const RimStage<4> st(rimSmem);
+  const int t = threadIdx.x;
+  const uint32_t total = workTotal(bt, FP_WORK_TILES);
+  for (uint32_t item = blockIdx.x; item < total; item += gridDim.x) {
+    uint32_t local;
+    const SimParams& P = *workSim(bt, FP_WORK_TILES, item, local).vview;
+    const Args A = resolve(P, Sl);
+    if (A.skip) continue;  // the same for the whole CTA
+    const int tile = P.liveTiles[local];
+    if (__ldg(&P.tileRec[tile]).w == 0) continue;
+    __syncthreads();  // the previous tile's stage has been read
+    if (t < 32) {
+      bool live = false;
+      if (t < 27) {
+        const int n = checkTile(P, FP_SITE_TILE_NBR, __ldg(&P.tileNbr[(size_t)tile * 27 + t]));
+        nbr[t] = n;
+        live = n >= 0 && P.tileIndex[n] >= 0 && __ldg(&P.tileRec[n]).w != 0;
+        masks[t] = live ? P.tileMask[n] : 0ull;
+      }
+      const uint32_t b = __ballot_sync(0xffffffffu, live);
+      if (t == 0) liveBits = b;
+    }
+    __syncthreads();
+    const uint32_t live = liveBits;
+    stageRim<4>(nbr, A.pin, A.pinN, A.rhs, A.rhsN, P.topo[A.level], st.val, st.rh, st.fl,
+                [&](int n, unsigned, int cell) { return ((masks[n] >> cell) & 1ull) != 0ull; },
+                [&](int n) { return ((live >> n) & 1u) == 0u; });
+    sweepAll<4, KIND>(st.val, st.rh, st.fl, st.other, A.poutN, [&](int c, float v) { stBf(A.pout, (long)tile * 64 + c, v, A.poutN); });
+    if (KIND == DOWN && t < 8) {
+      bool every;
+      const float r = restrictRim<4>(st.val, st.rh, st.fl, t, every);
+      storeCoarse(P, A, (long)tile * 8 + t, r, every);
+    }
+  }
+}
+
 // Every cell of `A.level` (a tile level of CELLS cells a tile) in every tile: a thread per
 // cell, 64 / CELLS tiles per CTA; no barriers, so threads of dead tiles just move on.
 template <int OP, int CELLS>
@@ -1408,6 +1685,34 @@ static void tileStagedLaunch(const FpBatch& bt, const MgSel& S, int sms, cudaStr
   k_level_tiles_staged<OP, TS><<<sms * tileStagedCtas<OP, TS>(), 256, TileStaged<OP, TS>::SMEM, st>>>(bt, S);
 }
 
+// Resident CTAs per SM of each sweep kernel, from the occupancy calculator.
+template <int OWN, int KIND, bool TILES>
+static int& sweepCtas() {
+  static int n = 4;
+  return n;
+}
+template <int OWN, int KIND, bool TILES>
+static void configureSweeps() {
+  using K = Rim<OWN>;
+  int n = 0;
+  cudaError_t e;
+  if constexpr (TILES)
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sweep_tiles<KIND>, K::THREADS, K::SMEM);
+  else
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sweep_bricks<OWN, KIND>, K::THREADS, K::SMEM);
+  sweepCtas<OWN, KIND, TILES>() = e == cudaSuccess && n > 0 ? n : 4;
+}
+template <int OWN, int KIND, bool TILES>
+static void sweepLaunch(const FpBatch& bt, const MgSel& S, int sms, cudaStream_t st) {
+  using K = Rim<OWN>;
+  static_assert(K::SMEM <= 48 * 1024, "within the limit a kernel needs no attribute for");
+  const int grid = sms * sweepCtas<OWN, KIND, TILES>();
+  if constexpr (TILES)
+    k_sweep_tiles<KIND><<<grid, K::THREADS, K::SMEM, st>>>(bt, S);
+  else
+    k_sweep_bricks<OWN, KIND><<<grid, K::THREADS, K::SMEM, st>>>(bt, S);
+}
+
 // Resident CTAs per SM of each staged instantiation, from the occupancy calculator.
 template <int OP, int SB>
 static int& stagedCtas() {
@@ -1440,6 +1745,12 @@ void fp_mg_configure(int B) {
   configureStaged<PROLONG, 4>();
   configureStaged<PROLONG, 2>();
   configureStaged<PROLONG, 1>();
+  configureSweeps<8, DOWN, false>();
+  configureSweeps<8, UP, false>();
+  configureSweeps<4, DOWN, false>();
+  configureSweeps<4, UP, false>();
+  configureSweeps<4, DOWN, true>();
+  configureSweeps<4, UP, true>();
   configureTileStaged<RELAX, 4>();
   configureTileStaged<RESTRICT, 4>();
   configureTileStaged<PROLONG, 2>();
@@ -1526,6 +1837,28 @@ static void levelLaunch(const FpBatch& bt, const MgSel& S, bool tiles, int B, in
 }
 void fp_launch_relax(const FpBatch& bt, const MgSel& S, bool tiles, int B, int sms, cudaStream_t st) {
   levelLaunch<RELAX>(bt, S, tiles, B, sms, st);
+}
+// The levels whose sweeps run several a launch: brick levels of 8^3 and 4^3 cells a brick, and the
+// first tile level. (A brick's 2^3 cells have no three-cell rim in their neighbours; at 16^3 and 32^3
+// a box does not fit several to an SM, and a sweep is no longer mostly latency.)
+bool fp_sweeps_fused(int level, int B) {
+  const int bl = log2i(B), side = level < bl ? B >> level : 0;
+  return side == 8 || side == 4 || level == bl;
+}
+template <int KIND>
+static void sweepsLaunch(const FpBatch& bt, const MgSel& S, int B, int sms, cudaStream_t st) {
+  if (S.level == log2i(B))
+    sweepLaunch<4, KIND, true>(bt, S, sms, st);
+  else if (B >> S.level == 8)
+    sweepLaunch<8, KIND, false>(bt, S, sms, st);
+  else
+    sweepLaunch<4, KIND, false>(bt, S, sms, st);
+}
+void fp_launch_sweeps_down(const FpBatch& bt, const MgSel& S, int B, int sms, cudaStream_t st) {
+  sweepsLaunch<DOWN>(bt, S, B, sms, st);
+}
+void fp_launch_sweeps_up(const FpBatch& bt, const MgSel& S, int B, int sms, cudaStream_t st) {
+  sweepsLaunch<UP>(bt, S, B, sms, st);
 }
 void fp_launch_restrict(const FpBatch& bt, const MgSel& S, bool tiles, int B, int sms, cudaStream_t st) {
   levelLaunch<RESTRICT>(bt, S, tiles, B, sms, st);

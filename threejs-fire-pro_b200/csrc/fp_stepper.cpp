@@ -381,18 +381,33 @@ void Stepper::vcycle(int level, int cur[], uint64_t& launches) {
       cur[level] = 1 - cur[level];
     }
   };
-  if (level > 0) relax(2);
-  int coarse = level + 1;
-  MgSel R{coarse, level == 0 ? rhs0Sel_ : sel(level, 2), sel(level, cur[level]), -1, sel(coarse, 2), sel(coarse, 1), cycle_};
-  fp_launch_restrict(batch(), R, coarse >= brickLevels_, B_ / vd_, sms_, stream_);
-  launches++;
+  const bool fused = fp_sweeps_fused(level, B_ / vd_);
+  const int rhs = level == 0 ? rhs0Sel_ : sel(level, 2), coarse = level + 1;
+  if (level > 0 && fused) {
+    MgSel D{level, rhs, sel(level, cur[level]), sel(coarse, 2), sel(level, 1 - cur[level]), sel(coarse, 1), cycle_, 0};
+    fp_launch_sweeps_down(batch(), D, B_ / vd_, sms_, stream_);
+    launches++;
+    cur[level] = 1 - cur[level];
+  } else {
+    if (level > 0) relax(2);
+    MgSel R{coarse, rhs, sel(level, cur[level]), -1, sel(coarse, 2), sel(coarse, 1), cycle_, 0};
+    fp_launch_restrict(batch(), R, coarse >= brickLevels_, B_ / vd_, sms_, stream_);
+    launches++;
+  }
   cur[coarse] = 1;
   vcycle(coarse, cur, launches);
-  MgSel Pr{level, -1, sel(level, cur[level]), sel(coarse, cur[coarse]), sel(level, 1 - cur[level]), -1, cycle_};
+  MgSel Pr{level, -1, sel(level, cur[level]), sel(coarse, cur[coarse]), sel(level, 1 - cur[level]), -1, cycle_, 0};
   fp_launch_prolong(batch(), Pr, tiles, B_ / vd_, sms_, stream_);
   launches++;
   cur[level] = 1 - cur[level];
-  relax(3);
+  if (fused) {
+    MgSel U{level, rhs, sel(level, cur[level]), -1, sel(level, 1 - cur[level]), -1, cycle_, 0};
+    fp_launch_sweeps_up(batch(), U, B_ / vd_, sms_, stream_);
+    launches++;
+    cur[level] = 1 - cur[level];
+  } else {
+    relax(3);
+  }
 }
 
 // One V-cycle of the red-black schedule (fp_solver_schedule) from `level` down: every level in
@@ -587,7 +602,7 @@ void Stepper::enqueue(bool solidsFresh, bool solidsAll, bool topoAll, bool curl,
     latest = 0;
   } else {
     // Up to `vcycles` V-cycles. Each leaves the finest level's result in the buffer it started
-    // from (four flips: prolongation and three sweeps), so a simulation that converged and
+    // from (an even number of flips: prolongation and its sweeps), so a simulation that converged and
     // skips the later cycles ends in the same buffer. After each cycle, when measured, the
     // FP64 residual decides convergence.
     for (int c = 0; c < vcycles; c++) {
