@@ -108,6 +108,7 @@ class Engine {
   bool solidsAll() const { return solidsStale_; }
   bool topoAll() const { return geometryDirty_ || schedule_.topology != 0; }
   int capacity() const { return capacity_; }
+  uint32_t activeBricks() const { return activeBricks_; }
   int liveTiles() const { return (int)liveTiles_.size(); }
   int smokeDivisor() const { return smokeDiv_; }
   int velocityDivisor() const { return vd_; }
@@ -353,6 +354,15 @@ class Stepper {
                uint64_t& launches);
   int cycle_ = 0;             // the V-cycle being enqueued
   bool fusedCoarse_ = false;  // the V-cycle below the first tile level runs as k_coarse
+  // From about this many computing bricks in a launch the finest level's restriction and the brick
+  // levels' prolongation run apart from the sweeps: over a wide rim they do their work several times
+  // over (finest level up, us: 98 together, 87 apart on 3.1k bricks; 12 and 17 on 90).
+  static constexpr uint64_t MANY_BRICKS = 1000;
+  bool manyBricks_ = false;
+  bool coarseSmall_ = false;  // k_coarse in its small form (fp_coarse_small)
+  bool single_ = false;       // one simulation
+  bool chain_ = false;        // the last multigrid launch was a leg, which the next may overlap
+  bool evenFlips_ = false;    // several V-cycles: the finest level ends in the buffer it started from
   bool anySmoke_ = false;     // a simulation of the launch keeps coarse smoke
   int smokeDiv_ = 0;          // the finest coarse smoke grid's divisor among them (0: none)
   fp_solver_schedule schedule_{};  // the launch's pressure-solve schedule (its simulations')

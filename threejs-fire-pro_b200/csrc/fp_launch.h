@@ -38,25 +38,32 @@ struct MgSel {
   // Relaxation: 0 weighted Jacobi (pin -> pout); 1 or 2 red-black Gauss-Seidel in place
   // (pin = pout) of the cells with x + y + z even (1) or odd (2).
   int colour;
+  // Launched while the kernel before it on the stream, a leg too, may still run.
+  bool overlap;
 };
 inline int fp_mg_sel(int level, int which) { return level * 4 + which; }
 void fp_launch_topology(const FpBatch& bt, bool anyAll, int sms, cudaStream_t st);
 void fp_launch_relax(const FpBatch& bt, const MgSel& S, bool tiles, int B, int sms, cudaStream_t st);
 void fp_launch_restrict(const FpBatch& bt, const MgSel& S, bool tiles, int B, int sms, cudaStream_t st);
 void fp_launch_prolong(const FpBatch& bt, const MgSel& S, bool tiles, int B, int sms, cudaStream_t st);
-// Jacobi sweeps several a launch, on the levels fp_sweeps_fused names (B velocity cells a brick):
-// S.pin -> S.pout, the level's other buffer. Down: two sweeps, and the restriction of the result into
-// S.coarse (the level below's right-hand side) and S.cfirst (its first iterate); up: three sweeps.
-bool fp_sweeps_fused(int level, int B);
-void fp_launch_sweeps_down(const FpBatch& bt, const MgSel& S, int B, int sms, cudaStream_t st);
-void fp_launch_sweeps_up(const FpBatch& bt, const MgSel& S, int B, int sms, cudaStream_t st);
+// A leg of the Jacobi V-cycle on a level in one launch, on the levels fp_legs_fused names (B velocity
+// cells a brick). Down: two sweeps from S.pin to S.pout, the level's other buffer (none at the finest
+// level, which starts from the first iterate as it is), and the restriction of the result into
+// S.coarse (the level below's right-hand side) and S.cfirst (its first iterate). Up: prolongation
+// from S.coarse (the level below; -1: none, S.pin is prolongated already) and three sweeps, S.pin to
+// S.pout.
+bool fp_legs_fused(int level, int B);
+bool fp_leg_per_brick(int level, int B);  // a CTA a brick (the others a CTA a tile)
+void fp_launch_leg_down(const FpBatch& bt, const MgSel& S, int B, int sms, cudaStream_t st);
+void fp_launch_leg_up(const FpBatch& bt, const MgSel& S, int B, int sms, cudaStream_t st);
 // The bottom level's iterations, a CTA per simulation.
 void fp_launch_bottom(const FpBatch& bt, const MgSel& S, int iterations, int sms, cudaStream_t st);
 // The V-cycle from the second tile level down in one CTA per simulation (k_coarse): S.level is
 // that level, S.rhs its right-hand side, S.pin its first iterate, S.pout its result, S.cfirst
 // the bottom's result. Usable when every simulation's live tiles fit (fp_coarse_fits).
 bool fp_coarse_fits(int liveTiles);
-void fp_launch_coarse(const FpBatch& bt, const MgSel& S, int iterations, int sms, cudaStream_t st);
+bool fp_coarse_small(int liveTiles);
+void fp_launch_coarse(const FpBatch& bt, const MgSel& S, int iterations, bool small, int sims, int sms, cudaStream_t st);
 // After V-cycle `cycle`: the FP64 sums of squares of the finest level's residual (and, after
 // the first, of its right-hand side) over the unknowns, then each simulation's convergence
 // decision. A simulation that converged skips the later cycles.

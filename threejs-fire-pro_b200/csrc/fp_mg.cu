@@ -485,176 +485,227 @@ FP_DEV Home enterTile(const SimParams& P, int t, int4 rec) {
   return H;
 }
 
-// Several Jacobi sweeps of a level in one launch: a CTA stages a box of values three cells beyond what
-// it owns, and sweeps it there, each sweep a cell less far out, until the last covers its own cells.
-// The cells of the rim are swept by their own CTA too, with the same arithmetic from the same values
-// (each sweep's result rounded as the level stores it), so all agree. The result goes to the level's
-// other buffer, since the neighbours read this one.
+// The Jacobi V-cycle's work on a level in one launch a leg: a CTA stages a box of values three cells
+// beyond what it owns, and works on it there, each sweep a cell less far out, until the last covers
+// its own cells. The cells of the rim are worked on by their own CTA too, with the same arithmetic
+// from the same values (each step's result rounded as the level stores it), so all agree. The result
+// goes to the level's other buffer, since the neighbours read this one.
+//   REST   the restriction alone (the finest level, whose first iterate the divergence left)
 //   DOWN   two sweeps (written: prolongation adds to them) and the restriction of the result
 //   UP     three sweeps
-// A sweep alone is a launch that waits for its work list, its brick's neighbours and one stage: 4 to
-// 5 us however small the level, 24 us at the finest level of 3.1k bricks, most of it latency.
-enum Sweeps { DOWN = 0, UP = 1 };
+//   PUP    prolongation from the level below, and three sweeps
+// A step alone is a launch that waits for its work list, its brick's neighbours and one stage: 4 to
+// 9 us however small the level, 24 us a sweep at the finest level of 3.1k bricks, most of it latency.
+enum Leg { REST = 0, DOWN = 1, UP = 2, PUP = 3 };
+
+// Legs may be launched while the one before still runs (MgSel::overlap): a leg lets its successor start
+// at once, and waits for its predecessor where it first reads what that wrote. What it reads before
+// then (parameters, lists, records, flags) was complete before the first of the legs started, which is
+// launched without overlap. Every thread waits before it ends, so that a leg's end is its
+// predecessors' end too. Without overlap both are nothing.
+FP_DEV void letNextStart() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+FP_DEV void waitForPrevious() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // A staged cell's flags: 0 for no unknown (its value becomes zero), else one of
 constexpr uint8_t RIM_OPEN = 0x80;   // an unknown, not solid: the sweeps update it (bits 0-5: its open sides)
-constexpr uint8_t RIM_KEEP = 0x40;   // no part of the solve this step: its value stays
 constexpr uint8_t RIM_SOLID = 0x01;  // an unknown that is solid: zero too
 
 // The shapes: OWN cells a side, pieces of 4 values (16 bytes, or 8 in BF16) a row: one before, one
 // after, so that every piece lies in one owner's row.
 template <int OWN>
 struct Rim {
-  static constexpr int R = 3, S = OWN + 2 * R;       // the box of values
+  static constexpr int R = 3, S = OWN + 2 * R;       // the box of values and flags
   static constexpr int PIECES = OWN / 4 + 2, P = OWN == 8 ? 20 : 12;  // a row's pieces; its pitch (bank spread)
-  static constexpr int X0 = 4 - R;                   // the box's first cell in a row
-  static constexpr int C = OWN + 4;                  // the box the first sweep covers
+  static constexpr int C = OWN + 4;                  // the box the first sweep covers, and the right-hand sides'
+  static constexpr int H = OWN / 2, G = H + 4;       // the level below: cells a side, and with a rim of two
   static constexpr int THREADS = OWN == 8 ? 256 : 128;
-  static constexpr int VALUES = S * S * P, SWEPT = C * C * P, FLAGS = C * C * P;
-  static constexpr size_t SMEM = (VALUES + 2 * SWEPT) * sizeof(float) + FLAGS;
+  static constexpr int VALUES = S * S * P, SWEPT = C * C * P;
+  static constexpr size_t SMEM = (VALUES + 2 * SWEPT + G * G * G) * sizeof(float) + VALUES;
 };
-
-// Four values of a level from index a.
-FP_DEV float4 ld4(const float* p, long a, bool narrow) {
-  if (!narrow) return *reinterpret_cast<const float4*>(p + a);
-  const __nv_bfloat162* q = reinterpret_cast<const __nv_bfloat162*>(reinterpret_cast<const __nv_bfloat16*>(p) + a);
-  const float2 u = __bfloat1622float2(q[0]), v = __bfloat1622float2(q[1]);
-  return make_float4(u.x, u.y, v.x, v.y);
-}
-
-// Fill the stage of the box of an owner of OWN^3 cells whose 27 neighbours' storage is nbr[] (their
-// slots, -1 none): values from `src`, right-hand sides, and flags from `topo`, `open(n, low, cell)`
-// (whether cell `cell` of neighbour n, on its low faces on the axes of bits `low`, is an unknown) and
-// `keep(n)` (whether n is no part of the solve this step).
-template <int OWN, class Open, class Keep>
-FP_DEV void stageRim(const int* nbr, const float* src, bool srcN, const float* rhs, bool rhsN, const uint8_t* topo,
-                     float* val, float* rh, uint8_t* fl, Open open, Keep keep) {
-  using K = Rim<OWN>;
-  constexpr int M = OWN - 1, CELLS = OWN * OWN * OWN;
-  for (int i = threadIdx.x; i < K::S * K::S * K::PIECES; i += K::THREADS) {
-    const int piece = i % K::PIECES, row = i / K::PIECES, ry = row % K::S, rz = row / K::S;
-    const int y = ry - K::R, z = rz - K::R;
-    const int dx = piece == 0 ? -1 : (piece == K::PIECES - 1 ? 1 : 0), dy = y < 0 ? -1 : (y >= OWN ? 1 : 0),
-              dz = z < 0 ? -1 : (z >= OWN ? 1 : 0);
-    const int n = nbrIndex(dx, dy, dz), s = nbr[n];
-    const int cx = piece == 0 ? OWN - 4 : (dx > 0 ? 0 : (piece - 1) * 4);
-    const long at = (long)s * CELLS + ((z & M) * OWN + (y & M)) * OWN + cx;
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (s >= 0) v = ld4(src, at, srcN);
-    *reinterpret_cast<float4*>(val + (rz * K::S + ry) * K::P + piece * 4) = v;
-    if (ry < 1 || ry > K::C || rz < 1 || rz > K::C) continue;
-    // The box of the first sweep: a cell less on every side.
-    const int o = ((rz - 1) * K::C + (ry - 1)) * K::P + piece * 4;
-    float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
-    uchar4 f = make_uchar4(0, 0, 0, 0);
-    if (s >= 0) {
-      r = ld4(rhs, at, rhsN);
-      const uchar4 t = *reinterpret_cast<const uchar4*>(topo + at);
-      const unsigned low = ((y & M) == 0 ? 2u : 0u) | ((z & M) == 0 ? 4u : 0u);
-      if (keep(n)) {
-        f = make_uchar4(RIM_KEEP, RIM_KEEP, RIM_KEEP, RIM_KEEP);
-      } else {
-        const int cell = ((z & M) * OWN + (y & M)) * OWN + cx;
-        // The piece before the row starts on no low face that a sweep reaches (OWN > R).
-        const unsigned edge = (cx == 0 && dx >= 0) ? low | 1u : low;
-        auto flag = [](uint8_t t, bool on) {
-          return (uint8_t)(!on ? 0u : ((t & FP_STORED_SOLID) ? RIM_SOLID : (RIM_OPEN | (t & 63u))));
-        };
-        f = make_uchar4(flag(t.x, open(n, edge, cell)), flag(t.y, open(n, low, cell + 1)),
-                        flag(t.z, open(n, low, cell + 2)), flag(t.w, open(n, low, cell + 3)));
-      }
-    }
-    *reinterpret_cast<float4*>(rh + o) = r;
-    *reinterpret_cast<uchar4*>(fl + o) = f;
-  }
-  __syncthreads();
-}
-
-// One sweep over the box `E` cells a side around the owner's (E = OWN + 2 rim): `get` and `put` are
-// given a cell's place from the box's first cell on each axis.
-template <int OWN, int E, class Put>
-FP_DEV void sweepBox(const float* in, int inS, int inOff, const float* rh, const uint8_t* fl, bool narrow, Put put) {
-  using K = Rim<OWN>;
-  constexpr int W = (K::C - E) / 2;  // the sweep's box starts this far into the first sweep's
-  for (int i = threadIdx.x; i < E * E * E; i += K::THREADS) {
-    const int x = i % E, y = i / E % E, z = i / (E * E);
-    const int o = ((z + W) * K::C + y + W) * K::P + x + W + K::X0 + 1;  // in the first sweep's box
-    const int c = ((z + W + inOff) * inS + y + W + inOff) * K::P + x + W + K::X0 + 1;  // in the values read
-    const uint32_t f = fl[o];
-    float v = 0.f;
-    if (f & RIM_OPEN) {
-      const int sy = K::P, sz = inS * K::P;
-      const float v0 = (f & 1u) ? in[c + 1] : 0.f, v1 = (f & 2u) ? in[c - 1] : 0.f;
-      const float v2 = (f & 4u) ? in[c + sy] : 0.f, v3 = (f & 8u) ? in[c - sy] : 0.f;
-      const float v4 = (f & 16u) ? in[c + sz] : 0.f, v5 = (f & 32u) ? in[c - sz] : 0.f;
-      const float sum = (v0 + v1) + (v2 + v3) + (v4 + v5);
-      const float cand = (sum - rh[o]) / fmaxf(diagOf(f & 63u), 1e-12f);
-      v = mixf(in[c], cand, 0.8f);
-      if (narrow) v = __bfloat162float(__float2bfloat16_rn(v));
-    } else if (f & RIM_KEEP) {
-      v = in[c];
-    }
-    put(x, y, z, o, v);
-  }
-}
-
-// The sweeps of a staged box. `own(index in the owner's cells, value)` takes the last sweep's values;
-// DOWN's restriction takes them from shared memory (the box of the second sweep) through `coarse`.
-template <int OWN, int KIND, class Own>
-FP_DEV void sweepAll(float* val, float* rh, const uint8_t* fl, float* other, bool narrow, Own own) {
-  using K = Rim<OWN>;
-  // The first sweep: from the staged values to `other`.
-  sweepBox<OWN, K::C>(val, K::S, 1, rh, fl, narrow, [&](int, int, int, int o, float v) { other[o] = v; });
-  __syncthreads();
-  // The second: back into the staged values' memory, laid out as the first sweep's box.
-  sweepBox<OWN, OWN + 2>(other, K::C, 0, rh, fl, narrow, [&](int x, int y, int z, int o, float v) {
-    val[o] = v;
-    if (KIND == DOWN && x >= 1 && x <= OWN && y >= 1 && y <= OWN && z >= 1 && z <= OWN)
-      own(((z - 1) * OWN + y - 1) * OWN + x - 1, v);
-  });
-  __syncthreads();
-  if (KIND == UP)
-    sweepBox<OWN, OWN>(val, K::C, 0, rh, fl, narrow,
-                       [&](int x, int y, int z, int, float v) { own((z * OWN + y) * OWN + x, v); });
-}
-// The restriction of coarse cell q (of the owner's (OWN / 2)^3) after DOWN's sweeps.
-template <int OWN>
-FP_DEV float restrictRim(const float* val, const float* rh, const uint8_t* fl, int q, bool& every) {
-  using K = Rim<OWN>;
-  constexpr int H = OWN / 2;
-  const int cx = q % H, cy = q / H % H, cz = q / (H * H);
-  float residual = 0.f;
-  every = true;
-#pragma unroll
-  for (int k = 0; k < 8; k++) {
-    const int x = cx * 2 + (k & 1), y = cy * 2 + ((k >> 1) & 1), z = cz * 2 + (k >> 2);
-    const int o = ((z + 2) * K::C + y + 2) * K::P + x + 2 + K::X0 + 1;
-    const uint32_t f = fl[o];
-    every = every && f != 0u;
-    if (f & RIM_OPEN) {
-      const float v0 = (f & 1u) ? val[o + 1] : 0.f, v1 = (f & 2u) ? val[o - 1] : 0.f;
-      const float v2 = (f & 4u) ? val[o + K::P] : 0.f, v3 = (f & 8u) ? val[o - K::P] : 0.f;
-      const float v4 = (f & 16u) ? val[o + K::C * K::P] : 0.f, v5 = (f & 32u) ? val[o - K::C * K::P] : 0.f;
-      const float sum = (v0 + v1) + (v2 + v3) + (v4 + v5);
-      residual += rh[o] - (sum - diagOf(f & 63u) * val[o]);
-    }
-  }
-  return residual * 0.5f;
-}
-
 // The shared memory of a box, carved.
 template <int OWN>
 struct RimStage {
-  float *val, *rh, *other;
+  float *val, *rh, *other, *below;
   uint8_t* fl;
   FP_DEV explicit RimStage(float* smem) {
     using K = Rim<OWN>;
     val = smem;
     rh = val + K::VALUES;
     other = rh + K::SWEPT;
-    fl = reinterpret_cast<uint8_t*>(other + K::SWEPT);
+    below = other + K::SWEPT;
+    fl = reinterpret_cast<uint8_t*>(below + K::G * K::G * K::G);
   }
+  // The place of cell (x,y,z), from the owner's first, among the values and flags; among the rest.
+  FP_DEV static int at(int x, int y, int z) { return ((z + 3) * Rim<OWN>::S + y + 3) * Rim<OWN>::P + x + 4; }
+  FP_DEV static int in(int x, int y, int z) { return ((z + 2) * Rim<OWN>::C + y + 2) * Rim<OWN>::P + x + 4; }
 };
-// What DOWN writes of coarse cell `out` of the level below from restriction r.
+
+// Four, or two, values of a level from index a.
+FP_DEV float4 ld4(const float* p, long a, bool narrow) {
+  if (!narrow) return *reinterpret_cast<const float4*>(p + a);
+  const __nv_bfloat162* q = reinterpret_cast<const __nv_bfloat162*>(reinterpret_cast<const __nv_bfloat16*>(p) + a);
+  const float2 u = __bfloat1622float2(q[0]), v = __bfloat1622float2(q[1]);
+  return make_float4(u.x, u.y, v.x, v.y);
+}
+FP_DEV float2 ld2(const float* p, long a, bool narrow) {
+  if (!narrow) return *reinterpret_cast<const float2*>(p + a);
+  return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(reinterpret_cast<const __nv_bfloat16*>(p) + a));
+}
+FP_DEV uint8_t rimFlag(uint8_t topo, bool unknown) {
+  return (uint8_t)(!unknown ? 0u : ((topo & FP_STORED_SOLID) ? RIM_SOLID : (RIM_OPEN | (topo & 63u))));
+}
+
+// Fill the stage of the box of an owner of OWN^3 cells whose 27 neighbours' storage is nbr[] (their
+// slots, -1 none), RV cells out for values, RR for right-hand sides, RF for flags: from `topo` and
+// `open(n, low, cell)`, whether cell `cell` of neighbour n, on its low faces on the axes of bits
+// `low`, is an unknown.
+template <int OWN, int RV, int RR, int RF, class Open>
+FP_DEV void stageRim(const RimStage<OWN>& st, const int* nbr, const Args& A, const uint8_t* topo, Open open) {
+  using K = Rim<OWN>;
+  constexpr int M = OWN - 1, CELLS = OWN * OWN * OWN, E = OWN + 2 * RV;
+  static_assert(RV >= RR && RV >= RF, "the values' box holds the others");
+  for (int i = threadIdx.x; i < E * E * K::PIECES; i += K::THREADS) {
+    const int piece = i % K::PIECES, row = i / K::PIECES, y = row % E - RV, z = row / E - RV;
+    const int dx = piece == 0 ? -1 : (piece == K::PIECES - 1 ? 1 : 0), dy = y < 0 ? -1 : (y >= OWN ? 1 : 0),
+              dz = z < 0 ? -1 : (z >= OWN ? 1 : 0);
+    const int n = nbrIndex(dx, dy, dz), s = nbr[n], x = piece * 4 - 4;
+    const int cell = ((z & M) * OWN + (y & M)) * OWN + (x & M);
+    const long at = (long)s * CELLS + cell;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (s >= 0) v = ld4(A.pin, at, A.pinN);
+    *reinterpret_cast<float4*>(st.val + st.at(x, y, z)) = v;
+    auto within = [&](int r) { return y >= -r && y < OWN + r && z >= -r && z < OWN + r; };
+    if (within(RR)) {
+      float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (s >= 0) r = ld4(A.rhs, at, A.rhsN);
+      *reinterpret_cast<float4*>(st.rh + st.in(x, y, z)) = r;
+    }
+    if (within(RF)) {
+      uchar4 f = make_uchar4(0, 0, 0, 0);
+      if (s >= 0) {
+        const uchar4 t = *reinterpret_cast<const uchar4*>(topo + at);
+        const unsigned low = ((y & M) == 0 ? 2u : 0u) | ((z & M) == 0 ? 4u : 0u);
+        // The piece before the row starts on no low face that a box reaches (OWN > R).
+        const unsigned edge = ((x & M) == 0 && dx >= 0) ? low | 1u : low;
+        f = make_uchar4(rimFlag(t.x, open(n, edge, cell)), rimFlag(t.y, open(n, low, cell + 1)),
+                        rimFlag(t.z, open(n, low, cell + 2)), rimFlag(t.w, open(n, low, cell + 3)));
+      }
+      *reinterpret_cast<uchar4*>(st.fl + st.at(x, y, z)) = f;
+    }
+  }
+}
+// The level below around the owner, a rim of two, as prolongation reads it: coarseValue of every
+// cell. `below(c, n)` gives a cell's index in the level's storage (-1 none) from its neighbour n and
+// its place there; a solid cell's ghost comes through the directory (few cells, near colliders).
+template <int OWN, class Below>
+FP_DEV void stageBelow(const SimParams& P, const Home& H, const RimStage<OWN>& st, const Args& A, int bx, int by, int bz,
+                       Below below) {
+  using K = Rim<OWN>;
+  for (int i = threadIdx.x; i < K::G * K::G * K::G; i += K::THREADS) {
+    const int x = i % K::G - 2, y = i / K::G % K::G - 2, z = i / (K::G * K::G) - 2;
+    const int dx = x < 0 ? -1 : (x >= K::H ? 1 : 0), dy = y < 0 ? -1 : (y >= K::H ? 1 : 0), dz = z < 0 ? -1 : (z >= K::H ? 1 : 0);
+    const long a = below(nbrIndex(dx, dy, dz), ((z & (K::H - 1)) * K::H + (y & (K::H - 1))) * K::H + (x & (K::H - 1)));
+    float v = 0.f;
+    if (a >= 0)
+      v = (P.colliderCount > 0 && (P.topo[A.level + 1][a] & FP_STORED_SOLID)) 
+              ? coarseValue(P, H, A.coarse, A.level + 1, bx + x, by + y, bz + z)
+              : ldBf(A.coarse, a, A.coarseN);
+    st.below[i] = v;
+  }
+}
+// prolongCell of the box, in place; `groundRow`: the lowest row of the level below that is not below
+// the ground (its ghosts mirror the ground).
+template <int OWN>
+FP_DEV void prolongRim(const RimStage<OWN>& st, int groundRow, bool narrow) {
+  using K = Rim<OWN>;
+  for (int i = threadIdx.x; i < K::S * K::S * K::S; i += K::THREADS) {
+    const int x = i % K::S - K::R, y = i / K::S % K::S - K::R, z = i / (K::S * K::S) - K::R, o = st.at(x, y, z);
+    float v = 0.f;
+    if (st.fl[o] & RIM_OPEN) {
+      // Cell p lies a quarter of a coarse cell past centre (p - 1) >> 1 when odd, three when even.
+      const int ix = ((x - 1) >> 1) + 2, iz = ((z - 1) >> 1) + 2;
+      const int iy[2] = {min(max((y - 1) >> 1, groundRow) + 2, K::G - 1), min(max(((y - 1) >> 1) + 1, groundRow) + 2, K::G - 1)};
+      const float fx = (x & 1) ? 0.25f : 0.75f, fy = (y & 1) ? 0.25f : 0.75f, fz = (z & 1) ? 0.25f : 0.75f;
+      float c[8];
+#pragma unroll
+      for (int k = 0; k < 8; k++) c[k] = st.below[((iz + (k >> 2)) * K::G + iy[(k >> 1) & 1]) * K::G + ix + (k & 1)];
+      const float corr = mixf(mixf(mixf(c[0], c[1], fx), mixf(c[2], c[3], fx), fy),
+                              mixf(mixf(c[4], c[5], fx), mixf(c[6], c[7], fx), fy), fz);
+      v = st.val[o] + corr;
+      if (narrow) v = __bfloat162float(__float2bfloat16_rn(v));
+    }
+    st.val[o] = v;
+  }
+}
+
+// One sweep over the box RIM cells around the owner's cells, from `in` (whose cell (x,y,z) is at
+// place(x,y,z), its rows SZ a layer).
+template <int OWN, int RIM, int SZ, class Place, class Put>
+FP_DEV void sweepBox(const RimStage<OWN>& st, const float* in, Place place, bool narrow, Put put) {
+  using K = Rim<OWN>;
+  constexpr int E = OWN + 2 * RIM;
+  for (int i = threadIdx.x; i < E * E * E; i += K::THREADS) {
+    const int x = i % E - RIM, y = i / E % E - RIM, z = i / (E * E) - RIM;
+    const int c = place(x, y, z);
+    const uint32_t f = st.fl[st.at(x, y, z)];
+    float v = 0.f;
+    if (f & RIM_OPEN) {
+      constexpr int sy = K::P, sz = SZ * K::P;
+      const float v0 = (f & 1u) ? in[c + 1] : 0.f, v1 = (f & 2u) ? in[c - 1] : 0.f;
+      const float v2 = (f & 4u) ? in[c + sy] : 0.f, v3 = (f & 8u) ? in[c - sy] : 0.f;
+      const float v4 = (f & 16u) ? in[c + sz] : 0.f, v5 = (f & 32u) ? in[c - sz] : 0.f;
+      const float sum = (v0 + v1) + (v2 + v3) + (v4 + v5);
+      const float cand = (sum - st.rh[st.in(x, y, z)]) / fmaxf(diagOf(f & 63u), 1e-12f);
+      v = mixf(in[c], cand, 0.8f);
+      if (narrow) v = __bfloat162float(__float2bfloat16_rn(v));
+    }
+    put(x, y, z, v);
+  }
+}
+// The leg on a staged box; `own(cell, value)` takes the owner's results. DOWN leaves them (and a rim of
+// one) in st.val at st.in for the restriction.
+template <int OWN, int LEG, class Own>
+FP_DEV void sweepRim(const RimStage<OWN>& st, bool narrow, Own own) {
+  using K = Rim<OWN>;
+  if constexpr (LEG == REST) return;
+  auto at = [&](int x, int y, int z) { return st.at(x, y, z); };
+  auto in = [&](int x, int y, int z) { return st.in(x, y, z); };
+  auto cell = [](int x, int y, int z) { return (z * OWN + y) * OWN + x; };
+  sweepBox<OWN, 2, K::S>(st, st.val, at, narrow, [&](int x, int y, int z, float v) { st.other[st.in(x, y, z)] = v; });
+  __syncthreads();
+  sweepBox<OWN, 1, K::C>(st, st.other, in, narrow, [&](int x, int y, int z, float v) {
+    st.val[st.in(x, y, z)] = v;
+    if (LEG == DOWN && x >= 0 && x < OWN && y >= 0 && y < OWN && z >= 0 && z < OWN) own(cell(x, y, z), v);
+  });
+  __syncthreads();
+  if constexpr (LEG == UP || LEG == PUP)
+    sweepBox<OWN, 0, K::C>(st, st.val, in, narrow, [&](int x, int y, int z, float v) { own(cell(x, y, z), v); });
+}
+// restrictCell of coarse cell q of the owner's (OWN / 2)^3 from the values after DOWN's sweeps, or as
+// staged; whether all its cells are unknowns.
+template <int OWN, int LEG>
+FP_DEV float restrictRim(const RimStage<OWN>& st, int q, bool& every) {
+  using K = Rim<OWN>;
+  const int cx = q % K::H, cy = q / K::H % K::H, cz = q / (K::H * K::H);
+  constexpr int sy = K::P, sz = (LEG == DOWN ? K::C : K::S) * K::P;
+  float residual = 0.f;
+  every = true;
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    const int x = cx * 2 + (k & 1), y = cy * 2 + ((k >> 1) & 1), z = cz * 2 + (k >> 2);
+    const int o = LEG == DOWN ? st.in(x, y, z) : st.at(x, y, z);
+    const uint32_t f = st.fl[st.at(x, y, z)];
+    every = every && f != 0u;
+    if (f & RIM_OPEN) {
+      const float v0 = (f & 1u) ? st.val[o + 1] : 0.f, v1 = (f & 2u) ? st.val[o - 1] : 0.f;
+      const float v2 = (f & 4u) ? st.val[o + sy] : 0.f, v3 = (f & 8u) ? st.val[o - sy] : 0.f;
+      const float v4 = (f & 16u) ? st.val[o + sz] : 0.f, v5 = (f & 32u) ? st.val[o - sz] : 0.f;
+      const float sum = (v0 + v1) + (v2 + v3) + (v4 + v5);
+      residual += st.rh[st.in(x, y, z)] - (sum - diagOf(f & 63u) * st.val[o]);
+    }
+  }
+  return residual * 0.5f;
+}
+// What the restriction writes of coarse cell `out` of the level below.
 FP_DEV void storeCoarse(const SimParams& P, const Args& A, long out, float r, bool every) {
   stBf(const_cast<float*>(A.coarse), out, r, A.coarseN);  // the coarse right-hand side
   float first = 0.f;
@@ -664,16 +715,38 @@ FP_DEV void storeCoarse(const SimParams& P, const Args& A, long out, float r, bo
   }
   stBf(A.cfirst, out, first, A.cfirstN);
 }
+template <int OWN, int LEG, class Open>
+FP_DEV void stageLeg(const RimStage<OWN>& st, const int* nbr, const Args& A, const uint8_t* topo, Open open) {
+  if constexpr (LEG == REST)
+    stageRim<OWN, 1, 0, 0>(st, nbr, A, topo, open);
+  else if constexpr (LEG == PUP)
+    stageRim<OWN, 3, 2, 3>(st, nbr, A, topo, open);
+  else
+    stageRim<OWN, 3, 2, 2>(st, nbr, A, topo, open);
+}
+// activeCell on a brick level: a cell is an unknown when its brick and those before it on the axes of
+// its low faces compute. Bit n of `ok`: neighbour n does, or lies below the ground (not asked).
+FP_DEV bool openIn(uint32_t ok, int n, unsigned low) {
+  uint32_t need = 1u << n;
+  if (low & 1u) need |= need >> 1;
+  if (low & 2u) need |= need >> 3;
+  if (low & 4u) need |= need >> 9;
+  return (ok & need) == need;
+}
+FP_DEV int groundRowOf(const SimParams& P, int firstRow) { return P.ground ? -firstRow : -(1 << 20); }
 
 // Brick levels of OWN^3 cells a brick (8 or 4), a CTA a brick. A.pin: the level's values; A.pout: the
-// result, the other buffer; DOWN: A.coarse the coarse right-hand side, A.cfirst its first iterate.
-template <int OWN, int KIND>
-__global__ void __launch_bounds__(Rim<OWN>::THREADS) k_sweep_bricks(FpBatch bt, MgSel Sl) {
+// result, the other buffer; REST, DOWN: A.coarse the coarse right-hand side, A.cfirst its first
+// iterate; PUP: A.coarse the level below.
+template <int OWN, int LEG>
+__global__ void __launch_bounds__(Rim<OWN>::THREADS) k_leg_bricks(FpBatch bt, MgSel Sl) {
+  using K = Rim<OWN>;
   __shared__ int nslot[27];
   __shared__ uint32_t okBits;
   extern __shared__ __align__(16) float rimSmem[];
   const RimStage<OWN> st(rimSmem);
   const int t = threadIdx.x;
+  letNextStart();
   const uint32_t total = workTotal(bt, FP_WORK_ACTIVE);
   for (uint32_t item = blockIdx.x; item < total; item += gridDim.x) {
     uint32_t i;
@@ -695,39 +768,40 @@ __global__ void __launch_bounds__(Rim<OWN>::THREADS) k_sweep_bricks(FpBatch bt, 
       if (t == 0) okBits = b;
     }
     __syncthreads();
-    // activeCell: a cell is an unknown when its brick and those before it on the axes of its low
-    // faces compute (below the ground none are asked).
     const uint32_t ok = okBits;
-    auto open = [&](int n, unsigned low, int) {
-      uint32_t need = 1u << n;
-      if (low & 1u) need |= need >> 1;
-      if (low & 2u) need |= need >> 3;
-      if (low & 4u) need |= need >> 9;
-      return (ok & need) == need;
-    };
-    stageRim<OWN>(nslot, A.pin, A.pinN, A.rhs, A.rhsN, P.topo[A.level], st.val, st.rh, st.fl, open, [](int) { return false; });
+    waitForPrevious();
+    stageLeg<OWN, LEG>(st, nslot, A, P.topo[A.level], [&](int n, unsigned low, int) { return openIn(ok, n, low); });
+    if constexpr (LEG == PUP) {
+      stageBelow<OWN>(P, H, st, A, H.bx * K::H, H.by * K::H, H.bz * K::H,
+                      [&](int n, int c) { return nslot[n] < 0 ? -1l : (long)nslot[n] * (K::H * K::H * K::H) + c; });
+      __syncthreads();
+      prolongRim<OWN>(st, groundRowOf(P, H.by * K::H), A.poutN);
+    }
+    __syncthreads();
     const long slot = nslot[13];
     constexpr int CELLS = OWN * OWN * OWN;
-    sweepAll<OWN, KIND>(st.val, st.rh, st.fl, st.other, A.poutN, [&](int c, float v) { stBf(A.pout, slot * CELLS + c, v, A.poutN); });
-    if (KIND == DOWN)
-      for (int q = t; q < CELLS / 8; q += Rim<OWN>::THREADS) {
+    sweepRim<OWN, LEG>(st, A.poutN, [&](int c, float v) { stBf(A.pout, slot * CELLS + c, v, A.poutN); });
+    if constexpr (LEG == DOWN || LEG == REST)
+      for (int q = t; q < CELLS / 8; q += K::THREADS) {
         bool every;
-        const float r = restrictRim<OWN>(st.val, st.rh, st.fl, q, every);
+        const float r = restrictRim<OWN, LEG>(st, q, every);
         storeCoarse(P, A, slot * (CELLS / 8) + q, r, every);
       }
   }
+  waitForPrevious();
 }
 
-// The first tile level (4^3 cells a tile, a cell a brick), a CTA a live tile. The cells of neighbour
-// tiles that are not live are no part of the solve.
-template <int KIND>
-__global__ void __launch_bounds__(Rim<4>::THREADS) k_sweep_tiles(FpBatch bt, MgSel Sl) {
+// The first tile level (4^3 cells a tile, a cell a brick), a CTA a live tile (a neighbour tile that
+// exists is live).
+template <int LEG>
+__global__ void __launch_bounds__(Rim<4>::THREADS) k_leg_tiles(FpBatch bt, MgSel Sl) {
+  using K = Rim<4>;
   __shared__ int nbr[27];
   __shared__ uint64_t masks[27];
-  __shared__ uint32_t liveBits;
   extern __shared__ __align__(16) float rimSmem[];
   const RimStage<4> st(rimSmem);
   const int t = threadIdx.x;
+  letNextStart();
   const uint32_t total = workTotal(bt, FP_WORK_TILES);
   for (uint32_t item = blockIdx.x; item < total; item += gridDim.x) {
     uint32_t local;
@@ -735,31 +809,128 @@ __global__ void __launch_bounds__(Rim<4>::THREADS) k_sweep_tiles(FpBatch bt, MgS
     const Args A = resolve(P, Sl);
     if (A.skip) continue;  // the same for the whole CTA
     const int tile = P.liveTiles[local];
-    if (__ldg(&P.tileRec[tile]).w == 0) continue;
+    const int4 rec = __ldg(&P.tileRec[tile]);
+    if (rec.w == 0) continue;
     __syncthreads();  // the previous tile's stage has been read
-    if (t < 32) {
-      bool live = false;
-      if (t < 27) {
-        const int n = checkTile(P, FP_SITE_TILE_NBR, __ldg(&P.tileNbr[(size_t)tile * 27 + t]));
-        nbr[t] = n;
-        live = n >= 0 && P.tileIndex[n] >= 0 && __ldg(&P.tileRec[n]).w != 0;
-        masks[t] = live ? P.tileMask[n] : 0ull;
-      }
-      const uint32_t b = __ballot_sync(0xffffffffu, live);
-      if (t == 0) liveBits = b;
+    if (t < 27) {
+      const int n = checkTile(P, FP_SITE_TILE_NBR, __ldg(&P.tileNbr[(size_t)tile * 27 + t]));
+      nbr[t] = n;
+      masks[t] = n >= 0 ? P.tileMask[n] : 0ull;
     }
     __syncthreads();
-    const uint32_t live = liveBits;
-    stageRim<4>(nbr, A.pin, A.pinN, A.rhs, A.rhsN, P.topo[A.level], st.val, st.rh, st.fl,
-                [&](int n, unsigned, int cell) { return ((masks[n] >> cell) & 1ull) != 0ull; },
-                [&](int n) { return ((live >> n) & 1u) == 0u; });
-    sweepAll<4, KIND>(st.val, st.rh, st.fl, st.other, A.poutN, [&](int c, float v) { stBf(A.pout, (long)tile * 64 + c, v, A.poutN); });
-    if (KIND == DOWN && t < 8) {
+    waitForPrevious();
+    stageLeg<4, LEG>(st, nbr, A, P.topo[A.level], [&](int n, unsigned, int cell) { return ((masks[n] >> cell) & 1ull) != 0ull; });
+    if constexpr (LEG == PUP) {
+      const Home H = enterTile(P, tile, rec);
+      stageBelow<4>(P, H, st, A, rec.x * K::H, rec.y * K::H, rec.z * K::H,
+                    [&](int n, int c) { return nbr[n] < 0 ? -1l : (long)nbr[n] * 8 + c; });
+      __syncthreads();
+      prolongRim<4>(st, groundRowOf(P, rec.y * K::H), A.poutN);
+    }
+    __syncthreads();
+    sweepRim<4, LEG>(st, A.poutN, [&](int c, float v) { stBf(A.pout, (long)tile * 64 + c, v, A.poutN); });
+    if (LEG == DOWN && t < 8) {
       bool every;
-      const float r = restrictRim<4>(st.val, st.rh, st.fl, t, every);
+      const float r = restrictRim<4, LEG>(st, t, every);
       storeCoarse(P, A, (long)tile * 8 + t, r, every);
     }
   }
+  waitForPrevious();
+}
+
+// The last brick level (2^3 cells a brick), whose three-cell rim reaches past a brick's neighbours: a
+// CTA a live tile, the tile's 8^3 cells read and written through its bricks' slots, and those of the
+// two bricks around it.
+template <int LEG>
+__global__ void __launch_bounds__(Rim<8>::THREADS) k_leg_pairs(FpBatch bt, MgSel Sl) {
+  using K = Rim<8>;
+  constexpr int N = 8;  // bricks a side: the tile's four and two on either side
+  __shared__ int nbr[27];
+  __shared__ int slots[N * N * N];
+  __shared__ uint32_t ok[N * N * N / 32];
+  extern __shared__ __align__(16) float rimSmem[];
+  const RimStage<8> st(rimSmem);
+  const int t = threadIdx.x;
+  letNextStart();
+  const uint32_t total = workTotal(bt, FP_WORK_TILES);
+  for (uint32_t item = blockIdx.x; item < total; item += gridDim.x) {
+    uint32_t local;
+    const SimParams& P = *workSim(bt, FP_WORK_TILES, item, local).vview;
+    const Args A = resolve(P, Sl);
+    if (A.skip) continue;  // the same for the whole CTA
+    const int tile = P.liveTiles[local];
+    const int4 rec = __ldg(&P.tileRec[tile]);
+    if (rec.w == 0) continue;
+    __syncthreads();  // the previous tile's stage has been read
+    if (t < 27) nbr[t] = checkTile(P, FP_SITE_TILE_NBR, __ldg(&P.tileNbr[(size_t)tile * 27 + t]));
+    __syncthreads();
+    for (int i = t; i < N * N * N; i += K::THREADS) {
+      const int bx = i % N - 2, by = i / N % N - 2, bz = i / (N * N) - 2;
+      const int n = nbr[nbrIndex(bx >> 2, by >> 2, bz >> 2)];
+      int s = -1;
+      if (n >= 0) s = checkSlot(P, FP_SITE_ENTRY, entryPage(P.entries[(size_t)n * 64 + ((bz & 3) * 4 + (by & 3)) * 4 + (bx & 3)]));
+      slots[i] = s;
+      const uint32_t b = __ballot_sync(0xffffffffu, s >= 0 || (P.ground && rec.y * 4 + by < 0));
+      if ((t & 31) == 0) ok[i >> 5] = b;
+    }
+    __syncthreads();
+    auto okAt = [&](int i) { return ((ok[i >> 5] >> (i & 31)) & 1u) != 0u; };
+    waitForPrevious();
+    // Pairs of cells along x: a row of the box lies in eight bricks.
+    const uint8_t* topo = P.topo[A.level];
+    for (int i = t; i < K::S * K::S * N; i += K::THREADS) {
+      const int px = i % N, row = i / N, x = px * 2 - 4, y = row % K::S - K::R, z = row / K::S - K::R;
+      const int b = (((z >> 1) + 2) * N + (y >> 1) + 2) * N + px, s = slots[b];
+      const long at = (long)s * 8 + ((z & 1) * 2 + (y & 1)) * 2;
+      float2 v = make_float2(0.f, 0.f), r = v;
+      uchar2 f = make_uchar2(0, 0);
+      if (s >= 0) {
+        v = ld2(A.pin, at, A.pinN);
+        const uchar2 q = *reinterpret_cast<const uchar2*>(topo + at);
+        // The cells of the outermost bricks that a box reaches are on no low face.
+        bool in = okAt(b);
+        if (!(y & 1) && b >= N) in = in && okAt(b - N);
+        if (!(z & 1) && b >= N * N) in = in && okAt(b - N * N);
+        if (!(y & 1) && !(z & 1) && b >= N * N + N) in = in && okAt(b - N * N - N);
+        bool edge = in;
+        if (px > 0) {
+          edge = edge && okAt(b - 1);
+          if (!(y & 1) && b >= N + 1) edge = edge && okAt(b - N - 1);
+          if (!(z & 1) && b >= N * N + 1) edge = edge && okAt(b - N * N - 1);
+          if (!(y & 1) && !(z & 1) && b >= N * N + N + 1) edge = edge && okAt(b - N * N - N - 1);
+        }
+        f = make_uchar2(rimFlag(q.x, edge), rimFlag(q.y, in));
+      }
+      const int o = st.at(x, y, z);
+      *reinterpret_cast<float2*>(st.val + o) = v;
+      *reinterpret_cast<uchar2*>(st.fl + o) = f;
+      if (y >= -2 && y < 10 && z >= -2 && z < 10) {
+        if (s >= 0) r = ld2(A.rhs, at, A.rhsN);
+        *reinterpret_cast<float2*>(st.rh + st.in(x, y, z)) = r;
+      }
+    }
+    if constexpr (LEG == PUP) {
+      const Home H = enterTile(P, tile, rec);
+      stageBelow<8>(P, H, st, A, rec.x * K::H, rec.y * K::H, rec.z * K::H,
+                    [&](int n, int c) { return nbr[n] < 0 ? -1l : (long)nbr[n] * 64 + c; });
+      __syncthreads();
+      prolongRim<8>(st, groundRowOf(P, rec.y * K::H), A.poutN);
+    }
+    __syncthreads();
+    auto slotOf = [&](int bx, int by, int bz) { return slots[((bz + 2) * N + by + 2) * N + bx + 2]; };
+    sweepRim<8, LEG>(st, A.poutN, [&](int c, float v) {
+      const int x = c & 7, y = (c >> 3) & 7, z = c >> 6, s = slotOf(x >> 1, y >> 1, z >> 1);
+      if (s >= 0) stBf(A.pout, (long)s * 8 + ((z & 1) * 2 + (y & 1)) * 2 + (x & 1), v, A.poutN);
+    });
+    // A coarse cell is a brick's, at the brick's own id; those of bricks without a slot are cleared
+    // with the tile masks.
+    if (LEG == DOWN && t < 64 && slotOf(t & 3, (t >> 2) & 3, t >> 4) >= 0) {
+      bool every;
+      const float r = restrictRim<8, LEG>(st, t, every);
+      storeCoarse(P, A, (long)tile * 64 + t, r, every);
+    }
+  }
+  waitForPrevious();
 }
 
 // Every cell of `A.level` (a tile level of CELLS cells a tile) in every tile: a thread per
@@ -1103,18 +1274,16 @@ constexpr uint8_t UNKNOWN = 0x80;  // level bl + 1 flag byte: activeCell; bit 6 
 
 // The level bl + 1 cell next to cell o of tile t on side k (+x, -x, +y, -y, +z, -z), as an
 // index of the level's tile-slot arrays; -1 without a tile there.
-// `faces` holds each live tile's six face neighbours as live positions (-1 without one).
+// `faces` holds each live tile's six face neighbours as live positions (-1 without one). Either way
+// the cell's place in its tile is o with the axis' bit turned.
 FP_DEV int coarseNbr(const int16_t* faces, int j, int o, int k) {
-  int l[3] = {o & 1, (o >> 1) & 1, o >> 2};
-  const int ax = k >> 1, step = (k & 1) ? -1 : 1;
-  int v = l[ax] + step;
-  l[ax] = v & 1;
-  const int nj = (v < 0 || v > 1) ? faces[j * 6 + k] : j;
-  return nj < 0 ? -1 : nj * 8 + ((l[2] * 2 + l[1]) * 2 + l[0]);
+  const int ax = k >> 1, nj = ((o >> ax) & 1) == (k & 1) ? j : faces[j * 6 + k];
+  return nj < 0 ? -1 : nj * 8 + (o ^ (1 << ax));
 }
 
-__global__ void __launch_bounds__(1024) k_coarse(FpBatch bt, MgSel Sl, int iterations) {
+__global__ void __launch_bounds__(1024) k_coarse(FpBatch bt, MgSel Sl, int iterations, int smemBytes) {
   extern __shared__ float coarseSmem[];
+  letNextStart();
   const int nbIndex[6] = {nbrIndex(1, 0, 0), nbrIndex(-1, 0, 0), nbrIndex(0, 1, 0),
                           nbrIndex(0, -1, 0), nbrIndex(0, 0, 1), nbrIndex(0, 0, -1)};
   const int sims = batchCount(bt);
@@ -1124,7 +1293,7 @@ __global__ void __launch_bounds__(1024) k_coarse(FpBatch bt, MgSel Sl, int itera
     if (A.skip) continue;  // the same for the whole CTA
     // Shared arrays by live position j (tile slot P.liveTiles[j]); level L cells at j * 8 + o.
     const int L = A.level, BL = L + 1, nt = P.liveCount, n4 = nt * 8;
-    if ((long)nt * COARSE_SLOT_BYTES > COARSE_SMEM) continue;  // the host sizes batches to fit
+    if ((long)nt * COARSE_SLOT_BYTES > smemBytes) continue;  // the host sizes launches to fit
     const bool nL = narrowLevel(P, L), nB = narrowLevel(P, BL);
     float* pa = coarseSmem;  // level L: iterates, right-hand side
     float* pb = pa + n4;
@@ -1139,25 +1308,47 @@ __global__ void __launch_bounds__(1024) k_coarse(FpBatch bt, MgSel Sl, int itera
     // live (its stored values are read from global memory), -1 for none.
     int16_t* nb27 = faces + nt * 6;
     bool solidNear = false;  // a bottom cell of a neighbour tile is solid
-    for (int q = threadIdx.x; q < nt * 27; q += blockDim.x) {
-      const int j = q / 27, k = q % 27;
-      const int n = checkTile(P, FP_SITE_TILE_NBR, __ldg(&P.tileNbr[P.liveTiles[j] * 27 + k]));
-      const int pos = n >= 0 ? P.tileIndex[n] : -1;
-      nb27[q] = (int16_t)(n < 0 ? -1 : (pos >= 0 ? pos : -2));
-      solidNear = solidNear || (n >= 0 && (P.topo[BL][n] & FP_STORED_SOLID));
-      const int dx = k % 3 - 1, dy = (k / 3) % 3 - 1, dz = k / 9 - 1;
-      if ((dx != 0) + (dy != 0) + (dz != 0) == 1) {  // a face: +x, -x, +y, -y, +z, -z
-        const int f = dx != 0 ? (dx > 0 ? 0 : 1) : (dy != 0 ? (dy > 0 ? 2 : 3) : (dz > 0 ? 4 : 5));
-        faces[j * 6 + f] = (int16_t)pos;
+    // Setting up is chains of dependent loads (a tile, its neighbour, what that holds): several at a
+    // time, so that their latencies overlap.
+    int* live = reinterpret_cast<int*>(cb);  // until the bottom's iterations
+    for (int j = threadIdx.x; j < nt; j += blockDim.x) live[j] = P.liveTiles[j];
+    __syncthreads();
+    constexpr int AHEAD = 8;
+    for (int base = threadIdx.x; base < nt * 27; base += AHEAD * blockDim.x) {
+      int n[AHEAD], pos[AHEAD];
+      uint8_t tb[AHEAD];
+#pragma unroll
+      for (int u = 0; u < AHEAD; u++) {
+        const int q = base + u * blockDim.x;
+        n[u] = q < nt * 27 ? checkTile(P, FP_SITE_TILE_NBR, __ldg(&P.tileNbr[live[q / 27] * 27 + q % 27])) : -1;
+      }
+#pragma unroll
+      for (int u = 0; u < AHEAD; u++) {
+        pos[u] = n[u] >= 0 ? P.tileIndex[n[u]] : -1;
+        tb[u] = n[u] >= 0 ? P.topo[BL][n[u]] : 0;
+      }
+#pragma unroll
+      for (int u = 0; u < AHEAD; u++) {
+        const int q = base + u * blockDim.x;
+        if (q >= nt * 27) break;
+        const int j = q / 27, k = q % 27;
+        nb27[q] = (int16_t)(n[u] < 0 ? -1 : (pos[u] >= 0 ? pos[u] : -2));
+        solidNear = solidNear || (tb[u] & FP_STORED_SOLID);
+        const int dx = k % 3 - 1, dy = (k / 3) % 3 - 1, dz = k / 9 - 1;
+        if ((dx != 0) + (dy != 0) + (dz != 0) == 1) {  // a face: +x, -x, +y, -y, +z, -z
+          const int f = dx != 0 ? (dx > 0 ? 0 : 1) : (dy != 0 ? (dy > 0 ? 2 : 3) : (dz > 0 ? 4 : 5));
+          faces[j * 6 + f] = (int16_t)pos[u];
+        }
       }
     }
+    waitForPrevious();
+#pragma unroll 4
     for (int c = threadIdx.x; c < n4; c += blockDim.x) {
-      const int t = P.liveTiles[c >> 3], o = c & 7;
+      const int t = live[c >> 3], o = c & 7;
       const long a = (long)t * 8 + o;  // the cell's storage
-      int4 rec = __ldg(&P.tileRec[t]);
-      Home H = enterTile(P, t, rec);
-      int px = rec.x * 2 + (o & 1), py = rec.y * 2 + ((o >> 1) & 1), pz = rec.z * 2 + (o >> 2);
-      fl[c] = (uint8_t)(P.topo[L][a] | (activeCell(P, H, px, py, pz, L) ? UNKNOWN : 0));
+      // activeCell of a live tile's own cell: its eight bricks compute (tileCellActive).
+      const uint64_t bricks = 0x0000000000330033ull << (2 * (o & 1) + 8 * ((o >> 1) & 1) + 32 * (o >> 2));
+      fl[c] = (uint8_t)(P.topo[L][a] | ((P.tileMask[t] & bricks) == bricks ? UNKNOWN : 0));
       pa[c] = ldBf(A.pin, a, nL);
       rh[c] = ldBf(A.rhs, a, nL);
     }
@@ -1218,8 +1409,32 @@ __global__ void __launch_bounds__(1024) k_coarse(FpBatch bt, MgSel Sl, int itera
     // relaxCoarse (pressure.wgsl:549-599): FP32 iterates in shared memory.
     float* cur = ca;
     float* nxt = cb;
+    // A thread keeps its first tile's flags, neighbours and right-hand side over the iterations (most
+    // simulations have a tile a thread at most).
+    const int own = threadIdx.x;
+    uint32_t ownFlags = SOLIDF;
+    float ownRhs = 0.f, ownDiag = 1.f;
+    int ownNbr[6] = {-1, -1, -1, -1, -1, -1};
+    if (own < nt) {
+      ownFlags = fb[own];
+      ownRhs = cr[own];
+      ownDiag = fmaxf(diagOf(ownFlags & 63u), 1e-12f);
+#pragma unroll
+      for (int k = 0; k < 6; k++) ownNbr[k] = ((ownFlags >> k) & 1u) ? faces[own * 6 + k] : -1;
+    }
     for (int it = 0; it < iterations; it++) {
-      for (int j = threadIdx.x; j < nt; j += blockDim.x) {
+      if (own < nt) {
+        float next = 0.f;
+        if (!(ownFlags & SOLIDF)) {
+          float w[6];
+#pragma unroll
+          for (int k = 0; k < 6; k++) w[k] = ownNbr[k] >= 0 ? cur[ownNbr[k]] : 0.f;
+          const float sum = (w[0] + w[1]) + (w[2] + w[3]) + (w[4] + w[5]);
+          next = mixf(cur[own], (sum - ownRhs) / ownDiag, 0.8f);
+        }
+        nxt[own] = next;
+      }
+      for (int j = own + blockDim.x; j < nt; j += blockDim.x) {
         const uint32_t f = fb[j];
         float next = 0.f;
         if (!(f & SOLIDF)) {
@@ -1290,6 +1505,7 @@ __global__ void __launch_bounds__(1024) k_coarse(FpBatch bt, MgSel Sl, int itera
     for (int c = threadIdx.x; c < n4; c += blockDim.x) stBf(A.pout, (long)P.liveTiles[c >> 3] * 8 + (c & 7), pa[c], nL);
     __syncthreads();
   }
+  waitForPrevious();
 }
 
 // The finest level's residual rhs - (sum - diag p) over its unknowns, as restrictCell forms
@@ -1685,32 +1901,48 @@ static void tileStagedLaunch(const FpBatch& bt, const MgSel& S, int sms, cudaStr
   k_level_tiles_staged<OP, TS><<<sms * tileStagedCtas<OP, TS>(), 256, TileStaged<OP, TS>::SMEM, st>>>(bt, S);
 }
 
-// Resident CTAs per SM of each sweep kernel, from the occupancy calculator.
-template <int OWN, int KIND, bool TILES>
-static int& sweepCtas() {
+// The leg kernels: which cells a CTA owns.
+enum Owner { BRICK8, BRICK4, PAIRS, TILE4 };
+template <int OWNER, int LEG>
+static auto legKernel() {
+  if constexpr (OWNER == BRICK8) return k_leg_bricks<8, LEG>;
+  else if constexpr (OWNER == BRICK4) return k_leg_bricks<4, LEG>;
+  else if constexpr (OWNER == PAIRS) return k_leg_pairs<LEG>;
+  else return k_leg_tiles<LEG>;
+}
+// Resident CTAs per SM of each, from the occupancy calculator.
+template <int OWNER, int LEG>
+static int& legCtas() {
   static int n = 4;
   return n;
 }
-template <int OWN, int KIND, bool TILES>
-static void configureSweeps() {
-  using K = Rim<OWN>;
+template <int OWNER, int LEG>
+static void configureLeg() {
+  using K = Rim<OWNER == BRICK8 || OWNER == PAIRS ? 8 : 4>;
+  static_assert(K::SMEM <= 46 * 1024, "with the static arrays within the limit a kernel needs no attribute for");
   int n = 0;
-  cudaError_t e;
-  if constexpr (TILES)
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sweep_tiles<KIND>, K::THREADS, K::SMEM);
-  else
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sweep_bricks<OWN, KIND>, K::THREADS, K::SMEM);
-  sweepCtas<OWN, KIND, TILES>() = e == cudaSuccess && n > 0 ? n : 4;
+  const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, legKernel<OWNER, LEG>(), K::THREADS, K::SMEM);
+  legCtas<OWNER, LEG>() = e == cudaSuccess && n > 0 ? n : 4;
 }
-template <int OWN, int KIND, bool TILES>
-static void sweepLaunch(const FpBatch& bt, const MgSel& S, int sms, cudaStream_t st) {
-  using K = Rim<OWN>;
-  static_assert(K::SMEM <= 48 * 1024, "within the limit a kernel needs no attribute for");
-  const int grid = sms * sweepCtas<OWN, KIND, TILES>();
-  if constexpr (TILES)
-    k_sweep_tiles<KIND><<<grid, K::THREADS, K::SMEM, st>>>(bt, S);
-  else
-    k_sweep_bricks<OWN, KIND><<<grid, K::THREADS, K::SMEM, st>>>(bt, S);
+// A launch that may start while the one before it on the stream still runs.
+template <class Kernel, class... Args>
+static void launch(bool overlap, Kernel kernel, int grid, int threads, size_t smem, cudaStream_t st, Args... args) {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3((unsigned)grid);
+  c.blockDim = dim3((unsigned)threads);
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  cudaLaunchAttribute a = {};
+  a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  a.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &a;
+  c.numAttrs = overlap ? 1 : 0;
+  cudaLaunchKernelEx(&c, kernel, args...);
+}
+template <int OWNER, int LEG>
+static void legLaunch(const FpBatch& bt, const MgSel& S, int sms, cudaStream_t st) {
+  using K = Rim<OWNER == BRICK8 || OWNER == PAIRS ? 8 : 4>;
+  launch(S.overlap, legKernel<OWNER, LEG>(), sms * legCtas<OWNER, LEG>(), K::THREADS, K::SMEM, st, bt, S);
 }
 
 // Resident CTAs per SM of each staged instantiation, from the occupancy calculator.
@@ -1745,12 +1977,18 @@ void fp_mg_configure(int B) {
   configureStaged<PROLONG, 4>();
   configureStaged<PROLONG, 2>();
   configureStaged<PROLONG, 1>();
-  configureSweeps<8, DOWN, false>();
-  configureSweeps<8, UP, false>();
-  configureSweeps<4, DOWN, false>();
-  configureSweeps<4, UP, false>();
-  configureSweeps<4, DOWN, true>();
-  configureSweeps<4, UP, true>();
+  configureLeg<BRICK8, REST>();
+  configureLeg<BRICK8, DOWN>();
+  configureLeg<BRICK8, UP>();
+  configureLeg<BRICK8, PUP>();
+  configureLeg<BRICK4, REST>();
+  configureLeg<BRICK4, DOWN>();
+  configureLeg<BRICK4, UP>();
+  configureLeg<BRICK4, PUP>();
+  configureLeg<PAIRS, DOWN>();
+  configureLeg<PAIRS, PUP>();
+  configureLeg<TILE4, DOWN>();
+  configureLeg<TILE4, PUP>();
   configureTileStaged<RELAX, 4>();
   configureTileStaged<RESTRICT, 4>();
   configureTileStaged<PROLONG, 2>();
@@ -1838,27 +2076,39 @@ static void levelLaunch(const FpBatch& bt, const MgSel& S, bool tiles, int B, in
 void fp_launch_relax(const FpBatch& bt, const MgSel& S, bool tiles, int B, int sms, cudaStream_t st) {
   levelLaunch<RELAX>(bt, S, tiles, B, sms, st);
 }
-// The levels whose sweeps run several a launch: brick levels of 8^3 and 4^3 cells a brick, and the
-// first tile level. (A brick's 2^3 cells have no three-cell rim in their neighbours; at 16^3 and 32^3
-// a box does not fit several to an SM, and a sweep is no longer mostly latency.)
-bool fp_sweeps_fused(int level, int B) {
+// The levels whose legs are one launch: brick levels of 8^3, 4^3 and 2^3 cells a brick, and the first
+// tile level. (At 16^3 and 32^3 a box does not fit several to an SM, and a step is no longer mostly
+// latency; the levels below are k_coarse's.)
+bool fp_legs_fused(int level, int B) {
   const int bl = log2i(B), side = level < bl ? B >> level : 0;
-  return side == 8 || side == 4 || level == bl;
+  return side == 8 || side == 4 || (side == 2 && level > 0) || level == bl;
 }
-template <int KIND>
-static void sweepsLaunch(const FpBatch& bt, const MgSel& S, int B, int sms, cudaStream_t st) {
-  if (S.level == log2i(B))
-    sweepLaunch<4, KIND, true>(bt, S, sms, st);
-  else if (B >> S.level == 8)
-    sweepLaunch<8, KIND, false>(bt, S, sms, st);
+bool fp_leg_per_brick(int level, int B) { return level < log2i(B) && (B >> level) >= 4; }
+template <int LEG>
+static void legsLaunch(const FpBatch& bt, const MgSel& S, int B, int sms, cudaStream_t st) {
+  const int side = S.level < log2i(B) ? B >> S.level : 0;
+  if (side == 8) {
+    legLaunch<BRICK8, LEG>(bt, S, sms, st);
+  } else if (side == 4) {
+    legLaunch<BRICK4, LEG>(bt, S, sms, st);
+  } else if constexpr (LEG == DOWN || LEG == PUP) {
+    if (side == 2)
+      legLaunch<PAIRS, LEG>(bt, S, sms, st);
+    else
+      legLaunch<TILE4, LEG>(bt, S, sms, st);
+  }
+}
+void fp_launch_leg_down(const FpBatch& bt, const MgSel& S, int B, int sms, cudaStream_t st) {
+  if (S.level == 0)
+    legsLaunch<REST>(bt, S, B, sms, st);
   else
-    sweepLaunch<4, KIND, false>(bt, S, sms, st);
+    legsLaunch<DOWN>(bt, S, B, sms, st);
 }
-void fp_launch_sweeps_down(const FpBatch& bt, const MgSel& S, int B, int sms, cudaStream_t st) {
-  sweepsLaunch<DOWN>(bt, S, B, sms, st);
-}
-void fp_launch_sweeps_up(const FpBatch& bt, const MgSel& S, int B, int sms, cudaStream_t st) {
-  sweepsLaunch<UP>(bt, S, B, sms, st);
+void fp_launch_leg_up(const FpBatch& bt, const MgSel& S, int B, int sms, cudaStream_t st) {
+  if (S.coarse < 0)
+    legsLaunch<UP>(bt, S, B, sms, st);
+  else
+    legsLaunch<PUP>(bt, S, B, sms, st);
 }
 void fp_launch_restrict(const FpBatch& bt, const MgSel& S, bool tiles, int B, int sms, cudaStream_t st) {
   levelLaunch<RESTRICT>(bt, S, tiles, B, sms, st);
@@ -1870,8 +2120,13 @@ void fp_launch_bottom(const FpBatch& bt, const MgSel& S, int iterations, int sms
   k_bottom<<<sms, 1024, BOTTOM_SMEM, st>>>(bt, S, iterations, BOTTOM_SMEM);
 }
 bool fp_coarse_fits(int liveTiles) { return (long)liveTiles * COARSE_SLOT_BYTES <= COARSE_SMEM; }
-void fp_launch_coarse(const FpBatch& bt, const MgSel& S, int iterations, int sms, cudaStream_t st) {
-  k_coarse<<<sms, 1024, COARSE_SMEM, st>>>(bt, S, iterations);
+// `small`: every simulation has at most COARSE_SMALL live tiles; a CTA a simulation of up to `sims`.
+// Fewer warps meet at a barrier sooner, and little shared memory leaves the neighbours' CTAs room.
+constexpr int COARSE_SMALL = 64;
+bool fp_coarse_small(int liveTiles) { return liveTiles <= COARSE_SMALL; }
+void fp_launch_coarse(const FpBatch& bt, const MgSel& S, int iterations, bool small, int sims, int sms, cudaStream_t st) {
+  const int smem = small ? COARSE_SMALL * COARSE_SLOT_BYTES : COARSE_SMEM;
+  launch(S.overlap, k_coarse, sims < sms ? sims : sms, small ? 256 : 1024, (size_t)smem, st, bt, S, iterations, smem);
 }
 
 void fp_launch_residual(const FpBatch& bt, int pSel, int cycle, int sms, cudaStream_t st) {

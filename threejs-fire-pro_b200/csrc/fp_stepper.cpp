@@ -230,8 +230,15 @@ int Stepper::step(Engine* const* sims, const fp_frame* const* frames, const floa
   size_t word = 0;
   bool solidsFresh = false, solidsAll = false, topoAll = false, curl = false, measure = false;
   schedule_ = sims[0]->schedule();
+  // About how many bricks compute, as of the latest measurement: which of two forms with the same
+  // results the multigrid's legs take (kept within a margin, so that a count near the line does not
+  // alternate between two graphs).
+  uint64_t bricks = 0;
+  for (int i = 0; i < count; i++) bricks += sims[i]->activeBricks();
+  manyBricks_ = bricks > (manyBricks_ ? MANY_BRICKS * 7 / 8 : MANY_BRICKS);
   int vcycles = 1;
-  fusedCoarse_ = true;
+  fusedCoarse_ = coarseSmall_ = true;
+  single_ = count == 1;
   anySmoke_ = false;
   smokeDiv_ = 0;
   pending_.clear();
@@ -239,6 +246,7 @@ int Stepper::step(Engine* const* sims, const fp_frame* const* frames, const floa
     Engine* e = sims[i];
     uint32_t cap = (uint32_t)e->capacity();
     fusedCoarse_ = fusedCoarse_ && fp_coarse_fits(e->liveTiles());
+    coarseSmall_ = coarseSmall_ && fp_coarse_small(e->liveTiles());
     anySmoke_ = anySmoke_ || e->smokeDivisor() > 1;
     if (e->smokeDivisor() > 1 && (smokeDiv_ == 0 || e->smokeDivisor() < smokeDiv_)) smokeDiv_ = e->smokeDivisor();
     rowBlocks[i] = blocks;
@@ -278,7 +286,8 @@ int Stepper::step(Engine* const* sims, const fp_frame* const* frames, const floa
                    ((uint64_t)anySmoke_ << 17) | ((uint64_t)schedule_.smoother << 18) |
                    ((uint64_t)schedule_.krylov << 19) | ((uint64_t)schedule_.levels << 20) |
                    ((uint64_t)schedule_.pre_sweeps << 24) | ((uint64_t)schedule_.post_sweeps << 28) |
-                   ((uint64_t)schedule_.bottom_sweeps << 32) | ((uint64_t)smokeDiv_ << 40);
+                   ((uint64_t)schedule_.bottom_sweeps << 32) | ((uint64_t)smokeDiv_ << 40) |
+                   ((uint64_t)manyBricks_ << 44) | ((uint64_t)coarseSmall_ << 45) | ((uint64_t)single_ << 46);
     auto it = graphs_.find(key);
     if (it == graphs_.end()) {
       GraphEntry ge{};
@@ -357,11 +366,18 @@ int Stepper::readProfile(fp_phase* out, uint32_t* count) {
 void Stepper::vcycle(int level, int cur[], uint64_t& launches) {
   auto sel = [](int l, int which) { return fp_mg_sel(l, which); };
   bool tiles = level >= brickLevels_;
+  if (level == 0) chain_ = false;
+  // Whether a leg may overlap the launch before it: one that lets its successor start early.
+  auto chained = [&]() {
+    const bool overlap = chain_ && !manyBricks_;
+    chain_ = true;
+    return overlap;
+  };
   if (fusedCoarse_ && level == brickLevels_ + 1) {
     // Two relaxations, restriction, the bottom, prolongation, three relaxations: an even
     // number of flips leaves the result in the buffer of the first iterate.
-    MgSel S{level, sel(level, 2), sel(level, cur[level]), -1, sel(level, cur[level]), sel(bottom_, 0), cycle_};
-    fp_launch_coarse(batch(), S, 19, sms_, stream_);
+    MgSel S{level, sel(level, 2), sel(level, cur[level]), -1, sel(level, cur[level]), sel(bottom_, 0), cycle_, 0, chained()};
+    fp_launch_coarse(batch(), S, 19, coarseSmall_, single_ ? 1 : sms_, sms_, stream_);
     launches++;
     cur[bottom_] = 0;
     return;
@@ -369,6 +385,7 @@ void Stepper::vcycle(int level, int cur[], uint64_t& launches) {
   if (level == bottom_) {
     MgSel S{level, sel(level, 2), sel(level, cur[level]), -1, sel(level, 1 - cur[level]), -1, cycle_};
     fp_launch_bottom(batch(), S, 19, sms_, stream_);
+    chain_ = false;
     launches++;
     cur[level] = 1 - cur[level];
     return;
@@ -377,32 +394,41 @@ void Stepper::vcycle(int level, int cur[], uint64_t& launches) {
     for (int i = 0; i < n; i++) {
       MgSel S{level, level == 0 ? rhs0Sel_ : sel(level, 2), sel(level, cur[level]), -1, sel(level, 1 - cur[level]), -1, cycle_};
       fp_launch_relax(batch(), S, tiles, B_ / vd_, sms_, stream_);
+      chain_ = false;
       launches++;
       cur[level] = 1 - cur[level];
     }
   };
-  const bool fused = fp_sweeps_fused(level, B_ / vd_);
+  const bool fused = fp_legs_fused(level, B_ / vd_);
   const int rhs = level == 0 ? rhs0Sel_ : sel(level, 2), coarse = level + 1;
-  if (level > 0 && fused) {
-    MgSel D{level, rhs, sel(level, cur[level]), sel(coarse, 2), sel(level, 1 - cur[level]), sel(coarse, 1), cycle_, 0};
-    fp_launch_sweeps_down(batch(), D, B_ / vd_, sms_, stream_);
+  if (fused && (level > 0 || !manyBricks_)) {
+    const bool sweeps = level > 0;
+    MgSel D{level, rhs, sel(level, cur[level]), sel(coarse, 2), sweeps ? sel(level, 1 - cur[level]) : -1, sel(coarse, 1), cycle_, 0, chained()};
+    fp_launch_leg_down(batch(), D, B_ / vd_, sms_, stream_);
     launches++;
-    cur[level] = 1 - cur[level];
+    if (sweeps) cur[level] = 1 - cur[level];
   } else {
     if (level > 0) relax(2);
     MgSel R{coarse, rhs, sel(level, cur[level]), -1, sel(coarse, 2), sel(coarse, 1), cycle_, 0};
     fp_launch_restrict(batch(), R, coarse >= brickLevels_, B_ / vd_, sms_, stream_);
+    chain_ = false;
     launches++;
   }
   cur[coarse] = 1;
   vcycle(coarse, cur, launches);
-  MgSel Pr{level, -1, sel(level, cur[level]), sel(coarse, cur[coarse]), sel(level, 1 - cur[level]), -1, cycle_, 0};
-  fp_launch_prolong(batch(), Pr, tiles, B_ / vd_, sms_, stream_);
-  launches++;
-  cur[level] = 1 - cur[level];
+  // With several V-cycles the finest level's result has to end in the buffer it started from (a
+  // converged simulation skips the later ones): prolongation and sweeps then flip it once each.
+  const bool apart = !fused || (level == 0 && evenFlips_) || (manyBricks_ && fp_leg_per_brick(level, B_ / vd_));
+  if (apart) {
+    MgSel Pr{level, -1, sel(level, cur[level]), sel(coarse, cur[coarse]), sel(level, 1 - cur[level]), -1, cycle_, 0};
+    fp_launch_prolong(batch(), Pr, tiles, B_ / vd_, sms_, stream_);
+    chain_ = false;
+    launches++;
+    cur[level] = 1 - cur[level];
+  }
   if (fused) {
-    MgSel U{level, rhs, sel(level, cur[level]), -1, sel(level, 1 - cur[level]), -1, cycle_, 0};
-    fp_launch_sweeps_up(batch(), U, B_ / vd_, sms_, stream_);
+    MgSel U{level, rhs, sel(level, cur[level]), apart ? -1 : sel(coarse, cur[coarse]), sel(level, 1 - cur[level]), -1, cycle_, 0, chained()};
+    fp_launch_leg_up(batch(), U, B_ / vd_, sms_, stream_);
     launches++;
     cur[level] = 1 - cur[level];
   } else {
@@ -553,6 +579,7 @@ void Stepper::enqueue(bool solidsFresh, bool solidsAll, bool topoAll, bool curl,
   phaseBegin(PH_MULTIGRID);
   uint64_t mg = 0;
   rhs0Sel_ = fp_mg_sel(0, 2);
+  evenFlips_ = vcycles > 1 && schedule_.krylov != FP_KRYLOV_FCG;
   const bool redBlack = schedule_.smoother == FP_SMOOTHER_REDBLACK;
   if (schedule_.krylov == FP_KRYLOV_FCG) {
     // Flexible CG: V-cycle 0 from the divergence gives the start x (the CG iterate, p0[2]);
