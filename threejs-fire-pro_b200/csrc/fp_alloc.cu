@@ -9,6 +9,7 @@
 // the oracle. Every kernel covers all simulations of a batch (FpBatch) in one launch.
 #include "fp_device.cuh"
 #include "fp_launch.h"
+#include "fp_overlap.cuh"
 
 namespace {
 
@@ -64,9 +65,43 @@ __device__ void blockScan2(uint32_t a, uint32_t b, uint32_t& ra, uint32_t& rb, u
   __syncthreads();
 }
 
+// Exclusive scan of one value a thread over the CTA (warps of 32); `total` the sum. Every thread of
+// the CTA calls it; `sums` is shared, 32 words.
+__device__ uint32_t blockScan(uint32_t v, uint32_t* sums, uint32_t& total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  uint32_t incl = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t u = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += u;
+  }
+  __syncthreads();  // the previous scan's sums have been read
+  if (lane == 31) sums[warp] = incl;
+  __syncthreads();
+  // Every warp scans the warps' sums for itself.
+  const uint32_t w = lane < warps ? sums[lane] : 0u;
+  uint32_t wi = w;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t u = __shfl_up_sync(0xffffffffu, wi, o);
+    if (lane >= o) wi += u;
+  }
+  total = __shfl_sync(0xffffffffu, wi, 31);
+  return __shfl_sync(0xffffffffu, wi - w, warp) + incl - v;
+}
+
+// The id of a brick at most one past the home tile of H, or -1 without a tile there (brickIdAt without
+// its way out of the neighbour tiles: the lookups of a brick's 27 neighbours then run together).
+__device__ __forceinline__ int nearBrickId(const SimParams& P, const Home& H, int bx, int by, int bz) {
+  const int t = checkTile(P, FP_SITE_TILE_NBR,
+                          __ldg(&P.tileNbr[H.tile * 27 + nbrIndex((bx >> 2) - H.tx, (by >> 2) - H.ty, (bz >> 2) - H.tz)]));
+  return t < 0 ? -1 : t * 64 + (((bz & 3) * 4 + (by & 3)) * 4 + (bx & 3));
+}
+
 // Blocks of 256 brick ids of every simulation in the launch, grid-stride; `b` is the block
 // within its simulation, `index` this thread's brick id.
 __global__ void __launch_bounds__(RANK_BLOCK) k_build_bricks(FpBatch bt) {
+  enterChain();
   uint32_t blocks = workTotal(bt, FP_WORK_IDBLOCKS);
   for (uint32_t item = blockIdx.x; item < blocks; item += gridDim.x) {
     uint32_t b;
@@ -88,14 +123,18 @@ __global__ void __launch_bounds__(RANK_BLOCK) k_build_bricks(FpBatch bt) {
         H.tz = rec.z;
         bool open = rec.w != 2;
         bool listed = false;
-        for (int z = -1; z <= 1 && open && !listed; z++)
-          for (int y = -1; y <= 1 && !listed; y++)
-            for (int x = -1; x <= 1 && !listed; x++) {
-              int nb = brickIdAt(P, H, bx + x, by + y, bz + z);
-              if (nb < 0) continue;
-              int toward = nbrIndex(-x, -y, -z);
-              listed = ((P.activity[nb] >> 3u) & (1u << toward)) != 0u || (P.meshCount > 0 && P.meshTables[nb] >= 0);
-            }
+        if (open) {
+          // All 27 neighbours at once: stopping at the first that lists the brick made the others'
+          // lookups wait for one another (11.7 -> 6 us on 90 bricks).
+          const bool meshes = P.meshCount > 0;
+#pragma unroll
+          for (int k = 0; k < 27; k++) {
+            const int nb = nearBrickId(P, H, bx + k % 3 - 1, by + (k / 3) % 3 - 1, bz + k / 9 - 1);
+            const uint32_t flags = nb >= 0 ? P.activity[nb] : 0u;
+            listed = listed || ((flags >> 3u) & (1u << (26 - k))) != 0u;  // nbrIndex(-x, -y, -z) = 26 - k
+            if (meshes && nb >= 0) listed = listed || P.meshTables[nb] >= 0;
+          }
+        }
         if (open && !listed) listed = sourceNear(P, tile, bx, by, bz);
         int page = P.pages[index];
         bool wasListed = (P.state[index] & 1u) != 0u;
@@ -121,81 +160,57 @@ __global__ void __launch_bounds__(RANK_BLOCK) k_build_bricks(FpBatch bt) {
 // A CTA per simulation: exclusive offsets of frees, requests and computing bricks per block,
 // and the step's totals (finishBricks' arithmetic, fluid-allocation.wgsl:352-358).
 __global__ void __launch_bounds__(1024) k_scan_blocks(FpBatch bt) {
-  __shared__ uint32_t sf[1024], sr[1024], sk[1024];
-  __shared__ uint32_t carry[3];
-  int sims = batchCount(bt);
+  enterChain();
+  __shared__ uint32_t sums[32];
+  const int sims = batchCount(bt);
   for (int sim = blockIdx.x; sim < sims; sim += gridDim.x) {
     const SimParams& P = bt.sims[sim];
-    uint32_t count = (uint32_t)P.capacity * 64u;
-    int blocks = (int)((count + RANK_BLOCK - 1) / RANK_BLOCK);
-    if (threadIdx.x == 0) carry[0] = carry[1] = carry[2] = 0;
-    __syncthreads();
+    const uint32_t count = (uint32_t)P.capacity * 64u;
+    const int blocks = (int)((count + RANK_BLOCK - 1) / RANK_BLOCK);
+    uint32_t frees = 0, requests = 0, active = 0, total;
     // Pass 1: frees and requests offsets.
-    for (int base = 0; base < blocks; base += 1024) {
-      int b = base + threadIdx.x;
-      uint32_t f = b < blocks ? P.blockCounts[b * 4 + 0] : 0, r = b < blocks ? P.blockCounts[b * 4 + 1] : 0;
-      sf[threadIdx.x] = f;
-      sr[threadIdx.x] = r;
-      __syncthreads();
-      for (int off = 1; off < 1024; off <<= 1) {
-        uint32_t a = threadIdx.x >= off ? sf[threadIdx.x - off] : 0, c = threadIdx.x >= off ? sr[threadIdx.x - off] : 0;
-        __syncthreads();
-        sf[threadIdx.x] += a;
-        sr[threadIdx.x] += c;
-        __syncthreads();
-      }
+    for (int base = 0; base < blocks; base += blockDim.x) {
+      const int b = base + threadIdx.x;
+      const uint32_t f = b < blocks ? P.blockCounts[b * 4 + 0] : 0, r = b < blocks ? P.blockCounts[b * 4 + 1] : 0;
+      const uint32_t before = blockScan(f, sums, total);
+      if (b < blocks) P.blockCounts[b * 4 + 0] = frees + before;
+      frees += total;
+      const uint32_t asked = blockScan(r, sums, total);
       if (b < blocks) {
-        P.blockCounts[b * 4 + 0] = carry[0] + sf[threadIdx.x] - f;  // exclusive
-        P.blockCounts[b * 4 + 1] = carry[1] + sr[threadIdx.x] - r;
+        P.blockCounts[b * 4 + 1] = requests + asked;
         P.blockCounts[b * 4 + 3] = r;  // keep the block's request count
       }
-      __syncthreads();
-      if (threadIdx.x == 1023) {
-        carry[0] += sf[1023];
-        carry[1] += sr[1023];
-      }
-      __syncthreads();
+      requests += total;
     }
-    uint32_t frees = carry[0], requests = carry[1];
-    int32_t freeCount = P.counters->freeCount;
-    int32_t avail = freeCount + (int32_t)frees - P.held;
-    uint32_t granted = (uint32_t)min((int32_t)requests, max(avail, 0));
+    const int32_t freeCount = P.counters->freeCount;
+    const int32_t avail = freeCount + (int32_t)frees - P.held;
+    const uint32_t granted = (uint32_t)min((int32_t)requests, max(avail, 0));
     // Pass 2: computing bricks per block = kept + granted requests of the block.
-    for (int base = 0; base < blocks; base += 1024) {
-      int b = base + threadIdx.x;
+    for (int base = 0; base < blocks; base += blockDim.x) {
+      const int b = base + threadIdx.x;
       uint32_t k = 0;
       if (b < blocks) {
-        uint32_t roff = P.blockCounts[b * 4 + 1], rcount = P.blockCounts[b * 4 + 3];
-        uint32_t g = granted > roff ? min(granted - roff, rcount) : 0u;
-        k = P.blockCounts[b * 4 + 2] + g;
+        const uint32_t roff = P.blockCounts[b * 4 + 1], rcount = P.blockCounts[b * 4 + 3];
+        k = P.blockCounts[b * 4 + 2] + (granted > roff ? min(granted - roff, rcount) : 0u);
       }
-      sk[threadIdx.x] = k;
-      __syncthreads();
-      for (int off = 1; off < 1024; off <<= 1) {
-        uint32_t a = threadIdx.x >= off ? sk[threadIdx.x - off] : 0;
-        __syncthreads();
-        sk[threadIdx.x] += a;
-        __syncthreads();
-      }
-      if (b < blocks) P.blockCounts[b * 4 + 2] = carry[2] + sk[threadIdx.x] - k;
-      __syncthreads();
-      if (threadIdx.x == 1023) carry[2] += sk[1023];
-      __syncthreads();
+      const uint32_t before = blockScan(k, sums, total);
+      if (b < blocks) P.blockCounts[b * 4 + 2] = active + before;
+      active += total;
     }
     if (threadIdx.x == 0) {
       FpCounters* C = P.counters;
       C->frees = frees;
       C->requests = requests;
       C->granted = granted;
-      C->active = carry[2];
+      C->active = active;
       C->fresh = granted;
     }
-    __syncthreads();
   }
 }
 
 // freeBricks: push freed slots in brick order.
 __global__ void __launch_bounds__(RANK_BLOCK) k_free_bricks(FpBatch bt) {
+  enterChain();
   uint32_t blocks = workTotal(bt, FP_WORK_IDBLOCKS);
   for (uint32_t item = blockIdx.x; item < blocks; item += gridDim.x) {
     uint32_t b;
@@ -214,6 +229,7 @@ __global__ void __launch_bounds__(RANK_BLOCK) k_free_bricks(FpBatch bt) {
 // allocateBricks: grants pop from the stack top in brick order; publish entries and the
 // ascending list of computing bricks; restart each brick's activity flags.
 __global__ void __launch_bounds__(RANK_BLOCK) k_allocate_bricks(FpBatch bt) {
+  enterChain();
   uint32_t blocks = workTotal(bt, FP_WORK_IDBLOCKS);
   for (uint32_t item = blockIdx.x; item < blocks; item += gridDim.x) {
     uint32_t b;
@@ -254,10 +270,48 @@ __global__ void __launch_bounds__(RANK_BLOCK) k_allocate_bricks(FpBatch bt) {
   }
 }
 
-// linkBricks: each slotted brick's 27 neighbour entries and its pressure-unknown flag.
+// finishBricks' commit of each simulation's stack (fluid-allocation.wgsl:354-358), then the
+// prefix offsets of the launch's computing bricks and granted slots. One CTA.
+__device__ void finishBricks(const FpBatch& bt) {
+  __shared__ uint32_t sums[32];
+  const int sims = batchCount(bt);
+  uint32_t* active = bt.work + 1 + FP_WORK_ACTIVE * bt.stride;
+  uint32_t* fresh = bt.work + 1 + FP_WORK_FRESH * bt.stride;
+  uint32_t actives = 0, grants = 0, total;
+  for (int base = 0; base < sims; base += blockDim.x) {
+    const int sim = base + threadIdx.x;
+    uint32_t a = 0, g = 0;
+    if (sim < sims) {
+      FpCounters* C = bt.sims[sim].counters;
+      const int32_t fr = C->freeCount + (int32_t)C->frees;
+      C->freeCount = fr - (int32_t)C->granted;
+      C->failures += C->requests - C->granted;
+      a = C->active;
+      g = C->fresh;
+    }
+    const uint32_t before = blockScan(a, sums, total);
+    if (sim < sims) active[sim] = actives + before;
+    actives += total;
+    const uint32_t granted = blockScan(g, sums, total);
+    if (sim < sims) fresh[sim] = grants + granted;
+    grants += total;
+  }
+  if (threadIdx.x == 0) {
+    active[sims] = actives;
+    fresh[sims] = grants;
+  }
+}
+
+// linkBricks: each slotted brick's 27 neighbour entries and its pressure-unknown flag. The last CTA
+// commits the allocation beside it (neither reads what the other writes).
 __global__ void __launch_bounds__(RANK_BLOCK) k_link_bricks(FpBatch bt) {
+  enterChain();
+  if (blockIdx.x == gridDim.x - 1) {
+    finishBricks(bt);
+    return;
+  }
   uint32_t blocks = workTotal(bt, FP_WORK_IDBLOCKS);
-  for (uint32_t item = blockIdx.x; item < blocks; item += gridDim.x) {
+  for (uint32_t item = blockIdx.x; item < blocks; item += gridDim.x - 1) {
     uint32_t b;
     const SimParams& P = workSim(bt, FP_WORK_IDBLOCKS, item, b);
     uint32_t count = (uint32_t)P.capacity * 64u;
@@ -272,67 +326,22 @@ __global__ void __launch_bounds__(RANK_BLOCK) k_link_bricks(FpBatch bt) {
     H.tx = rec.x;
     H.ty = rec.y;
     H.tz = rec.z;
-    int w[27];
+    int w[28];
+#pragma unroll
     for (int k = 0; k < 27; k++) {
-      int nb = brickIdAt(P, H, bx + k % 3 - 1, by + (k / 3) % 3 - 1, bz + k / 9 - 1);
+      const int nb = nearBrickId(P, H, bx + k % 3 - 1, by + (k / 3) % 3 - 1, bz + k / 9 - 1);
       w[k] = nb >= 0 ? P.entries[nb] : -1;
-      P.records[(size_t)index * FP_RECORD_WORDS + k] = w[k];
     }
-    int unknowns = 1;
+    w[27] = 1;
+#pragma unroll
     for (int k = 0; k < 8; k++) {
-      int dx = -(k & 1), dy = -((k >> 1) & 1), dz = -((k >> 2) & 1);
+      const int dx = -(k & 1), dy = -((k >> 1) & 1), dz = -((k >> 2) & 1);
       if (P.ground && by + dy < 0) continue;
-      if (w[nbrIndex(dx, dy, dz)] < 0) unknowns = 0;
+      if (w[nbrIndex(dx, dy, dz)] < 0) w[27] = 0;
     }
-    P.records[(size_t)index * FP_RECORD_WORDS + 27] = unknowns;
-  }
-}
-
-// finishBricks' commit of each simulation's stack (fluid-allocation.wgsl:354-358), then the
-// prefix offsets of the launch's computing bricks and granted slots. One CTA.
-__global__ void __launch_bounds__(1024) k_finish_bricks(FpBatch bt) {
-  __shared__ uint32_t sa[1024], sg[1024];
-  __shared__ uint32_t carry[2];
-  int sims = batchCount(bt);
-  uint32_t* active = bt.work + 1 + FP_WORK_ACTIVE * bt.stride;
-  uint32_t* fresh = bt.work + 1 + FP_WORK_FRESH * bt.stride;
-  if (threadIdx.x == 0) carry[0] = carry[1] = 0;
-  __syncthreads();
-  for (int base = 0; base < sims; base += 1024) {
-    int sim = base + threadIdx.x;
-    uint32_t a = 0, g = 0;
-    if (sim < sims) {
-      FpCounters* C = bt.sims[sim].counters;
-      int32_t fr = C->freeCount + (int32_t)C->frees;
-      C->freeCount = fr - (int32_t)C->granted;
-      C->failures += C->requests - C->granted;
-      a = C->active;
-      g = C->fresh;
-    }
-    sa[threadIdx.x] = a;
-    sg[threadIdx.x] = g;
-    __syncthreads();
-    for (int off = 1; off < 1024; off <<= 1) {
-      uint32_t x = threadIdx.x >= off ? sa[threadIdx.x - off] : 0, y = threadIdx.x >= off ? sg[threadIdx.x - off] : 0;
-      __syncthreads();
-      sa[threadIdx.x] += x;
-      sg[threadIdx.x] += y;
-      __syncthreads();
-    }
-    if (sim < sims) {
-      active[sim] = carry[0] + sa[threadIdx.x] - a;
-      fresh[sim] = carry[1] + sg[threadIdx.x] - g;
-    }
-    __syncthreads();
-    if (threadIdx.x == 1023) {
-      carry[0] += sa[1023];
-      carry[1] += sg[1023];
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    active[sims] = carry[0];
-    fresh[sims] = carry[1];
+    int4* out = reinterpret_cast<int4*>(P.records + (size_t)index * FP_RECORD_WORDS);
+#pragma unroll
+    for (int k = 0; k < 7; k++) out[k] = make_int4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]);
   }
 }
 
@@ -367,6 +376,7 @@ __device__ bool insideCollider(const SimParams& P, const FpCollider& c, int x, i
 // otherwise the slots granted this step in the simulations that have colliders.
 template <bool ALL>
 __global__ void __launch_bounds__(128) k_build_solids(FpBatch bt) {
+  enterChain();
   const int kind = ALL ? FP_WORK_IDS : FP_WORK_FRESH;
   uint32_t total = workTotal(bt, kind);
   for (uint32_t item = blockIdx.x; item < total; item += gridDim.x) {
@@ -405,6 +415,7 @@ __global__ void __launch_bounds__(128) k_build_solids(FpBatch bt) {
 // A fresh slot starts as still, empty air (fluid-zeroing.wgsl:75-105). Pools every step
 // rewrites before reading need no clearing.
 __global__ void __launch_bounds__(256) k_zero_fresh(FpBatch bt) {
+  enterChain();
   uint32_t total = workTotal(bt, FP_WORK_FRESH);
   for (uint32_t item = blockIdx.x; item < total; item += gridDim.x) {
     uint32_t i;
@@ -434,6 +445,7 @@ __global__ void __launch_bounds__(256) k_zero_fresh(FpBatch bt) {
 // into host-mapped memory; then failed allocations count afresh and the solve's
 // measurements start over. A CTA per simulation.
 __global__ void __launch_bounds__(256) k_readback(FpBatch bt) {
+  enterChain();
   int sims = batchCount(bt);
   const int cw = (int)(sizeof(FpCounters) / 4), sw = (int)(sizeof(FpSolver) / 4);
   for (int sim = blockIdx.x; sim < sims; sim += gridDim.x) {
@@ -463,19 +475,20 @@ __global__ void __launch_bounds__(256) k_readback(FpBatch bt) {
 
 }  // namespace
 
-void fp_launch_allocation(const FpBatch& bt, bool solidsFresh, bool solidsAll, int sms, cudaStream_t st) {
+void fp_launch_allocation(const FpBatch& bt, bool solidsFresh, bool solidsAll, bool overlap, int sms, cudaStream_t st) {
   int grid = sms * 8;
-  k_build_bricks<<<grid, RANK_BLOCK, 0, st>>>(bt);
-  k_scan_blocks<<<sms, 1024, 0, st>>>(bt);
-  k_free_bricks<<<grid, RANK_BLOCK, 0, st>>>(bt);
-  k_allocate_bricks<<<grid, RANK_BLOCK, 0, st>>>(bt);
-  k_link_bricks<<<grid, RANK_BLOCK, 0, st>>>(bt);
-  k_finish_bricks<<<1, 1024, 0, st>>>(bt);
-  if (solidsFresh) k_build_solids<false><<<sms * 4, 128, 0, st>>>(bt);
-  if (solidsAll) k_build_solids<true><<<sms * 4, 128, 0, st>>>(bt);
-  k_zero_fresh<<<sms * 2, 256, 0, st>>>(bt);
+  launchChained(false, k_build_bricks, grid, RANK_BLOCK, 0, st, bt);
+  launchChained(overlap, k_scan_blocks, sms, 1024, 0, st, bt);
+  launchChained(overlap, k_free_bricks, grid, RANK_BLOCK, 0, st, bt);
+  launchChained(overlap, k_allocate_bricks, grid, RANK_BLOCK, 0, st, bt);
+  launchChained(overlap, k_link_bricks, grid + 1, RANK_BLOCK, 0, st, bt);
+  if (solidsFresh) launchChained(overlap, k_build_solids<false>, sms * 4, 128, 0, st, bt);
+  if (solidsAll) launchChained(overlap, k_build_solids<true>, sms * 4, 128, 0, st, bt);
+  launchChained(overlap, k_zero_fresh, sms * 2, 256, 0, st, bt);
 }
 
-int fp_allocation_launches(bool solidsFresh, bool solidsAll) { return 7 + (solidsFresh ? 1 : 0) + (solidsAll ? 1 : 0); }
+int fp_allocation_launches(bool solidsFresh, bool solidsAll) { return 6 + (solidsFresh ? 1 : 0) + (solidsAll ? 1 : 0); }
 
-void fp_launch_readback(const FpBatch& bt, int sms, cudaStream_t st) { k_readback<<<sms, 256, 0, st>>>(bt); }
+void fp_launch_readback(const FpBatch& bt, bool overlap, int sms, cudaStream_t st) {
+  launchChained(overlap, k_readback, sms, 256, 0, st, bt);
+}

@@ -7,13 +7,15 @@
 
 #include "fp_types.h"
 
-void fp_launch_allocation(const FpBatch& bt, bool solidsFresh, bool solidsAll, int sms, cudaStream_t st);
+// `overlap`, here and below: launched while the kernel before it on the stream may still run
+// (fp_overlap.cuh); that one must be the kernel that comes before it in the step.
+void fp_launch_allocation(const FpBatch& bt, bool solidsFresh, bool solidsAll, bool overlap, int sms, cudaStream_t st);
 int fp_allocation_launches(bool solidsFresh, bool solidsAll);
 // The measurement of every simulation into its host-mapped readback words.
-void fp_launch_readback(const FpBatch& bt, int sms, cudaStream_t st);
-void fp_launch_predict(const FpBatch& bt, int B, int vd, int sms, cudaStream_t st);
-void fp_launch_correct(const FpBatch& bt, int B, int vd, int sms, cudaStream_t st);
-void fp_launch_evolve(const FpBatch& bt, int B, int vd, int sms, cudaStream_t st);
+void fp_launch_readback(const FpBatch& bt, bool overlap, int sms, cudaStream_t st);
+void fp_launch_predict(const FpBatch& bt, int B, int vd, bool overlap, int sms, cudaStream_t st);
+void fp_launch_correct(const FpBatch& bt, int B, int vd, bool overlap, int sms, cudaStream_t st);
+void fp_launch_evolve(const FpBatch& bt, int B, int vd, bool overlap, int sms, cudaStream_t st);
 // Coarse smoke (smoke_divisor > 1): advection with the donors' range (it reads only the
 // start-of-step state), then evolution with source production and content flags (after the
 // fine fields' evolution); simulations without coarse smoke skip both. B field cells a brick
@@ -24,7 +26,7 @@ void fp_launch_curl(const FpBatch& bt, int B, int vd, int sms, cudaStream_t st);
 void fp_launch_forces(const FpBatch& bt, int B, int vd, int sms, cudaStream_t st);
 // Divergence with the finest level's first iterate into p0[pSel]; projection with p0[pSel].
 void fp_launch_divergence(const FpBatch& bt, int pSel, int vd, int sms, cudaStream_t st);
-void fp_launch_project(const FpBatch& bt, int pSel, int vd, int sms, cudaStream_t st);
+void fp_launch_project(const FpBatch& bt, int pSel, int vd, bool overlap, int sms, cudaStream_t st);
 void fp_launch_noise(float4* noise, cudaStream_t st);
 
 // Multigrid (pressure.wgsl). Levels below the brick levels live in brick slots, the rest in

@@ -6,6 +6,7 @@
 // solve in one CTA. Brick levels run a CTA per computing brick; tile levels a CTA per tile.
 #include "fp_device.cuh"
 #include "fp_launch.h"
+#include "fp_overlap.cuh"
 
 namespace {
 
@@ -498,13 +499,10 @@ FP_DEV Home enterTile(const SimParams& P, int t, int4 rec) {
 // 9 us however small the level, 24 us a sweep at the finest level of 3.1k bricks, most of it latency.
 enum Leg { REST = 0, DOWN = 1, UP = 2, PUP = 3 };
 
-// Legs may be launched while the one before still runs (MgSel::overlap): a leg lets its successor start
-// at once, and waits for its predecessor where it first reads what that wrote. What it reads before
-// then (parameters, lists, records, flags) was complete before the first of the legs started, which is
-// launched without overlap. Every thread waits before it ends, so that a leg's end is its
-// predecessors' end too. Without overlap both are nothing.
-FP_DEV void letNextStart() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-FP_DEV void waitForPrevious() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Legs may be launched while the one before still runs (MgSel::overlap, fp_overlap.cuh): a leg lets its
+// successor start at once, and waits for its predecessor where it first reads what that wrote. What it
+// reads before then (parameters, lists, records) was complete before the kernel ahead of the first of
+// the legs started.
 // A staged cell's flags: 0 for no unknown (its value becomes zero), else one of
 constexpr uint8_t RIM_OPEN = 0x80;   // an unknown, not solid: the sweeps update it (bits 0-5: its open sides)
 constexpr uint8_t RIM_SOLID = 0x01;  // an unknown that is solid: zero too
@@ -1924,25 +1922,10 @@ static void configureLeg() {
   const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, legKernel<OWNER, LEG>(), K::THREADS, K::SMEM);
   legCtas<OWNER, LEG>() = e == cudaSuccess && n > 0 ? n : 4;
 }
-// A launch that may start while the one before it on the stream still runs.
-template <class Kernel, class... Args>
-static void launch(bool overlap, Kernel kernel, int grid, int threads, size_t smem, cudaStream_t st, Args... args) {
-  cudaLaunchConfig_t c = {};
-  c.gridDim = dim3((unsigned)grid);
-  c.blockDim = dim3((unsigned)threads);
-  c.dynamicSmemBytes = smem;
-  c.stream = st;
-  cudaLaunchAttribute a = {};
-  a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  a.val.programmaticStreamSerializationAllowed = 1;
-  c.attrs = &a;
-  c.numAttrs = overlap ? 1 : 0;
-  cudaLaunchKernelEx(&c, kernel, args...);
-}
 template <int OWNER, int LEG>
 static void legLaunch(const FpBatch& bt, const MgSel& S, int sms, cudaStream_t st) {
   using K = Rim<OWNER == BRICK8 || OWNER == PAIRS ? 8 : 4>;
-  launch(S.overlap, legKernel<OWNER, LEG>(), sms * legCtas<OWNER, LEG>(), K::THREADS, K::SMEM, st, bt, S);
+  launchChained(S.overlap, legKernel<OWNER, LEG>(), sms * legCtas<OWNER, LEG>(), K::THREADS, K::SMEM, st, bt, S);
 }
 
 // Resident CTAs per SM of each staged instantiation, from the occupancy calculator.
@@ -2126,7 +2109,7 @@ constexpr int COARSE_SMALL = 64;
 bool fp_coarse_small(int liveTiles) { return liveTiles <= COARSE_SMALL; }
 void fp_launch_coarse(const FpBatch& bt, const MgSel& S, int iterations, bool small, int sims, int sms, cudaStream_t st) {
   const int smem = small ? COARSE_SMALL * COARSE_SLOT_BYTES : COARSE_SMEM;
-  launch(S.overlap, k_coarse, sims < sms ? sims : sms, small ? 256 : 1024, (size_t)smem, st, bt, S, iterations, smem);
+  launchChained(S.overlap, k_coarse, sims < sms ? sims : sms, small ? 256 : 1024, (size_t)smem, st, bt, S, iterations, smem);
 }
 
 void fp_launch_residual(const FpBatch& bt, int pSel, int cycle, int sms, cudaStream_t st) {

@@ -15,6 +15,7 @@
 // paths compute the same sums in the same order.
 #include "fp_device.cuh"
 #include "fp_launch.h"
+#include "fp_overlap.cuh"
 
 namespace {
 
@@ -556,6 +557,7 @@ FP_DEV void brick_predict(const SimParams* __restrict__ Pp, uint32_t i) {
 }
 template <int MODE>
 __global__ void __launch_bounds__(THREADS, FP_TRANSPORT_CTAS) k_predict(FpBatch bt) {
+  enterChain();
   uint32_t total = workTotal(bt, FP_WORK_ACTIVE);
   for (uint32_t item = blockIdx.x; item < total; item += gridDim.x) {
     uint32_t i;
@@ -658,6 +660,7 @@ FP_DEV void brick_correct(const SimParams* __restrict__ Pp, uint32_t i) {
 }
 template <int MODE>
 __global__ void __launch_bounds__(THREADS, FP_TRANSPORT_CTAS) k_correct(FpBatch bt) {
+  enterChain();
   uint32_t total = workTotal(bt, FP_WORK_ACTIVE);
   for (uint32_t item = blockIdx.x; item < total; item += gridDim.x) {
     uint32_t i;
@@ -901,6 +904,7 @@ FP_DEV void brick_evolve(const SimParams* __restrict__ Pp, uint32_t i) {
 }
 template <int MODE>
 __global__ void __launch_bounds__(THREADS, FP_TRANSPORT_CTAS) k_evolve(FpBatch bt) {
+  enterChain();
   uint32_t total = workTotal(bt, FP_WORK_ACTIVE);
   for (uint32_t item = blockIdx.x; item < total; item += gridDim.x) {
     uint32_t i;
@@ -1307,6 +1311,7 @@ FP_DEV void brick_divergence(const SimParams* __restrict__ Pp, uint32_t i, int p
 }
 template <bool ONE>
 __global__ void __launch_bounds__(THREADS, 6) k_divergence(FpBatch bt, int pSel) {
+  enterChain();
   uint32_t total = workTotal(bt, FP_WORK_ACTIVE);
   for (uint32_t item = blockIdx.x; item < total; item += gridDim.x) {
     uint32_t i;
@@ -1354,6 +1359,7 @@ FP_DEV void brick_project(const SimParams* __restrict__ Pp, uint32_t i, int pSel
 }
 template <bool ONE>
 __global__ void __launch_bounds__(THREADS) k_project(FpBatch bt, int pSel) {
+  enterChain();
   uint32_t total = workTotal(bt, FP_WORK_ACTIVE);
   for (uint32_t item = blockIdx.x; item < total; item += gridDim.x) {
     uint32_t i;
@@ -1731,32 +1737,32 @@ void fp_step_configure(int B) {
 
 // The transport kernels' form for bricks of B field cells and velocity divisor vd.
 static int transportMode(int B, int vd) { return (B == 8 && vd == 1) ? 1 : ((vd > 1 && B == CUBE * vd) ? 2 : 0); }
-void fp_launch_predict(const FpBatch& bt, int B, int vd, int sms, cudaStream_t st) {
+void fp_launch_predict(const FpBatch& bt, int B, int vd, bool overlap, int sms, cudaStream_t st) {
   const int mode = transportMode(B, vd);
   if (mode == 1)
-    k_predict<1><<<sms * FP_TRANSPORT_CTAS, THREADS, stagedBytes(7), st>>>(bt);
+    launchChained(overlap, k_predict<1>, sms * FP_TRANSPORT_CTAS, THREADS, stagedBytes(7), st, bt);
   else if (mode == 2)
-    k_predict<2><<<sms * FP_TRANSPORT_CTAS, THREADS, stagedBytes(7), st>>>(bt);
+    launchChained(overlap, k_predict<2>, sms * FP_TRANSPORT_CTAS, THREADS, stagedBytes(7), st, bt);
   else
-    k_predict<0><<<sms * FP_TRANSPORT_CTAS, THREADS, 0, st>>>(bt);
+    launchChained(overlap, k_predict<0>, sms * FP_TRANSPORT_CTAS, THREADS, 0, st, bt);
 }
-void fp_launch_correct(const FpBatch& bt, int B, int vd, int sms, cudaStream_t st) {
+void fp_launch_correct(const FpBatch& bt, int B, int vd, bool overlap, int sms, cudaStream_t st) {
   const int mode = transportMode(B, vd);
   if (mode == 1)
-    k_correct<1><<<sms * FP_TRANSPORT_CTAS, THREADS, stagedBytes(6), st>>>(bt);
+    launchChained(overlap, k_correct<1>, sms * FP_TRANSPORT_CTAS, THREADS, stagedBytes(6), st, bt);
   else if (mode == 2)
-    k_correct<2><<<sms * FP_TRANSPORT_CTAS, THREADS, stagedBytes(6), st>>>(bt);
+    launchChained(overlap, k_correct<2>, sms * FP_TRANSPORT_CTAS, THREADS, stagedBytes(6), st, bt);
   else
-    k_correct<0><<<sms * FP_TRANSPORT_CTAS, THREADS, 0, st>>>(bt);
+    launchChained(overlap, k_correct<0>, sms * FP_TRANSPORT_CTAS, THREADS, 0, st, bt);
 }
-void fp_launch_evolve(const FpBatch& bt, int B, int vd, int sms, cudaStream_t st) {
+void fp_launch_evolve(const FpBatch& bt, int B, int vd, bool overlap, int sms, cudaStream_t st) {
   const int mode = transportMode(B, vd);
   if (mode == 1)
-    k_evolve<1><<<sms * FP_TRANSPORT_CTAS, THREADS, stagedBytes(7), st>>>(bt);
+    launchChained(overlap, k_evolve<1>, sms * FP_TRANSPORT_CTAS, THREADS, stagedBytes(7), st, bt);
   else if (mode == 2)
-    k_evolve<2><<<sms * FP_TRANSPORT_CTAS, THREADS, stagedBytes(7), st>>>(bt);
+    launchChained(overlap, k_evolve<2>, sms * FP_TRANSPORT_CTAS, THREADS, stagedBytes(7), st, bt);
   else
-    k_evolve<0><<<sms * FP_TRANSPORT_CTAS, THREADS, 0, st>>>(bt);
+    launchChained(overlap, k_evolve<0>, sms * FP_TRANSPORT_CTAS, THREADS, 0, st, bt);
 }
 void fp_launch_curl(const FpBatch& bt, int B, int vd, int sms, cudaStream_t st) {
   if (B == 8 && vd == 1)  // staged: 8^3 bricks, one lattice
@@ -1783,11 +1789,11 @@ void fp_launch_divergence(const FpBatch& bt, int pSel, int vd, int sms, cudaStre
   else
     k_divergence<false><<<sms * 6, THREADS, 0, st>>>(bt, pSel);
 }
-void fp_launch_project(const FpBatch& bt, int pSel, int vd, int sms, cudaStream_t st) {
+void fp_launch_project(const FpBatch& bt, int pSel, int vd, bool overlap, int sms, cudaStream_t st) {
   if (vd == 1)
-    k_project<true><<<sms * 4, THREADS, 0, st>>>(bt, pSel);
+    launchChained(overlap, k_project<true>, sms * 4, THREADS, 0, st, bt, pSel);
   else
-    k_project<false><<<sms * 4, THREADS, 0, st>>>(bt, pSel);
+    launchChained(overlap, k_project<false>, sms * 4, THREADS, 0, st, bt, pSel);
 }
 void fp_launch_noise(float4* noise, cudaStream_t st) { k_noise<<<64 * 64 * 64 / 256, 256, 0, st>>>(noise); }
 void fp_launch_post_divergence(const FpBatch& bt, int sms, cudaStream_t st) {

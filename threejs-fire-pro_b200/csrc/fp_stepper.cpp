@@ -220,7 +220,8 @@ int Stepper::step(Engine* const* sims, const fp_frame* const* frames, const floa
   if ((rc = reserve(header + scene, count, words))) return done(rc);
   FpBatch bt = batch();
   size_t paramsOff = (size_t)((const uint8_t*)bt.sims - arenaD_);
-  size_t off = paramsOff + (size_t)maxSims_ * sizeof(SimParams);
+  // The scenes follow this launch's parameters: room for more simulations is not copied each step.
+  size_t off = align256(paramsOff + (size_t)count * sizeof(SimParams));
   uint32_t* work = reinterpret_cast<uint32_t*>(arenaH_);
   work[0] = (uint32_t)count;
   uint32_t* rowBlocks = work + 1 + FP_WORK_IDBLOCKS * bt.stride;
@@ -366,10 +367,9 @@ int Stepper::readProfile(fp_phase* out, uint32_t* count) {
 void Stepper::vcycle(int level, int cur[], uint64_t& launches) {
   auto sel = [](int l, int which) { return fp_mg_sel(l, which); };
   bool tiles = level >= brickLevels_;
-  if (level == 0) chain_ = false;
   // Whether a leg may overlap the launch before it: one that lets its successor start early.
   auto chained = [&]() {
-    const bool overlap = chain_ && !manyBricks_;
+    const bool overlap = chain_ && !manyBricks_ && !profiling_;
     chain_ = true;
     return overlap;
   };
@@ -446,6 +446,7 @@ void Stepper::vcycleRB(int level, bool zero, uint64_t& launches) {
   const fp_solver_schedule& sc = schedule_;
   const int coarsest = sc.levels > 0 ? std::min(sc.levels - 1, bottom_) : bottom_;
   const bool tiles = level >= brickLevels_;
+  chain_ = false;  // none of these launches is a leg
   const int rhs = level == 0 ? rhs0Sel_ : sel(level, 2), buf = sel(level, 0);
   auto half = [&](int parity, bool fromZero) {
     MgSel S{level, rhs, fromZero ? -1 : buf, -1, buf, -1, cycle_, parity + 1};
@@ -488,7 +489,10 @@ void Stepper::enqueue(bool solidsFresh, bool solidsAll, bool topoAll, bool curl,
   FpBatch bt = batch();
   launches = 0;
   phaseBegin(PH_ALLOC);
-  fp_launch_allocation(bt, solidsFresh, solidsAll, sms_, stream_);
+  // Small launches are latency: each may start while the one before still runs. With many bricks the
+  // chip is full until a kernel's end, and the next one's blocks would only take room.
+  const bool overlap = !profiling_ && !manyBricks_;
+  fp_launch_allocation(bt, solidsFresh, solidsAll, overlap, sms_, stream_);
   int n = fp_allocation_launches(solidsFresh, solidsAll);
   launches += n;
   phaseEnd(PH_ALLOC, n);
@@ -515,10 +519,10 @@ void Stepper::enqueue(bool solidsFresh, bool solidsAll, bool topoAll, bool curl,
   }
   launches += topoAll ? 4 : 2;
   phaseBegin(PH_PREDICT);
-  fp_launch_predict(bt, B_, vd_, sms_, stream_);
+  fp_launch_predict(bt, B_, vd_, overlap, sms_, stream_);
   phaseEnd(PH_PREDICT, 1);
   phaseBegin(PH_CORRECT);
-  fp_launch_correct(bt, B_, vd_, sms_, stream_);
+  fp_launch_correct(bt, B_, vd_, overlap, sms_, stream_);
   phaseEnd(PH_CORRECT, 1);
   // The curl reads only the corrected velocity, and only the forces read it: beside evolution.
   if (fork && curl) {
@@ -528,7 +532,7 @@ void Stepper::enqueue(bool solidsFresh, bool solidsAll, bool topoAll, bool curl,
     cudaEventRecord(joinCurl_, side_);
   }
   phaseBegin(PH_EVOLVE);
-  fp_launch_evolve(bt, B_, vd_, sms_, stream_);
+  fp_launch_evolve(bt, B_, vd_, overlap, sms_, stream_);
   phaseEnd(PH_EVOLVE, 1);
   // Coarse smoke evolves after the fine fields, whose source production it averages, and
   // records content before the measurement.
@@ -546,7 +550,7 @@ void Stepper::enqueue(bool solidsFresh, bool solidsAll, bool topoAll, bool curl,
   // Measurement: counters and the tiles' content flags are final once evolution ran, so they
   // are read here; the next step waits for this event only and prepares while the GPU runs
   // the rest of this step. Failed allocations count from one measurement to the next.
-  fp_launch_readback(bt, sms_, stream_);
+  fp_launch_readback(bt, overlap && !anySmoke_, sms_, stream_);
   launches++;
   // Under capture, external: an event-record node the graph replays.
   if (profiling_)
@@ -576,6 +580,7 @@ void Stepper::enqueue(bool solidsFresh, bool solidsAll, bool topoAll, bool curl,
   launches++;
   phaseEnd(PH_DIVERGENCE, 1);
   cur[0] = 1;
+  chain_ = true;  // the divergence lets its successor start early
   phaseBegin(PH_MULTIGRID);
   uint64_t mg = 0;
   rhs0Sel_ = fp_mg_sel(0, 2);
@@ -594,6 +599,7 @@ void Stepper::enqueue(bool solidsFresh, bool solidsAll, bool topoAll, bool curl,
       x0 = cur[0];
     }
     fp_launch_fcg_begin(bt, x0, sms_, stream_);
+    chain_ = false;
     mg += 2;
     rhs0Sel_ = fp_mg_sel(0, 3);
     for (int c = 1; c < vcycles; c++) {
@@ -607,10 +613,12 @@ void Stepper::enqueue(bool solidsFresh, bool solidsAll, bool topoAll, bool curl,
         fp_launch_relax(bt, S, false, B_ / vd_, sms_, stream_);
         mg++;
         cur[0] = 1;
+        chain_ = false;
         vcycle(0, cur, mg);
         z = cur[0];
       }
       fp_launch_fcg_iterate(bt, z, c, sms_, stream_);
+      chain_ = false;
       mg += fp_fcg_iterate_launches(c);
     }
     rhs0Sel_ = fp_mg_sel(0, 2);
@@ -637,6 +645,7 @@ void Stepper::enqueue(bool solidsFresh, bool solidsAll, bool topoAll, bool curl,
       vcycle(0, cur, mg);
       if (vcycles > 1 || measure) {
         fp_launch_residual(bt, cur[0], c, sms_, stream_);
+        chain_ = false;
         mg += 2;
       }
     }
@@ -646,7 +655,7 @@ void Stepper::enqueue(bool solidsFresh, bool solidsAll, bool topoAll, bool curl,
   launches += mg;
   phaseEnd(PH_MULTIGRID, (int)mg);
   phaseBegin(PH_PROJECT);
-  fp_launch_project(bt, latest, vd_, sms_, stream_);
+  fp_launch_project(bt, latest, vd_, overlap && chain_, sms_, stream_);
   launches++;
   if (measure) {
     fp_launch_post_divergence(bt, sms_, stream_);
