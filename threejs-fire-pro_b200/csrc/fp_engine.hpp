@@ -358,7 +358,10 @@ class Stepper {
   // levels' prolongation run apart from the sweeps: over a wide rim they do their work several times
   // over (finest level up, us: 98 together, 87 apart on 3.1k bricks; 12 and 17 on 90).
   static constexpr uint64_t MANY_BRICKS = 1000;
-  bool manyBricks_ = false;
+  // 8^3-cell blocks of computing bricks an SM up to which the step's launches overlap (a plume of 750
+  // bricks: 457 us a frame with, 481 without; the default grid, 34 blocks an SM: 2842 and 2800).
+  static constexpr uint64_t OVERLAP_BLOCKS = 6;
+  bool manyBricks_ = false, fewBricks_ = false;
   bool coarseSmall_ = false;  // k_coarse in its small form (fp_coarse_small)
   bool single_ = false;       // one simulation
   bool chain_ = false;        // the last multigrid launch was a leg, which the next may overlap

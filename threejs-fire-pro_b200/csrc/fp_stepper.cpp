@@ -237,6 +237,8 @@ int Stepper::step(Engine* const* sims, const fp_frame* const* frames, const floa
   uint64_t bricks = 0;
   for (int i = 0; i < count; i++) bricks += sims[i]->activeBricks();
   manyBricks_ = bricks > (manyBricks_ ? MANY_BRICKS * 7 / 8 : MANY_BRICKS);
+  const uint64_t blocks8 = bricks * (uint64_t)((B_ / 8) * (B_ / 8) * (B_ / 8)), few = (uint64_t)sms_ * OVERLAP_BLOCKS;
+  fewBricks_ = blocks8 <= (fewBricks_ ? few * 9 / 8 : few);
   int vcycles = 1;
   fusedCoarse_ = coarseSmall_ = true;
   single_ = count == 1;
@@ -288,7 +290,7 @@ int Stepper::step(Engine* const* sims, const fp_frame* const* frames, const floa
                    ((uint64_t)schedule_.krylov << 19) | ((uint64_t)schedule_.levels << 20) |
                    ((uint64_t)schedule_.pre_sweeps << 24) | ((uint64_t)schedule_.post_sweeps << 28) |
                    ((uint64_t)schedule_.bottom_sweeps << 32) | ((uint64_t)smokeDiv_ << 40) |
-                   ((uint64_t)manyBricks_ << 44) | ((uint64_t)coarseSmall_ << 45) | ((uint64_t)single_ << 46);
+                   ((uint64_t)manyBricks_ << 44) | ((uint64_t)fewBricks_ << 47) | ((uint64_t)coarseSmall_ << 45) | ((uint64_t)single_ << 46);
     auto it = graphs_.find(key);
     if (it == graphs_.end()) {
       GraphEntry ge{};
@@ -369,7 +371,7 @@ void Stepper::vcycle(int level, int cur[], uint64_t& launches) {
   bool tiles = level >= brickLevels_;
   // Whether a leg may overlap the launch before it: one that lets its successor start early.
   auto chained = [&]() {
-    const bool overlap = chain_ && !manyBricks_ && !profiling_;
+    const bool overlap = chain_ && fewBricks_ && !profiling_;
     chain_ = true;
     return overlap;
   };
@@ -489,9 +491,10 @@ void Stepper::enqueue(bool solidsFresh, bool solidsAll, bool topoAll, bool curl,
   FpBatch bt = batch();
   launches = 0;
   phaseBegin(PH_ALLOC);
-  // Small launches are latency: each may start while the one before still runs. With many bricks the
-  // chip is full until a kernel's end, and the next one's blocks would only take room.
-  const bool overlap = !profiling_ && !manyBricks_;
+  // Small launches are latency: each may start while the one before still runs. With more bricks the
+  // chip is full until a kernel's end, and the next one's waiting blocks take room from the other
+  // stream's kernels.
+  const bool overlap = !profiling_ && fewBricks_;
   fp_launch_allocation(bt, solidsFresh, solidsAll, overlap, sms_, stream_);
   int n = fp_allocation_launches(solidsFresh, solidsAll);
   launches += n;
