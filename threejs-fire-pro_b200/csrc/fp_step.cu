@@ -473,8 +473,16 @@ FP_DEV void cubeOrigin(int B, int k, int& ox, int& oy, int& oz) {
   oz = k / (per * per) * CUBE;
 }
 
+// Form 2 takes a brick in parts, each a CTA's work of its own that stages the velocity again: 630 bricks
+// of 16^3 cells taken whole are a round and a half of the chip, and the default grid's prediction was
+// 223 us (173 in parts), its evolution 318 (239).
+FP_DEV int cubesOf(const FpBatch& bt) {  // of field cells in a brick (one brick size a launch)
+  const int per = bt.sims[0].B / CUBE;
+  return per * per * per;
+}
+// `part` of form 2: 0 the velocity's cells, k the scalars of cube k - 1.
 template <int MODE>
-FP_DEV void brick_predict(const SimParams* __restrict__ Pp, uint32_t i) {
+FP_DEV void brick_predict(const SimParams* __restrict__ Pp, uint32_t i, int part) {
   __shared__ int nslot[27];
   extern __shared__ float smem[];
   const SimParams& P = *Pp;
@@ -495,23 +503,22 @@ FP_DEV void brick_predict(const SimParams* __restrict__ Pp, uint32_t i) {
     float* out = P.velP + slot * 3 * CELLS;
     uint16_t* donors = P.donors + slot * 3 * CELLS;
     stageField<3>(H, 3, CELLS, GV, st, P.vel, 3);
-    stageWait();
-    for (int c = threadIdx.x; c < CELLS; c += THREADS)
-      predictVelocity<CELLS>(VP, H, VL, GV, V, out, donors, c, H.bx * 8 + (c & 7), H.by * 8 + ((c >> 3) & 7),
-                             H.bz * 8 + (c >> 6));
-    const int cubes = (P.B / CUBE) * (P.B / CUBE) * (P.B / CUBE);
-    for (int k = 0; k < cubes; k++) {
+    if (part == 0) {
+      stageWait();
+      for (int c = threadIdx.x; c < CELLS; c += THREADS)
+        predictVelocity<CELLS>(VP, H, VL, GV, V, out, donors, c, H.bx * 8 + (c & 7), H.by * 8 + ((c >> 3) & 7),
+                               H.bz * 8 + (c >> 6));
+    } else {
       int ox, oy, oz;
-      cubeOrigin(P.B, k, ox, oy, oz);
+      cubeOrigin(P.B, part - 1, ox, oy, oz);
       const TransportStage<true> GF =
           stageAt<8 + 2 * HALO>(H.bx * P.B + ox - HALO, H.by * P.B + oy - HALO, H.bz * P.B + oz - HALO);
-      __syncthreads();  // the previous cube's stage has been read
       stageField<4>(H, P.shift, P.N, GF, st + 3 * GV.S3, P.fld, 4, F.half);
       stageWait();
       for (int q = threadIdx.x; q < CUBE * CUBE * CUBE; q += THREADS) {
         const int lx = ox + (q & 7), ly = oy + ((q >> 3) & 7), lz = oz + (q >> 6);
         predictScalars<0, false>(P, VP, H, L, VL, GV, V, GF, F, O, maccormack, noLife, noSmoke,
-                          (lz * P.B + ly) * P.B + lx, H.bx * P.B + lx, H.by * P.B + ly, H.bz * P.B + lz);
+                                 (lz * P.B + ly) * P.B + lx, H.bx * P.B + lx, H.by * P.B + ly, H.bz * P.B + lz);
       }
     }
   } else if constexpr (MODE == 1) {
@@ -559,10 +566,11 @@ template <int MODE>
 __global__ void __launch_bounds__(THREADS, FP_TRANSPORT_CTAS) k_predict(FpBatch bt) {
   enterChain();
   uint32_t total = workTotal(bt, FP_WORK_ACTIVE);
-  for (uint32_t item = blockIdx.x; item < total; item += gridDim.x) {
+  const uint32_t parts = MODE == 2 ? 1 + cubesOf(bt) : 1;
+  for (uint32_t item = blockIdx.x; item < total * parts; item += gridDim.x) {
     uint32_t i;
-    const SimParams& P = workSim(bt, FP_WORK_ACTIVE, item, i);
-    brick_predict<MODE>(&P, i);
+    const SimParams& P = workSim(bt, FP_WORK_ACTIVE, item / parts, i);
+    brick_predict<MODE>(&P, i, (int)(item % parts));
   }
 }
 
@@ -673,8 +681,9 @@ __global__ void __launch_bounds__(THREADS, FP_TRANSPORT_CTAS) k_correct(FpBatch 
 // ---------------------------------------------------------------------------------------
 // evolveFields (fluid-field-evolution.wgsl:9-84) with correctedScalars
 // (fluid-scalar-transport.wgsl:144-199) and recordContent (fluid-content.wgsl:29-64).
+// `part` of form 2: the cube.
 template <int MODE>
-FP_DEV void brick_evolve(const SimParams* __restrict__ Pp, uint32_t i) {
+FP_DEV void brick_evolve(const SimParams* __restrict__ Pp, uint32_t i, int part) {
   __shared__ int nslot[27];
   __shared__ uint32_t busyAll, expandsAll;
   extern __shared__ float smem[];
@@ -853,19 +862,15 @@ FP_DEV void brick_evolve(const SimParams* __restrict__ Pp, uint32_t i) {
   if constexpr (MODE == 2) {
     const TransportStage<true> GV = velocityStage(VP, H);
     stageField<3>(H, 3, CELLS, GV, st, P.vel, 3);
-    const int cubes = (P.B / CUBE) * (P.B / CUBE) * (P.B / CUBE);
-    for (int k = 0; k < cubes; k++) {
-      int ox, oy, oz;
-      cubeOrigin(P.B, k, ox, oy, oz);
-      const TransportStage<true> GF =
-          stageAt<8 + 2 * HALO>(H.bx * P.B + ox - HALO, H.by * P.B + oy - HALO, H.bz * P.B + oz - HALO);
-      if (k > 0) __syncthreads();  // the previous cube's stage has been read
-      stageField<4>(H, P.shift, P.N, GF, st + 3 * GV.S3, P.fldP, 4);
-      stageWait();
-      for (int q = threadIdx.x; q < CUBE * CUBE * CUBE; q += blockDim.x) {
-        const int lx = ox + (q & 7), ly = oy + ((q >> 3) & 7), lz = oz + (q >> 6);
-        cell(GV, GF, (lz * P.B + ly) * P.B + lx, H.bx * P.B + lx, H.by * P.B + ly, H.bz * P.B + lz);
-      }
+    int ox, oy, oz;
+    cubeOrigin(P.B, part, ox, oy, oz);
+    const TransportStage<true> GF =
+        stageAt<8 + 2 * HALO>(H.bx * P.B + ox - HALO, H.by * P.B + oy - HALO, H.bz * P.B + oz - HALO);
+    stageField<4>(H, P.shift, P.N, GF, st + 3 * GV.S3, P.fldP, 4);
+    stageWait();
+    for (int q = threadIdx.x; q < CUBE * CUBE * CUBE; q += THREADS) {
+      const int lx = ox + (q & 7), ly = oy + ((q >> 3) & 7), lz = oz + (q >> 6);
+      cell(GV, GF, (lz * P.B + ly) * P.B + lx, H.bx * P.B + lx, H.by * P.B + ly, H.bz * P.B + lz);
     }
   } else if constexpr (MODE == 1) {
     const TransportStage<true> G = stageOf<true>(P, H);
@@ -881,7 +886,7 @@ FP_DEV void brick_evolve(const SimParams* __restrict__ Pp, uint32_t i) {
       cell(G, G, c, x, y, z);
     }
   }
-  // recordContent (fluid-content.wgsl:43-64): one update per brick.
+  // recordContent (fluid-content.wgsl:43-64): one update per brick, or part of one.
   busy = __reduce_or_sync(0xffffffffu, busy);
   uint32_t ex = __reduce_or_sync(0xffffffffu, (uint32_t)expands);
   if ((threadIdx.x & 31) == 0) {
@@ -898,7 +903,7 @@ FP_DEV void brick_evolve(const SimParams* __restrict__ Pp, uint32_t i) {
       atomicOr(&P.activity[(size_t)P.capacity * 64u + (id >> 6)], bits);
     }
     if (expandsAll) flags |= FP_EXPANDS;
-    if (flags) P.activity[id] |= flags;
+    if (flags) atomicOr(&P.activity[id], flags);
   }
   __syncthreads();
 }
@@ -906,10 +911,11 @@ template <int MODE>
 __global__ void __launch_bounds__(THREADS, FP_TRANSPORT_CTAS) k_evolve(FpBatch bt) {
   enterChain();
   uint32_t total = workTotal(bt, FP_WORK_ACTIVE);
-  for (uint32_t item = blockIdx.x; item < total; item += gridDim.x) {
+  const uint32_t parts = MODE == 2 ? cubesOf(bt) : 1;
+  for (uint32_t item = blockIdx.x; item < total * parts; item += gridDim.x) {
     uint32_t i;
-    const SimParams& P = workSim(bt, FP_WORK_ACTIVE, item, i);
-    brick_evolve<MODE>(&P, i);
+    const SimParams& P = workSim(bt, FP_WORK_ACTIVE, item / parts, i);
+    brick_evolve<MODE>(&P, i, (int)(item % parts));
   }
 }
 
