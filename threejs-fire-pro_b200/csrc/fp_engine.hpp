@@ -296,8 +296,14 @@ class Stepper {
   uint64_t lastUploadBytes() const { return lastUpload_; }
   uint64_t lastReadbackBytes() const { return lastReadback_; }
   const float4* noise() const { return (const float4*)noise_; }
+  // Room to widen FP16 pools in, a piece at a time, before they are copied to the host: allocated by
+  // the first such read and kept; null where the device has none left.
+  float* widenBuffer();
+  cudaError_t readWidened(const void* halves, size_t count, float* host);
 
  private:
+  static constexpr size_t WIDEN_VALUES = (size_t)1 << 21;  // 8 MB
+  float* widen_ = nullptr;
   int device_, B_, brickLevels_, bottom_;
   int vd_ = 0;  // the simulations' velocity divisor, from the first step
   int sms_ = 148;

@@ -28,6 +28,8 @@ void fp_launch_forces(const FpBatch& bt, int B, int vd, int sms, cudaStream_t st
 void fp_launch_divergence(const FpBatch& bt, int pSel, int vd, int sms, cudaStream_t st);
 void fp_launch_project(const FpBatch& bt, int pSel, int vd, bool overlap, int sms, cudaStream_t st);
 void fp_launch_noise(float4* noise, cudaStream_t st);
+// out[i] = the i-th of `count` (a multiple of 4, as every field's is) FP16 values.
+void fp_launch_widen(float* out, const uint16_t* halves, size_t count, int sms, cudaStream_t st);
 
 // Multigrid (pressure.wgsl). Levels below the brick levels live in brick slots, the rest in
 // tile slots. Buffers are named by selector, level * 4 + which: which 0 and 1 are the level's

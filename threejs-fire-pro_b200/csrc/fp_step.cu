@@ -1409,6 +1409,15 @@ __device__ float3 noiseGradient(float px, float py, float pz) {
                      mixf(mixf(c - a, d - b, s[0]), mixf(g - e, h - f1, s[0]), s[2]) * ds[1],
                      mixf(mixf(e - a, f1 - b, s[0]), mixf(g - c, h - d, s[0]), s[1]) * ds[2]);
 }
+// FP16 pools widened for a read-back: bound by the copy to the host that follows (9 us for the 2M
+// values of a buffer, the copy several hundred).
+__global__ void k_widen(float4* __restrict__ out, const ushort4* __restrict__ halves, size_t quads) {
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < quads; i += (size_t)gridDim.x * blockDim.x) {
+    const ushort4 h = halves[i];
+    out[i] = make_float4(__half2float(__ushort_as_half(h.x)), __half2float(__ushort_as_half(h.y)),
+                         __half2float(__ushort_as_half(h.z)), __half2float(__ushort_as_half(h.w)));
+  }
+}
 __global__ void k_noise(float4* __restrict__ out) {
   int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= 64 * 64 * 64) return;
@@ -1803,6 +1812,9 @@ void fp_launch_project(const FpBatch& bt, int pSel, int vd, bool overlap, int sm
     launchChained(overlap, k_project<true>, sms * 4, THREADS, 0, st, bt, pSel);
   else
     launchChained(overlap, k_project<false>, sms * 4, THREADS, 0, st, bt, pSel);
+}
+void fp_launch_widen(float* out, const uint16_t* halves, size_t count, int sms, cudaStream_t st) {
+  k_widen<<<sms * 8, 256, 0, st>>>((float4*)out, (const ushort4*)halves, count / 4);
 }
 void fp_launch_noise(float4* noise, cudaStream_t st) { k_noise<<<64 * 64 * 64 / 256, 256, 0, st>>>(noise); }
 void fp_launch_post_divergence(const FpBatch& bt, int sms, cudaStream_t st) {

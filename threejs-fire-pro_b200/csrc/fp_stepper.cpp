@@ -30,6 +30,7 @@ Stepper::~Stepper() {
   if (arenaD_) cudaFree(arenaD_);
   if (readH_) cudaFreeHost(readH_);
   if (noise_) cudaFree(noise_);
+  if (widen_) cudaFree(widen_);
   if (readEvent_) cudaEventDestroy(readEvent_);
   for (cudaEvent_t e : {forkTopo_, joinTopo_, forkCurl_, joinCurl_, joinSmoke_})
     if (e) cudaEventDestroy(e);
@@ -45,6 +46,39 @@ int Stepper::check(cudaError_t e, const char* what) {
   if (e == cudaSuccess) return FP_OK;
   error_ = std::string(what) + ": " + cudaGetErrorString(e);
   return e == cudaErrorMemoryAllocation ? FP_ENOMEM : FP_EDEVICE;
+}
+
+namespace {
+struct OnDevice {  // the stepper's device, and the caller's again afterwards
+  int before = 0;
+  explicit OnDevice(int device) {
+    cudaGetDevice(&before);
+    if (before != device) cudaSetDevice(device);
+  }
+  ~OnDevice() { cudaSetDevice(before); }
+};
+}  // namespace
+
+float* Stepper::widenBuffer() {
+  OnDevice here(device_);
+  if (!widen_ && cudaMalloc(&widen_, WIDEN_VALUES * sizeof(float)) != cudaSuccess) {
+    cudaGetLastError();  // not an error of the read
+    widen_ = nullptr;
+  }
+  return widen_;
+}
+
+cudaError_t Stepper::readWidened(const void* halves, size_t count, float* host) {
+  OnDevice here(device_);
+  cudaError_t e = cudaSuccess;
+  for (size_t at = 0; at < count && e == cudaSuccess; at += WIDEN_VALUES) {
+    const size_t n = std::min(WIDEN_VALUES, count - at);
+    fp_launch_widen(widen_, (const uint16_t*)halves + at, n, sms_, stream_);
+    if ((e = cudaGetLastError()) == cudaSuccess)
+      e = cudaMemcpyAsync(host + at, widen_, n * sizeof(float), cudaMemcpyDeviceToHost, stream_);
+  }
+  const cudaError_t done = cudaStreamSynchronize(stream_);
+  return e != cudaSuccess ? e : done;
 }
 
 int Stepper::initialize() {
