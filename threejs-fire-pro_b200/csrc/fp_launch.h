@@ -85,7 +85,7 @@ void fp_launch_fcg_iterate(const FpBatch& bt, int zSel, int cycle, int sms, cuda
 int fp_fcg_iterate_launches(int cycle);
 // After the projection: FP64 sums of squares of h x divergence and of the face velocities over
 // the interior unknowns.
-void fp_launch_post_divergence(const FpBatch& bt, int sms, cudaStream_t st);
+void fp_launch_post_divergence(const FpBatch& bt, int vd, int sms, cudaStream_t st);
 // Size the staged brick-level multigrid kernels for bricks of B cells (once per brick size).
 void fp_mg_configure(int B);
 // Set the step kernels' shared-memory limits (before any launch or stream capture).

@@ -695,7 +695,7 @@ void Stepper::enqueue(bool solidsFresh, bool solidsAll, bool topoAll, bool curl,
   fp_launch_project(bt, latest, vd_, overlap && chain_, sms_, stream_);
   launches++;
   if (measure) {
-    fp_launch_post_divergence(bt, sms_, stream_);
+    fp_launch_post_divergence(bt, vd_, sms_, stream_);
     launches++;
   }
   phaseEnd(PH_PROJECT, measure ? 2 : 1);
