@@ -378,7 +378,7 @@ class Stepper {
   int rhs0Sel_ = 2;           // the finest level's right-hand side: the divergence, or the CG residual
   void vcycle(int level, int cur[], uint64_t& launches);
   // One red-black V-cycle from `level` down, in place; from zero when `zero`.
-  void vcycleRB(int level, bool zero, uint64_t& launches);
+  void vcycleRB(int level, bool zero, int cur[], uint64_t& launches);
   int check(cudaError_t e, const char* what);
   int reserve(size_t arenaBytes, int sims, size_t readWords);
 };

@@ -44,6 +44,8 @@ struct MgSel {
   int colour;
   // Launched while the kernel before it on the stream, a leg too, may still run.
   bool overlap;
+  // A red-black leg: its half-sweeps, 2 or 4, alternating from `colour`'s.
+  int halves;
 };
 inline int fp_mg_sel(int level, int which) { return level * 4 + which; }
 void fp_launch_topology(const FpBatch& bt, bool anyAll, int sms, cudaStream_t st);
@@ -60,6 +62,9 @@ bool fp_legs_fused(int level, int B);
 bool fp_leg_per_brick(int level, int B);  // a CTA a brick (the others a CTA a tile)
 void fp_launch_leg_down(const FpBatch& bt, const MgSel& S, int B, int sms, cudaStream_t st);
 void fp_launch_leg_up(const FpBatch& bt, const MgSel& S, int B, int sms, cudaStream_t st);
+// One or two red-black sweeps of such a level in one launch, from S.pin (-1: from zero) to S.pout, the
+// level's other buffer.
+void fp_launch_leg_rb(const FpBatch& bt, const MgSel& S, int B, int sms, cudaStream_t st);
 // The bottom level's iterations, a CTA per simulation.
 void fp_launch_bottom(const FpBatch& bt, const MgSel& S, int iterations, int sms, cudaStream_t st);
 // The V-cycle from the second tile level down in one CTA per simulation (k_coarse): S.level is

@@ -126,7 +126,7 @@ struct Args {
   float* cfirst;
   bool rhsN, pinN, coarseN, poutN, cfirstN;  // the buffer holds BF16
   bool skip;                                 // a later V-cycle of a converged solve: no work
-  int colour;                                // MgSel::colour
+  int colour, halves;                        // MgSel::colour, MgSel::halves
 };
 
 // A launch names its buffers by selector, level * 4 + which (0 and 1 the level's pressure
@@ -153,6 +153,7 @@ FP_DEV Args resolve(const SimParams& P, const MgSel& S) {
   A.cfirstN = S.cfirst >= 0 && narrowLevel(P, S.cfirst >> 2);
   A.skip = S.cycle > 0 && P.solver->converged != 0;
   A.colour = S.colour;
+  A.halves = S.halves;
   return A;
 }
 
@@ -495,9 +496,12 @@ FP_DEV Home enterTile(const SimParams& P, int t, int4 rec) {
 //   DOWN   two sweeps (written: prolongation adds to them) and the restriction of the result
 //   UP     three sweeps
 //   PUP    prolongation from the level below, and three sweeps
+//   RB     red-black, a box four cells out: one or two sweeps (MgSel::halves half-sweeps, in place in the
+//          stage, the first of MgSel::colour), from zero or from the level's values
 // A step alone is a launch that waits for its work list, its brick's neighbours and one stage: 4 to
 // 9 us however small the level, 24 us a sweep at the finest level of 3.1k bricks, most of it latency.
-enum Leg { REST = 0, DOWN = 1, UP = 2, PUP = 3 };
+enum Leg { REST = 0, DOWN = 1, UP = 2, PUP = 3, RB = 4 };
+constexpr int rimOf(int leg) { return leg == RB ? 4 : 3; }
 
 // Legs may be launched while the one before still runs (MgSel::overlap, fp_overlap.cuh): a leg lets its
 // successor start at once, and waits for its predecessor where it first reads what that wrote. What it
@@ -509,32 +513,33 @@ constexpr uint8_t RIM_SOLID = 0x01;  // an unknown that is solid: zero too
 
 // The shapes: OWN cells a side, pieces of 4 values (16 bytes, or 8 in BF16) a row: one before, one
 // after, so that every piece lies in one owner's row.
-template <int OWN>
+template <int OWN, int RIM>
 struct Rim {
-  static constexpr int R = 3, S = OWN + 2 * R;       // the box of values and flags
+  static constexpr int R = RIM, S = OWN + 2 * R;     // the box of values and flags
   static constexpr int PIECES = OWN / 4 + 2, P = OWN == 8 ? 20 : 12;  // a row's pieces; its pitch (bank spread)
-  static constexpr int C = OWN + 4;                  // the box the first sweep covers, and the right-hand sides'
+  static constexpr int C = S - 2;                    // the box the first sweep covers, and the right-hand sides'
   static constexpr int H = OWN / 2, G = H + 4;       // the level below: cells a side, and with a rim of two
   static constexpr int THREADS = OWN == 8 ? 256 : 128;
   static constexpr int VALUES = S * S * P, SWEPT = C * C * P;
-  static constexpr size_t SMEM = (VALUES + 2 * SWEPT + G * G * G) * sizeof(float) + VALUES;
+  static constexpr int OTHER = R == 4 ? 0 : SWEPT, BELOW = R == 4 ? 0 : G * G * G;  // red-black works in place
+  static constexpr size_t SMEM = (VALUES + SWEPT + OTHER + BELOW) * sizeof(float) + VALUES;
 };
 // The shared memory of a box, carved.
-template <int OWN>
+template <int OWN, int R>
 struct RimStage {
   float *val, *rh, *other, *below;
   uint8_t* fl;
   FP_DEV explicit RimStage(float* smem) {
-    using K = Rim<OWN>;
+    using K = Rim<OWN, R>;
     val = smem;
     rh = val + K::VALUES;
     other = rh + K::SWEPT;
-    below = other + K::SWEPT;
-    fl = reinterpret_cast<uint8_t*>(below + K::G * K::G * K::G);
+    below = other + K::OTHER;
+    fl = reinterpret_cast<uint8_t*>(below + K::BELOW);
   }
   // The place of cell (x,y,z), from the owner's first, among the values and flags; among the rest.
-  FP_DEV static int at(int x, int y, int z) { return ((z + 3) * Rim<OWN>::S + y + 3) * Rim<OWN>::P + x + 4; }
-  FP_DEV static int in(int x, int y, int z) { return ((z + 2) * Rim<OWN>::C + y + 2) * Rim<OWN>::P + x + 4; }
+  FP_DEV static int at(int x, int y, int z) { return ((z + R) * Rim<OWN, R>::S + y + R) * Rim<OWN, R>::P + x + 4; }
+  FP_DEV static int in(int x, int y, int z) { return ((z + R - 1) * Rim<OWN, R>::C + y + R - 1) * Rim<OWN, R>::P + x + 4; }
 };
 
 // Four, or two, values of a level from index a.
@@ -556,9 +561,9 @@ FP_DEV uint8_t rimFlag(uint8_t topo, bool unknown) {
 // slots, -1 none), RV cells out for values, RR for right-hand sides, RF for flags: from `topo` and
 // `open(n, low, cell)`, whether cell `cell` of neighbour n, on its low faces on the axes of bits
 // `low`, is an unknown.
-template <int OWN, int RV, int RR, int RF, class Open>
-FP_DEV void stageRim(const RimStage<OWN>& st, const int* nbr, const Args& A, const uint8_t* topo, Open open) {
-  using K = Rim<OWN>;
+template <int RV, int RR, int RF, int OWN, int R, class Open>
+FP_DEV void stageRim(const RimStage<OWN, R>& st, const int* nbr, const Args& A, const uint8_t* topo, Open open) {
+  using K = Rim<OWN, R>;
   constexpr int M = OWN - 1, CELLS = OWN * OWN * OWN, E = OWN + 2 * RV;
   static_assert(RV >= RR && RV >= RF, "the values' box holds the others");
   for (int i = threadIdx.x; i < E * E * K::PIECES; i += K::THREADS) {
@@ -569,7 +574,7 @@ FP_DEV void stageRim(const RimStage<OWN>& st, const int* nbr, const Args& A, con
     const int cell = ((z & M) * OWN + (y & M)) * OWN + (x & M);
     const long at = (long)s * CELLS + cell;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (s >= 0) v = ld4(A.pin, at, A.pinN);
+    if (s >= 0 && (R != 4 || A.pin)) v = ld4(A.pin, at, A.pinN);
     *reinterpret_cast<float4*>(st.val + st.at(x, y, z)) = v;
     auto within = [&](int r) { return y >= -r && y < OWN + r && z >= -r && z < OWN + r; };
     if (within(RR)) {
@@ -582,7 +587,7 @@ FP_DEV void stageRim(const RimStage<OWN>& st, const int* nbr, const Args& A, con
       if (s >= 0) {
         const uchar4 t = *reinterpret_cast<const uchar4*>(topo + at);
         const unsigned low = ((y & M) == 0 ? 2u : 0u) | ((z & M) == 0 ? 4u : 0u);
-        // The piece before the row starts on no low face that a box reaches (OWN > R).
+        // The piece before the row starts on no low face that flags are asked of (OWN > RF).
         const unsigned edge = ((x & M) == 0 && dx >= 0) ? low | 1u : low;
         f = make_uchar4(rimFlag(t.x, open(n, edge, cell)), rimFlag(t.y, open(n, low, cell + 1)),
                         rimFlag(t.z, open(n, low, cell + 2)), rimFlag(t.w, open(n, low, cell + 3)));
@@ -594,10 +599,10 @@ FP_DEV void stageRim(const RimStage<OWN>& st, const int* nbr, const Args& A, con
 // The level below around the owner, a rim of two, as prolongation reads it: coarseValue of every
 // cell. `below(c, n)` gives a cell's index in the level's storage (-1 none) from its neighbour n and
 // its place there; a solid cell's ghost comes through the directory (few cells, near colliders).
-template <int OWN, class Below>
-FP_DEV void stageBelow(const SimParams& P, const Home& H, const RimStage<OWN>& st, const Args& A, int bx, int by, int bz,
+template <int OWN, int R, class Below>
+FP_DEV void stageBelow(const SimParams& P, const Home& H, const RimStage<OWN, R>& st, const Args& A, int bx, int by, int bz,
                        Below below) {
-  using K = Rim<OWN>;
+  using K = Rim<OWN, R>;
   for (int i = threadIdx.x; i < K::G * K::G * K::G; i += K::THREADS) {
     const int x = i % K::G - 2, y = i / K::G % K::G - 2, z = i / (K::G * K::G) - 2;
     const int dx = x < 0 ? -1 : (x >= K::H ? 1 : 0), dy = y < 0 ? -1 : (y >= K::H ? 1 : 0), dz = z < 0 ? -1 : (z >= K::H ? 1 : 0);
@@ -612,9 +617,9 @@ FP_DEV void stageBelow(const SimParams& P, const Home& H, const RimStage<OWN>& s
 }
 // prolongCell of the box, in place; `groundRow`: the lowest row of the level below that is not below
 // the ground (its ghosts mirror the ground).
-template <int OWN>
-FP_DEV void prolongRim(const RimStage<OWN>& st, int groundRow, bool narrow) {
-  using K = Rim<OWN>;
+template <int OWN, int R>
+FP_DEV void prolongRim(const RimStage<OWN, R>& st, int groundRow, bool narrow) {
+  using K = Rim<OWN, R>;
   for (int i = threadIdx.x; i < K::S * K::S * K::S; i += K::THREADS) {
     const int x = i % K::S - K::R, y = i / K::S % K::S - K::R, z = i / (K::S * K::S) - K::R, o = st.at(x, y, z);
     float v = 0.f;
@@ -637,9 +642,9 @@ FP_DEV void prolongRim(const RimStage<OWN>& st, int groundRow, bool narrow) {
 
 // One sweep over the box RIM cells around the owner's cells, from `in` (whose cell (x,y,z) is at
 // place(x,y,z), its rows SZ a layer).
-template <int OWN, int RIM, int SZ, class Place, class Put>
-FP_DEV void sweepBox(const RimStage<OWN>& st, const float* in, Place place, bool narrow, Put put) {
-  using K = Rim<OWN>;
+template <int RIM, int SZ, int OWN, int R, class Place, class Put>
+FP_DEV void sweepBox(const RimStage<OWN, R>& st, const float* in, Place place, bool narrow, Put put) {
+  using K = Rim<OWN, R>;
   constexpr int E = OWN + 2 * RIM;
   for (int i = threadIdx.x; i < E * E * E; i += K::THREADS) {
     const int x = i % E - RIM, y = i / E % E - RIM, z = i / (E * E) - RIM;
@@ -659,30 +664,68 @@ FP_DEV void sweepBox(const RimStage<OWN>& st, const float* in, Place place, bool
     put(x, y, z, v);
   }
 }
+// A red-black half-sweep over the box RIM cells around the owner's, in place: relaxCell's red-black branch,
+// the colour's other cells not touched. The box's last half-sweep is that of RIM 0, so this is the one
+// before it RIM times; nothing where the launch has fewer.
+template <int RIM, int OWN, int R>
+FP_DEV void halfSweep(const RimStage<OWN, R>& st, const Args& A) {
+  using K = Rim<OWN, R>;
+  constexpr int E = OWN + 2 * RIM, HALF = E / 2, sy = K::P, sz = K::S * K::P;
+  if (A.halves <= RIM) return;  // the same for the whole CTA
+  const int colour = (A.colour - 1 + A.halves - 1 - RIM) & 1;
+  for (int i = threadIdx.x; i < E * E * HALF; i += K::THREADS) {
+    const int row = i / HALF, y = row % E - RIM, z = row / E - RIM;
+    // An owner's first cell is even on each axis: the colour's cells of a row from its first or second.
+    const int x = i % HALF * 2 - RIM + ((colour + RIM + y + z) & 1);
+    const int c = st.at(x, y, z);
+    const uint32_t f = st.fl[c];
+    float v = 0.f;
+    if (f & RIM_OPEN) {
+      const float v0 = (f & 1u) ? st.val[c + 1] : 0.f, v1 = (f & 2u) ? st.val[c - 1] : 0.f;
+      const float v2 = (f & 4u) ? st.val[c + sy] : 0.f, v3 = (f & 8u) ? st.val[c - sy] : 0.f;
+      const float v4 = (f & 16u) ? st.val[c + sz] : 0.f, v5 = (f & 32u) ? st.val[c - sz] : 0.f;
+      const float sum = (v0 + v1) + (v2 + v3) + (v4 + v5);
+      v = (sum - st.rh[st.in(x, y, z)]) / fmaxf(diagOf(f & 63u), 1e-12f);
+      if (A.poutN) v = __bfloat162float(__float2bfloat16_rn(v));
+    }
+    st.val[c] = v;
+  }
+  __syncthreads();
+}
 // The leg on a staged box; `own(cell, value)` takes the owner's results. DOWN leaves them (and a rim of
 // one) in st.val at st.in for the restriction.
-template <int OWN, int LEG, class Own>
-FP_DEV void sweepRim(const RimStage<OWN>& st, bool narrow, Own own) {
-  using K = Rim<OWN>;
+template <int LEG, int OWN, int R, class Own>
+FP_DEV void sweepRim(const RimStage<OWN, R>& st, const Args& A, Own own) {
+  using K = Rim<OWN, R>;
+  const bool narrow = A.poutN;
   if constexpr (LEG == REST) return;
+  if constexpr (LEG == RB) {
+    halfSweep<3>(st, A);
+    halfSweep<2>(st, A);
+    halfSweep<1>(st, A);
+    halfSweep<0>(st, A);
+    for (int c = threadIdx.x; c < OWN * OWN * OWN; c += K::THREADS)
+      own(c, st.val[st.at(c % OWN, c / OWN % OWN, c / (OWN * OWN))]);
+    return;
+  }
   auto at = [&](int x, int y, int z) { return st.at(x, y, z); };
   auto in = [&](int x, int y, int z) { return st.in(x, y, z); };
   auto cell = [](int x, int y, int z) { return (z * OWN + y) * OWN + x; };
-  sweepBox<OWN, 2, K::S>(st, st.val, at, narrow, [&](int x, int y, int z, float v) { st.other[st.in(x, y, z)] = v; });
+  sweepBox<2, K::S>(st, st.val, at, narrow, [&](int x, int y, int z, float v) { st.other[st.in(x, y, z)] = v; });
   __syncthreads();
-  sweepBox<OWN, 1, K::C>(st, st.other, in, narrow, [&](int x, int y, int z, float v) {
+  sweepBox<1, K::C>(st, st.other, in, narrow, [&](int x, int y, int z, float v) {
     st.val[st.in(x, y, z)] = v;
     if (LEG == DOWN && x >= 0 && x < OWN && y >= 0 && y < OWN && z >= 0 && z < OWN) own(cell(x, y, z), v);
   });
   __syncthreads();
   if constexpr (LEG == UP || LEG == PUP)
-    sweepBox<OWN, 0, K::C>(st, st.val, in, narrow, [&](int x, int y, int z, float v) { own(cell(x, y, z), v); });
+    sweepBox<0, K::C>(st, st.val, in, narrow, [&](int x, int y, int z, float v) { own(cell(x, y, z), v); });
 }
 // restrictCell of coarse cell q of the owner's (OWN / 2)^3 from the values after DOWN's sweeps, or as
 // staged; whether all its cells are unknowns.
-template <int OWN, int LEG>
-FP_DEV float restrictRim(const RimStage<OWN>& st, int q, bool& every) {
-  using K = Rim<OWN>;
+template <int LEG, int OWN, int R>
+FP_DEV float restrictRim(const RimStage<OWN, R>& st, int q, bool& every) {
+  using K = Rim<OWN, R>;
   const int cx = q % K::H, cy = q / K::H % K::H, cz = q / (K::H * K::H);
   constexpr int sy = K::P, sz = (LEG == DOWN ? K::C : K::S) * K::P;
   float residual = 0.f;
@@ -713,14 +756,16 @@ FP_DEV void storeCoarse(const SimParams& P, const Args& A, long out, float r, bo
   }
   stBf(A.cfirst, out, first, A.cfirstN);
 }
-template <int OWN, int LEG, class Open>
-FP_DEV void stageLeg(const RimStage<OWN>& st, const int* nbr, const Args& A, const uint8_t* topo, Open open) {
+template <int LEG, int OWN, int R, class Open>
+FP_DEV void stageLeg(const RimStage<OWN, R>& st, const int* nbr, const Args& A, const uint8_t* topo, Open open) {
   if constexpr (LEG == REST)
-    stageRim<OWN, 1, 0, 0>(st, nbr, A, topo, open);
+    stageRim<1, 0, 0>(st, nbr, A, topo, open);
+  else if constexpr (LEG == RB)
+    stageRim<4, 3, 3>(st, nbr, A, topo, open);
   else if constexpr (LEG == PUP)
-    stageRim<OWN, 3, 2, 3>(st, nbr, A, topo, open);
+    stageRim<3, 2, 3>(st, nbr, A, topo, open);
   else
-    stageRim<OWN, 3, 2, 2>(st, nbr, A, topo, open);
+    stageRim<3, 2, 2>(st, nbr, A, topo, open);
 }
 // activeCell on a brick level: a cell is an unknown when its brick and those before it on the axes of
 // its low faces compute. Bit n of `ok`: neighbour n does, or lies below the ground (not asked).
@@ -737,12 +782,12 @@ FP_DEV int groundRowOf(const SimParams& P, int firstRow) { return P.ground ? -fi
 // result, the other buffer; REST, DOWN: A.coarse the coarse right-hand side, A.cfirst its first
 // iterate; PUP: A.coarse the level below.
 template <int OWN, int LEG>
-__global__ void __launch_bounds__(Rim<OWN>::THREADS) k_leg_bricks(FpBatch bt, MgSel Sl) {
-  using K = Rim<OWN>;
+__global__ void __launch_bounds__(Rim<OWN, rimOf(LEG)>::THREADS) k_leg_bricks(FpBatch bt, MgSel Sl) {
+  using K = Rim<OWN, rimOf(LEG)>;
   __shared__ int nslot[27];
   __shared__ uint32_t okBits;
   extern __shared__ __align__(16) float rimSmem[];
-  const RimStage<OWN> st(rimSmem);
+  const RimStage<OWN, K::R> st(rimSmem);
   const int t = threadIdx.x;
   letNextStart();
   const uint32_t total = workTotal(bt, FP_WORK_ACTIVE);
@@ -768,21 +813,21 @@ __global__ void __launch_bounds__(Rim<OWN>::THREADS) k_leg_bricks(FpBatch bt, Mg
     __syncthreads();
     const uint32_t ok = okBits;
     waitForPrevious();
-    stageLeg<OWN, LEG>(st, nslot, A, P.topo[A.level], [&](int n, unsigned low, int) { return openIn(ok, n, low); });
+    stageLeg<LEG>(st, nslot, A, P.topo[A.level], [&](int n, unsigned low, int) { return openIn(ok, n, low); });
     if constexpr (LEG == PUP) {
-      stageBelow<OWN>(P, H, st, A, H.bx * K::H, H.by * K::H, H.bz * K::H,
+      stageBelow(P, H, st, A, H.bx * K::H, H.by * K::H, H.bz * K::H,
                       [&](int n, int c) { return nslot[n] < 0 ? -1l : (long)nslot[n] * (K::H * K::H * K::H) + c; });
       __syncthreads();
-      prolongRim<OWN>(st, groundRowOf(P, H.by * K::H), A.poutN);
+      prolongRim(st, groundRowOf(P, H.by * K::H), A.poutN);
     }
     __syncthreads();
     const long slot = nslot[13];
     constexpr int CELLS = OWN * OWN * OWN;
-    sweepRim<OWN, LEG>(st, A.poutN, [&](int c, float v) { stBf(A.pout, slot * CELLS + c, v, A.poutN); });
+    sweepRim<LEG>(st, A, [&](int c, float v) { stBf(A.pout, slot * CELLS + c, v, A.poutN); });
     if constexpr (LEG == DOWN || LEG == REST)
       for (int q = t; q < CELLS / 8; q += K::THREADS) {
         bool every;
-        const float r = restrictRim<OWN, LEG>(st, q, every);
+        const float r = restrictRim<LEG>(st, q, every);
         storeCoarse(P, A, slot * (CELLS / 8) + q, r, every);
       }
   }
@@ -792,12 +837,12 @@ __global__ void __launch_bounds__(Rim<OWN>::THREADS) k_leg_bricks(FpBatch bt, Mg
 // The first tile level (4^3 cells a tile, a cell a brick), a CTA a live tile (a neighbour tile that
 // exists is live).
 template <int LEG>
-__global__ void __launch_bounds__(Rim<4>::THREADS) k_leg_tiles(FpBatch bt, MgSel Sl) {
-  using K = Rim<4>;
+__global__ void __launch_bounds__(Rim<4, rimOf(LEG)>::THREADS) k_leg_tiles(FpBatch bt, MgSel Sl) {
+  using K = Rim<4, rimOf(LEG)>;
   __shared__ int nbr[27];
   __shared__ uint64_t masks[27];
   extern __shared__ __align__(16) float rimSmem[];
-  const RimStage<4> st(rimSmem);
+  const RimStage<4, K::R> st(rimSmem);
   const int t = threadIdx.x;
   letNextStart();
   const uint32_t total = workTotal(bt, FP_WORK_TILES);
@@ -817,19 +862,19 @@ __global__ void __launch_bounds__(Rim<4>::THREADS) k_leg_tiles(FpBatch bt, MgSel
     }
     __syncthreads();
     waitForPrevious();
-    stageLeg<4, LEG>(st, nbr, A, P.topo[A.level], [&](int n, unsigned, int cell) { return ((masks[n] >> cell) & 1ull) != 0ull; });
+    stageLeg<LEG>(st, nbr, A, P.topo[A.level], [&](int n, unsigned, int cell) { return ((masks[n] >> cell) & 1ull) != 0ull; });
     if constexpr (LEG == PUP) {
       const Home H = enterTile(P, tile, rec);
-      stageBelow<4>(P, H, st, A, rec.x * K::H, rec.y * K::H, rec.z * K::H,
+      stageBelow(P, H, st, A, rec.x * K::H, rec.y * K::H, rec.z * K::H,
                     [&](int n, int c) { return nbr[n] < 0 ? -1l : (long)nbr[n] * 8 + c; });
       __syncthreads();
-      prolongRim<4>(st, groundRowOf(P, rec.y * K::H), A.poutN);
+      prolongRim(st, groundRowOf(P, rec.y * K::H), A.poutN);
     }
     __syncthreads();
-    sweepRim<4, LEG>(st, A.poutN, [&](int c, float v) { stBf(A.pout, (long)tile * 64 + c, v, A.poutN); });
+    sweepRim<LEG>(st, A, [&](int c, float v) { stBf(A.pout, (long)tile * 64 + c, v, A.poutN); });
     if (LEG == DOWN && t < 8) {
       bool every;
-      const float r = restrictRim<4, LEG>(st, t, every);
+      const float r = restrictRim<LEG>(st, t, every);
       storeCoarse(P, A, (long)tile * 8 + t, r, every);
     }
   }
@@ -840,14 +885,14 @@ __global__ void __launch_bounds__(Rim<4>::THREADS) k_leg_tiles(FpBatch bt, MgSel
 // CTA a live tile, the tile's 8^3 cells read and written through its bricks' slots, and those of the
 // two bricks around it.
 template <int LEG>
-__global__ void __launch_bounds__(Rim<8>::THREADS) k_leg_pairs(FpBatch bt, MgSel Sl) {
-  using K = Rim<8>;
+__global__ void __launch_bounds__(Rim<8, rimOf(LEG)>::THREADS) k_leg_pairs(FpBatch bt, MgSel Sl) {
+  using K = Rim<8, rimOf(LEG)>;
   constexpr int N = 8;  // bricks a side: the tile's four and two on either side
   __shared__ int nbr[27];
   __shared__ int slots[N * N * N];
   __shared__ uint32_t ok[N * N * N / 32];
   extern __shared__ __align__(16) float rimSmem[];
-  const RimStage<8> st(rimSmem);
+  const RimStage<8, K::R> st(rimSmem);
   const int t = threadIdx.x;
   letNextStart();
   const uint32_t total = workTotal(bt, FP_WORK_TILES);
@@ -883,7 +928,7 @@ __global__ void __launch_bounds__(Rim<8>::THREADS) k_leg_pairs(FpBatch bt, MgSel
       float2 v = make_float2(0.f, 0.f), r = v;
       uchar2 f = make_uchar2(0, 0);
       if (s >= 0) {
-        v = ld2(A.pin, at, A.pinN);
+        if (LEG != RB || A.pin) v = ld2(A.pin, at, A.pinN);
         const uchar2 q = *reinterpret_cast<const uchar2*>(topo + at);
         // The cells of the outermost bricks that a box reaches are on no low face.
         bool in = okAt(b);
@@ -902,21 +947,21 @@ __global__ void __launch_bounds__(Rim<8>::THREADS) k_leg_pairs(FpBatch bt, MgSel
       const int o = st.at(x, y, z);
       *reinterpret_cast<float2*>(st.val + o) = v;
       *reinterpret_cast<uchar2*>(st.fl + o) = f;
-      if (y >= -2 && y < 10 && z >= -2 && z < 10) {
+      if (y > -K::R && y < 7 + K::R && z > -K::R && z < 7 + K::R) {
         if (s >= 0) r = ld2(A.rhs, at, A.rhsN);
         *reinterpret_cast<float2*>(st.rh + st.in(x, y, z)) = r;
       }
     }
     if constexpr (LEG == PUP) {
       const Home H = enterTile(P, tile, rec);
-      stageBelow<8>(P, H, st, A, rec.x * K::H, rec.y * K::H, rec.z * K::H,
+      stageBelow(P, H, st, A, rec.x * K::H, rec.y * K::H, rec.z * K::H,
                     [&](int n, int c) { return nbr[n] < 0 ? -1l : (long)nbr[n] * 64 + c; });
       __syncthreads();
-      prolongRim<8>(st, groundRowOf(P, rec.y * K::H), A.poutN);
+      prolongRim(st, groundRowOf(P, rec.y * K::H), A.poutN);
     }
     __syncthreads();
     auto slotOf = [&](int bx, int by, int bz) { return slots[((bz + 2) * N + by + 2) * N + bx + 2]; };
-    sweepRim<8, LEG>(st, A.poutN, [&](int c, float v) {
+    sweepRim<LEG>(st, A, [&](int c, float v) {
       const int x = c & 7, y = (c >> 3) & 7, z = c >> 6, s = slotOf(x >> 1, y >> 1, z >> 1);
       if (s >= 0) stBf(A.pout, (long)s * 8 + ((z & 1) * 2 + (y & 1)) * 2 + (x & 1), v, A.poutN);
     });
@@ -924,7 +969,7 @@ __global__ void __launch_bounds__(Rim<8>::THREADS) k_leg_pairs(FpBatch bt, MgSel
     // with the tile masks.
     if (LEG == DOWN && t < 64 && slotOf(t & 3, (t >> 2) & 3, t >> 4) >= 0) {
       bool every;
-      const float r = restrictRim<8, LEG>(st, t, every);
+      const float r = restrictRim<LEG>(st, t, every);
       storeCoarse(P, A, (long)tile * 64 + t, r, every);
     }
   }
@@ -1916,7 +1961,7 @@ static int& legCtas() {
 }
 template <int OWNER, int LEG>
 static void configureLeg() {
-  using K = Rim<OWNER == BRICK8 || OWNER == PAIRS ? 8 : 4>;
+  using K = Rim<OWNER == BRICK8 || OWNER == PAIRS ? 8 : 4, rimOf(LEG)>;
   static_assert(K::SMEM <= 46 * 1024, "with the static arrays within the limit a kernel needs no attribute for");
   int n = 0;
   const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, legKernel<OWNER, LEG>(), K::THREADS, K::SMEM);
@@ -1924,7 +1969,7 @@ static void configureLeg() {
 }
 template <int OWNER, int LEG>
 static void legLaunch(const FpBatch& bt, const MgSel& S, int sms, cudaStream_t st) {
-  using K = Rim<OWNER == BRICK8 || OWNER == PAIRS ? 8 : 4>;
+  using K = Rim<OWNER == BRICK8 || OWNER == PAIRS ? 8 : 4, rimOf(LEG)>;
   launchChained(S.overlap, legKernel<OWNER, LEG>(), sms * legCtas<OWNER, LEG>(), K::THREADS, K::SMEM, st, bt, S);
 }
 
@@ -1972,6 +2017,10 @@ void fp_mg_configure(int B) {
   configureLeg<PAIRS, PUP>();
   configureLeg<TILE4, DOWN>();
   configureLeg<TILE4, PUP>();
+  configureLeg<BRICK8, RB>();
+  configureLeg<BRICK4, RB>();
+  configureLeg<PAIRS, RB>();
+  configureLeg<TILE4, RB>();
   configureTileStaged<RELAX, 4>();
   configureTileStaged<RESTRICT, 4>();
   configureTileStaged<PROLONG, 2>();
@@ -2074,7 +2123,7 @@ static void legsLaunch(const FpBatch& bt, const MgSel& S, int B, int sms, cudaSt
     legLaunch<BRICK8, LEG>(bt, S, sms, st);
   } else if (side == 4) {
     legLaunch<BRICK4, LEG>(bt, S, sms, st);
-  } else if constexpr (LEG == DOWN || LEG == PUP) {
+  } else if constexpr (LEG == DOWN || LEG == PUP || LEG == RB) {
     if (side == 2)
       legLaunch<PAIRS, LEG>(bt, S, sms, st);
     else
@@ -2092,6 +2141,9 @@ void fp_launch_leg_up(const FpBatch& bt, const MgSel& S, int B, int sms, cudaStr
     legsLaunch<UP>(bt, S, B, sms, st);
   else
     legsLaunch<PUP>(bt, S, B, sms, st);
+}
+void fp_launch_leg_rb(const FpBatch& bt, const MgSel& S, int B, int sms, cudaStream_t st) {
+  legsLaunch<RB>(bt, S, B, sms, st);
 }
 void fp_launch_restrict(const FpBatch& bt, const MgSel& S, bool tiles, int B, int sms, cudaStream_t st) {
   levelLaunch<RESTRICT>(bt, S, tiles, B, sms, st);

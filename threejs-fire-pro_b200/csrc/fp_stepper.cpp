@@ -472,32 +472,48 @@ void Stepper::vcycle(int level, int cur[], uint64_t& launches) {
   }
 }
 
-// One V-cycle of the red-black schedule (fp_solver_schedule) from `level` down: every level in
-// place in its first buffer, `pre_sweeps` before each restriction, the coarse level from zero,
-// prolongation in place, `post_sweeps` (odd cells first) after it; the coarsest of the
-// schedule's levels takes `bottom_sweeps` (the bottom level in one CTA per simulation). The
-// restriction's first iterate of the coarse level goes to its second buffer, unused.
-void Stepper::vcycleRB(int level, bool zero, uint64_t& launches) {
+// One V-cycle of the red-black schedule (fp_solver_schedule) from `level` down: `pre_sweeps` before each
+// restriction, the coarse level from zero, prolongation in place, `post_sweeps` (odd cells first) after
+// it; the coarsest of the schedule's levels takes `bottom_sweeps` (the bottom level in one CTA per
+// simulation). `cur`: each level's current buffer. The restriction's first iterate of the coarse level
+// goes to its second buffer, unused.
+void Stepper::vcycleRB(int level, bool zero, int cur[], uint64_t& launches) {
   auto sel = [](int l, int which) { return fp_mg_sel(l, which); };
   const fp_solver_schedule& sc = schedule_;
   const int coarsest = sc.levels > 0 ? std::min(sc.levels - 1, bottom_) : bottom_;
   const bool tiles = level >= brickLevels_;
-  chain_ = false;  // none of these launches is a leg
-  const int rhs = level == 0 ? rhs0Sel_ : sel(level, 2), buf = sel(level, 0);
+  chain_ = false;  // none of these launches is overlapped
+  const int rhs = level == 0 ? rhs0Sel_ : sel(level, 2);
+  // Two sweeps a launch where the level has them, each into the level's other buffer; the finest level has
+  // to end in the buffer it started from (a converged simulation skips the later V-cycles).
+  const int flips = level == coarsest ? (sc.bottom_sweeps + 1) / 2 : (sc.pre_sweeps + 1) / 2 + (sc.post_sweeps + 1) / 2;
+  const bool legs = fp_legs_fused(level, B_ / vd_) && (level > 0 || flips % 2 == 0);
   auto half = [&](int parity, bool fromZero) {
+    const int buf = sel(level, cur[level]);
     MgSel S{level, rhs, fromZero ? -1 : buf, -1, buf, -1, cycle_, parity + 1};
     fp_launch_relax(batch(), S, tiles, B_ / vd_, sms_, stream_);
     launches++;
   };
   auto sweeps = [&](int n, bool fromZero, bool post) {
-    for (int i = 0; i < n; i++) {
-      const int first = post ? 1 : 0;
-      half(first, fromZero && i == 0);
-      half(1 - first, false);
+    const int first = post ? 1 : 0;
+    while (n > 0) {
+      const int k = legs ? std::min(n, 2) : 1;
+      if (legs) {
+        MgSel S{level, rhs, fromZero ? -1 : sel(level, cur[level]), -1, sel(level, 1 - cur[level]), -1, cycle_, first + 1, false, 2 * k};
+        fp_launch_leg_rb(batch(), S, B_ / vd_, sms_, stream_);
+        launches++;
+        cur[level] = 1 - cur[level];
+      } else {
+        half(first, fromZero);
+        half(1 - first, false);
+      }
+      fromZero = false;
+      n -= k;
     }
   };
   if (level == coarsest) {
     if (level == bottom_) {
+      const int buf = sel(level, cur[level]);
       MgSel S{level, rhs, zero ? -1 : buf, -1, buf, -1, cycle_, 1};
       fp_launch_bottom_rb(batch(), S, sc.bottom_sweeps, sms_, stream_);
       launches++;
@@ -508,11 +524,13 @@ void Stepper::vcycleRB(int level, bool zero, uint64_t& launches) {
   }
   sweeps(sc.pre_sweeps, zero, false);
   const int coarse = level + 1;
-  MgSel R{coarse, rhs, buf, -1, sel(coarse, 2), sel(coarse, 1), cycle_, 0};
+  MgSel R{coarse, rhs, sel(level, cur[level]), -1, sel(coarse, 2), sel(coarse, 1), cycle_, 0};
   fp_launch_restrict(batch(), R, coarse >= brickLevels_, B_ / vd_, sms_, stream_);
   launches++;
-  vcycleRB(coarse, true, launches);
-  MgSel Pr{level, -1, buf, sel(coarse, 0), buf, -1, cycle_, 0};
+  cur[coarse] = 0;
+  vcycleRB(coarse, true, cur, launches);
+  const int buf = sel(level, cur[level]);
+  MgSel Pr{level, -1, buf, sel(coarse, cur[coarse]), buf, -1, cycle_, 0};
   fp_launch_prolong(batch(), Pr, tiles, B_ / vd_, sms_, stream_);
   launches++;
   sweeps(sc.post_sweeps, false, true);
@@ -628,22 +646,22 @@ void Stepper::enqueue(bool solidsFresh, bool solidsAll, bool topoAll, bool curl,
     // each later V-cycle, from zero on the residual s (level 0's selector 3), gives z, the next
     // direction and step. Simulations that converged skip the later cycles' work.
     cycle_ = 0;
-    int x0 = 0;
     if (redBlack) {
-      vcycleRB(0, true, mg);
+      cur[0] = 0;
+      vcycleRB(0, true, cur, mg);
     } else {
       vcycle(0, cur, mg);
-      x0 = cur[0];
     }
+    const int x0 = cur[0];
     fp_launch_fcg_begin(bt, x0, sms_, stream_);
     chain_ = false;
     mg += 2;
     rhs0Sel_ = fp_mg_sel(0, 3);
     for (int c = 1; c < vcycles; c++) {
       cycle_ = c;
-      int z = 0;
       if (redBlack) {
-        vcycleRB(0, true, mg);
+        cur[0] = 0;
+        vcycleRB(0, true, cur, mg);
       } else {
         // The first iterate from zero (as the divergence kernel writes it for V-cycle 0).
         MgSel S{0, rhs0Sel_, -1, -1, fp_mg_sel(0, 1), -1, cycle_, 0};
@@ -652,8 +670,8 @@ void Stepper::enqueue(bool solidsFresh, bool solidsAll, bool topoAll, bool curl,
         cur[0] = 1;
         chain_ = false;
         vcycle(0, cur, mg);
-        z = cur[0];
       }
+      const int z = cur[0];
       fp_launch_fcg_iterate(bt, z, c, sms_, stream_);
       chain_ = false;
       mg += fp_fcg_iterate_launches(c);
@@ -665,7 +683,8 @@ void Stepper::enqueue(bool solidsFresh, bool solidsAll, bool topoAll, bool curl,
     // skips it and keeps its result in the same buffer).
     for (int c = 0; c < vcycles; c++) {
       cycle_ = c;
-      vcycleRB(0, c == 0, mg);
+      cur[0] = 0;
+      vcycleRB(0, c == 0, cur, mg);
       if (vcycles > 1 || measure) {
         fp_launch_residual(bt, 0, c, sms_, stream_);
         mg += 2;
