@@ -73,6 +73,8 @@ void fp_launch_bottom(const FpBatch& bt, const MgSel& S, int iterations, int sms
 bool fp_coarse_fits(int liveTiles);
 bool fp_coarse_small(int liveTiles);
 void fp_launch_coarse(const FpBatch& bt, const MgSel& S, int iterations, bool small, int sims, int sms, cudaStream_t st);
+// The same of the red-black V-cycle, the second tile level from zero.
+void fp_launch_coarse_rb(const FpBatch& bt, const MgSel& S, int pre, int bottom, int post, bool small, int sims, int sms, cudaStream_t st);
 // After V-cycle `cycle`: the FP64 sums of squares of the finest level's residual (and, after
 // the first, of its right-hand side) over the unknowns, then each simulation's convergence
 // decision. A simulation that converged skips the later cycles.

@@ -484,6 +484,12 @@ void Stepper::vcycleRB(int level, bool zero, int cur[], uint64_t& launches) {
   const bool tiles = level >= brickLevels_;
   chain_ = false;  // none of these launches is overlapped
   const int rhs = level == 0 ? rhs0Sel_ : sel(level, 2);
+  if (fusedCoarse_ && zero && level == brickLevels_ + 1 && coarsest == bottom_) {
+    MgSel S{level, rhs, -1, -1, sel(level, cur[level]), sel(bottom_, 0), cycle_, 0};
+    fp_launch_coarse_rb(batch(), S, sc.pre_sweeps, sc.bottom_sweeps, sc.post_sweeps, coarseSmall_, single_ ? 1 : sms_, sms_, stream_);
+    launches++;
+    return;
+  }
   // Two sweeps a launch where the level has them, each into the level's other buffer; the finest level has
   // to end in the buffer it started from (a converged simulation skips the later V-cycles).
   const int flips = level == coarsest ? (sc.bottom_sweeps + 1) / 2 : (sc.pre_sweeps + 1) / 2 + (sc.post_sweeps + 1) / 2;
