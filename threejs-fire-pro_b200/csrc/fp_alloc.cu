@@ -275,8 +275,8 @@ __global__ void __launch_bounds__(RANK_BLOCK) k_allocate_bricks(FpBatch bt) {
 __device__ void finishBricks(const FpBatch& bt) {
   __shared__ uint32_t sums[32];
   const int sims = batchCount(bt);
-  uint32_t* active = bt.work + 1 + FP_WORK_ACTIVE * bt.stride;
-  uint32_t* fresh = bt.work + 1 + FP_WORK_FRESH * bt.stride;
+  uint32_t* active = bt.work + FP_WORK_HEAD + FP_WORK_ACTIVE * bt.stride;
+  uint32_t* fresh = bt.work + FP_WORK_HEAD + FP_WORK_FRESH * bt.stride;
   uint32_t actives = 0, grants = 0, total;
   for (int base = 0; base < sims; base += blockDim.x) {
     const int sim = base + threadIdx.x;

@@ -14,7 +14,7 @@
 // Work lists of a batch (fp_types.h): the simulations in the launch, a list's total, and the
 // simulation an item belongs to with the item's index in that simulation's own list.
 FP_DEV int batchCount(const FpBatch& b) { return (int)b.work[0]; }
-FP_DEV const uint32_t* workRow(const FpBatch& b, int kind) { return b.work + 1 + kind * b.stride; }
+FP_DEV const uint32_t* workRow(const FpBatch& b, int kind) { return b.work + FP_WORK_HEAD + kind * b.stride; }
 FP_DEV uint32_t workTotal(const FpBatch& b, int kind) { return workRow(b, kind)[batchCount(b)]; }
 FP_DEV const SimParams& workSim(const FpBatch& b, int kind, uint32_t item, uint32_t& local) {
   const uint32_t* row = workRow(b, kind);

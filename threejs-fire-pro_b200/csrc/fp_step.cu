@@ -441,6 +441,31 @@ FP_DEV void predictScalars(const SimParams& P, const SimParams& VP, const Home& 
   for (int k = 0; k < 4; k++) O.pred[k * N + c] = out[k];
 }
 
+// The transport kernels' CTAs take their bricks off a queue: what a brick costs depends on what
+// is in it (every 444th brick a CTA's own: 170, 150 and 151 us to predict, correct and evolve 3.1k bricks;
+// off the queue 161, 148 and 141).
+template <class Work>
+FP_DEV void eachItem(const FpBatch& bt, int queue, uint32_t total, Work work) {
+  __shared__ uint32_t next[2];
+  int k = 0;
+  for (uint32_t item = blockIdx.x; item < total; k ^= 1) {
+    uint32_t taken = 0;
+    if (threadIdx.x == 0) taken = atomicAdd(&bt.work[1 + queue], 1u);  // arrives while the brick is worked on
+    work(item);
+    if (threadIdx.x == 0) next[k] = gridDim.x + taken;
+    __syncthreads();  // the brick's stage has been read, too
+    item = next[k];
+  }
+}
+
+// With fewer bricks than CTAs a launch is as long as a brick: 2, 4 or 8 CTAs then share one, each staging all
+// of it and working on some of its layers.
+FP_DEV int layerParts(uint32_t bricks) {
+  int parts = 1;
+  while (parts < 8 && bricks * parts * 2 <= gridDim.x) parts *= 2;
+  return parts;
+}
+
 // Transport kernels' forms. 0: unstaged (any grid). 1: staged, 8^3 bricks on one lattice.
 // 2: staged, a velocity lattice of 8^3 cells a brick under a finer field lattice (velocity
 // divisor d > 1 with 8 d field cells a brick side): the velocity is staged once over the brick
@@ -480,9 +505,10 @@ FP_DEV int cubesOf(const FpBatch& bt) {  // of field cells in a brick (one brick
   const int per = bt.sims[0].B / CUBE;
   return per * per * per;
 }
-// `part` of form 2: 0 the velocity's cells, k the scalars of cube k - 1.
+// `part` of form 1: of `parts` equal shares of the brick's layers; of form 2: 0 the velocity's cells, k the
+// scalars of cube k - 1.
 template <int MODE>
-FP_DEV void brick_predict(const SimParams* __restrict__ Pp, uint32_t i, int part) {
+FP_DEV void brick_predict(const SimParams* __restrict__ Pp, uint32_t i, int part, int parts) {
   __shared__ int nslot[27];
   extern __shared__ float smem[];
   const SimParams& P = *Pp;
@@ -531,7 +557,8 @@ FP_DEV void brick_predict(const SimParams* __restrict__ Pp, uint32_t i, int part
     stageField<3>(H, 3, CELLS, G, st, P.vel, 3);
     stageField<4>(H, 3, CELLS, G, st + 3 * G.S3, P.fld, 4, F.half);
     stageWait();
-    for (int c = threadIdx.x; c < CELLS; c += THREADS) {
+    const int cells = CELLS / parts;
+    for (int c = part * cells + threadIdx.x; c < (part + 1) * cells; c += THREADS) {
       const int x = H.bx * 8 + (c & 7), y = H.by * 8 + ((c >> 3) & 7), z = H.bz * 8 + (c >> 6);
       predictVelocity<CELLS>(P, H, L, G, V, out, donors, c, x, y, z);
       predictScalars<CELLS, true>(P, P, H, L, L, G, V, G, F, O, maccormack, noLife, noSmoke, c, x, y, z);
@@ -560,25 +587,25 @@ FP_DEV void brick_predict(const SimParams* __restrict__ Pp, uint32_t i, int part
         predictScalars<0, false>(P, VP, H, L, VL, G, V, G, F, O, maccormack, noLife, noSmoke, c, x, y, z);
     }
   }
-  __syncthreads();
 }
 template <int MODE>
 __global__ void __launch_bounds__(THREADS, FP_TRANSPORT_CTAS) k_predict(FpBatch bt) {
   enterChain();
   uint32_t total = workTotal(bt, FP_WORK_ACTIVE);
-  const uint32_t parts = MODE == 2 ? 1 + cubesOf(bt) : 1;
-  for (uint32_t item = blockIdx.x; item < total * parts; item += gridDim.x) {
+  const uint32_t parts = MODE == 2 ? 1 + cubesOf(bt) : (MODE == 1 ? layerParts(total) : 1);
+  eachItem(bt, FP_QUEUE_PREDICT, total * parts, [&](uint32_t item) {
     uint32_t i;
     const SimParams& P = workSim(bt, FP_WORK_ACTIVE, item / parts, i);
-    brick_predict<MODE>(&P, i, (int)(item % parts));
-  }
+    brick_predict<MODE>(&P, i, (int)(item % parts), (int)parts);
+  });
 }
 
 // ---------------------------------------------------------------------------------------
 // correctVelocity (fluid-velocity-transport.wgsl:104-179): bounded MacCormack correction.
 // ONE: the velocity lattice is the field lattice (velocity divisor 1), known at compile time.
+// `part`: staged, of `parts` equal shares of the brick's layers.
 template <bool STAGED, bool ONE>
-FP_DEV void brick_correct(const SimParams* __restrict__ Pp, uint32_t i) {
+FP_DEV void brick_correct(const SimParams* __restrict__ Pp, uint32_t i, int part, int parts) {
   __shared__ int nslot[27];
   extern __shared__ float smem[];
   const SimParams& P = *Pp;
@@ -599,7 +626,8 @@ FP_DEV void brick_correct(const SimParams* __restrict__ Pp, uint32_t i) {
   const int N = STAGED ? CELLS : P.N, shift = STAGED ? 3 : P.shift;
   const uint16_t* __restrict__ donors = P.donors + slot * 3 * N;
   float* __restrict__ out = P.velC + slot * 3 * N;
-  for (int c = threadIdx.x; c < N; c += THREADS) {
+  const int first = STAGED ? part * (CELLS / parts) : 0, end = STAGED ? first + CELLS / parts : N;
+  for (int c = first + threadIdx.x; c < end; c += THREADS) {
     int x, y, z;
     if constexpr (STAGED) {
       x = H.bx * 8 + (c & 7);
@@ -664,26 +692,26 @@ FP_DEV void brick_correct(const SimParams* __restrict__ Pp, uint32_t i) {
       out[comp * N + c] = result;
     }
   }
-  __syncthreads();
 }
 template <int MODE>
 __global__ void __launch_bounds__(THREADS, FP_TRANSPORT_CTAS) k_correct(FpBatch bt) {
   enterChain();
   uint32_t total = workTotal(bt, FP_WORK_ACTIVE);
-  for (uint32_t item = blockIdx.x; item < total; item += gridDim.x) {
+  const uint32_t parts = MODE != 0 ? layerParts(total) : 1;
+  eachItem(bt, FP_QUEUE_CORRECT, total * parts, [&](uint32_t item) {
     uint32_t i;
-    const SimParams& P = workSim(bt, FP_WORK_ACTIVE, item, i);
+    const SimParams& P = workSim(bt, FP_WORK_ACTIVE, item / parts, i);
     // the velocity lattice, 8^3 cells a brick in the staged forms
-    brick_correct<MODE != 0, MODE == 1>(MODE == 1 ? &P : P.vview, i);
-  }
+    brick_correct<MODE != 0, MODE == 1>(MODE == 1 ? &P : P.vview, i, (int)(item % parts), (int)parts);
+  });
 }
 
 // ---------------------------------------------------------------------------------------
 // evolveFields (fluid-field-evolution.wgsl:9-84) with correctedScalars
 // (fluid-scalar-transport.wgsl:144-199) and recordContent (fluid-content.wgsl:29-64).
-// `part` of form 2: the cube.
+// `part` of form 1: of `parts` shares of the layers; of form 2: the cube.
 template <int MODE>
-FP_DEV void brick_evolve(const SimParams* __restrict__ Pp, uint32_t i, int part) {
+FP_DEV void brick_evolve(const SimParams* __restrict__ Pp, uint32_t i, int part, int parts) {
   __shared__ int nslot[27];
   __shared__ uint32_t busyAll, expandsAll;
   extern __shared__ float smem[];
@@ -877,7 +905,9 @@ FP_DEV void brick_evolve(const SimParams* __restrict__ Pp, uint32_t i, int part)
     stageField<3>(H, 3, CELLS, G, st, P.vel, 3);
     stageField<4>(H, 3, CELLS, G, st + 3 * G.S3, P.fldP, 4);
     stageWait();
-    for (int c = threadIdx.x; c < CELLS; c += THREADS) cell(G, G, c, H.bx * 8 + (c & 7), H.by * 8 + ((c >> 3) & 7), H.bz * 8 + (c >> 6));
+    const int cells = CELLS / parts;
+    for (int c = part * cells + threadIdx.x; c < (part + 1) * cells; c += THREADS)
+      cell(G, G, c, H.bx * 8 + (c & 7), H.by * 8 + ((c >> 3) & 7), H.bz * 8 + (c >> 6));
   } else {
     const TransportStage<false> G = stageOf<false>(P, H);
     for (int c = threadIdx.x; c < P.N; c += blockDim.x) {
@@ -905,18 +935,17 @@ FP_DEV void brick_evolve(const SimParams* __restrict__ Pp, uint32_t i, int part)
     if (expandsAll) flags |= FP_EXPANDS;
     if (flags) atomicOr(&P.activity[id], flags);
   }
-  __syncthreads();
 }
 template <int MODE>
 __global__ void __launch_bounds__(THREADS, FP_TRANSPORT_CTAS) k_evolve(FpBatch bt) {
   enterChain();
   uint32_t total = workTotal(bt, FP_WORK_ACTIVE);
-  const uint32_t parts = MODE == 2 ? cubesOf(bt) : 1;
-  for (uint32_t item = blockIdx.x; item < total * parts; item += gridDim.x) {
+  const uint32_t parts = MODE == 2 ? cubesOf(bt) : (MODE == 1 ? layerParts(total) : 1);
+  eachItem(bt, FP_QUEUE_EVOLVE, total * parts, [&](uint32_t item) {
     uint32_t i;
     const SimParams& P = workSim(bt, FP_WORK_ACTIVE, item / parts, i);
-    brick_evolve<MODE>(&P, i, (int)(item % parts));
-  }
+    brick_evolve<MODE>(&P, i, (int)(item % parts), (int)parts);
+  });
 }
 
 // ---------------------------------------------------------------------------------------

@@ -104,7 +104,7 @@ int Stepper::initialize() {
 
 FpBatch Stepper::batch() const {
   FpBatch b;
-  b.sims = reinterpret_cast<const SimParams*>(arenaD_ + align256((size_t)(1 + FP_WORK_KINDS * (maxSims_ + 1)) * 4));
+  b.sims = reinterpret_cast<const SimParams*>(arenaD_ + align256((size_t)(FP_WORK_HEAD + FP_WORK_KINDS * (maxSims_ + 1)) * 4));
   b.work = reinterpret_cast<uint32_t*>(arenaD_);
   b.stride = maxSims_ + 1;
   return b;
@@ -118,7 +118,7 @@ int Stepper::reserve(size_t arenaBytes, int sims, size_t readWords) {
     cudaStreamSynchronize(stream_);
     clearGraphs();
     int nextSims = std::max(sims, maxSims_ * 2);
-    size_t header = align256((size_t)(1 + FP_WORK_KINDS * (nextSims + 1)) * 4) + (size_t)nextSims * sizeof(SimParams);
+    size_t header = align256((size_t)(FP_WORK_HEAD + FP_WORK_KINDS * (nextSims + 1)) * 4) + (size_t)nextSims * sizeof(SimParams);
     size_t cap = std::max(arenaBytes + header, arenaCap_ * 2);
     if (arenaH_) cudaFreeHost(arenaH_);
     if (arenaD_) cudaFree(arenaD_);
@@ -249,7 +249,7 @@ int Stepper::step(Engine* const* sims, const fp_frame* const* frames, const floa
     scene += sims[i]->sceneBytes();
     words += sims[i]->readbackWords();
   }
-  size_t header = align256((size_t)(1 + FP_WORK_KINDS * (std::max(count, maxSims_) + 1)) * 4) +
+  size_t header = align256((size_t)(FP_WORK_HEAD + FP_WORK_KINDS * (std::max(count, maxSims_) + 1)) * 4) +
                   (size_t)std::max(count, maxSims_) * sizeof(SimParams);
   if ((rc = reserve(header + scene, count, words))) return done(rc);
   FpBatch bt = batch();
@@ -258,9 +258,10 @@ int Stepper::step(Engine* const* sims, const fp_frame* const* frames, const floa
   size_t off = align256(paramsOff + (size_t)count * sizeof(SimParams));
   uint32_t* work = reinterpret_cast<uint32_t*>(arenaH_);
   work[0] = (uint32_t)count;
-  uint32_t* rowBlocks = work + 1 + FP_WORK_IDBLOCKS * bt.stride;
-  uint32_t* rowTiles = work + 1 + FP_WORK_TILES * bt.stride;
-  uint32_t* rowIds = work + 1 + FP_WORK_IDS * bt.stride;
+  for (int q = 0; q < FP_QUEUES; q++) work[1 + q] = 0;
+  uint32_t* rowBlocks = work + FP_WORK_HEAD + FP_WORK_IDBLOCKS * bt.stride;
+  uint32_t* rowTiles = work + FP_WORK_HEAD + FP_WORK_TILES * bt.stride;
+  uint32_t* rowIds = work + FP_WORK_HEAD + FP_WORK_IDS * bt.stride;
   uint32_t blocks = 0, tiles = 0, ids = 0;
   size_t word = 0;
   bool solidsFresh = false, solidsAll = false, topoAll = false, curl = false, measure = false;

@@ -252,8 +252,17 @@ enum FpWork {
   FP_WORK_FRESH,     // slots granted this step
   FP_WORK_KINDS
 };
+// Kernels whose CTAs take bricks off a queue: how many were taken beyond each CTA's first, a word a kernel
+// (zeroed by each step's upload).
+enum {
+  FP_QUEUE_PREDICT,
+  FP_QUEUE_CORRECT,
+  FP_QUEUE_EVOLVE,
+  FP_QUEUES
+};
+#define FP_WORK_HEAD (1 + FP_QUEUES)
 struct FpBatch {
   const SimParams* sims;  // one per simulation of the launch
-  uint32_t* work;         // work[0] = simulations; row k at work + 1 + k * stride
+  uint32_t* work;         // work[0] = simulations, then the queues; row k at work + FP_WORK_HEAD + k * stride
   int stride;             // most simulations + 1
 };
