@@ -441,9 +441,9 @@ FP_DEV void predictScalars(const SimParams& P, const SimParams& VP, const Home& 
   for (int k = 0; k < 4; k++) O.pred[k * N + c] = out[k];
 }
 
-// The transport kernels' CTAs take their bricks off a queue: what a brick costs depends on what
-// is in it (every 444th brick a CTA's own: 170, 150 and 151 us to predict, correct and evolve 3.1k bricks;
-// off the queue 161, 148 and 141).
+// The transport kernels' CTAs take their bricks off a queue: what a brick costs depends on what is in it
+// (every 444th brick a CTA's own: 170, 150 and 151 us to predict, correct and evolve 3.1k bricks; off the
+// queue 160, 147 and 143).
 template <class Work>
 FP_DEV void eachItem(const FpBatch& bt, int queue, uint32_t total, Work work) {
   __shared__ uint32_t next[2];
@@ -458,8 +458,8 @@ FP_DEV void eachItem(const FpBatch& bt, int queue, uint32_t total, Work work) {
   }
 }
 
-// With fewer bricks than CTAs a launch is as long as a brick: 2, 4 or 8 CTAs then share one, each staging all
-// of it and working on some of its layers.
+// With fewer bricks than CTAs a launch is as long as a brick: 2, 4 or 8 CTAs then share one, each staging
+// all of it and working on some of its layers (a step of 90 bricks 196 us apart, 189 so).
 FP_DEV int layerParts(uint32_t bricks) {
   int parts = 1;
   while (parts < 8 && bricks * parts * 2 <= gridDim.x) parts *= 2;
@@ -1453,7 +1453,8 @@ __global__ void k_noise(float4* __restrict__ out) {
 // Bound by its reads of the velocity. Whether a cell and its six neighbours are unknowns is asked of one
 // word, the neighbourhood's bricks that compute, and of the neighbours' solids only where that word does
 // not already answer (inside the flow it is full); the sums leave a thread's registers once per simulation
-// that its CTA meets. Asking every cell's bricks through the directory took 139 us a launch on 2.3k bricks, and 64 on 1k; now 28 and 15.
+// that its CTA meets. Asking every cell's bricks through the directory took 139 us a launch on 2.3k bricks
+// and 64 on 1k, this 28 and 15.
 // ONE: one lattice (velocity divisor 1) known at compile time.
 template <bool ONE>
 __global__ void __launch_bounds__(THREADS, 4) k_post_divergence(FpBatch bt) {

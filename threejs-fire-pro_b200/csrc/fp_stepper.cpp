@@ -325,7 +325,8 @@ int Stepper::step(Engine* const* sims, const fp_frame* const* frames, const floa
                    ((uint64_t)schedule_.krylov << 19) | ((uint64_t)schedule_.levels << 20) |
                    ((uint64_t)schedule_.pre_sweeps << 24) | ((uint64_t)schedule_.post_sweeps << 28) |
                    ((uint64_t)schedule_.bottom_sweeps << 32) | ((uint64_t)smokeDiv_ << 40) |
-                   ((uint64_t)manyBricks_ << 44) | ((uint64_t)fewBricks_ << 47) | ((uint64_t)coarseSmall_ << 45) | ((uint64_t)single_ << 46);
+                   ((uint64_t)manyBricks_ << 44) | ((uint64_t)coarseSmall_ << 45) | ((uint64_t)single_ << 46) |
+                   ((uint64_t)fewBricks_ << 47);
     auto it = graphs_.find(key);
     if (it == graphs_.end()) {
       GraphEntry ge{};
