@@ -635,19 +635,23 @@ void Stepper::enqueue(bool solidsFresh, bool solidsAll, bool topoAll, bool curl,
   fp_launch_forces(bt, B_, vd_, sms_, stream_);
   launches++;
   phaseEnd(PH_FORCES, 1);
-  // Cold start every step: the divergence writes the first iterate into p0[1].
+  // Cold start every step. The divergence writes the first iterate into the buffer from which the V-cycles
+  // end in p0[0], whichever form the finest level takes: so a simulation's pools hold the same alone and in
+  // a batch, freed slots too (one flip where prolongation and sweeps are one launch, else two or four).
+  evenFlips_ = vcycles > 1 && schedule_.krylov != FP_KRYLOV_FCG;
+  const bool oneFlip = fp_legs_fused(0, B_ / vd_) && !evenFlips_ && !(manyBricks_ && fp_leg_per_brick(0, B_ / vd_));
+  const int start = oneFlip || schedule_.smoother == FP_SMOOTHER_REDBLACK ? 1 : 0;
   int cur[FP_MAX_LEVELS] = {0};
   if (fork) cudaStreamWaitEvent(stream_, joinTopo_, 0);  // the first iterate reads the topology
   phaseBegin(PH_DIVERGENCE);
-  fp_launch_divergence(bt, 1, vd_, sms_, stream_);
+  fp_launch_divergence(bt, start, vd_, sms_, stream_);
   launches++;
   phaseEnd(PH_DIVERGENCE, 1);
-  cur[0] = 1;
+  cur[0] = start;
   chain_ = true;  // the divergence lets its successor start early
   phaseBegin(PH_MULTIGRID);
   uint64_t mg = 0;
   rhs0Sel_ = fp_mg_sel(0, 2);
-  evenFlips_ = vcycles > 1 && schedule_.krylov != FP_KRYLOV_FCG;
   const bool redBlack = schedule_.smoother == FP_SMOOTHER_REDBLACK;
   if (schedule_.krylov == FP_KRYLOV_FCG) {
     // Flexible CG: V-cycle 0 from the divergence gives the start x (the CG iterate, p0[2]);
