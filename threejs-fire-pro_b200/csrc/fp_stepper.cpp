@@ -13,10 +13,9 @@
 
 #include "fp_engine.hpp"
 #include "fp_launch.h"
+#include "fp_upload.h"
 
 namespace fp {
-
-static size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 
 Stepper::Stepper(int device, int brickSize) : device_(device), B_(brickSize) {
   brickLevels_ = B_ == 8 ? 3 : (B_ == 16 ? 4 : 5);
@@ -104,7 +103,7 @@ int Stepper::initialize() {
 
 FpBatch Stepper::batch() const {
   FpBatch b;
-  b.sims = reinterpret_cast<const SimParams*>(arenaD_ + align256((size_t)(FP_WORK_HEAD + FP_WORK_KINDS * (maxSims_ + 1)) * 4));
+  b.sims = reinterpret_cast<const SimParams*>(arenaD_ + fp_upload_params(maxSims_));
   b.work = reinterpret_cast<uint32_t*>(arenaD_);
   b.stride = maxSims_ + 1;
   return b;
@@ -118,8 +117,7 @@ int Stepper::reserve(size_t arenaBytes, int sims, size_t readWords) {
     cudaStreamSynchronize(stream_);
     clearGraphs();
     int nextSims = std::max(sims, maxSims_ * 2);
-    size_t header = align256((size_t)(FP_WORK_HEAD + FP_WORK_KINDS * (nextSims + 1)) * 4) + (size_t)nextSims * sizeof(SimParams);
-    size_t cap = std::max(arenaBytes + header, arenaCap_ * 2);
+    size_t cap = std::max(arenaBytes + fp_upload_bytes(nextSims, 0), arenaCap_ * 2);
     if (arenaH_) cudaFreeHost(arenaH_);
     if (arenaD_) cudaFree(arenaD_);
     arenaH_ = arenaD_ = nullptr;
@@ -249,13 +247,11 @@ int Stepper::step(Engine* const* sims, const fp_frame* const* frames, const floa
     scene += sims[i]->sceneBytes();
     words += sims[i]->readbackWords();
   }
-  size_t header = align256((size_t)(FP_WORK_HEAD + FP_WORK_KINDS * (std::max(count, maxSims_) + 1)) * 4) +
-                  (size_t)std::max(count, maxSims_) * sizeof(SimParams);
-  if ((rc = reserve(header + scene, count, words))) return done(rc);
+  if ((rc = reserve(fp_upload_bytes(std::max(count, maxSims_), scene), count, words))) return done(rc);
   FpBatch bt = batch();
-  size_t paramsOff = (size_t)((const uint8_t*)bt.sims - arenaD_);
+  size_t paramsOff = fp_upload_params(maxSims_);
   // The scenes follow this launch's parameters: room for more simulations is not copied each step.
-  size_t off = align256(paramsOff + (size_t)count * sizeof(SimParams));
+  size_t off = fp_upload_scenes(maxSims_, count);
   uint32_t* work = reinterpret_cast<uint32_t*>(arenaH_);
   work[0] = (uint32_t)count;
   for (int q = 0; q < FP_QUEUES; q++) work[1 + q] = 0;
