@@ -11,6 +11,7 @@ ROOT = Path(__file__).resolve().parent.parent
 CSRC = ROOT / "threejs-fire-pro_b200" / "csrc"
 PROGRAM = r"""
 #include <cstdio>
+#include <initializer_list>
 #include "fp_upload.h"
 int main() {
   for (int room : {1, 2, 3, 31, 256, 511, 512, 513, 517, 600, 1023, 1025, 4099})
