@@ -3,6 +3,7 @@
 // that their addresses stay the same while simulations come and go; the scenes follow the parameters
 // of the `count` simulations that the step has.
 #pragma once
+#include <cuda_runtime.h>
 #include <stddef.h>
 
 #include "fp_types.h"
