@@ -1,0 +1,63 @@
+"""The render's forms by what the device has room for and by the image's size, against the oracle.
+
+The tolerance is test_gpu_render's: relative L2 2e-3 between the FP32 image and the oracle's FP64
+one of the same state.
+"""
+import numpy as np
+import pytest
+
+from firepro import render, scenes
+from firepro.engine import FluidSimulation
+import parity
+
+pytestmark = pytest.mark.gpu
+
+RENDER_TOL = 2e-3
+
+
+class DiagonalScene(scenes.Scene):
+    """A small fire in every tile along a diagonal: the tiles touch, so one box spans them all,
+    `count` tiles (four bricks each) a side."""
+
+    name = "diagonal"
+
+    def __init__(self, count, seed=1):
+        self.count = count
+        self.settings = scenes.settings(buoyancy=1.0, vorticity=0.0, seed=seed)
+        self.comb = scenes.combustion()
+
+    def frame(self, step):
+        tile = 4 * 8 * self.voxel_size
+        srcs = [scenes.source(1 + k, "sphere", ((k + 0.4) * tile,) * 3, (0.12, 0.12, 0.12), flame=0.8, heat=3.0,
+                              smoke=8.0, velocity=(0.0, 1.0, 0.0), response=30.0) for k in range(self.count)]
+        return scenes.make_frame(self.settings, self.comb, True, srcs)
+
+
+def images(scene, steps, cameras, settings, budget):
+    """Each camera's image of the last step's state, the simulation's and the oracle's."""
+    out = []
+
+    def after(gpu, orc):
+        out.extend((gpu.render(cam, settings), orc.render(cam, settings)) for cam in cameras)
+
+    parity.lockstep(scene, steps, lambda g: FluidSimulation(g), budget=budget, after=after)
+    return out
+
+
+def check(gpu, orc):
+    assert np.isfinite(gpu).all()
+    assert orc[..., 3].max() > 0.05, "something should be visible"
+    assert parity.rel_l2(gpu, orc.astype(np.float64)) <= RENDER_TOL
+
+
+def test_box_too_large_for_tables():
+    """A box of more than 2^24 bricks (66 tiles a side: 258^3 at the least) renders through the tile
+    hash, at both resolutions."""
+    cams = []
+    for half in (0, 1):
+        cam = render.look_at((2.6, 1.3, -1.2), (1.1, 1.1, 1.1), 97, 65, time=0.5)
+        cam.half_resolution = half
+        cams.append(cam)
+    st = render.default_settings(ray_steps=1024, shadow_samples=8)
+    for gpu, orc in images(DiagonalScene(66), 3, cams, st, 2 ** 22):
+        check(gpu, orc)

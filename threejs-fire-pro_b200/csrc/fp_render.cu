@@ -16,6 +16,8 @@
 #include "fp_device.cuh"
 #include "fp_render.h"
 
+#include <type_traits>
+
 namespace {
 
 constexpr int RTHREADS = 128;
@@ -23,29 +25,40 @@ constexpr int RTHREADS = 128;
 // 7 % and 20 % on the slice pass, two 15 %.
 constexpr int MARCH_CTAS = 3;
 
-// A thread's current box: the bricks its samples read.
-struct BoxCursor {
+// A thread's current box, the bricks its samples read, and how it finds a brick's slot: through the
+// boxes' tables, or (no tables, FpRender::pages null) through the tile hash. What follows is compiled for
+// each, so that neither's kernels hold the other's code: one cursor that asks at each lookup took the
+// hash form 10.6 ms for 231,401 rays of 700 bricks, 7.5 for 129,600 of a 1.8k-brick jet and 24.7 for
+// 518,400 of 3.7k bricks (now 6.5, 4.5 and 22.8), the tables 0.95, 0.95 and 4.2 ms (0.87, 0.89, 3.8).
+// Remembering the last two lookups loses: lanes that hit wait for those that miss (24.7 -> 25.9 ms).
+struct TableCursor {
   int lo[3], hi[3];  // in bricks, inclusive
   int first;         // its first entry in FpRender::pages
 };
-FP_DEV BoxCursor noBox() {
-  BoxCursor c;
+struct HashCursor {
+  int lo[3], hi[3];
+};
+template <class Cursor>
+FP_DEV Cursor noBox() {
+  Cursor c;
   for (int a = 0; a < 3; a++) {
     c.lo[a] = 0;
     c.hi[a] = -1;
   }
-  c.first = 0;
+  if constexpr (std::is_same_v<Cursor, TableCursor>) c.first = 0;
   return c;
 }
 // Box k becomes the current one.
-FP_DEV void useBox(const FpRender& R, BoxCursor& c, int k) {
+template <class Cursor>
+FP_DEV void useBox(const FpRender& R, Cursor& c, int k) {
   for (int a = 0; a < 3; a++) {
     c.lo[a] = R.boxes[FP_BOX_INTS * k + a];
     c.hi[a] = R.boxes[FP_BOX_INTS * k + 3 + a];
   }
-  c.first = R.boxes[FP_BOX_INTS * k + 6];
+  if constexpr (std::is_same_v<Cursor, TableCursor>) c.first = R.boxes[FP_BOX_INTS * k + 6];
 }
-FP_DEV bool inBox(const BoxCursor& c, int bx, int by, int bz) {
+template <class Cursor>
+FP_DEV bool inBox(const Cursor& c, int bx, int by, int bz) {
   return bx >= c.lo[0] && bx <= c.hi[0] && by >= c.lo[1] && by <= c.hi[1] && bz >= c.lo[2] && bz <= c.hi[2];
 }
 // The slot of world brick b, or -1, through the tile hash.
@@ -55,13 +68,16 @@ FP_DEV int hashedSlot(const SimParams& P, int bx, int by, int bz) {
   return checkSlot(P, FP_SITE_ENTRY, entryPage(P.entries[t * 64 + (((bz & 3) * 4 + (by & 3)) * 4 + (bx & 3))]));
 }
 // The entry of brick b of the current box in its table.
-FP_DEV int pageIndex(const BoxCursor& c, int bx, int by, int bz) {
+FP_DEV int pageIndex(const TableCursor& c, int bx, int by, int bz) {
   return c.first + ((bz - c.lo[2]) * (c.hi[1] - c.lo[1] + 1) + (by - c.lo[1])) * (c.hi[0] - c.lo[0] + 1) + (bx - c.lo[0]);
 }
 // fireProPage: the slot of world brick b inside the current box, or less than 0 (FpRender::pages).
-FP_DEV int slotAt(const SimParams& P, const FpRender& R, BoxCursor& c, int bx, int by, int bz) {
+FP_DEV int slotAt(const SimParams& P, const FpRender& R, TableCursor& c, int bx, int by, int bz) {
   if (!inBox(c, bx, by, bz)) return -1;
-  return R.pages ? __ldg(&R.pages[pageIndex(c, bx, by, bz)]) : hashedSlot(P, bx, by, bz);
+  return __ldg(&R.pages[pageIndex(c, bx, by, bz)]);
+}
+FP_DEV int slotAt(const SimParams& P, const FpRender&, HashCursor& c, int bx, int by, int bz) {
+  return inBox(c, bx, by, bz) ? hashedSlot(P, bx, by, bz) : -1;
 }
 // Of a low-face cell (lx,ly,lz) of a brick of `side` cells a side, its place in the brick's three
 // apron planes.
@@ -84,7 +100,8 @@ FP_DEV bool apronCell(int side, int i, unsigned before, int& lx, int& ly, int& l
     if ((k & ~on) == 0u && ((before >> k) & 1u)) return true;
   return false;
 }
-FP_DEV unsigned slottedBefore(const SimParams& P, const FpRender& R, BoxCursor& c, int bx, int by, int bz) {
+template <class Cursor>
+FP_DEV unsigned slottedBefore(const SimParams& P, const FpRender& R, Cursor& c, int bx, int by, int bz) {
   unsigned before = 0;
   for (int k = 1; k < 8; k++)
     if (slotAt(P, R, c, bx - (k & 1), by - ((k >> 1) & 1), bz - (k >> 2)) >= 0) before |= 1u << k;
@@ -94,9 +111,10 @@ FP_DEV unsigned slottedBefore(const SimParams& P, const FpRender& R, BoxCursor& 
 // the low (bit clear) or high (bit set) brick on x, y, z (bits 0, 1, 2). n is less than a brick,
 // `sh` the log2 of a brick's cells on the lattice asked about. False unless every one lies in the
 // current box and has a slot. The common case of a sample: its taps then need no lookup each.
-FP_DEV bool slots8(const FpRender& R, const BoxCursor& c, int sh, int x, int y, int z, int n, int* s) {
+FP_DEV bool slots8(const FpRender&, const HashCursor&, int, int, int, int, int, int*) { return false; }
+FP_DEV bool slots8(const FpRender& R, const TableCursor& c, int sh, int x, int y, int z, int n, int* s) {
   const int bx = x >> sh, by = y >> sh, bz = z >> sh, ex = (x + n) >> sh, ey = (y + n) >> sh, ez = (z + n) >> sh;
-  if (!R.pages || bx < c.lo[0] || by < c.lo[1] || bz < c.lo[2] || ex > c.hi[0] || ey > c.hi[1] || ez > c.hi[2])
+  if (bx < c.lo[0] || by < c.lo[1] || bz < c.lo[2] || ex > c.hi[0] || ey > c.hi[1] || ez > c.hi[2])
     return false;
   const int nx = c.hi[0] - c.lo[0] + 1, nxy = nx * (c.hi[1] - c.lo[1] + 1);
   const int* p = R.pages + pageIndex(c, bx, by, bz);
@@ -113,13 +131,15 @@ FP_DEV bool slots8(const FpRender& R, const BoxCursor& c, int sh, int x, int y, 
 FP_DEV float glowOf(float life) { return fminf(fmaxf(life * 5.f, 0.f), 1.f); }  // fireProGlow
 
 // The simulation's smoke at a world cell: zero outside the box or without a slot.
-FP_DEV float rawSmoke(const SimParams& P, const FpRender& R, BoxCursor& c, int x, int y, int z) {
+template <class Cursor>
+FP_DEV float rawSmoke(const SimParams& P, const FpRender& R, Cursor& c, int x, int y, int z) {
   int s = slotAt(P, R, c, x >> P.shift, y >> P.shift, z >> P.shift);
   if (s < 0) return 0.f;
   return ldHalf(P.fld, (size_t)s * 4 * P.N + localCell(P, x, y, z), P.scalarHalf != 0);
 }
 // fireProField of the smoke at `q` in cells: clamped to the box, trilinear.
-FP_DEV float smokeSample(const SimParams& P, const FpRender& R, BoxCursor& c, float qx, float qy, float qz) {
+template <class Cursor>
+FP_DEV float smokeSample(const SimParams& P, const FpRender& R, Cursor& c, float qx, float qy, float qz) {
   float B = (float)P.B;
   qx = fminf(fmaxf(qx, (float)c.lo[0] * B + .5f), (float)(c.hi[0] + 1) * B - .5f);
   qy = fminf(fmaxf(qy, (float)c.lo[1] * B + .5f), (float)(c.hi[1] + 1) * B - .5f);
@@ -136,7 +156,8 @@ FP_DEV float smokeSample(const SimParams& P, const FpRender& R, BoxCursor& c, fl
   return v;
 }
 // smoothSmoke's [1,2,1]/4 density at a world cell: eight half-offset samples.
-FP_DEV float smoothedSmoke(const SimParams& P, const FpRender& R, BoxCursor& c, int x, int y, int z) {
+template <class Cursor>
+FP_DEV float smoothedSmoke(const SimParams& P, const FpRender& R, Cursor& c, int x, int y, int z) {
   float d = 0.f;
   for (int k = 0; k < 8; k++)
     d += smokeSample(P, R, c, (float)(x + (k & 1)), (float)(y + ((k >> 1) & 1)), (float)(z + (k >> 2)));
@@ -145,14 +166,16 @@ FP_DEV float smoothedSmoke(const SimParams& P, const FpRender& R, BoxCursor& c, 
 
 // The coarse smoke grid (smoke_divisor d > 1): 2^P.smokeShift cells a brick side.
 // The simulation's coarse density at a coarse cell: zero outside the box or without a slot.
-FP_DEV float rawCoarse(const SimParams& P, const FpRender& R, BoxCursor& c, int x, int y, int z) {
+template <class Cursor>
+FP_DEV float rawCoarse(const SimParams& P, const FpRender& R, Cursor& c, int x, int y, int z) {
   const int sh = P.smokeShift, m = (1 << sh) - 1;
   int s = slotAt(P, R, c, x >> sh, y >> sh, z >> sh);
   if (s < 0) return 0.f;
   return ldHalf(P.smk, (size_t)s * P.smokeCells + (((z & m) << sh | (y & m)) << sh | (x & m)), P.scalarHalf != 0);
 }
 // fireProField of the coarse density at `q` in coarse cells: clamped to the box, trilinear.
-FP_DEV float coarseSample(const SimParams& P, const FpRender& R, BoxCursor& c, float qx, float qy, float qz) {
+template <class Cursor>
+FP_DEV float coarseSample(const SimParams& P, const FpRender& R, Cursor& c, float qx, float qy, float qz) {
   float S = (float)(1 << P.smokeShift);
   qx = fminf(fmaxf(qx, (float)c.lo[0] * S + .5f), (float)(c.hi[0] + 1) * S - .5f);
   qy = fminf(fmaxf(qy, (float)c.lo[1] * S + .5f), (float)(c.hi[1] + 1) * S - .5f);
@@ -169,7 +192,8 @@ FP_DEV float coarseSample(const SimParams& P, const FpRender& R, BoxCursor& c, f
   return v;
 }
 // smoothCoarseSmoke (lighting.wgsl:104-129): the [1,2,1]/4 density at a coarse cell.
-FP_DEV float smoothedCoarse(const SimParams& P, const FpRender& R, BoxCursor& c, int x, int y, int z) {
+template <class Cursor>
+FP_DEV float smoothedCoarse(const SimParams& P, const FpRender& R, Cursor& c, int x, int y, int z) {
   float d = 0.f;
   for (int k = 0; k < 8; k++)
     d += coarseSample(P, R, c, (float)(x + (k & 1)), (float)(y + ((k >> 1) & 1)), (float)(z + (k >> 2)));
@@ -177,7 +201,8 @@ FP_DEV float smoothedCoarse(const SimParams& P, const FpRender& R, BoxCursor& c,
 }
 // The smoothed coarse density at a coarse cell: the pool in a brick with a slot, else what a
 // sample based in a slotted brick reads from its apron (`apron`), else zero.
-FP_DEV float renderSmokeCell(const SimParams& P, const FpRender& R, BoxCursor& c, int x, int y, int z, bool apron) {
+template <class Cursor>
+FP_DEV float renderSmokeCell(const SimParams& P, const FpRender& R, Cursor& c, int x, int y, int z, bool apron) {
   const int sh = P.smokeShift, m = (1 << sh) - 1;
   int s = slotAt(P, R, c, x >> sh, y >> sh, z >> sh);
   if (s >= 0) return R.renderSmoke[(size_t)s * P.smokeCells + (((z & m) << sh | (y & m)) << sh | (x & m))];
@@ -187,7 +212,8 @@ FP_DEV float renderSmokeCell(const SimParams& P, const FpRender& R, BoxCursor& c
 }
 // renderSmokeAt (volume-common.wgsl:74-78): fireProField of the smoothed coarse density at `q`
 // in coarse cells.
-FP_DEV float renderSmokeAt(const SimParams& P, const FpRender& R, BoxCursor& c, float qx, float qy, float qz) {
+template <class Cursor>
+FP_DEV float renderSmokeAt(const SimParams& P, const FpRender& R, Cursor& c, float qx, float qy, float qz) {
   const int sh = P.smokeShift;
   float S = (float)(1 << sh);
   qx = fminf(fmaxf(qx, (float)c.lo[0] * S + .5f), (float)(c.hi[0] + 1) * S - .5f);
@@ -219,7 +245,8 @@ FP_DEV float renderSmokeAt(const SimParams& P, const FpRender& R, BoxCursor& c, 
 }
 // cachedSmokeCell (lighting.wgsl:133-156): the smoothed coarse density a conservative bound
 // reads at coarse cell (x,y,z): the pool, else the apron a previous neighbour holds.
-FP_DEV float cachedSmokeCell(const SimParams& P, const FpRender& R, BoxCursor& c, int x, int y, int z) {
+template <class Cursor>
+FP_DEV float cachedSmokeCell(const SimParams& P, const FpRender& R, Cursor& c, int x, int y, int z) {
   const int sh = P.smokeShift, m = (1 << sh) - 1;
   int bx = x >> sh, by = y >> sh, bz = z >> sh;
   int s = slotAt(P, R, c, bx, by, bz);
@@ -237,7 +264,8 @@ FP_DEV float cachedSmokeCell(const SimParams& P, const FpRender& R, BoxCursor& c
 // brick without one reads as the apron of a sample based in a slotted brick would hold it
 // (`apron`: the smoothed density, no heat, flame or fuel; all zero with coarse smoke, whose
 // field apron holds no neighbour), else zero.
-FP_DEV float4 renderCell(const SimParams& P, const FpRender& R, BoxCursor& c, int x, int y, int z, bool apron) {
+template <class Cursor>
+FP_DEV float4 renderCell(const SimParams& P, const FpRender& R, Cursor& c, int x, int y, int z, bool apron) {
   int s = slotAt(P, R, c, x >> P.shift, y >> P.shift, z >> P.shift);
   if (s >= 0) return __ldg(&R.renderField[(size_t)s * P.N + localCell(P, x, y, z)]);
   if (!apron || P.smokeDiv > 1) return make_float4(0.f, 0.f, 0.f, 0.f);
@@ -256,7 +284,8 @@ FP_DEV void add4(float4& a, const float4& b, float w) {
 // The trilinear sample of the 2x2x2 block from cell (x0,y0,z0) when a cell of it has no slot or
 // lies past the box: a lookup a cell. Out of line, so that the rare path costs the march and the
 // lighting neither registers nor instruction-cache space.
-static __device__ __noinline__ float4 renderSampleFar(const SimParams& P, const FpRender& R, BoxCursor c, int x0, int y0,
+template <class Cursor>
+static __device__ __noinline__ float4 renderSampleFar(const SimParams& P, const FpRender& R, Cursor c, int x0, int y0,
                                                       int z0, float fx, float fy, float fz) {
   bool based = slotAt(P, R, c, x0 >> P.shift, y0 >> P.shift, z0 >> P.shift) >= 0;
   float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -268,7 +297,8 @@ static __device__ __noinline__ float4 renderSampleFar(const SimParams& P, const 
   return v;
 }
 // fireProField of the render field at `q` in cells (fireProSample, volume-bricks.wgsl).
-FP_DEV float4 renderSample(const SimParams& P, const FpRender& R, BoxCursor& c, float qx, float qy, float qz) {
+template <class Cursor>
+FP_DEV float4 renderSample(const SimParams& P, const FpRender& R, Cursor& c, float qx, float qy, float qz) {
   float B = (float)P.B;
   qx = fminf(fmaxf(qx, (float)c.lo[0] * B + .5f), (float)(c.hi[0] + 1) * B - .5f);
   qy = fminf(fmaxf(qy, (float)c.lo[1] * B + .5f), (float)(c.hi[1] + 1) * B - .5f);
@@ -358,7 +388,8 @@ FP_DEV float4 tensorSample(const SimParams& P, const FpRender& R, const int* slo
 
 // The B-spline as eight trilinear samples, when a cell of its block has no slot or lies past the
 // box (each sample then decides by itself what the missing cells hold and where it clamps).
-static __device__ __noinline__ float4 reconstructFar(const SimParams& P, const FpRender& R, BoxCursor c, float px,
+template <class Cursor>
+static __device__ __noinline__ float4 reconstructFar(const SimParams& P, const FpRender& R, Cursor c, float px,
                                                      float py, float pz, int mode) {
   float pos[2][3], wt[2][3];
   float p[3] = {px, py, pz};
@@ -396,7 +427,8 @@ static __device__ __noinline__ float4 reconstructFar(const SimParams& P, const F
 // under the spline once each: with every one of them in a slotted brick of the box (the window then
 // clamps nowhere) the same sum is taken over the cells directly, one vector load and two packed
 // multiply-adds a cell.
-FP_DEV float4 reconstruct(const SimParams& P, const FpRender& R, BoxCursor& c, float px, float py, float pz, int mode) {
+template <class Cursor>
+FP_DEV float4 reconstruct(const SimParams& P, const FpRender& R, Cursor& c, float px, float py, float pz, int mode) {
   if (mode == 0) return renderSample(P, R, c, px, py, pz);
   float w[3][4];
   int first[3];
@@ -469,7 +501,8 @@ FP_DEV float3 emissionOf(const FpRender& R, const Tint& tint, const float4& f) {
 
 // sampleWorld (volume-common.wgsl:33-43): the render field at world point p, zero outside
 // the box.
-FP_DEV float4 sampleWorld(const SimParams& P, const FpRender& R, BoxCursor& c, float px, float py, float pz) {
+template <class Cursor>
+FP_DEV float4 sampleWorld(const SimParams& P, const FpRender& R, Cursor& c, float px, float py, float pz) {
   float size = (float)P.B * P.h;
   if (px < (float)c.lo[0] * size || py < (float)c.lo[1] * size || pz < (float)c.lo[2] * size ||
       px > (float)(c.hi[0] + 1) * size || py > (float)(c.hi[1] + 1) * size || pz > (float)(c.hi[2] + 1) * size)
@@ -483,7 +516,8 @@ FP_DEV float4 sampleWorld(const SimParams& P, const FpRender& R, BoxCursor& c, f
 }
 
 // exitDistance (lighting.wgsl:248-255).
-FP_DEV float exitDistance(const SimParams& P, const BoxCursor& c, float px, float py, float pz, float dx, float dy,
+template <class Cursor>
+FP_DEV float exitDistance(const SimParams& P, const Cursor& c, float px, float py, float pz, float dx, float dy,
                           float dz) {
   float size = (float)P.B * P.h;
   float p[3] = {px, py, pz}, d[3] = {dx, dy, dz}, m = 1e30f;
@@ -510,7 +544,8 @@ FP_DEV float glowRay(int d, int axis) {
   return sign * (axis == 0 ? .48f : (axis == 1 ? .64f : .6f));
 }
 // incidentLight (lighting.wgsl:257-310): glow RGB and the sun's transmittance at p.
-FP_DEV float4 incidentLight(const SimParams& P, const FpRender& R, BoxCursor& c, float px, float py, float pz) {
+template <class Cursor>
+FP_DEV float4 incidentLight(const SimParams& P, const FpRender& R, Cursor& c, float px, float py, float pz) {
   const Tint tint = tintOf(R);
   float4 local = sampleWorld(P, R, c, px, py, pz);
   if (local.x + glowOf(local.z) < 1e-5f) return make_float4(0.f, 0.f, 0.f, 1.f);
@@ -552,7 +587,8 @@ FP_DEV float4 incidentLight(const SimParams& P, const FpRender& R, BoxCursor& c,
 
 // The brick of computing brick `i` inside a box, that box made the current one, with its
 // slot; false when no box holds it.
-FP_DEV bool boxBrick(const SimParams& P, const FpRender& R, BoxCursor& c, uint32_t i, int& bx, int& by, int& bz,
+template <class Cursor>
+FP_DEV bool boxBrick(const SimParams& P, const FpRender& R, Cursor& c, uint32_t i, int& bx, int& by, int& bz,
                      int& slot) {
   uint32_t id = P.active[i];
   if (!homeOk(P, id)) return false;  // the bounds-checked build only
@@ -623,8 +659,8 @@ FP_DEV uint32_t apronTotal(const FpRender& R) { return R.apronCap ? (uint32_t)mi
 struct SmoothStage {
   float cells[1000], corners[729];
 };
-template <class Raw, class Put>
-FP_DEV void smoothBlock(const BoxCursor& c, SmoothStage& st, int sh, int ox, int oy, int oz, int bs, Raw raw, Put put) {
+template <class Cursor, class Raw, class Put>
+FP_DEV void smoothBlock(const Cursor& c, SmoothStage& st, int sh, int ox, int oy, int oz, int bs, Raw raw, Put put) {
   const int S = bs + 2, C = bs + 1;
   for (int i = threadIdx.x; i < S * S * S; i += RTHREADS)
     st.cells[i] = raw(ox - 1 + i % S, oy - 1 + i / S % S, oz - 1 + i / (S * S));
@@ -665,6 +701,7 @@ FP_DEV void smoothBlock(const BoxCursor& c, SmoothStage& st, int sh, int ox, int
 // fuel as they are; the coarse density smoothed on its own lattice; the aprons of both; and each
 // 2x2x2 cells' maxima for the occupancy. A CTA an 8^3 block, so that bricks of 16^3 and 32^3 spread
 // over the chip too.
+template <class Cursor>
 __global__ void __launch_bounds__(RTHREADS) k_render_field(const SimParams* __restrict__ Pp, const __grid_constant__ FpRender R) {
   const SimParams& P = *Pp;
   __shared__ SmoothStage st;
@@ -678,7 +715,7 @@ __global__ void __launch_bounds__(RTHREADS) k_render_field(const SimParams* __re
     const int b = item % blocks, ox = b % per * 8, oy = b / per % per * 8, oz = b / (per * per) * 8;
     const int sx = coarse ? b % sper * sbs : 0, sy = coarse ? b / sper % sper * sbs : 0,
               sz = coarse ? b / (sper * sper) * sbs : 0;  // the coarse block b, when there are that many
-    BoxCursor c = noBox();
+    Cursor c = noBox<Cursor>();
     auto fine = [&](int x, int y, int z) { return rawSmoke(P, R, c, x, y, z); };
     auto thin = [&](int x, int y, int z) { return rawCoarse(P, R, c, x, y, z); };
     __syncthreads();  // the previous block's stage has been read
@@ -742,6 +779,7 @@ __global__ void __launch_bounds__(RTHREADS) k_render_field(const SimParams* __re
 
 // buildOccupancy (lighting.wgsl:149-244), a warp an 8^3 block: what is visible in the block and two
 // cells around it, from the maxima of 2x2x2 cells (216 of them; each lies in one brick).
+template <class Cursor>
 __global__ void __launch_bounds__(RTHREADS) k_render_occupancy(const SimParams* __restrict__ Pp,
                                                                const __grid_constant__ FpRender R) {
   const SimParams& P = *Pp;
@@ -750,7 +788,7 @@ __global__ void __launch_bounds__(RTHREADS) k_render_occupancy(const SimParams* 
   const bool coarse = P.smokeDiv > 1;
   for (uint32_t item = blockIdx.x * (RTHREADS / 32) + (threadIdx.x >> 5); item < total * (uint32_t)blocks;
        item += gridDim.x * (RTHREADS / 32)) {
-    BoxCursor c = noBox();
+    Cursor c = noBox<Cursor>();
     int bx, by, bz, slot;
     if (!boxBrick(P, R, c, item / blocks, bx, by, bz, slot)) continue;  // the same for the whole warp
     const int b = item % blocks;
@@ -814,6 +852,7 @@ struct LightStage {
   int glows[LIGHT_TEXELS];
   int count;
 };
+template <class Cursor>
 __global__ void __launch_bounds__(RTHREADS) k_render_light(const SimParams* __restrict__ Pp, const __grid_constant__ FpRender R) {
   const SimParams& P = *Pp;
   __shared__ LightStage st;
@@ -826,7 +865,7 @@ __global__ void __launch_bounds__(RTHREADS) k_render_light(const SimParams* __re
   const float sx = R.light[0] / ln, sy = R.light[1] / ln, sz = R.light[2] / ln;
   const int count = R.light[3] > 0.f ? R.shadowSamples : 0, perTexel = count + (R.optical[1] > 0.f ? GLOW_SAMPLES : 0);
   for (uint32_t item = blockIdx.x; item < total * chunks + aprons * apronChunks; item += gridDim.x) {
-    BoxCursor c = noBox();
+    Cursor c = noBox<Cursor>();
     int bx, by, bz, slot = 0;
     unsigned before = 0;
     const bool apron = item >= total * chunks;
@@ -925,7 +964,8 @@ __global__ void __launch_bounds__(RTHREADS) k_render_light(const SimParams* __re
 }
 
 // The lighting sample whose texels' bricks are not all slotted: out of line, rare.
-static __device__ __noinline__ float4 lightSampleFar(const SimParams& P, const FpRender& R, BoxCursor c, int x0, int y0,
+template <class Cursor>
+static __device__ __noinline__ float4 lightSampleFar(const SimParams& P, const FpRender& R, Cursor c, int x0, int y0,
                                                      int z0, float fx, float fy, float fz) {
   const int L = 1 << R.lightShift, L3 = L * L * L;
   const float texel = P.h * (float)(P.B >> R.lightShift);
@@ -952,7 +992,8 @@ static __device__ __noinline__ float4 lightSampleFar(const SimParams& P, const F
   return v;
 }
 // fireProLight (volume-bricks.wgsl:158-178) at `q` in lighting texels.
-FP_DEV float4 lightSample(const SimParams& P, const FpRender& R, BoxCursor& c, float qx, float qy, float qz) {
+template <class Cursor>
+FP_DEV float4 lightSample(const SimParams& P, const FpRender& R, Cursor& c, float qx, float qy, float qz) {
   const int L = 1 << R.lightShift;
   qx = fminf(fmaxf(qx, (float)c.lo[0] * L + .5f), (float)(c.hi[0] + 1) * L - .5f);
   qy = fminf(fmaxf(qy, (float)c.lo[1] * L + .5f), (float)(c.hi[1] + 1) * L - .5f);
@@ -1057,7 +1098,8 @@ FP_DEV bool rayOf(const SimParams& P, const FpRender& R, float ux, float uy, Ray
 // fireProEnter (fireProNext): the box the ray is in at t, or the next one it enters, becomes the
 // current one with its exit, and t moves to its entry; false past the last box. Boxes never
 // overlap, so of the boxes the ray has not left, the one it enters first is the one.
-FP_DEV bool enterBox(const SimParams& P, const FpRender& R, const Ray& r, float& t, float& exit, BoxCursor& c) {
+template <class Cursor>
+FP_DEV bool enterBox(const SimParams& P, const FpRender& R, const Ray& r, float& t, float& exit, Cursor& c) {
   const float brickSize = P.h * (float)P.B;
   float entry = 1e30f, out = 0.f;
   int best = -1;
@@ -1084,7 +1126,8 @@ struct Sample {
   float cell[3];   // the sample point in field cells
   int filter;      // the reconstruction filter of its block
 };
-FP_DEV Sample sampleAt(const SimParams& P, const FpRender& R, BoxCursor& c, const Ray& r, float t, float ds, float exit) {
+template <class Cursor>
+FP_DEV Sample sampleAt(const SimParams& P, const FpRender& R, Cursor& c, const Ray& r, float t, float ds, float exit) {
   Sample s;
   float tt = t + r.jitter * ds;
   float p[3] = {r.ro[0] + r.rd[0] * tt, r.ro[1] + r.rd[1] * tt, r.ro[2] + r.rd[2] * tt};
@@ -1129,7 +1172,8 @@ FP_DEV Sample sampleAt(const SimParams& P, const FpRender& R, BoxCursor& c, cons
 }
 // The radiance a sample ds long adds per unit of the transmittance before it, and the factor it
 // leaves of that transmittance.
-FP_DEV float4 shade(const SimParams& P, const FpRender& R, BoxCursor& c, const Ray& r, const Tint& tint, const Sample& s,
+template <class Cursor>
+FP_DEV float4 shade(const SimParams& P, const FpRender& R, Cursor& c, const Ray& r, const Tint& tint, const Sample& s,
                     float ds) {
   const float texels = 1.f / (float)(P.B >> R.lightShift);  // lighting texels a cell: a power of two, exact
   float4 f = reconstruct(P, R, c, s.cell[0], s.cell[1], s.cell[2], s.filter);
@@ -1177,8 +1221,8 @@ struct Steps {
   Sample s;
 };
 // The group's next steps before `limit`, looked up.
-template <int G>
-FP_DEV Steps<G> lookAhead(const SimParams& P, const FpRender& R, BoxCursor& c, const Ray& r, float limit, bool on,
+template <int G, class Cursor>
+FP_DEV Steps<G> lookAhead(const SimParams& P, const FpRender& R, Cursor& c, const Ray& r, float limit, bool on,
                           const March& m) {
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & (G - 1);
@@ -1208,8 +1252,8 @@ FP_DEV Steps<G> lookAhead(const SimParams& P, const FpRender& R, BoxCursor& c, c
   return a;
 }
 // The group's lit steps shaded and composed into the ray.
-template <int G>
-FP_DEV void shadeSteps(const SimParams& P, const FpRender& R, BoxCursor& c, const Ray& r, const Tint& tint, bool on,
+template <int G, class Cursor>
+FP_DEV void shadeSteps(const SimParams& P, const FpRender& R, Cursor& c, const Ray& r, const Tint& tint, bool on,
                        const Steps<G>& a, March& m) {
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & (G - 1);
@@ -1255,12 +1299,12 @@ FP_DEV void shadeSteps(const SimParams& P, const FpRender& R, BoxCursor& c, cons
 // What bounds it is instruction issue (cells come from L1): about 98 % L1 hits, DRAM idle. Slice
 // pass, us: 14,400 rays of a small plume 2103 -> 85; 129,600 rays of a 1.8k-brick jet 8954 -> 845;
 // 518,400 rays of 3.7k bricks 20,889 -> 3025; full resolution, 231,401 rays, quadratic 12,807 -> 800.
-template <int G, class Limit, class Arrived>
+template <class Cursor, int G, class Limit, class Arrived>
 FP_DEV void marchRays(const SimParams& P, const FpRender& R, const Ray& r, bool alive, float end, March& m, Limit limitOf,
                       Arrived arrived) {
   const unsigned full = 0xffffffffu;
   const Tint tint = tintOf(R);
-  BoxCursor c = noBox();
+  Cursor c = noBox<Cursor>();
   while (true) {
     Steps<G> a;
     bool ready = false;  // this group's steps hold a lit one
@@ -1323,7 +1367,7 @@ static dim3 groupGrid(int w, int h) {
 // evenly spaced depths; depths passed by a skip or a jump between boxes keep the values of the
 // moment, those past the exit or an opaque ray the final ones. Without a scene depth every pixel
 // resumes from the last slice, so only that one is stored.
-template <int G>
+template <class Cursor, int G>
 __global__ void __launch_bounds__(RTHREADS, MARCH_CTAS) k_slices(const SimParams* __restrict__ Pp, const __grid_constant__ FpRender R) {
   const SimParams& P = *Pp;
   int px, py;
@@ -1349,7 +1393,7 @@ __global__ void __launch_bounds__(RTHREADS, MARCH_CTAS) k_slices(const SimParams
     m.t = m.exit = r.lo;
     depth = r.lo + spacing;
   }
-  marchRays<G>(P, R, r, alive, r.hi, m, [&]() { return depth; },
+  marchRays<Cursor, G>(P, R, r, alive, r.hi, m, [&]() { return depth; },
                [&]() {
                  while (recorded < FP_SLICES && m.t >= depth) {
                    record();
@@ -1362,7 +1406,7 @@ __global__ void __launch_bounds__(RTHREADS, MARCH_CTAS) k_slices(const SimParams
 // fireProSceneVolume (scene-volume.wgsl:39-44, 146-167): the march of each pixel's ray up to
 // the scene's depth through the boxes, from the last half-resolution slice in front of it when
 // slices exist.
-template <int G>
+template <class Cursor, int G>
 __global__ void __launch_bounds__(RTHREADS, MARCH_CTAS) k_march(const SimParams* __restrict__ Pp, const __grid_constant__ FpRender R) {
   const SimParams& P = *Pp;
   int px, py;
@@ -1421,7 +1465,7 @@ __global__ void __launch_bounds__(RTHREADS, MARCH_CTAS) k_march(const SimParams*
   // fireProMarch: the cursor starts exited, so the first pass enters the box at t.
   const bool drawn = alive;
   m.exit = m.t;
-  marchRays<G>(P, R, r, alive, end, m, [&]() { return end; }, []() {});
+  marchRays<Cursor, G>(P, R, r, alive, end, m, [&]() { return end; }, []() {});
   if (inside && (threadIdx.x & (G - 1)) == 0)
     reinterpret_cast<float4*>(R.image)[pix] =
         drawn ? make_float4(m.rad[0], m.rad[1], m.rad[2], 1.f - m.trans) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1540,36 +1584,45 @@ void fp_launch_collect_lights(const SimParams* dP, const FpRender& R, const floa
 // idle. Slice pass, us by lanes 1 / 2 / 4 / 8 / 16: 14,400 rays 308 / 198 / 138 / 112 / 82; 129,600
 // rays 925 / 818 / 940 / 1159 / 1429; 518,400 rays 2913 / 2958 / 3501 / 4363 / 5844; full
 // resolution with 231,401 rays 1046 / 773 / 714 / 798 / 1141.
-template <int G>
+template <class Cursor, int G>
 static void marchLaunch(const SimParams* dP, const FpRender& R, cudaStream_t st) {
   if (R.slices) {
-    k_slices<G><<<groupGrid<G>(R.sliceW, R.sliceH), RTHREADS, 0, st>>>(dP, R);
+    k_slices<Cursor, G><<<groupGrid<G>(R.sliceW, R.sliceH), RTHREADS, 0, st>>>(dP, R);
     // Every pixel resumes at its last slice: at most an eighth of its ray is left to march.
-    k_march<1><<<groupGrid<1>(R.width, R.height), RTHREADS, 0, st>>>(dP, R);
+    k_march<Cursor, 1><<<groupGrid<1>(R.width, R.height), RTHREADS, 0, st>>>(dP, R);
   } else {
-    k_march<G><<<groupGrid<G>(R.width, R.height), RTHREADS, 0, st>>>(dP, R);
+    k_march<Cursor, G><<<groupGrid<G>(R.width, R.height), RTHREADS, 0, st>>>(dP, R);
   }
 }
-void fp_launch_render(const SimParams* dP, const FpRender& R, int sms, cudaStream_t st) {
-  if (R.pages) {
-    const int rows = R.boxCount < 64 ? R.boxCount : 64;
-    const long long blocks = (R.pageCount / rows + 255) / 256;
-    k_render_pages<<<dim3((unsigned)(blocks < 1 ? 1 : (blocks < sms * 8 ? blocks : sms * 8)), rows), 256, 0, st>>>(dP, R);
-    if (R.apronCap)
-      k_render_aprons<<<dim3((unsigned)(blocks < 1 ? 1 : (blocks < sms * 8 ? blocks : sms * 8)), rows), 256, 0, st>>>(R);
-  }
-  k_render_field<<<sms * 24, RTHREADS, 0, st>>>(dP, R);
+template <class Cursor>
+static void poolsLaunch(const SimParams* dP, const FpRender& R, int sms, cudaStream_t st) {
+  k_render_field<Cursor><<<sms * 24, RTHREADS, 0, st>>>(dP, R);
   // More CTAs than reside: texels that nothing is at cost little, so equal shares of them are not
   // equal work (5 CTAs an SM 536 us, 20 474, 40 464 on the default grid).
-  k_render_light<<<sms * 40, RTHREADS, 0, st>>>(dP, R);
-  k_render_occupancy<<<sms * 8, RTHREADS, 0, st>>>(dP, R);
+  k_render_light<Cursor><<<sms * 40, RTHREADS, 0, st>>>(dP, R);
+  k_render_occupancy<Cursor><<<sms * 8, RTHREADS, 0, st>>>(dP, R);
+}
+void fp_launch_render(const SimParams* dP, const FpRender& R, int sms, cudaStream_t st) {
+  if (!R.pages) {
+    // Rare, so one form for every size: 2 and 4 lanes a ray 2220 and 1803 us (14,400 rays), 6.3 and 4.5 ms
+    // (129,600), 8.9 and 6.5 (231,401), 21.3 and 22.8 (518,400).
+    poolsLaunch<HashCursor>(dP, R, sms, st);
+    marchLaunch<HashCursor, 4>(dP, R, st);
+    return;
+  }
+  const int rows = R.boxCount < 64 ? R.boxCount : 64;
+  const long long blocks = (R.pageCount / rows + 255) / 256;
+  const dim3 grid((unsigned)(blocks < 1 ? 1 : (blocks < sms * 8 ? blocks : sms * 8)), rows);
+  k_render_pages<<<grid, 256, 0, st>>>(dP, R);
+  if (R.apronCap) k_render_aprons<<<grid, 256, 0, st>>>(R);
+  poolsLaunch<TableCursor>(dP, R, sms, st);
   const long long rays = R.slices ? (long long)R.sliceW * R.sliceH : (long long)R.width * R.height;
   if (rays >= 125000)
-    marchLaunch<2>(dP, R, st);
+    marchLaunch<TableCursor, 2>(dP, R, st);
   else if (rays >= 62500)
-    marchLaunch<4>(dP, R, st);
+    marchLaunch<TableCursor, 4>(dP, R, st);
   else if (rays >= 31250)
-    marchLaunch<8>(dP, R, st);
+    marchLaunch<TableCursor, 8>(dP, R, st);
   else
-    marchLaunch<16>(dP, R, st);
+    marchLaunch<TableCursor, 16>(dP, R, st);
 }
