@@ -61,3 +61,15 @@ def test_box_too_large_for_tables():
     st = render.default_settings(ray_steps=1024, shadow_samples=8)
     for gpu, orc in images(DiagonalScene(66), 3, cams, st, 2 ** 22):
         check(gpu, orc)
+
+
+@pytest.mark.parametrize("width,height", [(112, 96), (160, 160), (224, 208), (304, 272), (480, 400), (720, 560)])
+def test_opacity_below_zero(width, height):
+    """A negative flame opacity raises the transmittance along a ray: whatever number of lanes shares
+    it, the steps compose as one after the other."""
+    cam = render.look_at((1.4, 1.0, 2.0), (0.0, 0.45, 0.0), width, height, time=0.5)
+    st = render.default_settings(ray_steps=64, shadow_samples=8)
+    st.flame_opacity = -1.5
+    (gpu, orc), = images(scenes.ForceScene(), 10, [cam], st, 2 ** 20)
+    assert np.isfinite(gpu).all() and orc[..., 3].min() < -0.05, "some ray should gain"
+    assert parity.rel_l2(gpu, orc.astype(np.float64)) <= RENDER_TOL

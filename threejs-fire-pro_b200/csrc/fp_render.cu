@@ -1269,16 +1269,19 @@ FP_DEV void shadeSteps(const SimParams& P, const FpRender& R, Cursor& c, const R
     }
     const float before = __shfl_up_sync(full, incl, 1, G);
     const float tb = lane == 0 ? m.trans : m.trans * before;
-    const bool counts = tb >= OPAQUE;  // falls along the group: a prefix of it
+    // The steps before the first at which the serial march would have stopped count. (The transmittance
+    // need not fall along the group: an opacity below zero raises it.)
+    const unsigned stops = (__ballot_sync(full, !(tb >= OPAQUE)) >> ((threadIdx.x & 31) & ~(G - 1))) & ((1u << G) - 1u);
+    const int n = stops ? __ffs((int)stops) - 1 : G;
+    const bool counts = lane < n;
     float x = counts ? tb * q.x : 0.f, y = counts ? tb * q.y : 0.f, z = counts ? tb * q.z : 0.f;
-    float left = counts ? tb * q.w : m.trans;
 #pragma unroll
     for (int o = G / 2; o > 0; o >>= 1) {
       x += __shfl_xor_sync(full, x, o, G);
       y += __shfl_xor_sync(full, y, o, G);
       z += __shfl_xor_sync(full, z, o, G);
-      left = fminf(left, __shfl_xor_sync(full, left, o, G));
     }
+    const float left = __shfl_sync(full, tb * q.w, max(0, n - 1), G);
     if (on) {
       m.rad[0] += x;
       m.rad[1] += y;
