@@ -73,3 +73,43 @@ def test_opacity_below_zero(width, height):
     (gpu, orc), = images(scenes.ForceScene(), 10, [cam], st, 2 ** 20)
     assert np.isfinite(gpu).all() and orc[..., 3].min() < -0.05, "some ray should gain"
     assert parity.rel_l2(gpu, orc.astype(np.float64)) <= RENDER_TOL
+
+
+class SparseScene(scenes.Scene):
+    """`side`^3 puffs of smoke, each within a brick of its own, three bricks apart: every brick has its
+    seven apron bricks, more than the render keeps room for (two a slot)."""
+
+    name = "sparse"
+
+    def __init__(self, side=4, seed=1):
+        self.side = side
+        self.settings = scenes.settings(buoyancy=0.0, smoke_weight=0.0, vorticity=0.0, seed=seed)
+        self.comb = scenes.combustion()
+
+    def frame(self, step):
+        brick, n = 8 * self.voxel_size, range(self.side)
+        at = [((3 * x + 0.5) * brick, (3 * y + 0.5) * brick, (3 * z + 0.5) * brick) for z in n for y in n for x in n]
+        srcs = [scenes.source(1 + k, "sphere", p, (0.03, 0.03, 0.03), smoke=400.0 + k) for k, p in enumerate(at)]
+        return scenes.make_frame(self.settings, self.comb, False, srcs)
+
+
+@pytest.mark.parametrize("smoke_divisor", [1, 2])
+def test_more_aprons_than_room(smoke_divisor):
+    """With places for a third of the aprons a frame is still the oracle's, and repeats bit for bit."""
+    sc = SparseScene()
+    budget = sc.side ** 3 * 512
+    cam = render.look_at((3.2, 1.9, 3.6), (1.0, 1.0, 1.0), 200, 150, time=0.5)
+    st = render.default_settings(ray_steps=256, shadow_samples=16)
+    grid = sc.grid(budget=budget)
+    grid.smoke_divisor = smoke_divisor
+    out = {}
+
+    def after(gpu, orc):
+        assert gpu.stats().active_bricks == gpu.stats().pool_slots == sc.side ** 3
+        out["gpu"] = [gpu.render(cam, st) for _ in range(12)]
+        out["orc"] = orc.render(cam, st)
+
+    parity.lockstep(sc, 4, lambda g: FluidSimulation(g), budget=budget, grid=grid, after=after)
+    check(out["gpu"][0], out["orc"])
+    for img in out["gpu"][1:]:
+        assert np.array_equal(img, out["gpu"][0])
