@@ -3,10 +3,16 @@
 The tolerance is test_gpu_render's: relative L2 2e-3 between the FP32 image and the oracle's FP64
 one of the same state.
 """
+import json
+import os
+import subprocess
+import sys
+from pathlib import Path
+
 import numpy as np
 import pytest
 
-from firepro import render, scenes
+from firepro import abi, render, scenes
 from firepro.engine import FluidSimulation
 import parity
 
@@ -113,3 +119,59 @@ def test_more_aprons_than_room(smoke_divisor):
     check(out["gpu"][0], out["orc"])
     for img in out["gpu"][1:]:
         assert np.array_equal(img, out["gpu"][0])
+
+
+# Runs with and without memory to spare, which the checked build refuses when the environment says so.
+WITHOUT = r"""
+import json, os, sys
+sys.path[:0] = [{root!r}, {root!r} + "/threejs-fire-pro_b200", {root!r} + "/tests"]
+import numpy as np
+from firepro import abi, render, scenes
+from firepro.engine import FluidSimulation
+import parity
+
+sc = scenes.ForceScene()
+grid = sc.grid(budget=2 ** 20, precision=abi.FP_PRECISION_MIXED)
+grid.smoke_divisor = {divisor}
+out = {{}}
+
+def after(gpu, orc):
+    errors = []
+    before = gpu.lib.fp_last_error(gpu.h).decode()
+    for half in (0, 1):
+        cam = render.look_at((1.4, 1.0, 2.0), (0.0, 0.45, 0.0), 97, 65, time=0.5)
+        cam.half_resolution = half
+        st = render.default_settings(ray_steps=128, shadow_samples=16)
+        img, ref = gpu.render(cam, st), orc.render(cam, st)
+        assert ref[..., 3].max() > 0.05
+        errors.append(parity.rel_l2(img, ref.astype(np.float64)))
+    halves = gpu.field(abi.FP_FIELD_SCALARS)
+    blob = bytes(gpu.snapshot())
+    out.update(errors=errors, before=before, message=gpu.lib.fp_last_error(gpu.h).decode(), checked=gpu.read_bounds().checked,
+               bad=gpu.read_bounds().count, field=float(np.abs(halves).max()),
+               same=blob.find(halves.astype(np.float16).tobytes()) >= 0)
+
+os.environ["FIREPRO_SPARE"] = "{spare}"
+parity.lockstep(sc, 8, lambda g: FluidSimulation(g), budget=2 ** 20, grid=grid, after=after)
+print("WITHOUT " + json.dumps(out))
+"""
+
+
+@pytest.mark.parametrize("divisor", [1, 2])
+@pytest.mark.parametrize("spare", [0, 1])
+def test_no_memory_to_spare(spare, divisor):
+    """Without room for the boxes' tables, the aprons, the occupancy's maxima and the widening buffer
+    (and with all of it, in the same build): the images are the oracle's, FP16 pools read back as the
+    snapshot's halves, and a call that did without memory leaves no error behind."""
+    if not abi.DEBUG_LIB_PATH.exists():
+        pytest.fail("the bounds-checked build is missing: build.py --debug (or __graft_entry__.build())")
+    root = str(Path(__file__).resolve().parent.parent)
+    env = dict(os.environ, FIREPRO_LIBRARY=str(abi.DEBUG_LIB_PATH))
+    r = subprocess.run([sys.executable, "-c", WITHOUT.format(root=root, spare=spare, divisor=divisor)], env=env,
+                       capture_output=True, text=True, timeout=1200)
+    assert r.returncode == 0, r.stdout[-3000:] + r.stderr[-3000:]
+    out = json.loads([x for x in r.stdout.splitlines() if x.startswith("WITHOUT ")][-1][len("WITHOUT "):])
+    assert out["checked"] == 1 and out["bad"] == 0
+    assert max(out["errors"]) <= RENDER_TOL, out
+    assert out["field"] > 0 and out["same"], out
+    assert out["message"] == out["before"], out

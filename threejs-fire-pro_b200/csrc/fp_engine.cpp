@@ -89,12 +89,20 @@ int Engine::check(cudaError_t e, const char* what) {
   return e == cudaErrorMemoryAllocation ? FP_ENOMEM : FP_EDEVICE;
 }
 
+// cudaMalloc, once more without what the renders can do without.
+bool Engine::claim(void** p, size_t bytes) {
+  if (cudaMalloc(p, bytes) == cudaSuccess) return true;
+  if (!giveWay()) return false;
+  cudaGetLastError();
+  return cudaMalloc(p, bytes) == cudaSuccess;
+}
+
 bool Engine::alloc(DeviceBuffer& b, size_t bytes, bool zero) {
   if (b.ptr) cudaFree(b.ptr);
   b.ptr = nullptr;
   b.bytes = 0;
   if (bytes == 0) bytes = 16;
-  if (cudaMalloc(&b.ptr, bytes) != cudaSuccess) {
+  if (!claim(&b.ptr, bytes)) {
     b.ptr = nullptr;
     error_ = "device memory exhausted";
     return false;
@@ -107,7 +115,7 @@ bool Engine::alloc(DeviceBuffer& b, size_t bytes, bool zero) {
 bool Engine::grow(DeviceBuffer& b, size_t bytes, int fill) {
   if (bytes <= b.bytes && b.ptr) return true;
   void* p = nullptr;
-  if (cudaMalloc(&p, bytes) != cudaSuccess) {
+  if (!claim(&p, bytes)) {
     error_ = "device memory exhausted";
     return false;
   }

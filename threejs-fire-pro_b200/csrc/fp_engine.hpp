@@ -13,6 +13,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <cstdlib>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -64,6 +65,17 @@ struct DeviceBuffer {
   void* ptr = nullptr;
   size_t bytes = 0;
 };
+
+// Memory that a call can do without (tables and buffers that only make it faster) is refused in the
+// checked build with FIREPRO_SPARE=0 in the environment: how the tests reach what runs without it.
+#ifdef FP_BOUNDS
+inline bool spareRefused() {
+  const char* e = std::getenv("FIREPRO_SPARE");
+  return e && e[0] == '0';
+}
+#else
+constexpr bool spareRefused() { return false; }
+#endif
 
 class Stepper;
 
@@ -224,7 +236,11 @@ class Engine {
       renderPages_, apronList_, apronPools_, renderUnits_;
   SimParams* renderParamsH_ = nullptr;
   // The blackbody table and the render parameters of the latest state (device).
+  static constexpr int SPARE_WAIT = 64;  // renders
+  int spareWait_ = 0;  // renders until memory that was refused is asked for again
   bool spare(DeviceBuffer& b, size_t need, size_t want);
+  bool giveWay();
+  bool claim(void** p, size_t bytes);
   int renderInputs();
   void updateRenderBox();
 

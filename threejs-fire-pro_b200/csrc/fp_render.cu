@@ -763,7 +763,7 @@ __global__ void __launch_bounds__(RTHREADS) k_render_field(const SimParams* __re
       smoothBlock(c, st, P.shift, bx * P.B + ox, by * P.B + oy, bz * P.B + oz, 8, fine, put);
     }
     __syncthreads();
-    if (threadIdx.x < 64) {
+    if (R.units && threadIdx.x < 64) {
       const int u = threadIdx.x, first = ((u >> 4) * 2 * 8 + ((u >> 2) & 3) * 2) * 8 + (u & 3) * 2;
       float2 m = make_float2(0.f, 0.f);
 #pragma unroll
@@ -779,7 +779,8 @@ __global__ void __launch_bounds__(RTHREADS) k_render_field(const SimParams* __re
 
 // buildOccupancy (lighting.wgsl:149-244), a warp an 8^3 block: what is visible in the block and two
 // cells around it, from the maxima of 2x2x2 cells (216 of them; each lies in one brick).
-template <class Cursor>
+// UNITS: those maxima are there; else they are taken here, each some 27 times over.
+template <class Cursor, bool UNITS>
 __global__ void __launch_bounds__(RTHREADS) k_render_occupancy(const SimParams* __restrict__ Pp,
                                                                const __grid_constant__ FpRender R) {
   const SimParams& P = *Pp;
@@ -801,9 +802,19 @@ __global__ void __launch_bounds__(RTHREADS) k_render_occupancy(const SimParams* 
       if (s < 0) continue;
       const int block = (((uz & m) >> 3) * per + ((uy & m) >> 3)) * per + ((ux & m) >> 3);
       const int unit = (((uz & 7) >> 1) * 4 + ((uy & 7) >> 1)) * 4 + ((ux & 7) >> 1);
-      const float2 v = __ldg(&R.units[((size_t)s * blocks + block) * 64 + unit]);
-      glow = fmaxf(glow, v.x);
-      seen = fmaxf(seen, v.y);
+      if constexpr (UNITS) {
+        const float2 v = __ldg(&R.units[((size_t)s * blocks + block) * 64 + unit]);
+        glow = fmaxf(glow, v.x);
+        seen = fmaxf(seen, v.y);
+      } else {
+        for (int k = 0; k < 8; k++) {
+          const int cell = localCell(P, ux + (k & 1), uy + ((k >> 1) & 1), uz + (k >> 2));
+          const float4 f = __ldg(&R.renderField[(size_t)s * P.N + cell]);
+          const float g = glowOf(f.z);
+          glow = fmaxf(glow, g);
+          seen = fmaxf(seen, (coarse ? 0.f : f.x) + g);
+        }
+      }
     }
     float smoke = 0.f;
     if (coarse) {
@@ -1603,7 +1614,10 @@ static void poolsLaunch(const SimParams* dP, const FpRender& R, int sms, cudaStr
   // More CTAs than reside: texels that nothing is at cost little, so equal shares of them are not
   // equal work (5 CTAs an SM 536 us, 20 474, 40 464 on the default grid).
   k_render_light<Cursor><<<sms * 40, RTHREADS, 0, st>>>(dP, R);
-  k_render_occupancy<Cursor><<<sms * 8, RTHREADS, 0, st>>>(dP, R);
+  if (R.units)
+    k_render_occupancy<Cursor, true><<<sms * 8, RTHREADS, 0, st>>>(dP, R);
+  else
+    k_render_occupancy<Cursor, false><<<sms * 8, RTHREADS, 0, st>>>(dP, R);
 }
 void fp_launch_render(const SimParams* dP, const FpRender& R, int sms, cudaStream_t st) {
   if (!R.pages) {

@@ -49,7 +49,7 @@ struct FpRender {
   float4* renderField;  // [slot][cell]: smoothed smoke, heat, lifetime, fuel (coarse smoke: the
                         // simulation's fields as they are)
   float2* units;        // [slot][block][4^3]: of each 2x2x2 cells of an 8^3 block, the most flame glow
-                        // and the most smoke plus glow
+                        // and the most smoke plus glow; null without room (taken from renderField then)
   float* renderSmoke;   // coarse smoke (smokeDiv > 1): [slot][smoke cells], the smoothed density
   float4* lighting;     // [slot][texel]: glow RGB, sun transmittance
   uint8_t* occupancy;   // [slot]: bit 0 flame glow, bit 1 anything visible, in the block and halo

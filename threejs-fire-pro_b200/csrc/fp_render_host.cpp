@@ -233,13 +233,38 @@ int Engine::renderInputs() {
   return FP_OK;
 }
 
-// Room of at least `need` bytes in a buffer that a render can do without: `want` bytes when it has
-// to be allocated. False without it, the device's error state cleared.
+// Room of at least `need` bytes in a buffer that a render can do without: `want` bytes, or `need`, when
+// it has to be allocated. False without it, which is no error of the render's; the next renders then do
+// without too rather than ask each time.
 bool Engine::spare(DeviceBuffer& b, size_t need, size_t want) {
   if (b.ptr && b.bytes >= need) return true;
-  if (alloc(b, want, false)) return true;
-  cudaGetLastError();
+  if (spareWait_ > 0) return false;
+  if (b.ptr) cudaFree(b.ptr);
+  b = DeviceBuffer{};
+  for (size_t bytes : {want, need}) {
+    if (!spareRefused() && cudaMalloc(&b.ptr, bytes) == cudaSuccess) {
+      b.bytes = bytes;
+      return true;
+    }
+    b.ptr = nullptr;
+    cudaGetLastError();
+  }
+  spareWait_ = SPARE_WAIT;
   return false;
+}
+
+// What a render can do without is given back when the simulation needs the memory. (cudaFree waits for
+// the kernels that read it.)
+bool Engine::giveWay() {
+  bool freed = false;
+  for (DeviceBuffer* b : {&renderPages_, &apronList_, &apronPools_, &renderUnits_}) {
+    if (!b->ptr) continue;
+    cudaFree(b->ptr);
+    *b = DeviceBuffer{};
+    freed = true;
+  }
+  if (freed) spareWait_ = SPARE_WAIT;
+  return freed;
 }
 
 // The optical model's settings (fire-emission.wgsl's uniforms).
@@ -264,6 +289,7 @@ int Engine::render(const fp_camera& cam, const fp_render_settings& rs, float* im
   if (cam.half_resolution > 1) return fail(FP_EINVAL, "render: half_resolution must be 0 or 1.");
   int rc = consume();
   if (rc) return rc;
+  if (spareWait_ > 0) spareWait_--;
   const int divShift = rs.lighting_divisor == 1 ? 0 : (rs.lighting_divisor == 2 ? 1 : 2);
   const int lightShift = shift_ - divShift, L = 1 << lightShift, blocks = (B_ / 8) * (B_ / 8) * (B_ / 8);
   size_t pixels = (size_t)cam.width * cam.height;
@@ -272,7 +298,6 @@ int Engine::render(const fp_camera& cam, const fp_render_settings& rs, float* im
             (lighting_.bytes >= (size_t)slots_ * 4 * L * L * L * 4 ||
              grow(lighting_, (size_t)slots_ * 4 * L * L * L * 4, 0)) &&
             (occupancy_.bytes >= (size_t)slots_ * blocks || grow(occupancy_, (size_t)slots_ * blocks, 0)) &&
-            (renderUnits_.bytes >= (size_t)slots_ * N_ || grow(renderUnits_, (size_t)slots_ * N_, 0)) &&
             (smokeDiv_ == 1 || renderSmoke_.bytes >= (size_t)slots_ * SN_ * 4 ||
              grow(renderSmoke_, (size_t)slots_ * SN_ * 4, 0)) &&
             (renderParams_.ptr || alloc(renderParams_, sizeof(SimParams), false));
@@ -349,7 +374,7 @@ int Engine::render(const fp_camera& cam, const fp_render_settings& rs, float* im
   R.sliceW = sliceW;
   R.sliceH = sliceH;
   R.renderField = (float4*)renderField_.ptr;
-  R.units = (float2*)renderUnits_.ptr;
+  R.units = spare(renderUnits_, (size_t)slots_ * N_, (size_t)slots_ * N_) ? (float2*)renderUnits_.ptr : nullptr;
   R.renderSmoke = (float*)renderSmoke_.ptr;
   R.lighting = (float4*)lighting_.ptr;
   R.occupancy = (uint8_t*)occupancy_.ptr;

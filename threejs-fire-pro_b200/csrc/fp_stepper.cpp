@@ -60,7 +60,7 @@ struct OnDevice {  // the stepper's device, and the caller's again afterwards
 
 float* Stepper::widenBuffer() {
   OnDevice here(device_);
-  if (!widen_ && cudaMalloc(&widen_, WIDEN_VALUES * sizeof(float)) != cudaSuccess) {
+  if (!widen_ && (spareRefused() || cudaMalloc(&widen_, WIDEN_VALUES * sizeof(float)) != cudaSuccess)) {
     cudaGetLastError();  // not an error of the read
     widen_ = nullptr;
   }
