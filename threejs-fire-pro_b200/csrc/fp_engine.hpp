@@ -363,9 +363,12 @@ class Stepper {
   void phaseBegin(int id);
   void phaseEnd(int id, int launches);
 
-  // The step's launch sequence as CUDA graphs, one per combination of the optional launches.
+  // The step's launch sequence as CUDA graphs, one per combination of the optional launches and, in these
+  // bits of its key, of the forms that suit a step's size.
+  static constexpr uint64_t MANY_BIT = 1ull << 44, COARSE_SMALL_BIT = 1ull << 45, SINGLE_BIT = 1ull << 46,
+                            FEW_BIT = 1ull << 47, FORM_BITS = 15ull << 44;
   struct GraphEntry {
-    cudaGraphExec_t exec;
+    cudaGraphExec_t exec = nullptr;
     int latest;
     uint64_t launches;
   };

@@ -71,7 +71,8 @@ void fp_launch_bottom(const FpBatch& bt, const MgSel& S, int iterations, int sms
 // that level, S.rhs its right-hand side, S.pin its first iterate, S.pout its result, S.cfirst
 // the bottom's result. Usable when every simulation's live tiles fit (fp_coarse_fits).
 bool fp_coarse_fits(int liveTiles);
-bool fp_coarse_small(int liveTiles);
+bool fp_coarse_small(int liveTiles);        // the small form suits it
+bool fp_coarse_small_holds(int liveTiles);  // and still holds it
 void fp_launch_coarse(const FpBatch& bt, const MgSel& S, int iterations, bool small, int sims, int sms, cudaStream_t st);
 // The same of the red-black V-cycle, the second tile level from zero.
 void fp_launch_coarse_rb(const FpBatch& bt, const MgSel& S, int pre, int bottom, int post, bool small, int sims, int sms, cudaStream_t st);

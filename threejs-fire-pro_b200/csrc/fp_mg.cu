@@ -2293,15 +2293,17 @@ void fp_launch_bottom(const FpBatch& bt, const MgSel& S, int iterations, int sms
 }
 bool fp_coarse_fits(int liveTiles) { return (long)liveTiles * COARSE_SLOT_BYTES <= COARSE_SMEM; }
 // `small`: every simulation has at most COARSE_SMALL live tiles; a CTA a simulation of up to `sims`.
-// Fewer warps meet at a barrier sooner, and little shared memory leaves the neighbours' CTAs room.
-constexpr int COARSE_SMALL = 64;
+// Fewer warps meet at a barrier sooner, and little shared memory leaves the neighbours' CTAs room. It
+// holds a few more, so that a simulation that grows past the line steps on until the other form is there.
+constexpr int COARSE_SMALL = 64, COARSE_SMALL_ROOM = 80;
 bool fp_coarse_small(int liveTiles) { return liveTiles <= COARSE_SMALL; }
+bool fp_coarse_small_holds(int liveTiles) { return liveTiles <= COARSE_SMALL_ROOM; }
 void fp_launch_coarse(const FpBatch& bt, const MgSel& S, int iterations, bool small, int sims, int sms, cudaStream_t st) {
-  const int smem = small ? COARSE_SMALL * COARSE_SLOT_BYTES : COARSE_SMEM;
+  const int smem = small ? COARSE_SMALL_ROOM * COARSE_SLOT_BYTES : COARSE_SMEM;
   launchChained(S.overlap, k_coarse<false>, sims < sms ? sims : sms, small ? 256 : 1024, (size_t)smem, st, bt, S, iterations, smem, 0, 0);
 }
 void fp_launch_coarse_rb(const FpBatch& bt, const MgSel& S, int pre, int bottom, int post, bool small, int sims, int sms, cudaStream_t st) {
-  const int smem = small ? COARSE_SMALL * COARSE_SLOT_BYTES : COARSE_SMEM;
+  const int smem = small ? COARSE_SMALL_ROOM * COARSE_SLOT_BYTES : COARSE_SMEM;
   k_coarse<true><<<sims < sms ? sims : sms, small ? 256 : 1024, smem, st>>>(bt, S, bottom, smem, pre, post);
 }
 

@@ -272,6 +272,7 @@ int Stepper::step(Engine* const* sims, const fp_frame* const* frames, const floa
   fewBricks_ = blocks8 <= (fewBricks_ ? few * 9 / 8 : few);
   int vcycles = 1;
   fusedCoarse_ = coarseSmall_ = true;
+  bool coarseHolds = true;  // k_coarse's small form holds every simulation's tiles
   single_ = count == 1;
   anySmoke_ = false;
   smokeDiv_ = 0;
@@ -281,6 +282,7 @@ int Stepper::step(Engine* const* sims, const fp_frame* const* frames, const floa
     uint32_t cap = (uint32_t)e->capacity();
     fusedCoarse_ = fusedCoarse_ && fp_coarse_fits(e->liveTiles());
     coarseSmall_ = coarseSmall_ && fp_coarse_small(e->liveTiles());
+    coarseHolds = coarseHolds && fp_coarse_small_holds(e->liveTiles());
     anySmoke_ = anySmoke_ || e->smokeDivisor() > 1;
     if (e->smokeDivisor() > 1 && (smokeDiv_ == 0 || e->smokeDivisor() < smokeDiv_)) smokeDiv_ = e->smokeDivisor();
     rowBlocks[i] = blocks;
@@ -320,26 +322,43 @@ int Stepper::step(Engine* const* sims, const fp_frame* const* frames, const floa
                    ((uint64_t)anySmoke_ << 17) | ((uint64_t)schedule_.smoother << 18) |
                    ((uint64_t)schedule_.krylov << 19) | ((uint64_t)schedule_.levels << 20) |
                    ((uint64_t)schedule_.pre_sweeps << 24) | ((uint64_t)schedule_.post_sweeps << 28) |
-                   ((uint64_t)schedule_.bottom_sweeps << 32) | ((uint64_t)smokeDiv_ << 40) |
-                   ((uint64_t)manyBricks_ << 44) | ((uint64_t)coarseSmall_ << 45) | ((uint64_t)single_ << 46) |
-                   ((uint64_t)fewBricks_ << 47);
-    auto it = graphs_.find(key);
-    if (it == graphs_.end()) {
-      GraphEntry ge{};
-      if ((rc = check(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture")))
-        return done(rc);
+                   ((uint64_t)schedule_.bottom_sweeps << 32) | ((uint64_t)smokeDiv_ << 40);
+    const uint64_t forms = (manyBricks_ ? MANY_BIT : 0) | (coarseSmall_ ? COARSE_SMALL_BIT : 0) |
+                           (single_ ? SINGLE_BIT : 0) | (fewBricks_ ? FEW_BIT : 0);
+    auto capture = [&](GraphEntry& ge) {
+      cudaError_t e = cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal);
+      if (e != cudaSuccess) return e;
       enqueue(solidsFresh, solidsAll, topoAll, curl, vcycles, measure, ge.latest, ge.launches);
       cudaGraph_t g = nullptr;
-      rc = check(cudaStreamEndCapture(stream_, &g), "cudaStreamEndCapture");
-      if (rc) return done(rc);
-      rc = check(cudaGraphInstantiate(&ge.exec, g, 0), "cudaGraphInstantiate");
+      if ((e = cudaStreamEndCapture(stream_, &g)) != cudaSuccess) return e;
+      e = cudaGraphInstantiate(&ge.exec, g, 0);
       cudaGraphDestroy(g);
-      if (rc) return done(rc);
-      it = graphs_.emplace(key, ge).first;
+      return e;
+    };
+    // Of the forms that suit a step's size any that holds it gives the same results. A step that crosses a
+    // line replays what it has, and its own graph is captured while the device works on that (the step of a
+    // large scene at 1024 bricks, called and waited for, us: 1320 with the capture first, 922 so; 929 the
+    // step before).
+    auto it = graphs_.find(key | forms);
+    bool later = false;
+    if (it == graphs_.end()) {
+      for (auto g = graphs_.begin(); g != graphs_.end() && !later; ++g)
+        if ((g->first & ~FORM_BITS) == key && (coarseHolds || !(g->first & COARSE_SMALL_BIT))) {
+          it = g;
+          later = true;
+        }
+    }
+    if (it == graphs_.end()) {
+      GraphEntry ge{};
+      if ((rc = check(capture(ge), "step capture"))) return done(rc);
+      it = graphs_.emplace(key | forms, ge).first;
     }
     if ((rc = check(cudaGraphLaunch(it->second.exec, stream_), "cudaGraphLaunch"))) return done(rc);
     latest = it->second.latest;
     launches_ += it->second.launches;
+    GraphEntry own{};
+    if (later && capture(own) == cudaSuccess) graphs_.emplace(key | forms, own);
+    if (later && !own.exec) cudaGetLastError();  // the next step tries again
   }
   pendingRead_ = true;
   for (int i = 0; i < count; i++) sims[i]->launched(dts[i], latest);
