@@ -3,6 +3,7 @@
 The tolerance is test_gpu_render's: relative L2 2e-3 between the FP32 image and the oracle's FP64
 one of the same state.
 """
+import ctypes as C
 import json
 import os
 import subprocess
@@ -66,6 +67,34 @@ def test_box_too_large_for_tables():
         cams.append(cam)
     st = render.default_settings(ray_steps=1024, shadow_samples=8)
     for gpu, orc in images(DiagonalScene(66), 3, cams, st, 2 ** 22):
+        check(gpu, orc)
+
+
+# Rays: 15,931 (16 lanes a ray), 16,037 and 35,649 (8), 36,045 and 99,855 (4), 100,233 and 402,003 (2):
+# odd and either side of each line, so that every form has tiles partly outside.
+SIZES = [(179, 89), (203, 79), (233, 153), (267, 135), (317, 315), (333, 301), (709, 567)]
+
+
+@pytest.mark.parametrize("width,height", SIZES)
+def test_lanes_a_ray(width, height):
+    """Each number of lanes a ray: at full resolution, and in the half-resolution slices (of an odd
+    image), with a scene's depth through the flames, for which all slices are written and read, and
+    without."""
+    cams, depths = [], []
+    for half, depth in ((0, False), (0, True), (1, False), (1, True)):
+        w, h = (2 * width - 1, 2 * height - 1) if half else (width, height)
+        cam = render.look_at((1.4, 1.0, 2.0), (0.0, 0.45, 0.0), w, h, time=0.5)
+        cam.half_resolution = half
+        if depth:  # clip z of a plane 2.15 to 2.55 m from the eye, left to right; a band with nothing
+            near, far = 0.05, 50.0
+            d = 2.35 + 0.4 * ((np.arange(w) + 0.5) / w - 0.5) + np.zeros((h, 1))
+            z = np.ascontiguousarray((far * (d - near) / (d * (far - near))).astype(np.float32))
+            z[:, : w // 8] = 1.0
+            depths.append(z)  # the camera points into it
+            cam.scene_depth = z.ctypes.data_as(C.POINTER(C.c_float))
+        cams.append(cam)
+    st = render.default_settings(ray_steps=40, shadow_samples=4)
+    for gpu, orc in images(scenes.ForceScene(), 12, cams, st, 2 ** 20):
         check(gpu, orc)
 
 

@@ -1595,9 +1595,20 @@ void fp_launch_collect_lights(const SimParams* dP, const FpRender& R, const floa
 
 // Lanes a ray (marchRays): enough that the rays' lanes fill the chip several times over (148 SMs x
 // 12 warps), no more, since a group's lanes share the ray's own work and its last steps leave lanes
-// idle. Slice pass, us by lanes 1 / 2 / 4 / 8 / 16: 14,400 rays 308 / 198 / 138 / 112 / 82; 129,600
-// rays 925 / 818 / 940 / 1159 / 1429; 518,400 rays 2913 / 2958 / 3501 / 4363 / 5844; full
-// resolution with 231,401 rays 1046 / 773 / 714 / 798 / 1141.
+// idle. What is best moves with the scene and with the steps a ray takes; the lines lie where the means
+// over five scenes, both resolutions and 128 and 256 steps cross. A render relative to its best number
+// of lanes, the mean at half resolution, 128 / 256 steps:
+//   rays          1           2           4           8           16
+//   9,216     2.39/3.08   1.60/1.89   1.19/1.35   1.01/1.06   1.01/1.01
+//   17,280    2.12/2.59   1.43/1.59   1.09/1.17   1.00/1.00   1.07/1.04
+//   30,720    1.71/2.14   1.17/1.32   1.01/1.02   1.05/1.01   1.18/1.12
+//   43,200    1.63/1.95   1.12/1.30   1.00/1.00   1.08/1.04   1.27/1.20
+//   86,400    1.24/1.43   1.02/1.05   1.05/1.02   1.23/1.15   1.58/1.43
+//   129,600   1.09/1.22   1.00/1.01   1.10/1.07   1.35/1.27   1.81/1.65
+//   230,400   1.02/1.03   1.06/1.04   1.24/1.17   1.61/1.46   2.26/1.95
+//   518,400   1.02/1.02   1.11/1.08   1.38/1.27   1.88/1.67   2.77/2.34
+// Past 230,400 one lane would be better in most scenes and worse in the largest (518,400 rays of 256 steps
+// through 3.7k bricks: 3962 us, with two 3829); from 921,600 on in nearly all, by a tenth.
 template <class Cursor, int G>
 static void marchLaunch(const SimParams* dP, const FpRender& R, cudaStream_t st) {
   if (R.slices) {
@@ -1634,11 +1645,11 @@ void fp_launch_render(const SimParams* dP, const FpRender& R, int sms, cudaStrea
   if (R.apronCap) k_render_aprons<<<grid, 256, 0, st>>>(R);
   poolsLaunch<TableCursor>(dP, R, sms, st);
   const long long rays = R.slices ? (long long)R.sliceW * R.sliceH : (long long)R.width * R.height;
-  if (rays >= 125000)
+  if (rays >= 100000)
     marchLaunch<TableCursor, 2>(dP, R, st);
-  else if (rays >= 62500)
+  else if (rays >= 36000)
     marchLaunch<TableCursor, 4>(dP, R, st);
-  else if (rays >= 31250)
+  else if (rays >= 16000)
     marchLaunch<TableCursor, 8>(dP, R, st);
   else
     marchLaunch<TableCursor, 16>(dP, R, st);
