@@ -381,10 +381,13 @@ class Stepper {
   bool fusedCoarse_ = false;  // the V-cycle below the first tile level runs as k_coarse
   // From about this many computing bricks in a launch the finest level's restriction and the brick
   // levels' prolongation run apart from the sweeps: over a wide rim they do their work several times
-  // over (finest level up, us: 98 together, 87 apart on 3.1k bricks; 12 and 17 on 90).
+  // over. A large scene's step, us together / apart: 200 bricks 215 / 234, 400 259 / 276, 600 343 / 359,
+  // 800 407 / 409, 1000 496 / 503, 1250 572 / 569, 1500 647 / 630, 2000 780 / 770, 3000 1033 / 1000.
   static constexpr uint64_t MANY_BRICKS = 1000;
-  // 8^3-cell blocks of computing bricks an SM up to which the step's launches overlap (a plume of 750
-  // bricks: 457 us a frame with, 481 without; the default grid, 34 blocks an SM: 2842 and 2800).
+  // 8^3-cell blocks of computing bricks an SM up to which the step's launches overlap: where the chip is
+  // not full. A large scene's step, us with / without: 400 bricks 260 / 289, 700 370 / 401, 900 438 / 462
+  // (the line), 1400 574 / 597, 2000 761 / 769; past 3k bricks it lost up to 5 %, and on the default grid
+  // (34 blocks an SM) a frame took 2842 and 2800.
   static constexpr uint64_t OVERLAP_BLOCKS = 6;
   bool manyBricks_ = false, fewBricks_ = false;
   bool coarseSmall_ = false;  // k_coarse in its small form (fp_coarse_small)

@@ -976,11 +976,11 @@ __global__ void __launch_bounds__(Rim<8, rimOf(LEG)>::THREADS) k_leg_pairs(FpBat
   waitForPrevious();
 }
 
-// Every cell of `A.level` (a tile level of CELLS cells a tile) in every tile: a thread per
+// Every cell of `A.level` (a tile level of CELLS cells a tile, 8 or 1) in every tile: a thread per
 // cell, 64 / CELLS tiles per CTA; no barriers, so threads of dead tiles just move on.
 template <int OP, int CELLS>
 __global__ void __launch_bounds__(64) k_level_tiles(FpBatch bt, MgSel Sl) {
-  constexpr int NT = 64 / CELLS, s = CELLS == 64 ? 2 : (CELLS == 8 ? 1 : 0), side = 1 << s;
+  constexpr int NT = 64 / CELLS, s = CELLS == 8 ? 1 : 0, side = 1 << s;
   const int g = threadIdx.x / CELLS, o = threadIdx.x % CELLS;
   uint32_t total = workTotal(bt, FP_WORK_TILES);
   for (uint32_t item = blockIdx.x * NT + g; item < total; item += gridDim.x * NT) {
@@ -1000,10 +1000,9 @@ __global__ void __launch_bounds__(64) k_level_tiles(FpBatch bt, MgSel Sl) {
 // Staged tile levels: k_level_bricks_staged with a live tile in place of a brick. A group of 64
 // threads copies, for its tile, the values of the level it reads over the tile and a rim from
 // the tile's 27 neighbour tiles (tileNbr) into shared memory; a cell is an unknown when its
-// brick computes (the tile's mask, tileCellActive). Same arithmetic, same order as relaxCell /
-// restrictCell / prolongCell.
-//   RELAX     stage A.pin at A.level (TS = 4: the first tile level, a cell a brick)
-//   RESTRICT  stage A.pin at A.level - 1 (TS = 4); write A.pout, A.cfirst at A.level (2^3 a tile)
+// brick computes (the tile's mask, tileCellActive). Same arithmetic, same order as restrictCell and
+// prolongCell. (The first tile level's sweeps are legs.)
+//   RESTRICT  stage A.pin at A.level - 1 (TS = 4: the first tile level, a cell a brick); write A.pout, A.cfirst at A.level (2^3 a tile)
 //   PROLONG   stage A.coarse at A.level + 1 (TS = 2); write A.pout at A.level (4^3 a tile)
 template <int OP, int TS>
 struct TileStaged {
@@ -1045,14 +1044,14 @@ __global__ void __launch_bounds__(256) k_level_tiles_staged(FpBatch bt, MgSel Sl
     __syncthreads();
     // The stage's first cell, in cells of the staged level.
     const int ox = rec.x * TS - R, oy = rec.y * TS - R, oz = rec.z * TS - R;
-    // This thread's fine cell (RELAX, PROLONG): its flags and right-hand side or value, loaded
-    // before the stage so that both sets of loads are in flight together.
+    // This thread's fine cell (PROLONG): its flags and value, loaded before the stage so that both
+    // sets of loads are in flight together.
     const long own = (long)tile * FCELLS + t;
     uint8_t ownTopo = 0;
     float ownValue = 0.f;
-    if (OP != RESTRICT && has) {
+    if (OP == PROLONG && has) {
       ownTopo = P.topo[fineLevel][own];
-      ownValue = OP == RELAX ? ldBf(A.rhs, own, A.rhsN) : ldBf(A.pin, own, A.pinN);
+      ownValue = ldBf(A.pin, own, A.pinN);
     }
     bool solidStaged = false;
     if (has) {
@@ -1063,8 +1062,7 @@ __global__ void __launch_bounds__(256) k_level_tiles_staged(FpBatch bt, MgSel Sl
         const int n = nbr[nbrIndex(dx, dy, dz)];
         const int cx = (lx - R) & (TS - 1), cy = (ly - R) & (TS - 1), cz = (lz - R) & (TS - 1);
         const long a = n < 0 ? -1 : (long)n * TS3 + (cz * TS + cy) * TS + cx;
-        const bool skipLoad = OP == RELAX && (!src || (A.colour != 0 && ((ox + oy + oz + lx + ly + lz) & 1) == A.colour - 1));
-        st[q] = (a < 0 || skipLoad) ? 0.f : ldBf(src, a, srcN);
+        st[q] = a < 0 ? 0.f : ldBf(src, a, srcN);
         if (OP == PROLONG) {
           const bool solid = a >= 0 && (P.topo[stageLevel][a] & FP_STORED_SOLID);
           solidSt[q] = solid ? 1 : 0;
@@ -1089,24 +1087,7 @@ __global__ void __launch_bounds__(256) k_level_tiles_staged(FpBatch bt, MgSel Sl
       };
       const int lx = t & 3, ly = (t >> 2) & 3, lz = t >> 4;
       const int px = rec.x * 4 + lx, py = rec.y * 4 + ly, pz = rec.z * 4 + lz;
-      if (OP == RELAX) {
-        if (A.colour != 0 && parityOf(px, py, pz) != A.colour - 1) {
-          if (!src) stBf(A.pout, own, 0.f, A.poutN);  // the other colour: kept, or zero from zero
-        } else {
-          const uint32_t f = expandFlags(ownTopo);
-          if ((f & SOLIDF) || !unknown(lx, ly, lz)) {
-            stBf(A.pout, own, 0.f, A.poutN);
-          } else {
-            float cand = (sumAt(lx, ly, lz, f) - ownValue) / fmaxf(diagOf(f), 1e-12f);
-            if (A.colour != 0) {
-              stBf(A.pout, own, cand, A.poutN);  // Gauss-Seidel in place
-            } else {
-              float center = st[((lz + 1) * S + (ly + 1)) * S + (lx + 1)];
-              stBf(A.pout, own, mixf(center, cand, 0.8f), A.poutN);
-            }
-          }
-        }
-      } else if (OP == PROLONG) {
+      if (OP == PROLONG) {
         const uint32_t f = expandFlags(ownTopo);
         if ((f & SOLIDF) || !unknown(lx, ly, lz)) {
           stBf(A.pout, own, 0.f, A.poutN);
@@ -2157,7 +2138,6 @@ void fp_mg_configure(int B) {
   configureLeg<BRICK4, RB>();
   configureLeg<PAIRS, RB>();
   configureLeg<TILE4, RB>();
-  configureTileStaged<RELAX, 4>();
   configureTileStaged<RESTRICT, 4>();
   configureTileStaged<PROLONG, 2>();
   cudaFuncSetAttribute(k_bottom, cudaFuncAttributeMaxDynamicSharedMemorySize, BOTTOM_SMEM);
@@ -2197,13 +2177,9 @@ static void levelLaunch(const FpBatch& bt, const MgSel& S, bool tiles, int B, in
     }
   }
   if (tiles) {
-    // The tile levels hold 4^3, 2^3 and one cell a tile. Those that read or write the first
-    // (a cell a brick) are staged per tile.
+    // The tile levels hold 4^3, 2^3 and one cell a tile. Operations that read or write the first
+    // (a cell a brick) are staged per tile; its sweeps are legs (fp_legs_fused).
     const int below = S.level - log2i(B);
-    if (OP == RELAX && below == 0) {
-      tileStagedLaunch<RELAX, 4>(bt, S, sms, st);
-      return;
-    }
     if (OP == RESTRICT && below == 1) {
       tileStagedLaunch<RESTRICT, 4>(bt, S, sms, st);
       return;
@@ -2212,9 +2188,7 @@ static void levelLaunch(const FpBatch& bt, const MgSel& S, bool tiles, int B, in
       tileStagedLaunch<PROLONG, 2>(bt, S, sms, st);
       return;
     }
-    if (below == 0)
-      k_level_tiles<OP, 64><<<sms * 16, 64, 0, st>>>(bt, S);
-    else if (below == 1)
+    if (below == 1)
       k_level_tiles<OP, 8><<<sms * 16, 64, 0, st>>>(bt, S);
     else
       k_level_tiles<OP, 1><<<sms * 16, 64, 0, st>>>(bt, S);
