@@ -130,6 +130,13 @@ bool Engine::grow(DeviceBuffer& b, size_t bytes, int fill) {
   return true;
 }
 
+// Host memory to the device in the stream's order. The stream does not synchronise with the default one,
+// and a plain cudaMemcpy from pageable memory may return before the device has it: such a copy would be
+// ordered with neither a clear enqueued before it (alloc's, behind a step in flight) nor a kernel after it.
+int Engine::copyIn(void* dst, const void* src, size_t bytes) {
+  return check(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream()), "copy to the device");
+}
+
 // Host-to-device copies go through a pinned arena, so they are truly asynchronous. The arena
 // restarts each step: the previous step's copies ran before its allocation kernels, which
 // precede the measurement the step start waits for.
@@ -345,10 +352,10 @@ int Engine::allocatePools(uint32_t slots) {
   }
   std::vector<uint32_t> stack(slots);
   for (uint32_t i = 0; i < slots; i++) stack[i] = slots - 1 - i;
-  cudaMemcpy(freeStack_.ptr, stack.data(), s * 4, cudaMemcpyHostToDevice);
   FpCounters c{};
   c.freeCount = (int32_t)slots;
-  cudaMemcpy(counters_.ptr, &c, sizeof(c), cudaMemcpyHostToDevice);
+  int rc;
+  if ((rc = copyIn(freeStack_.ptr, stack.data(), s * 4)) || (rc = copyIn(counters_.ptr, &c, sizeof(c)))) return rc;
   slots_ = slots;
   return FP_OK;
 }
@@ -386,11 +393,11 @@ int Engine::growPool(uint32_t target) {
   for (uint32_t i = 0; i < added; i++) next[i] = slots_ + added - 1 - i;
   for (uint32_t i = 0; i < slots_; i++) next[added + i] = old[i];
   if (!alloc(freeStack_, s * 4, false)) return FP_ENOMEM;
-  cudaMemcpy(freeStack_.ptr, next.data(), s * 4, cudaMemcpyHostToDevice);
   FpCounters c;
   cudaMemcpy(&c, counters_.ptr, sizeof(c), cudaMemcpyDeviceToHost);
   c.freeCount += (int32_t)added;
-  cudaMemcpy(counters_.ptr, &c, sizeof(c), cudaMemcpyHostToDevice);
+  int rc;
+  if ((rc = copyIn(freeStack_.ptr, next.data(), s * 4)) || (rc = copyIn(counters_.ptr, &c, sizeof(c)))) return rc;
   slots_ = target;
   geometryDirty_ = true;
   return FP_OK;

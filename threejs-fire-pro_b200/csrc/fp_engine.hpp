@@ -240,6 +240,7 @@ class Engine {
   int spareWait_ = 0;  // renders until memory that was refused is asked for again
   bool spare(DeviceBuffer& b, size_t need, size_t want);
   bool giveWay();
+  int copyIn(void* dst, const void* src, size_t bytes);
   bool claim(void** p, size_t bytes);
   int renderInputs();
   void updateRenderBox();

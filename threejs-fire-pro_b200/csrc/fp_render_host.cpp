@@ -192,7 +192,7 @@ int Engine::renderInputs() {
     std::vector<float> table(FP_BLACKBODY_SIZE * 4);
     fp_blackbody_table(table.data());
     if (!alloc(lut_, table.size() * 4, false)) return FP_ENOMEM;
-    if ((rc = check(cudaMemcpy(lut_.ptr, table.data(), table.size() * 4, cudaMemcpyHostToDevice), "render"))) return rc;
+    if ((rc = copyIn(lut_.ptr, table.data(), table.size() * 4))) return rc;
   }
   if (!renderParams_.ptr && !alloc(renderParams_, sizeof(SimParams), false)) return FP_ENOMEM;
   if (!renderParamsH_ && (rc = check(cudaMallocHost(&renderParamsH_, sizeof(SimParams)), "cudaMallocHost"))) return rc;

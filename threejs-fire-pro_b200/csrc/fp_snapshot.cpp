@@ -337,7 +337,7 @@ int Engine::restore(const uint8_t* data, size_t bytes) {
       e.b = DeviceBuffer{};                                                                             \
     } else {                                                                                            \
       if (e.b.bytes != n && !alloc(e.b, n, false)) return fail(FP_ENOMEM, "out of device memory for the restore"); \
-      if ((rc = check(cudaMemcpy(e.b.ptr, r.p, n, cudaMemcpyHostToDevice), "restore"))) return rc;     \
+      if ((rc = copyIn(e.b.ptr, r.p, n))) return rc;                                                    \
       r.p += n;                                                                                         \
     }                                                                                                   \
   }
