@@ -852,7 +852,7 @@ __global__ void __launch_bounds__(RTHREADS) k_render_occupancy(const SimParams* 
 // six rays of six samples, each at a place known beforehand: the CTA takes the texels' samples as
 // one flat list, a thread each, into shared memory; then four lanes a texel add them up in the
 // serial order, one the sun's depth (with its early stop) and one each colour of the glow.
-// A warp a texel left 26 lanes idle while six walked the rays: 1.9 -> 0.46 ms on the default
+// A warp a texel left 26 lanes idle while six walked the rays: 1.9 -> 0.43 ms on the default
 // grid's 640 bricks of 64 texels, 0.66 -> 0.21 ms on 3.7k bricks of 8.
 constexpr int LIGHT_TEXELS = 16, GLOW_SAMPLES = 36, SUN_SAMPLES = 256;
 struct LightStage {
@@ -1311,8 +1311,8 @@ FP_DEV void shadeSteps(const SimParams& P, const FpRender& R, Cursor& c, const R
 // The rays of a warp cross their empty stretches together, by lookups alone, before any shades: a
 // ray in empty space then does not wait, step by step, for the others' shading.
 // What bounds it is instruction issue (cells come from L1): about 98 % L1 hits, DRAM idle. Slice
-// pass, us: 14,400 rays of a small plume 2103 -> 85; 129,600 rays of a 1.8k-brick jet 8954 -> 845;
-// 518,400 rays of 3.7k bricks 20,889 -> 3025; full resolution, 231,401 rays, quadratic 12,807 -> 800.
+// pass, us: 14,400 rays of a small plume 2103 -> 82; 129,600 rays of a 1.8k-brick jet 8954 -> 801;
+// 518,400 rays of 3.7k bricks 20,889 -> 2689; full resolution, 231,401 rays, quadratic 12,807 -> 722.
 template <class Cursor, int G, class Limit, class Arrived>
 FP_DEV void marchRays(const SimParams& P, const FpRender& R, const Ray& r, bool alive, float end, March& m, Limit limitOf,
                       Arrived arrived) {
@@ -1623,7 +1623,7 @@ template <class Cursor>
 static void poolsLaunch(const SimParams* dP, const FpRender& R, int sms, cudaStream_t st) {
   k_render_field<Cursor><<<sms * 24, RTHREADS, 0, st>>>(dP, R);
   // More CTAs than reside: texels that nothing is at cost little, so equal shares of them are not
-  // equal work (5 CTAs an SM 536 us, 20 474, 40 464 on the default grid).
+  // equal work (on the default grid 5 CTAs an SM took 16 % longer than 40, 20 took 2 %).
   k_render_light<Cursor><<<sms * 40, RTHREADS, 0, st>>>(dP, R);
   if (R.units)
     k_render_occupancy<Cursor, true><<<sms * 8, RTHREADS, 0, st>>>(dP, R);
