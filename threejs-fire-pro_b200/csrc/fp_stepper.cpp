@@ -5,8 +5,8 @@
 //   3. writes the work rows, every simulation's SimParams and scene into one pinned upload
 //      and copies it with one cudaMemcpyAsync;
 //   4. replays the CUDA graph of the step's kernels (captured once per combination of the
-//      optional launches: grids are fixed and buffers are read from SimParams, so growth of
-//      any simulation keeps the graph valid).
+//      optional launches and of the forms that suit the step's size: grids are fixed and buffers
+//      are read from SimParams, so growth of any simulation keeps the graph valid).
 #include <algorithm>
 #include <chrono>
 #include <cstring>
