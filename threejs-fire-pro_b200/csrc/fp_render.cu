@@ -852,6 +852,9 @@ __global__ void __launch_bounds__(RTHREADS) k_render_occupancy(const SimParams* 
 // six rays of six samples, each at a place known beforehand: the CTA takes the texels' samples as
 // one flat list, a thread each, into shared memory; then four lanes a texel add them up in the
 // serial order, one the sun's depth (with its early stop) and one each colour of the glow.
+// All the sun's samples are taken, those too past the depth at which the sum then stops: a small image
+// of 2.4k bricks takes 228 us with 16 samples a texel and 355 with 256 (in smoke fifty times as dense 346),
+// where a warp a texel that stopped after the 32 in which it got there took 1.9 and 2.5 to 2.7 ms.
 // A warp a texel left 26 lanes idle while six walked the rays: 1.9 -> 0.43 ms on the default
 // grid's 640 bricks of 64 texels, 0.66 -> 0.21 ms on 3.7k bricks of 8.
 constexpr int LIGHT_TEXELS = 16, GLOW_SAMPLES = 36, SUN_SAMPLES = 256;
